@@ -117,9 +117,10 @@ static void free_graph_data(grz_graph* g, uint64_t next_V = ~0ull)
         // the PageRank arrays are sized by V alone: kept, and refilled at the next grz_pr_init
         g->pr_lists_changed = 1;
     } else {
-        void* plain[] = { g->pr_fx[0], g->pr_fx[1], g->pr_sum, g->pr_K, g->pr_rowacc, g->pr_cut, g->pr_d[0], g->pr_d[1] };
+        void* plain[] = { g->pr_fx[0], g->pr_fx[1], g->pr_sum, g->pr_K, g->pr_rowacc, g->pr_cut, g->pr_pk[0], g->pr_pk[1], g->pr_hot[0], g->pr_hot[1] };
         for (void* p : plain) cudaFree(p);
-        g->pr_d[0] = g->pr_d[1] = nullptr;
+        g->pr_pk[0] = g->pr_pk[1] = nullptr;
+        g->pr_hot[0] = g->pr_hot[1] = nullptr;
         g->pr_fx[0] = g->pr_fx[1] = nullptr; g->pr_sum = nullptr; g->pr_K = nullptr; g->pr_rowacc = nullptr;
         g->pr_cut = nullptr;
     }
@@ -130,7 +131,15 @@ static void free_graph_data(grz_graph* g, uint64_t next_V = ~0ull)
     g->seg_bits = 0;
     g->nseg = 0;
     g->pr_segmode = 0;
-    g->pr_dmode = g->pr_fx_stale = g->pr_d_stale = 0;
+    g->pr_pkmode = g->pr_fx_stale = g->pr_pk_stale = 0;
+    g->pr_cut_vec = 0;
+    grz_dev_free(g, g->pr_hot_nbr);
+    grz_dev_free(g, g->pr_hotmap);
+    g->pr_hot_nbr = nullptr;
+    g->pr_hot_of = nullptr;
+    g->pr_hotmap = nullptr;
+    g->pr_nhot = 0;
+    g->pr_hot_known = 0;
     g->outdeg = nullptr; g->degree = nullptr; g->inv_deg = nullptr;
     g->pr_rowacc_stale = 0;
     g->prop = nullptr; g->accum = nullptr; g->glob = nullptr; g->scratch = nullptr;
@@ -634,7 +643,8 @@ extern "C" int grz_graph_get_info(const grz_graph* gc, grz_graph_info_t* out)
         if (L->nbr) b += L->nvec * ((L->vs ? 32 : 0) + 16 + 4) + (g->V + 64) * 8 + (g->V + 1) * 4;
     b += (g->V + 8) * 8 * 3 + g->V * 12;
     if (g->pr_fx[0]) b += g->V * (16 * 3 + 4);
-    if (g->pr_d[0]) b += g->V * 16;
+    if (g->pr_pk[0]) b += g->V * 16;
+    if (g->pr_hot_nbr) b += 16 * (g->pr_segmode ? g->seg_first[g->nseg] : g->pull.nvec);
     out->device_bytes = b;
     return GRZ_OK;
 }

@@ -145,6 +145,44 @@ __host__ __device__ __forceinline__ double fx_to_double(u128 a)
 #endif
 }
 
+// Packed prop: a 4.124 fixed-point value of at most 53 significant bits in 8 bytes.  Bits 63:7 hold
+// its significand with the leading bit at bit 63 (the low 11 of the 64 are zero, so bits 6:0 are
+// free), bits 6:0 hold s = 127 - (index of its leading bit): value = (significand << 64) >> s.  Zero
+// is 0.  A prop is the conversion of a double, so it always fits, and it unpacks to exactly the
+// value fx_from_double gives; the gathers read half the bytes of the 16-byte form and need two
+// mask and three shift operations instead of the double's exponent handling.
+__device__ __forceinline__ unsigned long long shl64_clamp(unsigned long long x, uint32_t n)
+{
+    unsigned long long r;  // shift counts above 63 give 0
+    asm("shl.b64 %0, %1, %2;" : "=l"(r) : "l"(x), "r"(n));
+    return r;
+}
+__device__ __forceinline__ unsigned long long shr64_clamp(unsigned long long x, uint32_t n)
+{
+    unsigned long long r;
+    asm("shr.u64 %0, %1, %2;" : "=l"(r) : "l"(x), "r"(n));
+    return r;
+}
+__device__ __forceinline__ u128 pk_to_fx(unsigned long long w)
+{
+    const uint32_t s = (uint32_t)w & 127u;
+    const unsigned long long x = w & ~127ull;
+    u128 r;
+    r.hi = shr64_clamp(x, s);
+    r.lo = shl64_clamp(x, 64u - s) | shr64_clamp(x, s - 64u);  // one of the two is 0 unless s = 64 (both are x)
+    return r;
+}
+// the packed form of fx_from_double(x), x in [0, 8)
+__device__ __forceinline__ unsigned long long pk_from_double(double x)
+{
+    const unsigned long long b = (unsigned long long)__double_as_longlong(x);
+    const int t = (int)(b >> 52) - 1022 + GRZ_FX_FRAC;  // leading bit's index + 1
+    if (t < 1) return 0ull;
+    unsigned long long m = (b << 11) | 0x8000000000000000ull;
+    if (t < 53) m &= ~0ull << (64 - t);  // bits below 2^-124 are cut off, as in fx_from_double
+    return m | (unsigned long long)(128 - t);
+}
+
 // Exact global u128 accumulation: two 64-bit atomics; the low-word wrap-around is carried.
 __device__ __forceinline__ void u128_atomic_add(u128* dst, u128 v)
 {
@@ -299,6 +337,12 @@ struct grz_list {
 #define GRZ_HUB_MAX 49152u
 #define GRZ_INGEST_MAX_CHUNKS 64
 #define GRZ_PR_MAX_SEGMENTS 256
+
+// hot sources of the PageRank gather: 12000 packed props are 96 KB of shared memory, the largest
+// table that fits the 100 KB carveout and so leaves L1 the rest (GB300, gather per iteration with
+// 768 threads: R-MAT 20 46.7 / 44.5 / 42.5 us, R-MAT 22 192 / 180 / 174 us, R-MAT 24 848 / 807 / 814
+// us with 4000 / 7800 / 12000 slots; a table past 128 KB starves L1 and loses)
+#define GRZ_PR_HOT_MAX 12000u
 
 #define GRZ_BATCH_K 8  // instances per graph of a batch (grz_batch.cu)
 
@@ -486,10 +530,19 @@ struct grz_graph {
     int pr_segmode;       // fused iterations gather segment by segment
     void* pr_bar;         // grid barrier and phase timer of the persistent PageRank kernel (device)
     void* pr_bar_host;    // pinned read-back of its error word and phase times
-    double* pr_d[2];      // double[V+1]: the props as doubles, gathered instead of pr_fx in pr_dmode
-    int pr_dmode;         // fused iterations gather pr_d
-    int pr_fx_stale;      // pr_fx[pr_cur] is behind pr_d[pr_cur]
-    int pr_d_stale;       // pr_d[pr_cur] is behind pr_fx[pr_cur]
+    unsigned long long* pr_pk[2];  // u64[V+1]: the props packed (pk_to_fx), gathered instead of pr_fx in pr_pkmode
+    int pr_pkmode;        // fused iterations gather pr_pk
+    int pr_fx_stale;      // pr_fx[pr_cur] is behind pr_pk[pr_cur]
+    int pr_pk_stale;      // pr_pk[pr_cur] is behind pr_fx[pr_cur]
+    uint64_t pr_cut_vec;  // vectors per gather range that pr_cut was made for (0: not made)
+    // hot sources of the packed gather (grz_pr.cu): the few of the highest out-degrees, whose props
+    // every block of the gather keeps in shared memory
+    uint4* pr_hot_nbr;    // the gathered list (pull, or its segments) with hot sources as GRZ_HUB_BASE + slot
+    const uint4* pr_hot_of;        // the list it encodes
+    unsigned long long* pr_hot[2]; // u64[GRZ_PR_HOT_MAX + 2]: packed props of the hot slots (ping-pong), then zeros
+    uint2* pr_hotmap;     // per 32 vertices: their hot bits, and the slot of the first
+    uint32_t pr_nhot;     // hot sources (0: none, or not worth it)
+    int pr_hot_known;     // chosen for the loaded lists
     double pr_damping;
     uint32_t pr_iters_done;
     double* prop;         // double[V+8]: reference-format vertex props (PR props, CC labels, BFS parents)

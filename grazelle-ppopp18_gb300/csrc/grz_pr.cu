@@ -11,12 +11,14 @@
 //     exact sum of the reference's double inputs, rounded once to double.  The result is
 //     independent of tile shape, thread count and scheduling.  GB300's FP64 pipe runs at ~1/58
 //     of its integer rate, so FP64 adds per edge would bound the kernel.
-//   * The gather kernel runs one thread per vector at full occupancy, so that as many random
-//     16-byte gathers as possible are in flight.  The gathers bound the iteration: about one line
-//     request per SM clock.  A warp-segmented scan sums the vectors of each destination.
-//     Destinations cut by a warp edge are combined with exact u128 atomics, in any order.
-//     This replaces the reference's work-unit merge buffer (source/phases.c:41-70); no thread
-//     ever waits on another.
+//   * The gathers bound the iteration: about one line request per SM clock.  The iterations of
+//     grz_pr_iterate therefore gather 8-byte packed props (pk_to_fx), and take those of the sources
+//     with the highest out-degrees from shared memory (k_pr_gather_pk): in a power-law graph 12000
+//     sources are half of the edges at R-MAT 20.  Each thread sums four consecutive vectors, a
+//     warp-segmented scan joins the threads, and a warp walks a contiguous range of the list, so
+//     only the destinations cut by the ends of a range are combined with exact u128 atomics, in any
+//     order.  This replaces the reference's work-unit merge buffer (source/phases.c:41-70); no
+//     thread ever waits on another.
 //   * The apply kernel is the vertex phase.  It also accumulates S_{k+1} = sum_u outdeg[u] *
 //     prop_{k+1}[u] exactly, which equals iteration k+1's sum of accumulators, so an iteration is
 //     two kernels with no host round trip.
@@ -49,10 +51,11 @@ __device__ __forceinline__ u128 ld_fx(const u128* p, uint32_t i)
 #endif
 }
 
-// a gathered prop as fixed point: stored so (16 bytes), or as the double it exactly converts
-// from (8 bytes: half the gathered working set, the same sums)
+// a gathered prop as fixed point: stored so (16 bytes), or packed (8 bytes: half the gathered
+// working set, the same sums)
+typedef unsigned long long pk_t;
 __device__ __forceinline__ u128 ld_prop(const u128* p, uint32_t i) { return ld_fx(p, i); }
-__device__ __forceinline__ u128 ld_prop(const double* p, uint32_t i) { return fx_from_double(__ldg(p + i)); }
+__device__ __forceinline__ u128 ld_prop(const pk_t* p, uint32_t i) { return pk_to_fx(__ldg(p + i)); }
 
 // The same through the coherent path (ld.global, L1-cached): for the persistent kernel, whose
 // apply phase rewrites the props that a later gather phase of the same launch reads, which the
@@ -63,11 +66,11 @@ __device__ __forceinline__ u128 ld_prop_coh(const u128* p, uint32_t i)
     asm volatile("ld.global.v2.u64 {%0, %1}, [%2];" : "=l"(r.lo), "=l"(r.hi) : "l"(p + i));
     return r;
 }
-__device__ __forceinline__ u128 ld_prop_coh(const double* p, uint32_t i)
+__device__ __forceinline__ u128 ld_prop_coh(const pk_t* p, uint32_t i)
 {
-    double x;
-    asm volatile("ld.global.f64 %0, [%1];" : "=d"(x) : "l"(p + i));
-    return fx_from_double(x);
+    pk_t x;
+    asm volatile("ld.global.u64 %0, [%1];" : "=l"(x) : "l"(p + i));
+    return pk_to_fx(x);
 }
 
 // per-iteration constants handed from the gather kernel to the apply kernel
@@ -96,7 +99,9 @@ __device__ __forceinline__ u128 u128_shfl_up(u128 v, int off)
 // accumulators must be zero on entry (the fused apply clears exactly those, marked in pr_cut).
 // A destination with no in-edges is never touched and stays 0.  The loads of nbr/dst are
 // streamed once (evict-first); the prop gathers go through L1.  P is the gathered props' type:
-// u128 fixed point, or double (converted exactly to fixed point after the load).
+// u128 fixed point, or packed.  This is the general form: the phases.h calls (any vector range),
+// hub-encoded lists, and 16-byte props when asked for; grz_pr_iterate's packed props go through
+// k_pr_gather_pk.
 __device__ __forceinline__ u128 block_reduce_u128(u128 s, u128* red);
 
 // shared memory of the gather's block combine
@@ -118,9 +123,9 @@ __device__ __forceinline__ void pr_publish_K(const PRConst& pc, u128* red)
     if (threadIdx.x == 0) *pc.K_out = __fma_rn((1.0 - fx_to_double(S)) / pc.nverts, pc.damping, pc.c);
 }
 
-// The gather over tiles blockIdx.x, blockIdx.x + nblocks, ... of PR_THREADS vectors.
-// ADD: the accumulators already hold the sums of earlier launches (source segments); a destination
-// owned by one warp or block is added by a plain read-modify-write, one cut by a tile edge atomically.
+// A destination's sum.  ADD: the accumulators already hold the sums of earlier launches (source
+// segments); a destination owned by one warp is added by a plain read-modify-write, one cut by the
+// edge of a range atomically.
 __device__ __forceinline__ void rowacc_put(u128* rowacc, uint32_t key, u128 val, bool add)
 {
     ulonglong2* p = reinterpret_cast<ulonglong2*>(rowacc) + key;
@@ -134,7 +139,8 @@ __device__ __forceinline__ void rowacc_put(u128* rowacc, uint32_t key, u128 val,
     __stcg(p, make_ulonglong2(val.lo, val.hi));
 }
 
-template <typename P, bool COH, bool ADD = false>
+// The gather over tiles blockIdx.x, blockIdx.x + nblocks, ... of PR_THREADS vectors.
+template <typename P, bool COH>
 __device__ __forceinline__ void pr_gather_tiles(const uint4* __restrict__ nbr, const uint32_t* __restrict__ dstv, uint64_t first,
                                                 uint64_t nvec, uint64_t list_nvec, const P* __restrict__ prop_fx, uint32_t V,
                                                 u128* __restrict__ rowacc, const uint32_t* __restrict__ hub_vid, uint32_t nhub,
@@ -184,7 +190,7 @@ __device__ __forceinline__ void pr_gather_tiles(const uint4* __restrict__ nbr, c
             const bool head_real = (real_heads >> segstart) & 1u;
             if (tail && head_real) {
                 // every vector of this destination is in this warp
-                rowacc_put(rowacc, key, val, ADD);
+                rowacc_put(rowacc, key, val, false);
             } else {
                 // open on the left (slot 0) or on the right only (slot 1): combined across the block below
                 const int slot = (segstart == 0 && !head_real) ? 0 : 1;
@@ -207,7 +213,7 @@ __device__ __forceinline__ void pr_gather_tiles(const uint4* __restrict__ nbr, c
                     if (!open) { open = true; open_head = false; ok = sm.key[0][w]; os = u128_zero(); }
                     os = u128_add(os, sm.sum[0][w]);
                     if (f0 & 4u) {
-                        if (open_head) rowacc_put(rowacc, ok, os, ADD);
+                        if (open_head) rowacc_put(rowacc, ok, os, false);
                         else if (os.lo | os.hi) u128_atomic_add(rowacc + ok, os);
                         open = false;
                     }
@@ -226,7 +232,7 @@ __device__ __forceinline__ void pr_gather_tiles(const uint4* __restrict__ nbr, c
 // per SM), which measured 47% slower at R-MAT 20.
 constexpr int PR_GATHER_MIN_BLOCKS = 8;
 
-template <typename P, bool ADD = false>
+template <typename P>
 __global__ void __launch_bounds__(PR_THREADS, PR_GATHER_MIN_BLOCKS) k_pr_gather(const uint4* __restrict__ nbr, const uint32_t* __restrict__ dstv,
                                                           uint64_t first, uint64_t nvec, uint64_t list_nvec,
                                                           const P* __restrict__ prop_fx, uint32_t V, u128* __restrict__ rowacc,
@@ -234,7 +240,188 @@ __global__ void __launch_bounds__(PR_THREADS, PR_GATHER_MIN_BLOCKS) k_pr_gather(
 {
     __shared__ GatherSmem sm;
     if (pc.K_out && blockIdx.x == 0) pr_publish_K(pc, sm.red);
-    pr_gather_tiles<P, false, ADD>(nbr, dstv, first, nvec, list_nvec, prop_fx, V, rowacc, hub_vid, nhub, blockIdx.x, gridDim.x, sm);
+    pr_gather_tiles<P, false>(nbr, dstv, first, nvec, list_nvec, prop_fx, V, rowacc, hub_vid, nhub, blockIdx.x, gridDim.x, sm);
+}
+
+// ---------------------------------------------------------------------------------------------
+// The gather of grz_pr_iterate over packed props.
+//
+// A random gather costs an L1 tag lookup per line, one per SM clock, and a miss about 1.9 clocks of
+// the SM's path to L2 (GB300: 160 G misses/s, at R-MAT 20 and on a uniform graph alike), whatever
+// its width.  So what helps is fewer gathers through L1 and fewer instructions around them:
+//   * HOT: the props of up to GRZ_PR_HOT_MAX sources of the highest out-degrees are copied into
+//     shared memory when the block starts, and lanes that name one
+//     (GRZ_HUB_BASE + slot in the encoded list) read them there.
+//   * A thread owns four consecutive vectors (two 32-byte loads and one of four destinations, the
+//     next group's issued before this one's sums): it joins vectors of one destination in registers,
+//     so the u128 scan over the warp runs once per 128 vectors, not once per 32.
+//   * A warp walks a contiguous range of `per` vectors and carries the open destination's sum from
+//     group to group.  There is no barrier, and only the two destinations cut by the range's ends
+//     are added atomically (the apply clears exactly those, marked in pr_cut).
+// One block of 768 threads per SM: 80 registers hold a thread's 16 gathers without spills, and the
+// table is copied once per SM.  GB300, gather per iteration (16-byte props, a thread per vector,
+// 2048 threads per SM -> this kernel): R-MAT 20 83 -> 43 us, R-MAT 24 1550 -> 810 us, uniform graph of
+// 3M vertices and 36M edges 200 -> 148 us.
+constexpr int PK_THREADS = 768;
+constexpr uint32_t PK_GROUP = 128;    // vectors a warp sums at a time
+constexpr uint32_t PK_MIN_RANGE = 32; // fewest vectors per warp: a small list spreads over the SMs
+
+struct PkVec8 {
+    uint32_t a[8];  // two vectors' sources
+};
+
+// two consecutive vectors, read once (32-byte aligned)
+__device__ __forceinline__ PkVec8 ld_vec8(const uint4* p)
+{
+    PkVec8 r;
+    asm volatile("ld.global.nc.L1::no_allocate.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(r.a[0]), "=r"(r.a[1]), "=r"(r.a[2]), "=r"(r.a[3]), "=r"(r.a[4]), "=r"(r.a[5]), "=r"(r.a[6]), "=r"(r.a[7])
+                 : "l"(p));
+    return r;
+}
+
+__device__ __forceinline__ u128 u128_shfl(u128 v, int src)
+{
+    u128 r;
+    r.lo = __shfl_sync(0xffffffffu, v.lo, src);
+    r.hi = __shfl_sync(0xffffffffu, v.hi, src);
+    return r;
+}
+
+// The vectors [first, end) of a list whose first vector is at a multiple of 16 bytes of `dstv`.
+// `base` is `first` rounded down to a multiple of 4 (vectors before `first` count as empty), so that
+// the wide loads are aligned; ranges are [base + w * per, base + (w + 1) * per), per a multiple of 4.
+template <bool HOT, bool ADD>
+__global__ void __launch_bounds__(PK_THREADS, 1) k_pr_gather_pk(const uint4* __restrict__ nbr, const uint32_t* __restrict__ dstv,
+                                                                uint32_t first, uint32_t end, uint32_t per,
+                                                                const pk_t* __restrict__ props, uint32_t V,
+                                                                const pk_t* __restrict__ hot, uint32_t nhot,
+                                                                u128* __restrict__ rowacc, const PRConst pc)
+{
+    extern __shared__ __align__(16) pk_t s_hot[];
+    const int lane = threadIdx.x & 31;
+    const uint32_t nwarps = gridDim.x * (PK_THREADS / 32);
+    const uint32_t wid = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;  // neighbouring ranges on different SMs
+    if (HOT) {
+        // 16 bytes per thread and step, all steps' loads in flight (the table ends in zeros)
+        const uint32_t n16 = (nhot + 2) / 2;
+#pragma unroll
+        for (uint32_t j = 0; j < (GRZ_PR_HOT_MAX / 2 + PK_THREADS) / PK_THREADS; ++j) {
+            const uint32_t i = j * PK_THREADS + threadIdx.x;
+            if (i < n16) reinterpret_cast<ulonglong2*>(s_hot)[i] = __ldg(reinterpret_cast<const ulonglong2*>(hot) + i);
+        }
+    }
+    // the iteration's constant (pr_publish_K), by the warp of the last range, which is usually empty
+    if (pc.K_out && wid == nwarps - 1) {
+        u128 S = u128_zero();
+        for (uint32_t b = lane; b < pc.nparts; b += 32) S = u128_add(S, pc.part_in[b]);
+        for (int o = 16; o > 0; o >>= 1) S = u128_add(S, u128_shfl_down(S, o));
+        if (lane == 0) *pc.K_out = __fma_rn((1.0 - fx_to_double(S)) / pc.nverts, pc.damping, pc.c);
+    }
+    const uint32_t base = first & ~3u;
+    const uint64_t lo64 = (uint64_t)base + (uint64_t)wid * per;
+    const uint32_t lo = (uint32_t)(lo64 < end ? lo64 : end);
+    const uint32_t hi = (uint32_t)(lo64 + per < end ? lo64 + per : end);
+    PkVec8 na, nb;
+    uint4 nk;
+    const uint32_t pad = HOT ? (GRZ_HUB_BASE | nhot) : GRZ_INVALID_ID;
+    auto load = [&](uint64_t v) {  // the lane's four vectors from v on
+        if (v >= first && v + 3 < hi) {
+            na = ld_vec8(nbr + v);
+            nb = ld_vec8(nbr + v + 2);
+            nk = __ldcs(reinterpret_cast<const uint4*>(dstv + v));
+        } else {
+            uint4 x[4];
+            uint32_t k[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const bool in = v + j >= first && v + j < hi;
+                x[j] = in ? __ldcs(nbr + v + j) : make_uint4(pad, pad, pad, pad);
+                k[j] = in ? __ldcs(dstv + v + j) : GRZ_INVALID_ID;
+            }
+            na.a[0] = x[0].x; na.a[1] = x[0].y; na.a[2] = x[0].z; na.a[3] = x[0].w;
+            na.a[4] = x[1].x; na.a[5] = x[1].y; na.a[6] = x[1].z; na.a[7] = x[1].w;
+            nb.a[0] = x[2].x; nb.a[1] = x[2].y; nb.a[2] = x[2].z; nb.a[3] = x[2].w;
+            nb.a[4] = x[3].x; nb.a[5] = x[3].y; nb.a[6] = x[3].z; nb.a[7] = x[3].w;
+            nk = make_uint4(k[0], k[1], k[2], k[3]);
+        }
+    };
+    uint32_t kbefore = GRZ_INVALID_ID - 1;  // destination of the vector before the range
+    if (lo < hi) {
+        load((uint64_t)lo + 4 * lane);
+        if (lo > first) kbefore = __ldg(dstv + lo - 1);
+    }
+    if (HOT) __syncthreads();
+    auto get = [&](uint32_t id) -> pk_t {
+        if (HOT) {
+            if ((int)id < 0) return s_hot[id & (GRZ_HUB_BASE - 1)];
+            return __ldg(props + id);
+        }
+        return __ldg(props + min(id, V));  // entry V is zero
+    };
+    auto put = [&](uint32_t key, u128 v) {
+        if (key == GRZ_INVALID_ID) return;
+        if (key != kbefore) rowacc_put(rowacc, key, v, ADD);
+        else u128_atomic_add(rowacc + key, v);  // cut by the start of the range
+    };
+    u128 carry = u128_zero();  // sum so far of the destination the previous group left open
+    uint32_t ckey = GRZ_INVALID_ID - 1;
+    for (uint64_t v = lo; v < hi; v += PK_GROUP) {  // warp-uniform
+        const uint4 k = nk;
+        u128 v0, v1, v2, v3;
+        {
+            pk_t p[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) p[j] = get(na.a[j]);
+            v0 = u128_add(u128_add(pk_to_fx(p[0]), pk_to_fx(p[1])), u128_add(pk_to_fx(p[2]), pk_to_fx(p[3])));
+            v1 = u128_add(u128_add(pk_to_fx(p[4]), pk_to_fx(p[5])), u128_add(pk_to_fx(p[6]), pk_to_fx(p[7])));
+#pragma unroll
+            for (int j = 0; j < 8; ++j) p[j] = get(nb.a[j]);
+            if (v + PK_GROUP < hi) {
+                load(v + PK_GROUP + 4 * lane);
+            } else {
+                nk.x = hi < end ? __ldg(dstv + hi) : GRZ_INVALID_ID;  // the next range's first destination
+            }
+            v2 = u128_add(u128_add(pk_to_fx(p[0]), pk_to_fx(p[1])), u128_add(pk_to_fx(p[2]), pk_to_fx(p[3])));
+            v3 = u128_add(u128_add(pk_to_fx(p[4]), pk_to_fx(p[5])), u128_add(pk_to_fx(p[6]), pk_to_fx(p[7])));
+        }
+        const uint32_t after = __shfl_sync(0xffffffffu, nk.x, 0);
+        uint32_t kp = __shfl_up_sync(0xffffffffu, k.w, 1), kn = __shfl_down_sync(0xffffffffu, k.x, 1);
+        if (lane == 0) kp = ckey;
+        const bool ends = v + PK_GROUP >= hi;  // the range's last group: its last vectors may not fill the warp
+        const int last = ends ? (int)((hi - (uint32_t)v + 3) / 4) - 1 : 31;
+        if (lane == last) kn = after;
+        // the thread's vectors: the first destination's sum if it ends here (`head`), destinations
+        // that start and end here (stored at once), and the last destination's sum (`cur`)
+        u128 cur = v0, head = u128_zero();
+        bool closed = false;
+        if (k.y == k.x) cur = u128_add(cur, v1);
+        else { head = cur; closed = true; cur = v1; }
+        if (k.z == k.y) cur = u128_add(cur, v2);
+        else { if (closed) put(k.y, cur); else { head = cur; closed = true; } cur = v2; }
+        if (k.w == k.z) cur = u128_add(cur, v3);
+        else { if (closed) put(k.z, cur); else { head = cur; closed = true; } cur = v3; }
+        if (lane == 0 && !closed && kp == k.x) cur = u128_add(cur, carry);
+        // segmented inclusive scan of `cur` over the threads
+        const unsigned heads = __ballot_sync(0xffffffffu, lane == 0 || closed || kp != k.x);
+        const int segstart = 31 - __clz(heads & (0xffffffffu >> (31 - lane)));
+        const int maxlen = __reduce_max_sync(0xffffffffu, (unsigned)(lane - segstart + 1));
+        for (int off = 1; off < maxlen; off <<= 1) {
+            const u128 o = u128_shfl_up(cur, off);
+            if (lane - off >= segstart) cur = u128_add(cur, o);
+        }
+        u128 before = u128_shfl_up(cur, 1);
+        if (lane == 0) before = carry;
+        if (closed) {
+            if (kp == k.x) head = u128_add(head, before);
+            put(k.x, head);
+        }
+        if (k.w != kn) put(k.w, cur);
+        carry = u128_shfl(cur, 31);
+        ckey = __shfl_sync(0xffffffffu, k.w, 31);
+        // the destination goes on in the next range
+        if (ends && lane == last && k.w == kn && k.w != GRZ_INVALID_ID) u128_atomic_add(rowacc + k.w, cur);
+    }
 }
 
 __device__ __forceinline__ u128 block_reduce_u128(u128 s, u128* red)
@@ -255,8 +442,8 @@ __device__ __forceinline__ u128 block_reduce_u128(u128 s, u128* red)
 // Vertex phase fused with reading the accumulators (phase_vertex_pr.asm:75-134):
 //   prop[v] = (acc[v]*d + G*d + (1-d)/V) / deg'[v],  G = (1 - S)/V
 // computed as fma + multiply by the precomputed 1/deg'.  It writes the new props in fixed point,
-// or as doubles when the next gather reads doubles (plus the reference-format doubles when
-// asked), and accumulates S' = sum deg[v]*prop[v] exactly; S' is the next
+// or packed when the next gather reads them packed (and then the hot sources' once more, into the
+// table of the next gather), plus the reference-format doubles when asked, and accumulates S' = sum deg[v]*prop[v] exactly; S' is the next
 // iteration's sum of accumulators.  Of the accumulators it clears only those the next gather
 // adds to atomically (bit set in `cut`); the others are overwritten by the next gather's stores.
 // The grid strides over the vertices, PR_APPLY_U vertices per thread at a time whose
@@ -273,14 +460,23 @@ __device__ __forceinline__ u128 block_reduce_u128(u128 s, u128* red)
 constexpr int PR_APPLY_U = GRZ_PR_APPLY_U;
 constexpr int PR_APPLY_RESIDENT = GRZ_PR_APPLY_MINB;  // blocks per SM that the launch bounds fit
 
+// vertex v's packed prop also into its slot of the hot table, if it has one (slots ascend by vertex)
+__device__ __forceinline__ void hot_put(const uint2* __restrict__ hotmap, pk_t* __restrict__ hot, uint64_t v, pk_t w)
+{
+    const uint2 m = __ldg(hotmap + (v >> 5));
+    const uint32_t bit = (uint32_t)v & 31u;
+    if ((m.x >> bit) & 1u) hot[m.y + __popc(m.x & ((1u << bit) - 1u))] = w;
+}
+
 // the apply over vertices block*PR_THREADS + tid, strided by nblocks*PR_THREADS, U vertices per
 // thread loaded before any is stored; returns the block's partial of S' (valid in thread 0;
 // every thread of the block must call it)
 template <int U>
 __device__ __forceinline__ u128 pr_apply_range(u128* __restrict__ rowacc, const uint32_t* __restrict__ cut, bool clear_all,
                                                const double* __restrict__ inv_deg, const uint32_t* __restrict__ degree, uint64_t V,
-                                               double sK, double damping, u128* __restrict__ prop_fx, double* __restrict__ prop_d,
-                                               double* __restrict__ prop_out, uint32_t block, uint32_t nblocks, u128* red)
+                                               double sK, double damping, u128* __restrict__ prop_fx, pk_t* __restrict__ prop_pk,
+                                               double* __restrict__ prop_out, const uint2* __restrict__ hotmap, pk_t* __restrict__ hot,
+                                               uint32_t block, uint32_t nblocks, u128* red)
 {
     const uint64_t stride = (uint64_t)nblocks * PR_THREADS;
     u128 s = u128_zero();
@@ -307,9 +503,16 @@ __device__ __forceinline__ u128 pr_apply_range(u128* __restrict__ rowacc, const 
             acc.lo = a[j].x;
             acc.hi = a[j].y;
             const double p = __dmul_rn(__fma_rn(fx_to_double(acc), damping, sK), __ldg(inv_deg + v));
-            const u128 pf = fx_from_double(p);
-            if (prop_d) __stcg(prop_d + v, p);  // the next gather reads doubles
-            else __stcg(reinterpret_cast<ulonglong2*>(prop_fx) + v, make_ulonglong2(pf.lo, pf.hi));
+            u128 pf;
+            if (prop_pk) {
+                const pk_t w = pk_from_double(p);
+                pf = pk_to_fx(w);
+                __stcg(prop_pk + v, w);
+                if (hotmap) hot_put(hotmap, hot, v, w);
+            } else {
+                pf = fx_from_double(p);
+                __stcg(reinterpret_cast<ulonglong2*>(prop_fx) + v, make_ulonglong2(pf.lo, pf.hi));
+            }
             if (prop_out) prop_out[v] = p;
             s = u128_add(s, u128_mul32(pf, __ldg(degree + v)));
         }
@@ -322,11 +525,12 @@ __global__ void __launch_bounds__(PR_THREADS, PR_APPLY_RESIDENT) k_pr_apply(u128
                                                                             const uint32_t* __restrict__ degree, uint64_t V,
                                                                             const double* __restrict__ Kp, u128* __restrict__ part_out,
                                                                             double damping, u128* __restrict__ prop_fx,
-                                                                            double* __restrict__ prop_d, double* __restrict__ prop_out)
+                                                                            pk_t* __restrict__ prop_pk, double* __restrict__ prop_out,
+                                                                            const uint2* __restrict__ hotmap, pk_t* __restrict__ hot)
 {
     __shared__ u128 red[PR_THREADS / 32];
-    const u128 s = pr_apply_range<PR_APPLY_U>(rowacc, cut, clear_all != 0, inv_deg, degree, V, *Kp, damping, prop_fx, prop_d, prop_out, blockIdx.x, gridDim.x,
-                                  red);
+    const u128 s = pr_apply_range<PR_APPLY_U>(rowacc, cut, clear_all != 0, inv_deg, degree, V, *Kp, damping, prop_fx, prop_pk, prop_out, hotmap, hot, blockIdx.x,
+                                  gridDim.x, red);
     if (threadIdx.x == 0) part_out[blockIdx.x] = s;  // summed by the next gather kernel's block 0
 }
 
@@ -404,8 +608,8 @@ struct PRPersist {
     const double* inv_deg;
     const uint32_t* degree;
     u128* fx[2];            // props, fixed point (ping-pong)
-    double* d[2];           // props, doubles (ping-pong; gathered in doubles mode)
-    int dmode;
+    pk_t* pk[2];            // props, packed (ping-pong; gathered in packed mode)
+    int pkmode;
     int cur;                // which buffer holds the current props
     u128* sum[2];           // per-block partials of S (ping-pong)
     uint32_t nparts0;       // partials in sum[sum_cur] at the start
@@ -445,14 +649,14 @@ __global__ void __launch_bounds__(PR_THREADS, MINB) k_pr_persistent(const PRPers
             pc.nverts = q.nverts;
             pr_publish_K(pc, sm.red);
         }
-        const P* props = q.dmode ? (const P*)q.d[cur] : (const P*)q.fx[cur];
+        const P* props = q.pkmode ? (const P*)q.pk[cur] : (const P*)q.fx[cur];
         pr_gather_tiles<P, true>(q.nbr, q.dstv, 0, q.nvec, q.nvec, props, q.V, q.rowacc, q.hub_vid, q.nhub, blockIdx.x, nb, sm);
         if (!pr_grid_barrier(q.bar, nb, q.limit_ns, ++bi, (int)blockIdx.x == q.withhold_block)) return;
         const unsigned long long t1 = (q.time_phases && blockIdx.x == 0 && threadIdx.x == 0) ? pr_now_ns() : 0ull;
         const double sK = *(volatile double*)q.K;
         const u128 s = pr_apply_range<PR_PERSIST_APPLY_U>(q.rowacc, q.cut, false, q.inv_deg, q.degree, q.V, sK, q.damping, q.fx[cur ^ 1],
-                                      q.dmode ? q.d[cur ^ 1] : nullptr, it + 1 == q.iters ? q.prop_out : nullptr, blockIdx.x, nb,
-                                      sm.red);
+                                      q.pkmode ? q.pk[cur ^ 1] : nullptr, it + 1 == q.iters ? q.prop_out : nullptr, nullptr, nullptr,
+                                      blockIdx.x, nb, sm.red);
         if (threadIdx.x == 0) q.sum[sc ^ 1][blockIdx.x] = s;
         if (!pr_grid_barrier(q.bar, nb, q.limit_ns, ++bi, false)) return;
         if (q.time_phases && blockIdx.x == 0 && threadIdx.x == 0 && it < 64) {
@@ -466,15 +670,15 @@ __global__ void __launch_bounds__(PR_THREADS, MINB) k_pr_persistent(const PRPers
     }
 }
 
-// bit j of word t: vertex 32t + j has pull vectors in two or more gather tiles of PR_THREADS
+// bit j of word t: vertex 32t + j has pull vectors in two or more of the gather's ranges of `per`
 // vectors (its accumulator is summed with atomics)
-__global__ void k_pr_cutbits(const uint32_t* __restrict__ rowptr, uint64_t V, uint32_t* __restrict__ cut)
+__global__ void k_pr_cutbits(const uint32_t* __restrict__ rowptr, uint64_t V, uint32_t per, uint32_t* __restrict__ cut)
 {
     const uint64_t v = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     bool c = false;
     if (v < V) {
         const uint32_t r0 = rowptr[v], r1 = rowptr[v + 1];
-        c = r1 > r0 && r0 / PR_THREADS != (r1 - 1) / PR_THREADS;
+        c = r1 > r0 && r0 / per != (r1 - 1) / per;
     }
     const unsigned m = __ballot_sync(0xffffffffu, c);
     if ((threadIdx.x & 31) == 0 && v < V) cut[v >> 5] = m;
@@ -633,7 +837,8 @@ __global__ void k_pr_vertex(const double* __restrict__ accum, const double* __re
 // execution_initialize_vertex_prop_pr (source/execution_pr.c:85-88): (1/V) / deg'
 __global__ void k_pr_init(const double* __restrict__ outdeg, const uint32_t* __restrict__ degree, uint64_t V,
                           double* __restrict__ prop, double* __restrict__ accum, u128* __restrict__ prop_fx,
-                          double* __restrict__ prop_d, u128* __restrict__ part0)
+                          pk_t* __restrict__ prop_pk, const uint2* __restrict__ hotmap, pk_t* __restrict__ hot,
+                          u128* __restrict__ part0)
 {
     __shared__ u128 red[PR_THREADS / 32];
     const uint64_t v = (uint64_t)blockIdx.x * PR_THREADS + threadIdx.x;
@@ -645,7 +850,11 @@ __global__ void k_pr_init(const double* __restrict__ outdeg, const uint32_t* __r
         accum[v] = 0.0;
         const u128 pf = fx_from_double(p);
         prop_fx[v] = pf;
-        if (prop_d) prop_d[v] = p;
+        if (prop_pk) {
+            const pk_t w = pk_from_double(p);
+            prop_pk[v] = w;
+            if (hotmap) hot_put(hotmap, hot, v, w);
+        }
         s = u128_mul32(pf, degree[v]);
     }
     s = block_reduce_u128(s, red);
@@ -658,15 +867,114 @@ __global__ void k_fx_to_double(const u128* __restrict__ fx, uint64_t V, double* 
     if (v < V) out[v] = fx_to_double(fx[v]);
 }
 
-// double props -> the fixed-point props they convert to (and, when asked, back to the double
-// the fixed-point value rounds to, which is what the fixed-point path reports)
-__global__ void k_double_to_fx(const double* __restrict__ d, uint64_t V, u128* __restrict__ fx, double* __restrict__ out)
+// packed props -> fixed point, or the doubles they are
+__global__ void k_pk_unpack(const pk_t* __restrict__ pk, uint64_t V, u128* __restrict__ fx, double* __restrict__ out)
 {
     const uint64_t v = (uint64_t)blockIdx.x * PR_THREADS + threadIdx.x;
     if (v >= V) return;
-    const u128 f = fx_from_double(d[v]);
+    const u128 f = pk_to_fx(pk[v]);
     if (fx) fx[v] = f;
     if (out) out[v] = fx_to_double(f);
+}
+
+// fixed-point props (each the conversion of a double) -> packed, and the hot table
+__global__ void k_pk_pack(const u128* __restrict__ fx, uint64_t V, pk_t* __restrict__ pk, const uint2* __restrict__ hotmap,
+                          pk_t* __restrict__ hot)
+{
+    const uint64_t v = (uint64_t)blockIdx.x * PR_THREADS + threadIdx.x;
+    if (v >= V) return;
+    const pk_t w = pk_from_double(fx_to_double(fx[v]));
+    pk[v] = w;
+    if (hotmap) hot_put(hotmap, hot, v, w);
+}
+
+// ---------------------------------------------------------------------------------------------
+// Hot sources: the vertices of the highest out-degrees, at most GRZ_PR_HOT_MAX of them, cut where a
+// degree bin ends (32 bins per octave above 64, exact below).
+
+constexpr uint32_t HOT_BINS = 64 + 26 * 32;
+
+__device__ __forceinline__ uint32_t hot_bin(uint32_t d)
+{
+    if (d < 64u) return d;
+    const uint32_t e = 31u - (uint32_t)__clz(d);
+    return 64u + (e - 6u) * 32u + ((d >> (e - 5u)) & 31u);
+}
+
+// vertices and out-edges per bin, of the vertices with out-degree `dmin` or more
+__global__ void __launch_bounds__(PR_THREADS) k_hot_hist(const uint32_t* __restrict__ degree, uint64_t V, uint32_t dmin,
+                                                         unsigned long long* __restrict__ hist)
+{
+    __shared__ uint32_t cnt[HOT_BINS];
+    __shared__ unsigned long long edges[HOT_BINS];
+    for (uint32_t b = threadIdx.x; b < HOT_BINS; b += PR_THREADS) { cnt[b] = 0; edges[b] = 0; }
+    __syncthreads();
+    for (uint64_t v = (uint64_t)blockIdx.x * PR_THREADS + threadIdx.x; v < V; v += (uint64_t)gridDim.x * PR_THREADS) {
+        const uint32_t d = __ldg(degree + v);
+        if (d < dmin) continue;
+        const uint32_t b = hot_bin(d);
+        atomicAdd(cnt + b, 1u);
+        atomicAdd(edges + b, (unsigned long long)d);
+    }
+    __syncthreads();
+    for (uint32_t b = threadIdx.x; b < HOT_BINS; b += PR_THREADS)
+        if (cnt[b]) {
+            atomicAdd(hist + b, (unsigned long long)cnt[b]);
+            atomicAdd(hist + HOT_BINS + b, edges[b]);
+        }
+}
+
+// out[0] = the lowest bin whose vertices and all above are at most `cap`, out[1] = how many they
+// are, out[2] = their out-edges.  One warp; 896 bins.
+__global__ void k_hot_pick(const unsigned long long* __restrict__ hist, uint32_t cap, unsigned long long* __restrict__ out)
+{
+    if (threadIdx.x) return;
+    unsigned long long n = 0, e = 0;
+    uint32_t b = HOT_BINS;
+    while (b > 0 && n + hist[b - 1] <= cap) {
+        --b;
+        n += hist[b];
+        e += hist[HOT_BINS + b];
+    }
+    out[0] = b;
+    out[1] = n;
+    out[2] = e;
+}
+
+// the hot bits of 32 vertices per warp, and how many there are (words: (V + 31) / 32)
+__global__ void __launch_bounds__(PR_THREADS) k_hot_mark(const uint32_t* __restrict__ degree, uint64_t V, uint32_t dmin, uint32_t bin,
+                                                         uint2* __restrict__ hotmap, uint32_t* __restrict__ count)
+{
+    const uint64_t v = (uint64_t)blockIdx.x * PR_THREADS + threadIdx.x;
+    const uint32_t d = v < V ? __ldg(degree + v) : 0u;
+    const unsigned m = __ballot_sync(0xffffffffu, d >= dmin && hot_bin(d) >= bin);
+    if ((threadIdx.x & 31) == 0 && v < V) {
+        hotmap[v >> 5].x = m;
+        count[v >> 5] = __popc(m);
+    }
+}
+
+__global__ void k_hot_base(const uint32_t* __restrict__ base, uint64_t words, uint2* __restrict__ hotmap)
+{
+    const uint64_t w = (uint64_t)blockIdx.x * PR_THREADS + threadIdx.x;
+    if (w < words) hotmap[w].y = base[w];
+}
+
+// the list with its hot sources as GRZ_HUB_BASE + slot and its empty lanes as the slot after the
+// last, which is zero
+__global__ void __launch_bounds__(PR_THREADS) k_hot_encode(const uint4* __restrict__ nbr, uint64_t nvec, const uint2* __restrict__ hotmap,
+                                                           uint32_t nhot, uint4* __restrict__ out)
+{
+    const uint64_t v = (uint64_t)blockIdx.x * PR_THREADS + threadIdx.x;
+    if (v >= nvec) return;
+    const uint4 s = __ldcs(nbr + v);
+    auto code = [&](uint32_t id) -> uint32_t {
+        if (id == GRZ_INVALID_ID) return GRZ_HUB_BASE | nhot;
+        const uint2 m = __ldg(hotmap + (id >> 5));
+        const uint32_t bit = id & 31u;
+        return (m.x >> bit) & 1u ? GRZ_HUB_BASE | (m.y + __popc(m.x & ((1u << bit) - 1u))) : id;
+    };
+    __stcs(out + v, make_uint4(code(s.x), code(s.y), code(s.z), code(s.w)));
 }
 
 unsigned blocks_for(uint64_t n) { return (unsigned)((n + PR_THREADS - 1) / PR_THREADS); }
@@ -674,23 +982,24 @@ unsigned blocks_for(uint64_t n) { return (unsigned)((n + PR_THREADS - 1) / PR_TH
 }  // namespace
 
 // The current props live in pr_fx[pr_cur] (fixed point) or, after fused iterations that gather
-// doubles, in pr_d[pr_cur]; each form is brought up to date from the other before a path that
+// packed props, in pr_pk[pr_cur]; each form is brought up to date from the other before a path that
 // reads it.
 static int pr_sync_fx(grz_graph* g)
 {
     if (!g->pr_fx_stale) return GRZ_OK;
-    k_double_to_fx<<<blocks_for(g->V), PR_THREADS, 0, g->stream>>>(g->pr_d[g->pr_cur], g->V, g->pr_fx[g->pr_cur], nullptr); GRZ_COUNT_LAUNCH(g);
+    k_pk_unpack<<<blocks_for(g->V), PR_THREADS, 0, g->stream>>>(g->pr_pk[g->pr_cur], g->V, g->pr_fx[g->pr_cur], nullptr); GRZ_COUNT_LAUNCH(g);
     GRZ_CK(g, cudaGetLastError());
     g->pr_fx_stale = 0;
     return GRZ_OK;
 }
 
-static int pr_sync_d(grz_graph* g)
+static int pr_sync_pk(grz_graph* g)
 {
-    if (!g->pr_d_stale) return GRZ_OK;
-    k_fx_to_double<<<blocks_for(g->V), PR_THREADS, 0, g->stream>>>(g->pr_fx[g->pr_cur], g->V, g->pr_d[g->pr_cur]); GRZ_COUNT_LAUNCH(g);
+    if (!g->pr_pk_stale) return GRZ_OK;
+    k_pk_pack<<<blocks_for(g->V), PR_THREADS, 0, g->stream>>>(g->pr_fx[g->pr_cur], g->V, g->pr_pk[g->pr_cur],
+                                                             g->pr_nhot ? g->pr_hotmap : nullptr, g->pr_hot[g->pr_cur]); GRZ_COUNT_LAUNCH(g);
     GRZ_CK(g, cudaGetLastError());
-    g->pr_d_stale = 0;
+    g->pr_pk_stale = 0;
     return GRZ_OK;
 }
 
@@ -702,6 +1011,84 @@ int grz_pr_rowacc_clean(grz_graph* g)
         GRZ_CK(g, cudaMemsetAsync(g->pr_rowacc, 0, sizeof(u128) * (g->V + 1), g->stream));
         g->pr_rowacc_stale = 0;
     }
+    return GRZ_OK;
+}
+
+// Marks the destinations cut by the gather's ranges of `per` vectors.  When the ranges change, the
+// accumulators that the old marks left uncleared are cleared.
+static int pr_cut_for(grz_graph* g, uint32_t per)
+{
+    if (g->pr_cut_vec == per || !g->V) return GRZ_OK;
+    GRZ_TRY(grz_pr_rowacc_clean(g));
+    k_pr_cutbits<<<blocks_for(g->V), PR_THREADS, 0, g->stream>>>(g->pull.rowptr, g->V, per, g->pr_cut); GRZ_COUNT_LAUNCH(g);
+    GRZ_CK(g, cudaGetLastError());
+    g->pr_cut_vec = per;
+    return GRZ_OK;
+}
+
+// Chooses the hot sources of the loaded lists and encodes the list that the packed gather reads
+// (the pull list, or its source segments).  Once per loaded lists; one read-back.  Worth it when
+// the hot sources are at least a tenth of the edges: with 1% (a uniform graph) the gather is no
+// faster, with 20% (R-MAT 24) it is 13% faster, with 52% (R-MAT 20) 20-30%.  Lists below 2^18
+// vectors stay as they are: their props fit L1.
+static int pr_hot_prepare(grz_graph* g, const uint4* list, uint64_t nvec)
+{
+    const uint64_t V = g->V;
+    if (g->pr_hot_known && (!g->pr_nhot || g->pr_hot_of == list)) return GRZ_OK;
+    cudaStream_t st = g->stream;
+    const uint64_t words = (V + 31) / 32;
+    if (!g->pr_hot_known) {
+        g->pr_nhot = 0;
+        if (nvec < (1ull << 18) || V >= GRZ_HUB_BASE) {
+            g->pr_hot_known = 1;
+            return GRZ_OK;
+        }
+        const uint32_t dmin = (uint32_t)std::min<uint64_t>(g->E / V + 1, 0xffffffffull);
+        unsigned long long* hist = nullptr;
+        uint32_t* cnt = nullptr;
+        unsigned long long pick[3] = { 0, 0, 0 };
+        int rc = grz_dev_alloc(g, (void**)&hist, sizeof(unsigned long long) * (2 * HOT_BINS + 3));
+        if (!rc) rc = grz_cuda_check(g, cudaMemsetAsync(hist, 0, sizeof(unsigned long long) * (2 * HOT_BINS + 3), st), "memset");
+        if (!rc) {
+            const unsigned grid = (unsigned)std::min<uint64_t>(blocks_for(V), (uint64_t)g->num_sms * 8);
+            k_hot_hist<<<grid, PR_THREADS, 0, st>>>(g->degree, V, dmin, hist); GRZ_COUNT_LAUNCH(g);
+            k_hot_pick<<<1, 32, 0, st>>>(hist, GRZ_PR_HOT_MAX, hist + 2 * HOT_BINS); GRZ_COUNT_LAUNCH(g);
+            rc = grz_cuda_check(g, cudaGetLastError(), "k_hot_pick");
+        }
+        if (!rc) rc = grz_cuda_check(g, cudaMemcpyAsync(pick, hist + 2 * HOT_BINS, sizeof(pick), cudaMemcpyDeviceToHost, st), "D2H");
+        if (!rc) rc = grz_cuda_check(g, cudaStreamSynchronize(st), "hot sources");
+        if (!rc && pick[1] && pick[2] * 10 >= g->E) {
+            rc = grz_dev_alloc(g, (void**)&g->pr_hotmap, sizeof(uint2) * words);
+            if (!rc) rc = grz_dev_alloc(g, (void**)&cnt, sizeof(uint32_t) * words);
+            if (!rc) {
+                k_hot_mark<<<blocks_for(V), PR_THREADS, 0, st>>>(g->degree, V, dmin, (uint32_t)pick[0], g->pr_hotmap, cnt); GRZ_COUNT_LAUNCH(g);
+                rc = grz_cuda_check(g, cudaGetLastError(), "k_hot_mark");
+            }
+            if (!rc) rc = grz_exclusive_sum_u32_on(g, cnt, cnt, words, nullptr, st);
+            if (!rc) {
+                k_hot_base<<<blocks_for(words), PR_THREADS, 0, st>>>(cnt, words, g->pr_hotmap); GRZ_COUNT_LAUNCH(g);
+                rc = grz_cuda_check(g, cudaGetLastError(), "k_hot_base");
+            }
+            for (int i = 0; i < 2 && !rc; ++i) {
+                if (!g->pr_hot[i]) rc = grz_cuda_check(g, cudaMalloc((void**)&g->pr_hot[i], sizeof(pk_t) * (GRZ_PR_HOT_MAX + 2)), "hot props");
+                // the slots past the last stay zero
+                if (!rc) rc = grz_cuda_check(g, cudaMemsetAsync(g->pr_hot[i], 0, sizeof(pk_t) * (GRZ_PR_HOT_MAX + 2), st), "memset");
+            }
+        }
+        grz_dev_free(g, hist);
+        grz_dev_free(g, cnt);
+        if (rc) return rc;
+        if (g->pr_hotmap) g->pr_nhot = (uint32_t)pick[1];
+        g->pr_hot_known = 1;
+        if (!g->pr_nhot) return GRZ_OK;
+    }
+    grz_dev_free(g, g->pr_hot_nbr);
+    g->pr_hot_nbr = nullptr;
+    g->pr_hot_of = nullptr;
+    GRZ_TRY(grz_dev_alloc(g, (void**)&g->pr_hot_nbr, sizeof(uint4) * nvec));
+    k_hot_encode<<<blocks_for(nvec), PR_THREADS, 0, st>>>(list, nvec, g->pr_hotmap, g->pr_nhot, g->pr_hot_nbr); GRZ_COUNT_LAUNCH(g);
+    GRZ_CK(g, cudaGetLastError());
+    g->pr_hot_of = list;
     return GRZ_OK;
 }
 
@@ -748,26 +1135,19 @@ int grz_pr_prepare(grz_graph* g)
         // (also after a reload with the same V, which kept the arrays)
         GRZ_CK(g, cudaMemsetAsync(g->pr_rowacc, 0, sizeof(u128) * (V + 1), g->stream));
         g->pr_rowacc_stale = 0;
-        if (V) {
-            k_pr_cutbits<<<blocks_for(V), PR_THREADS, 0, g->stream>>>(g->pull.rowptr, V, g->pr_cut); GRZ_COUNT_LAUNCH(g);
-            GRZ_CK(g, cudaGetLastError());
-        }
+        g->pr_cut_vec = 0;
         // entry V of both prop arrays is a permanent zero that invalid lanes gather
         GRZ_CK(g, cudaMemsetAsync(g->pr_fx[0], 0, sizeof(u128) * (V + 1), g->stream));
         GRZ_CK(g, cudaMemsetAsync(g->pr_fx[1], 0, sizeof(u128) * (V + 1), g->stream));
-        for (double* d : g->pr_d)
-            if (d) GRZ_CK(g, cudaMemsetAsync(d, 0, sizeof(double) * (V + 1), g->stream));
+        for (pk_t* p : g->pr_pk)
+            if (p) GRZ_CK(g, cudaMemsetAsync(p, 0, sizeof(pk_t) * (V + 1), g->stream));
         g->pr_lists_changed = 0;
     }
-    // Doubles gathered instead of 16-byte fixed point: chosen, or when the fixed-point props
-    // exceed 6x L2.  Below that the gathers are bound by the L1/L2 path and the per-edge
-    // conversion costs more than the smaller working set saves; above it the DRAM sectors of the
-    // random gathers dominate and halving the props wins.  GB300 sweep (16 iterations,
-    // fixed vs doubles): R-MAT 24 25.7 vs 31.8 ms, 25 64.6 vs 67.4 ms, 26 179.1 vs 156.4 ms,
-    // 27 413 vs 371 ms.
-    const int pick = g->tune.pr_props;
-    g->pr_dmode = pick == 2 || (pick == 0 && (uint64_t)sizeof(u128) * V > 6ull * (uint64_t)g->l2_bytes);
-    // Source segments when even the double props are far larger than L2 (or when chosen): each
+    // Packed props (8 bytes) unless 16-byte fixed point is asked for: half the gathered working set
+    // for a few integer instructions per edge (GB300, a thread per vector, gather per iteration, 16 ->
+    // 8 bytes: R-MAT 20 71 -> 63 us, R-MAT 24 1089 -> 938 us, uniform 3M vertices 153 -> 145 us).
+    g->pr_pkmode = g->tune.pr_props != 1;
+    // Source segments when even the packed props are far larger than L2 (or when chosen): each
     // segment's props (8 bytes x 2^bits) mostly stay in L2 while its edges stream, instead of one
     // random DRAM sector per gathered prop.  Segment props of about the size of L2 are best: on
     // GB300 at R-MAT 27 (16 iterations) the gather took 23.2 ms unsegmented and 17.8 / 18.1 /
@@ -781,14 +1161,16 @@ int grz_pr_prepare(grz_graph* g)
         const int rc = pr_build_segments(g, bits);
         if (rc) return rc;
         g->pr_segmode = 1;
-        g->pr_dmode = 1;  // the segments gather the props as doubles
+        g->pr_pkmode = 1;  // the segments gather the props packed
     }
-    if (g->pr_dmode && !g->pr_d[0]) {
-        GRZ_CK(g, cudaMalloc((void**)&g->pr_d[0], sizeof(double) * (V + 1)));
-        GRZ_CK(g, cudaMalloc((void**)&g->pr_d[1], sizeof(double) * (V + 1)));
-        GRZ_CK(g, cudaMemsetAsync(g->pr_d[0], 0, sizeof(double) * (V + 1), g->stream));
-        GRZ_CK(g, cudaMemsetAsync(g->pr_d[1], 0, sizeof(double) * (V + 1), g->stream));
+    if (g->pr_pkmode && !g->pr_pk[0]) {
+        GRZ_CK(g, cudaMalloc((void**)&g->pr_pk[0], sizeof(pk_t) * (V + 1)));
+        GRZ_CK(g, cudaMalloc((void**)&g->pr_pk[1], sizeof(pk_t) * (V + 1)));
+        GRZ_CK(g, cudaMemsetAsync(g->pr_pk[0], 0, sizeof(pk_t) * (V + 1), g->stream));
+        GRZ_CK(g, cudaMemsetAsync(g->pr_pk[1], 0, sizeof(pk_t) * (V + 1), g->stream));
     }
+    if (g->pr_pkmode && !g->pull.nhub && V)
+        GRZ_TRY(g->pr_segmode ? pr_hot_prepare(g, g->seg_nbr, g->seg_first[g->nseg]) : pr_hot_prepare(g, g->pull.nbr, g->pull.nvec));
     return GRZ_OK;
 }
 
@@ -866,7 +1248,7 @@ int grz_pr_init_state(grz_graph* g, double damping)
     if (rc) return rc;
     g->pr_damping = damping;
     g->pr_cur = 0;
-    g->pr_fx_stale = g->pr_d_stale = 0;
+    g->pr_fx_stale = g->pr_pk_stale = 0;
     g->pr_sum_cur = 0;
     g->pr_iters_done = 0;
     GRZ_CK(g, cudaMemsetAsync(g->pr_sum, 0, sizeof(u128) * 2 * (blocks_for(g->V) + 1), g->stream));
@@ -874,21 +1256,22 @@ int grz_pr_init_state(grz_graph* g, double damping)
     g->pr_nparts[0] = g->pr_nparts[1] = blocks_for(g->V);
     if (g->V) {
         k_pr_init<<<blocks_for(g->V), PR_THREADS, 0, g->stream>>>(g->outdeg, g->degree, g->V, g->prop, g->accum, g->pr_fx[0],
-                                                                 g->pr_dmode ? g->pr_d[0] : nullptr, g->pr_sum); GRZ_COUNT_LAUNCH(g);
+                                                                 g->pr_pkmode ? g->pr_pk[0] : nullptr, g->pr_nhot ? g->pr_hotmap : nullptr,
+                                                                 g->pr_hot[0], g->pr_sum); GRZ_COUNT_LAUNCH(g);
         GRZ_CK(g, cudaGetLastError());
     }
     return GRZ_OK;
 }
 
-// resident blocks per SM of the gather kernel (its grid is persistent: SMs x resident)
-template <typename P, bool ADD>
+// resident blocks per SM of the general gather kernel (its grid is persistent: SMs x resident)
+template <typename P>
 static int pr_gather_resident(grz_graph* g)
 {
     static int resident[64] = {};
     if (g->device < 0 || g->device >= 64) return 1;
     if (!resident[g->device]) {
         int r = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&r, k_pr_gather<P, ADD>, PR_THREADS, 0) != cudaSuccess || r < 1) {
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&r, k_pr_gather<P>, PR_THREADS, 0) != cudaSuccess || r < 1) {
             cudaGetLastError();
             r = 1;
         }
@@ -897,49 +1280,88 @@ static int pr_gather_resident(grz_graph* g)
     return resident[g->device];
 }
 
-// one gather launch over vectors [first, first + count) of a list of list_nvec vectors
-template <typename P, bool ADD>
-static void pr_gather_launch(grz_graph* g, const uint4* nbr, const uint32_t* dstv, uint64_t first, uint64_t count, uint64_t list_nvec,
-                             const P* props, const uint32_t* hub_vid, uint32_t nhub, const PRConst& pc)
-{
-    const uint64_t want = g->tune.pr_grid ? g->tune.pr_grid : (uint64_t)g->num_sms * pr_gather_resident<P, ADD>(g);
-    const unsigned grid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(blocks_for(count), want));
-    k_pr_gather<P, ADD><<<grid, PR_THREADS, 0, g->stream>>>(nbr, dstv, first, count, list_nvec, props, (uint32_t)g->V, g->pr_rowacc,
-                                                            hub_vid, nhub, pc);
-    GRZ_COUNT_LAUNCH(g);
-}
-
+// the general gather over vectors [first, first + count) of the pull list
 template <typename P>
 static int pr_gather(grz_graph* g, uint64_t first, uint64_t count, const PRConst& pc, const P* props)
 {
     if (count == 0) return GRZ_OK;
     grz_prof_begin(g, GRZ_PROF_PR_GATHER);
-    pr_gather_launch<P, false>(g, g->pull.nbr, g->pull.shared, first, count, g->pull.nvec, props, g->pull.hub_vid, g->pull.nhub, pc);
+    const uint64_t want = g->tune.pr_grid ? g->tune.pr_grid : (uint64_t)g->num_sms * pr_gather_resident<P>(g);
+    const unsigned grid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(blocks_for(count), want));
+    k_pr_gather<P><<<grid, PR_THREADS, 0, g->stream>>>(g->pull.nbr, g->pull.shared, first, count, g->pull.nvec, props, (uint32_t)g->V,
+                                                       g->pr_rowacc, g->pull.hub_vid, g->pull.nhub, pc);
+    GRZ_COUNT_LAUNCH(g);
     grz_prof_end(g);
     return grz_cuda_check(g, cudaGetLastError(), "k_pr_gather");
 }
 
+// shared-memory opt-in of the packed gather with a hot table, once per device
+static int pr_gather_pk_config(grz_graph* g)
+{
+    static bool done[64] = {};
+    if (g->device >= 0 && g->device < 64 && done[g->device]) return GRZ_OK;
+    const int bytes = (int)(sizeof(pk_t) * (GRZ_PR_HOT_MAX + 2));
+    GRZ_CK(g, cudaFuncSetAttribute(k_pr_gather_pk<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+    GRZ_CK(g, cudaFuncSetAttribute(k_pr_gather_pk<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+    if (g->device >= 0 && g->device < 64) done[g->device] = true;
+    return GRZ_OK;
+}
+
+static unsigned pr_gather_pk_grid(const grz_graph* g, uint64_t nvec)
+{
+    const uint64_t want = g->tune.pr_grid ? g->tune.pr_grid : (uint64_t)g->num_sms;
+    return (unsigned)std::max<uint64_t>(1, std::min<uint64_t>((nvec + PK_MIN_RANGE - 1) / PK_MIN_RANGE, want));
+}
+
+// vectors of a warp's range: an even share of the list, a multiple of 4
+static uint32_t pr_gather_pk_range(uint64_t nvec, unsigned grid)
+{
+    const uint64_t nwarps = (uint64_t)grid * (PK_THREADS / 32);
+    const uint64_t share = ((nvec + nwarps - 1) / nwarps + 3) & ~3ull;
+    return (uint32_t)std::max<uint64_t>(share, PK_MIN_RANGE);
+}
+
+// the packed gather over vectors [first, end) of `nbr` (encoded when there are hot sources)
+template <bool ADD>
+static int pr_gather_pk(grz_graph* g, const uint4* nbr, const uint32_t* dstv, uint64_t first, uint64_t end, const PRConst& pc)
+{
+    const uint64_t span = end - (first & ~3ull);
+    const unsigned grid = pr_gather_pk_grid(g, span);
+    const uint32_t per = pr_gather_pk_range(span, grid);
+    const pk_t* props = g->pr_pk[g->pr_cur];
+    if (g->pr_nhot) {
+        GRZ_TRY(pr_gather_pk_config(g));
+        const size_t smem = sizeof(pk_t) * 2 * ((g->pr_nhot + 2) / 2);
+        k_pr_gather_pk<true, ADD><<<grid, PK_THREADS, smem, g->stream>>>(nbr, dstv, (uint32_t)first, (uint32_t)end, per, props, (uint32_t)g->V,
+                                                                         g->pr_hot[g->pr_cur], g->pr_nhot, g->pr_rowacc, pc);
+    } else {
+        k_pr_gather_pk<false, ADD><<<grid, PK_THREADS, 0, g->stream>>>(nbr, dstv, (uint32_t)first, (uint32_t)end, per, props, (uint32_t)g->V,
+                                                                       nullptr, 0u, g->pr_rowacc, pc);
+    }
+    GRZ_COUNT_LAUNCH(g);
+    return grz_cuda_check(g, cudaGetLastError(), "k_pr_gather_pk");
+}
+
 // The gather over the source segments in order, each adding into the accumulators (which the
 // apply of segmented iterations leaves all zero).  One profiler record spans all segments.
-static int pr_gather_segments(grz_graph* g, const PRConst& pc0, const double* props)
+static int pr_gather_segments(grz_graph* g, const PRConst& pc0)
 {
     grz_prof_begin(g, GRZ_PROF_PR_GATHER);
+    const uint4* nbr = g->pr_nhot ? g->pr_hot_nbr : g->seg_nbr;
     bool first = true;
-    for (uint32_t sg = 0; sg < g->nseg; ++sg) {
-        const uint64_t a = g->seg_first[sg], n = g->seg_first[sg + 1] - a;
-        if (n == 0) continue;
+    int rc = GRZ_OK;
+    for (uint32_t sg = 0; sg < g->nseg && !rc; ++sg) {
+        const uint64_t a = g->seg_first[sg], b = g->seg_first[sg + 1];
+        if (a == b) continue;
         PRConst pc = pc0;
         if (!first) pc.K_out = nullptr;  // the iteration's constant once
         first = false;
-        pr_gather_launch<double, true>(g, g->seg_nbr, g->seg_dst, a, n, g->seg_first[g->nseg], props, nullptr, 0u, pc);
+        rc = pr_gather_pk<true>(g, nbr, g->seg_dst, a, b, pc);
     }
-    if (first) {
-        // no edges at all: the constant still has to be published
-        k_pr_gather<double, true><<<1, PR_THREADS, 0, g->stream>>>(g->seg_nbr, g->seg_dst, 0, 0, 0, props, (uint32_t)g->V, g->pr_rowacc,
-                                                                   nullptr, 0u, pc0); GRZ_COUNT_LAUNCH(g);
-    }
+    // no edges at all: the constant still has to be published
+    if (first && !rc) rc = pr_gather_pk<true>(g, nbr, g->seg_dst, 0, 0, pc0);
     grz_prof_end(g);
-    return grz_cuda_check(g, cudaGetLastError(), "k_pr_gather (segments)");
+    return rc;
 }
 
 // one PageRank iteration: edge-pull gather + vertex phase (two kernels)
@@ -956,30 +1378,38 @@ int grz_pr_fused_iteration(grz_graph* g, int write_double_props)
     pc.damping = g->pr_damping;
     pc.c = (1.0 - g->pr_damping) / dV;
     pc.nverts = dV;
-    int rc = GRZ_OK;
+    // hot sources are chosen by grz_pr_init for a list without hub encoding
+    const bool packed = g->pr_pkmode && !g->pull.nhub;
+    const uint64_t n = g->pull.nvec;
+    int rc = g->pr_pkmode ? pr_sync_pk(g) : pr_sync_fx(g);
+    if (rc) return rc;
     if (g->pr_segmode) {
-        rc = pr_sync_d(g);
-        if (rc == GRZ_OK) rc = pr_gather_segments(g, pc, (const double*)g->pr_d[g->pr_cur]);
-    } else if (g->pr_dmode) {
-        rc = pr_sync_d(g);
-        if (rc == GRZ_OK) rc = pr_gather(g, 0, g->pull.nvec, pc, (const double*)g->pr_d[g->pr_cur]);
+        rc = pr_gather_segments(g, pc);
+    } else if (packed) {
+        rc = pr_cut_for(g, pr_gather_pk_range(n, pr_gather_pk_grid(g, n)));
+        if (rc) return rc;
+        grz_prof_begin(g, GRZ_PROF_PR_GATHER);
+        rc = pr_gather_pk<false>(g, g->pr_nhot ? g->pr_hot_nbr : g->pull.nbr, g->pull.shared, 0, n, pc);
+        grz_prof_end(g);
     } else {
-        rc = pr_sync_fx(g);
-        if (rc == GRZ_OK) rc = pr_gather(g, 0, g->pull.nvec, pc, (const u128*)g->pr_fx[g->pr_cur]);
+        rc = pr_cut_for(g, PR_THREADS);
+        if (!rc) rc = g->pr_pkmode ? pr_gather(g, 0, n, pc, (const pk_t*)g->pr_pk[g->pr_cur]) : pr_gather(g, 0, n, pc, (const u128*)g->pr_fx[g->pr_cur]);
     }
     if (rc) return rc;
+    const bool hot = g->pr_pkmode && g->pr_nhot;
     grz_prof_begin(g, GRZ_PROF_PR_APPLY);
     const uint64_t agrid = std::max<uint64_t>(1, std::min<uint64_t>((g->V + (uint64_t)PR_THREADS * PR_APPLY_U - 1) /
                                                                         ((uint64_t)PR_THREADS * PR_APPLY_U),
                                                                     (uint64_t)g->num_sms * PR_APPLY_RESIDENT));
     k_pr_apply<<<(unsigned)agrid, PR_THREADS, 0, g->stream>>>(g->pr_rowacc, g->pr_cut, g->pr_segmode, g->inv_deg, g->degree, g->V, g->pr_K,
                                                               g->pr_sum + (size_t)(k ^ 1) * stride, g->pr_damping, g->pr_fx[g->pr_cur ^ 1],
-                                                              g->pr_dmode ? g->pr_d[g->pr_cur ^ 1] : nullptr,
-                                                              write_double_props ? g->prop : nullptr); GRZ_COUNT_LAUNCH(g);
+                                                              g->pr_pkmode ? g->pr_pk[g->pr_cur ^ 1] : nullptr,
+                                                              write_double_props ? g->prop : nullptr, hot ? g->pr_hotmap : nullptr,
+                                                              g->pr_hot[g->pr_cur ^ 1]); GRZ_COUNT_LAUNCH(g);
     grz_prof_end(g);
     GRZ_CK(g, cudaGetLastError());
     g->pr_nparts[k ^ 1] = (uint32_t)agrid;
-    g->pr_fx_stale = g->pr_dmode;  // the new props are only in pr_d
+    g->pr_fx_stale = g->pr_pkmode;  // the new props are only in pr_pk
     g->pr_rowacc_stale = 1;
     g->pr_cur ^= 1;
     g->pr_sum_cur = k ^ 1;
@@ -1020,11 +1450,12 @@ int grz_pr_persistent_iterations(grz_graph* g, uint32_t iters)
         GRZ_CK(g, cudaMalloc(&g->pr_bar, sizeof(PRBar)));
         GRZ_CK(g, cudaMallocHost(&g->pr_bar_host, sizeof(PRBar)));
     }
-    int rc = g->pr_dmode ? pr_sync_d(g) : pr_sync_fx(g);
+    int rc = g->pr_pkmode ? pr_sync_pk(g) : pr_sync_fx(g);
+    if (!rc) rc = pr_cut_for(g, PR_THREADS);
     if (rc) return rc;
     const bool eight = g->tune.pr_persistent == 3;
-    const int resident = eight ? (g->pr_dmode ? pr_persistent_resident<double, 8>(g) : pr_persistent_resident<u128, 8>(g))
-                               : (g->pr_dmode ? pr_persistent_resident<double, 6>(g) : pr_persistent_resident<u128, 6>(g));
+    const int resident = eight ? (g->pr_pkmode ? pr_persistent_resident<pk_t, 8>(g) : pr_persistent_resident<u128, 8>(g))
+                               : (g->pr_pkmode ? pr_persistent_resident<pk_t, 6>(g) : pr_persistent_resident<u128, 6>(g));
     uint64_t want = g->tune.pr_grid ? g->tune.pr_grid : (uint64_t)g->num_sms * resident;
     want = std::min<uint64_t>(want, (uint64_t)g->num_sms * resident);  // co-resident
     const unsigned grid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(want, blocks_for(g->V)));  // partial slots
@@ -1044,9 +1475,9 @@ int grz_pr_persistent_iterations(grz_graph* g, uint32_t iters)
     q.degree = g->degree;
     q.fx[0] = g->pr_fx[0];
     q.fx[1] = g->pr_fx[1];
-    q.d[0] = g->pr_d[0];
-    q.d[1] = g->pr_d[1];
-    q.dmode = g->pr_dmode;
+    q.pk[0] = g->pr_pk[0];
+    q.pk[1] = g->pr_pk[1];
+    q.pkmode = g->pr_pkmode;
     q.cur = g->pr_cur;
     q.sum[0] = g->pr_sum;
     q.sum[1] = g->pr_sum + stride;
@@ -1064,8 +1495,8 @@ int grz_pr_persistent_iterations(grz_graph* g, uint32_t iters)
     q.time_phases = timing ? 1 : 0;
     GRZ_CK(g, cudaMemsetAsync(g->pr_bar, 0, 4 * sizeof(unsigned int), g->stream));
     void* args[] = { &q };
-    const void* fn = eight ? (g->pr_dmode ? (const void*)k_pr_persistent<double, 8> : (const void*)k_pr_persistent<u128, 8>)
-                           : (g->pr_dmode ? (const void*)k_pr_persistent<double, 6> : (const void*)k_pr_persistent<u128, 6>);
+    const void* fn = eight ? (g->pr_pkmode ? (const void*)k_pr_persistent<pk_t, 8> : (const void*)k_pr_persistent<u128, 8>)
+                           : (g->pr_pkmode ? (const void*)k_pr_persistent<pk_t, 6> : (const void*)k_pr_persistent<u128, 6>);
     GRZ_CK(g, cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(PR_THREADS), args, 0, g->stream));
     GRZ_COUNT_LAUNCH(g);
     const size_t rb = timing ? sizeof(PRBar) : 4 * sizeof(unsigned int);
@@ -1090,7 +1521,12 @@ int grz_pr_persistent_iterations(grz_graph* g, uint32_t iters)
         g->pr_sum_cur ^= 1;
     }
     g->pr_nparts[g->pr_sum_cur] = grid;
-    g->pr_fx_stale = g->pr_dmode;
+    g->pr_fx_stale = g->pr_pkmode;
+    if (g->pr_nhot) {
+        // the persistent form does not keep the hot table: packed again before the next fused iteration
+        GRZ_TRY(pr_sync_fx(g));
+        g->pr_pk_stale = 1;
+    }
     g->pr_rowacc_stale = 1;
     g->pr_iters_done += iters;
     return GRZ_OK;
@@ -1126,7 +1562,7 @@ int grz_pr_vertex(grz_graph* g, uint64_t first, uint64_t count, double S)
     const double K = fma(G, g->pr_damping, c);
     int rc = pr_sync_fx(g);
     if (rc) return rc;
-    g->pr_d_stale = g->pr_d[0] != nullptr;  // the props change in the fixed-point form only
+    g->pr_pk_stale = g->pr_pk[0] != nullptr;  // the props change in the fixed-point form only
     // the props being gathered are rewritten in place: the boundary path keeps one live copy
     k_pr_vertex<<<blocks_for(count), PR_THREADS, 0, g->stream>>>(g->accum, g->inv_deg, g->prop, g->pr_fx[g->pr_cur],
                                                                  first, count, g->pr_damping, K); GRZ_COUNT_LAUNCH(g);
@@ -1139,8 +1575,7 @@ int grz_pr_props_to_double(grz_graph* g)
 {
     if (g->V == 0) return GRZ_OK;
     if (g->pr_fx_stale) {
-        // the double props convert exactly to the fixed-point ones; report what those round to
-        k_double_to_fx<<<blocks_for(g->V), PR_THREADS, 0, g->stream>>>(g->pr_d[g->pr_cur], g->V, nullptr, g->prop); GRZ_COUNT_LAUNCH(g);
+        k_pk_unpack<<<blocks_for(g->V), PR_THREADS, 0, g->stream>>>(g->pr_pk[g->pr_cur], g->V, nullptr, g->prop); GRZ_COUNT_LAUNCH(g);
     } else {
         k_fx_to_double<<<blocks_for(g->V), PR_THREADS, 0, g->stream>>>(g->pr_fx[g->pr_cur], g->V, g->prop); GRZ_COUNT_LAUNCH(g);
     }
