@@ -136,7 +136,8 @@ static void free_graph_data(grz_graph* g, uint64_t next_V = ~0ull)
     grz_dev_free(g, g->pr_hot_nbr);
     grz_dev_free(g, g->pr_hotmap);
     g->pr_hot_nbr = nullptr;
-    g->pr_hot_of = nullptr;
+    grz_dev_free(g, g->pr_hot_vid);
+    g->pr_hot_vid = nullptr;
     g->pr_hotmap = nullptr;
     g->pr_nhot = 0;
     g->pr_hot_known = 0;
@@ -644,7 +645,7 @@ extern "C" int grz_graph_get_info(const grz_graph* gc, grz_graph_info_t* out)
     b += (g->V + 8) * 8 * 3 + g->V * 12;
     if (g->pr_fx[0]) b += g->V * (16 * 3 + 4);
     if (g->pr_pk[0]) b += g->V * 16;
-    if (g->pr_hot_nbr) b += 16 * (g->pr_segmode ? g->seg_first[g->nseg] : g->pull.nvec);
+    if (g->pr_hot_nbr) b += 16 * g->pull.nvec;
     out->device_bytes = b;
     return GRZ_OK;
 }

@@ -1610,8 +1610,8 @@ static int launch_cc_pull_bt(grz_graph* g, uint64_t first, uint64_t count, const
             const uint64_t a = g->seg_first[sg], n = g->seg_first[sg + 1] - a;
             if (n == 0) continue;
             const uint64_t sgrid = std::max<uint64_t>(1, std::min<uint64_t>(grid, (n + BT - 1) / BT));
-            k_cc_pull<BT, false><<<(unsigned)sgrid, BT, 0, g->stream>>>(g->seg_nbr, g->seg_dst, a, n, (uint32_t)g->V, f.label, nullptr,
-                                                                       0u, 0u, f.has_next, vc, f.vote, f.chg, f.iter, f.level_dev, 2,
+            k_cc_pull<BT, false><<<(unsigned)sgrid, BT, 0, g->stream>>>(g->seg_nbr, g->seg_dst, a, n, (uint32_t)g->V, f.label,
+                                                                       g->pr_hot_vid, g->seg_nhot, 0u, f.has_next, vc, f.vote, f.chg, f.iter, f.level_dev, 2,
                                                                        f.dev_err); GRZ_COUNT_LAUNCH(g);
         }
         k_cc_pull<BT, BULK><<<(unsigned)grid, BT, smem, g->stream>>>(g->pull.nbr, g->pull.shared, first, count, (uint32_t)g->V, f.label,
@@ -2083,6 +2083,7 @@ static int build_run_graph(grz_graph* g)
     f.run_key[1] = f.flags;
     f.run_tune = g->tune;
     f.run_seg = cc_use_segments(g) ? g->seg_nbr : nullptr;
+    f.run_seg_gen = g->seg_gen;
     return GRZ_OK;
 }
 
@@ -2113,7 +2114,7 @@ int grz_frontier_run_graph(grz_graph* g, uint64_t* launches)
     if (rc) return rc;
     const bool same = f.run_exec && f.run_bm[0] == f.has && f.run_bm[1] == f.has_next && f.run_key[0] == f.app &&
                       f.run_key[1] == f.flags && !memcmp(&f.run_tune, &g->tune, sizeof(g->tune)) &&
-                      f.run_seg == (cc_use_segments(g) ? g->seg_nbr : nullptr);
+                      f.run_seg == (cc_use_segments(g) ? g->seg_nbr : nullptr) && f.run_seg_gen == g->seg_gen;
     if (!same) {
         int resident = 0;
         const size_t smem = sizeof(uint32_t) * std::min<uint32_t>(g->tune.cc_cache, g->pull.nhub);

@@ -486,6 +486,7 @@ struct grz_frontier_state {
     int run_key[2];                  // app, flags of the captured graph
     grz_tuning run_tune;             // kernel shapes of the captured graph
     const uint4* run_seg;            // source-segmented lists the captured graph reads (or null)
+    uint32_t run_seg_gen;            // their build
     // snapshot for timing both engines from one state
     void* snap;
     uint64_t snap_bytes;
@@ -525,8 +526,10 @@ struct grz_graph {
     uint32_t seg_bits;    // 0: not built
     uint32_t nseg;
     uint64_t seg_first[GRZ_PR_MAX_SEGMENTS + 1];
-    uint4* seg_nbr;
+    uint4* seg_nbr;       // hot sources as GRZ_HUB_BASE + slot (pr_hot_vid) when seg_nhot
     uint32_t* seg_dst;
+    uint32_t seg_nhot;    // hot sources encoded
+    uint32_t seg_gen;     // builds so far (a captured run names one of them)
     int pr_segmode;       // fused iterations gather segment by segment
     void* pr_bar;         // grid barrier and phase timer of the persistent PageRank kernel (device)
     void* pr_bar_host;    // pinned read-back of its error word and phase times
@@ -537,8 +540,8 @@ struct grz_graph {
     uint64_t pr_cut_vec;  // vectors per gather range that pr_cut was made for (0: not made)
     // hot sources of the packed gather (grz_pr.cu): the few of the highest out-degrees, whose props
     // every block of the gather keeps in shared memory
-    uint4* pr_hot_nbr;    // the gathered list (pull, or its segments) with hot sources as GRZ_HUB_BASE + slot
-    const uint4* pr_hot_of;        // the list it encodes
+    uint4* pr_hot_nbr;    // the pull list with hot sources as GRZ_HUB_BASE + slot
+    uint32_t* pr_hot_vid; // vertex of each slot
     unsigned long long* pr_hot[2]; // u64[GRZ_PR_HOT_MAX + 2]: packed props of the hot slots (ping-pong), then zeros
     uint2* pr_hotmap;     // per 32 vertices: their hot bits, and the slot of the first
     uint32_t pr_nhot;     // hot sources (0: none, or not worth it)

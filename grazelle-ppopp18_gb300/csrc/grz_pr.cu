@@ -689,118 +689,91 @@ __global__ void k_pr_cutbits(const uint32_t* __restrict__ rowptr, uint64_t V, ui
 // by source (the -pull order), so the edges from source segment s form one run of lanes
 // [a_s, b_s).  Segment s's list has ceil((b_s - a_s) / 4) vectors per destination, grouped by
 // destination in ascending order; the segment lists are concatenated in segment order.
+//
+// Both passes over the list run a thread per vector, so a hub's lanes are spread over the grid and
+// every read is coalesced (GB300, R-MAT 26 in 4 segments, against a thread per destination that
+// searched its lanes for each segment's run: 20.9 -> 9.3 ms of device time, hot
+// encoding included).
 
-// source of lane L of a destination whose vectors start at r0
-__device__ __forceinline__ uint32_t lane_src(const uint32_t* __restrict__ nbr32, uint32_t r0, uint32_t L)
+// a code of the gathered list: the slot of a hot source, the zero slot of an empty lane, else the ID
+__device__ __forceinline__ uint32_t hot_code(uint32_t id, const uint2* __restrict__ hotmap, uint32_t nhot)
 {
-    return __ldg(nbr32 + (uint64_t)r0 * 4 + L);
+    if (id == GRZ_INVALID_ID) return GRZ_HUB_BASE | nhot;
+    const uint2 m = __ldg(hotmap + (id >> 5));
+    const uint32_t bit = id & 31u;
+    return (m.x >> bit) & 1u ? GRZ_HUB_BASE | (m.y + __popc(m.x & ((1u << bit) - 1u))) : id;
 }
 
-// valid lanes of the destination with vectors [r0, r1) (only its last vector can be partial)
-__device__ __forceinline__ uint32_t dst_lanes(const uint4* __restrict__ nbr, uint32_t r0, uint32_t r1)
+// the source after vector v's lanes in its destination's order, or GRZ_INVALID_ID if v is its last
+__device__ __forceinline__ uint32_t seg_next_src(const uint4* __restrict__ nbr, uint32_t v, uint32_t r1)
 {
-    const uint4 t = __ldg(nbr + r1 - 1);
-    return 4 * (r1 - r0 - 1) + (t.x != GRZ_INVALID_ID) + (t.y != GRZ_INVALID_ID) + (t.z != GRZ_INVALID_ID) + (t.w != GRZ_INVALID_ID);
+    return v + 1 < r1 ? __ldg(&nbr[v + 1].x) : GRZ_INVALID_ID;
 }
 
-// first lane in [lo, hi) whose source is >= key, else hi
-__device__ __forceinline__ uint32_t lane_lower_bound(const uint32_t* __restrict__ nbr32, uint32_t r0, uint32_t lo, uint32_t hi,
-                                                     uint64_t key)
+// start and end lane of the run of every (segment, destination) pair: [s * (V + 1) + d], both 0 for
+// a pair without edges
+__global__ void __launch_bounds__(PR_THREADS) k_seg_bounds(const uint4* __restrict__ nbr, const uint32_t* __restrict__ dstv,
+                                                           const uint32_t* __restrict__ rowptr, uint64_t nvec, uint64_t V, uint32_t bits,
+                                                           uint32_t* __restrict__ start, uint32_t* __restrict__ end)
 {
-    while (lo < hi) {
-        const uint32_t mid = lo + (hi - lo) / 2;
-        if ((uint64_t)lane_src(nbr32, r0, mid) < key) lo = mid + 1;
-        else hi = mid;
-    }
-    return lo;
-}
-
-// first lane at or after p + 1 whose source is >= key (lane p's source is below key): galloping,
-// then a binary search, so a run of n lanes costs O(log n) reads
-__device__ __forceinline__ uint32_t lane_gallop(const uint32_t* __restrict__ nbr32, uint32_t r0, uint32_t p, uint32_t L, uint64_t key)
-{
-    uint32_t lo = p + 1, step = 1, hi = p + 1;
-    while (hi < L && (uint64_t)lane_src(nbr32, r0, hi) < key) {
-        lo = hi + 1;
-        step <<= 1;
-        hi = (p + step < L) ? p + step : L;
-    }
-    return lane_lower_bound(nbr32, r0, lo, hi < L ? hi : L, key);
-}
-
-// vectors of every (segment, destination): cnt[s * (V + 1) + d]; entries of empty pairs stay 0
-__global__ void k_seg_count(const uint4* __restrict__ nbr, const uint32_t* __restrict__ rowptr, uint32_t V, uint32_t bits,
-                            uint32_t* __restrict__ cnt)
-{
-    const uint32_t* nbr32 = reinterpret_cast<const uint32_t*>(nbr);
-    for (uint64_t d = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; d < V; d += (uint64_t)gridDim.x * blockDim.x) {
-        const uint32_t r0 = __ldg(rowptr + d), r1 = __ldg(rowptr + d + 1);
-        if (r0 == r1) continue;
-        const uint32_t L = dst_lanes(nbr, r0, r1);
-        uint32_t p = 0;
-        while (p < L) {
-            const uint32_t sg = lane_src(nbr32, r0, p) >> bits;
-            const uint32_t q = lane_gallop(nbr32, r0, p, L, (uint64_t)(sg + 1) << bits);
-            cnt[(uint64_t)sg * (V + 1) + d] = (q - p + 3) / 4;
-            p = q;
-        }
+    const uint64_t v = (uint64_t)blockIdx.x * PR_THREADS + threadIdx.x;
+    if (v >= nvec) return;
+    const uint32_t d = __ldg(dstv + v), r0 = __ldg(rowptr + d), r1 = __ldg(rowptr + d + 1);
+    const uint4 x = __ldg(nbr + v);
+    const uint32_t id[5] = { x.x, x.y, x.z, x.w, seg_next_src(nbr, (uint32_t)v, r1) };
+    const uint32_t pos = 4 * ((uint32_t)v - r0);
+    if (pos == 0) start[(uint64_t)(id[0] >> bits) * (V + 1) + d] = 0;
+#pragma unroll
+    for (int l = 0; l < 4; ++l) {
+        if (id[l] == GRZ_INVALID_ID) break;
+        const uint32_t sg = id[l] >> bits;
+        if (id[l + 1] != GRZ_INVALID_ID && id[l + 1] >> bits == sg) continue;
+        end[(uint64_t)sg * (V + 1) + d] = pos + l + 1;
+        if (id[l + 1] != GRZ_INVALID_ID) start[(uint64_t)(id[l + 1] >> bits) * (V + 1) + d] = pos + l + 1;
     }
 }
 
-// run of one (segment, destination) pair too long for one thread: written by a whole block
-struct SegBig {
-    uint32_t d, a, b, out;  // destination, lanes [a, b), first output vector (within the segment)
+// vectors of every pair, in place of its end
+__global__ void __launch_bounds__(PR_THREADS) k_seg_sizes(const uint32_t* __restrict__ start, uint32_t* __restrict__ end, uint64_t n)
+{
+    for (uint64_t i = (uint64_t)blockIdx.x * PR_THREADS + threadIdx.x; i < n; i += (uint64_t)gridDim.x * PR_THREADS)
+        end[i] = (end[i] - start[i] + 3) / 4;
+}
+
+// every lane to its place: the lane of rank r in its run goes to lane r % 4 of vector r / 4 of the
+// pair, whose vectors start at seg_first[s] + off[s][d]; the run's last lane also fills the vector
+struct SegFirst {
+    uint64_t at[GRZ_PR_MAX_SEGMENTS + 1];
 };
-constexpr uint32_t SEG_BIG_VECTORS = 32;
-
-__device__ __forceinline__ void seg_write_vector(const uint32_t* __restrict__ nbr32, uint32_t r0, uint32_t a, uint32_t b, uint32_t j,
-                                                 uint32_t d, uint4* __restrict__ out_nbr, uint32_t* __restrict__ out_dst, uint64_t o)
+__global__ void __launch_bounds__(PR_THREADS) k_seg_emit(const uint4* __restrict__ nbr, const uint32_t* __restrict__ dstv,
+                                                         const uint32_t* __restrict__ rowptr, uint64_t nvec, uint64_t V, uint32_t bits,
+                                                         const uint32_t* __restrict__ start, const uint32_t* __restrict__ off,
+                                                         const __grid_constant__ SegFirst first, const uint2* __restrict__ hotmap, uint32_t nhot,
+                                                         uint32_t* __restrict__ out_nbr, uint32_t* __restrict__ out_dst)
 {
-    const uint32_t L0 = a + 4 * j;
-    uint4 v;
-    v.x = L0 + 0 < b ? lane_src(nbr32, r0, L0 + 0) : GRZ_INVALID_ID;
-    v.y = L0 + 1 < b ? lane_src(nbr32, r0, L0 + 1) : GRZ_INVALID_ID;
-    v.z = L0 + 2 < b ? lane_src(nbr32, r0, L0 + 2) : GRZ_INVALID_ID;
-    v.w = L0 + 3 < b ? lane_src(nbr32, r0, L0 + 3) : GRZ_INVALID_ID;
-    out_nbr[o] = v;
-    out_dst[o] = d;
-}
-
-// segment sg: each destination with a run writes its vectors at base + off[d]; runs of more than
-// SEG_BIG_VECTORS vectors are listed for k_seg_write_big instead
-__global__ void k_seg_write(const uint4* __restrict__ nbr, const uint32_t* __restrict__ rowptr, uint32_t V, uint32_t bits, uint32_t sg,
-                            const uint32_t* __restrict__ off, uint64_t base, uint4* __restrict__ out_nbr, uint32_t* __restrict__ out_dst,
-                            SegBig* __restrict__ big, uint32_t* __restrict__ nbig)
-{
-    const uint32_t* nbr32 = reinterpret_cast<const uint32_t*>(nbr);
-    for (uint64_t d = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; d < V; d += (uint64_t)gridDim.x * blockDim.x) {
-        const uint32_t o0 = __ldg(off + d), n = __ldg(off + d + 1) - o0;
-        if (n == 0) continue;
-        const uint32_t r0 = __ldg(rowptr + d), r1 = __ldg(rowptr + d + 1);
-        const uint32_t L = dst_lanes(nbr, r0, r1);
-        const uint32_t a = lane_lower_bound(nbr32, r0, 0, L, (uint64_t)sg << bits);
-        const uint32_t b = lane_lower_bound(nbr32, r0, a, L, (uint64_t)(sg + 1) << bits);
-        if (n > SEG_BIG_VECTORS) {
-            const uint32_t k = atomicAdd(nbig, 1u);
-            SegBig e;
-            e.d = (uint32_t)d; e.a = a; e.b = b; e.out = o0;
-            big[k] = e;
-            continue;
+    const uint64_t v = (uint64_t)blockIdx.x * PR_THREADS + threadIdx.x;
+    if (v >= nvec) return;
+    const uint32_t d = __ldg(dstv + v), r0 = __ldg(rowptr + d), r1 = __ldg(rowptr + d + 1);
+    const uint4 x = __ldg(nbr + v);
+    const uint32_t id[5] = { x.x, x.y, x.z, x.w, seg_next_src(nbr, (uint32_t)v, r1) };
+    const uint32_t pos = 4 * ((uint32_t)v - r0);
+    const uint32_t pad = hotmap ? GRZ_HUB_BASE | nhot : GRZ_INVALID_ID;
+    uint32_t sg = 0xffffffffu, a = 0;
+    uint64_t o = 0;
+#pragma unroll
+    for (int l = 0; l < 4; ++l) {
+        if (id[l] == GRZ_INVALID_ID) break;
+        if (id[l] >> bits != sg) {
+            sg = id[l] >> bits;
+            a = __ldg(start + (uint64_t)sg * (V + 1) + d);
+            o = first.at[sg] + __ldg(off + (uint64_t)sg * (V + 1) + d);
         }
-        for (uint32_t j = 0; j < n; ++j) seg_write_vector(nbr32, r0, a, b, j, (uint32_t)d, out_nbr, out_dst, base + o0 + j);
-    }
-}
-
-__global__ void k_seg_write_big(const uint4* __restrict__ nbr, const uint32_t* __restrict__ rowptr, const SegBig* __restrict__ big,
-                                const uint32_t* __restrict__ nbig, uint64_t base, uint4* __restrict__ out_nbr, uint32_t* __restrict__ out_dst)
-{
-    const uint32_t* nbr32 = reinterpret_cast<const uint32_t*>(nbr);
-    const uint32_t m = *nbig;
-    for (uint32_t k = blockIdx.x; k < m; k += gridDim.x) {
-        const SegBig e = big[k];
-        const uint32_t r0 = __ldg(rowptr + e.d);
-        const uint32_t n = (e.b - e.a + 3) / 4;
-        for (uint32_t j = threadIdx.x; j < n; j += blockDim.x) seg_write_vector(nbr32, r0, e.a, e.b, j, e.d, out_nbr, out_dst, base + e.out + j);
+        const uint32_t r = pos + l - a;
+        const uint64_t at = 4 * o + r;
+        out_nbr[at] = hotmap ? hot_code(id[l], hotmap, nhot) : id[l];
+        if ((r & 3u) == 0) out_dst[at >> 2] = d;
+        if (id[l + 1] == GRZ_INVALID_ID || id[l + 1] >> bits != sg)
+            for (uint64_t q = at + 1; q & 3u; ++q) out_nbr[q] = pad;
     }
 }
 
@@ -834,28 +807,36 @@ __global__ void k_pr_vertex(const double* __restrict__ accum, const double* __re
     prop_fx[v] = fx_from_double(p);
 }
 
-// execution_initialize_vertex_prop_pr (source/execution_pr.c:85-88): (1/V) / deg'
-__global__ void k_pr_init(const double* __restrict__ outdeg, const uint32_t* __restrict__ degree, uint64_t V,
-                          double* __restrict__ prop, double* __restrict__ accum, u128* __restrict__ prop_fx,
-                          pk_t* __restrict__ prop_pk, const uint2* __restrict__ hotmap, pk_t* __restrict__ hot,
-                          u128* __restrict__ part0)
+// execution_initialize_vertex_prop_pr (source/execution_pr.c:85-88): c / deg' with c = 1/V, in the
+// form the first gather reads (packed with the hot table, or fixed point).  The division is one
+// Newton step on the reciprocal 1/deg' (Markstein 1990): q0 = c * inv, r = c - q0 * deg' exactly by
+// one fma, q = q0 + r * inv.  It gives the division's result for every degree up to 4M at 40 vertex
+// counts and up to 100k at 360 others (checked against the division on the CPU), at 3 FP64
+// operations instead of a division's; the grid strides, with one partial of S_0 per block.  GB300, with
+// the accumulators' clearing (a division per vertex, props also written as doubles and in fixed point
+// -> now): V = 2^26 1.94 -> 0.70 ms, 2^20 52 -> 20 us.
+__global__ void __launch_bounds__(PR_THREADS, 8) k_pr_init(const double* __restrict__ inv_deg, const uint32_t* __restrict__ degree, uint64_t V,
+                                                           double c, u128* __restrict__ prop_fx, pk_t* __restrict__ prop_pk,
+                                                           const uint2* __restrict__ hotmap, pk_t* __restrict__ hot, u128* __restrict__ part0)
 {
     __shared__ u128 red[PR_THREADS / 32];
-    const uint64_t v = (uint64_t)blockIdx.x * PR_THREADS + threadIdx.x;
     u128 s = u128_zero();
-    if (v < V) {
-        const double dV = (double)V;
-        const double p = (1.0 / dV) / (outdeg[v] == 0.0 ? dV : outdeg[v]);
-        prop[v] = p;
-        accum[v] = 0.0;
-        const u128 pf = fx_from_double(p);
-        prop_fx[v] = pf;
+    for (uint64_t v = (uint64_t)blockIdx.x * PR_THREADS + threadIdx.x; v < V; v += (uint64_t)gridDim.x * PR_THREADS) {
+        const uint32_t deg = __ldg(degree + v);
+        const double inv = __ldg(inv_deg + v), d = deg ? (double)deg : (double)V;
+        const double q0 = __dmul_rn(c, inv);
+        const double p = __fma_rn(__fma_rn(-q0, d, c), inv, q0);
+        u128 pf;
         if (prop_pk) {
             const pk_t w = pk_from_double(p);
+            pf = pk_to_fx(w);
             prop_pk[v] = w;
             if (hotmap) hot_put(hotmap, hot, v, w);
+        } else {
+            pf = fx_from_double(p);
+            prop_fx[v] = pf;
         }
-        s = u128_mul32(pf, degree[v]);
+        s = u128_add(s, u128_mul32(pf, deg));
     }
     s = block_reduce_u128(s, red);
     if (threadIdx.x == 0) part0[blockIdx.x] = s;
@@ -925,20 +906,28 @@ __global__ void __launch_bounds__(PR_THREADS) k_hot_hist(const uint32_t* __restr
 }
 
 // out[0] = the lowest bin whose vertices and all above are at most `cap`, out[1] = how many they
-// are, out[2] = their out-edges.  One warp; 896 bins.
-__global__ void k_hot_pick(const unsigned long long* __restrict__ hist, uint32_t cap, unsigned long long* __restrict__ out)
+// are, out[2] = their out-edges.  One block, thread t has the t-th bin from the top.
+constexpr int HOT_PICK_T = (HOT_BINS + 31) / 32 * 32;
+
+__global__ void __launch_bounds__(HOT_PICK_T) k_hot_pick(const unsigned long long* __restrict__ hist, uint32_t cap,
+                                                         unsigned long long* __restrict__ out)
 {
-    if (threadIdx.x) return;
-    unsigned long long n = 0, e = 0;
-    uint32_t b = HOT_BINS;
-    while (b > 0 && n + hist[b - 1] <= cap) {
-        --b;
-        n += hist[b];
-        e += hist[HOT_BINS + b];
+    __shared__ unsigned long long sn[HOT_PICK_T / 32], se[HOT_PICK_T / 32];
+    const int t = threadIdx.x, lane = t & 31;
+    unsigned long long n = t < (int)HOT_BINS ? hist[HOT_BINS - 1 - t] : 0ull;
+    unsigned long long e = t < (int)HOT_BINS ? hist[2 * HOT_BINS - 1 - t] : 0ull;
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned long long yn = __shfl_up_sync(0xffffffffu, n, o), ye = __shfl_up_sync(0xffffffffu, e, o);
+        if (lane >= o) { n += yn; e += ye; }
     }
-    out[0] = b;
-    out[1] = n;
-    out[2] = e;
+    if (lane == 31) { sn[t >> 5] = n; se[t >> 5] = e; }
+    __syncthreads();
+    for (int w = 0; w < t >> 5; ++w) { n += sn[w]; e += se[w]; }
+    // the running counts ascend, so the bins within the cap are the first `fit`
+    const int fit = __syncthreads_count(t < (int)HOT_BINS && n <= cap);
+    if (t == 0) { out[0] = HOT_BINS - (uint32_t)fit; }
+    if (fit == 0 && t == 0) { out[1] = 0; out[2] = 0; }
+    if (t == fit - 1) { out[1] = n; out[2] = e; }
 }
 
 // the hot bits of 32 vertices per warp, and how many there are (words: (V + 31) / 32)
@@ -954,10 +943,14 @@ __global__ void __launch_bounds__(PR_THREADS) k_hot_mark(const uint32_t* __restr
     }
 }
 
-__global__ void k_hot_base(const uint32_t* __restrict__ base, uint64_t words, uint2* __restrict__ hotmap)
+// the slot of each word's first hot vertex, and the vertex of each slot
+__global__ void k_hot_base(const uint32_t* __restrict__ base, uint64_t words, uint2* __restrict__ hotmap, uint32_t* __restrict__ vid)
 {
     const uint64_t w = (uint64_t)blockIdx.x * PR_THREADS + threadIdx.x;
-    if (w < words) hotmap[w].y = base[w];
+    if (w >= words) return;
+    uint32_t b = base[w];
+    hotmap[w].y = b;
+    for (uint32_t m = hotmap[w].x; m; m &= m - 1) vid[b++] = (uint32_t)(32 * w) + (uint32_t)(__ffs(m) - 1);
 }
 
 // the list with its hot sources as GRZ_HUB_BASE + slot and its empty lanes as the slot after the
@@ -968,13 +961,7 @@ __global__ void __launch_bounds__(PR_THREADS) k_hot_encode(const uint4* __restri
     const uint64_t v = (uint64_t)blockIdx.x * PR_THREADS + threadIdx.x;
     if (v >= nvec) return;
     const uint4 s = __ldcs(nbr + v);
-    auto code = [&](uint32_t id) -> uint32_t {
-        if (id == GRZ_INVALID_ID) return GRZ_HUB_BASE | nhot;
-        const uint2 m = __ldg(hotmap + (id >> 5));
-        const uint32_t bit = id & 31u;
-        return (m.x >> bit) & 1u ? GRZ_HUB_BASE | (m.y + __popc(m.x & ((1u << bit) - 1u))) : id;
-    };
-    __stcs(out + v, make_uint4(code(s.x), code(s.y), code(s.z), code(s.w)));
+    __stcs(out + v, make_uint4(hot_code(s.x, hotmap, nhot), hot_code(s.y, hotmap, nhot), hot_code(s.z, hotmap, nhot), hot_code(s.w, hotmap, nhot)));
 }
 
 unsigned blocks_for(uint64_t n) { return (unsigned)((n + PR_THREADS - 1) / PR_THREADS); }
@@ -1026,77 +1013,92 @@ static int pr_cut_for(grz_graph* g, uint32_t per)
     return GRZ_OK;
 }
 
-// Chooses the hot sources of the loaded lists and encodes the list that the packed gather reads
-// (the pull list, or its source segments).  Once per loaded lists; one read-back.  Worth it when
-// the hot sources are at least a tenth of the edges: with 1% (a uniform graph) the gather is no
+// Chooses the hot sources of the loaded lists.  Once per loaded lists; one read-back.  Worth it
+// when the hot sources are at least a tenth of the edges: with 1% (a uniform graph) the gather is no
 // faster, with 20% (R-MAT 24) it is 13% faster, with 52% (R-MAT 20) 20-30%.  Lists below 2^18
 // vectors stay as they are: their props fit L1.
-static int pr_hot_prepare(grz_graph* g, const uint4* list, uint64_t nvec)
+static int pr_hot_choose(grz_graph* g)
 {
     const uint64_t V = g->V;
-    if (g->pr_hot_known && (!g->pr_nhot || g->pr_hot_of == list)) return GRZ_OK;
+    if (g->pr_hot_known) return GRZ_OK;
     cudaStream_t st = g->stream;
     const uint64_t words = (V + 31) / 32;
-    if (!g->pr_hot_known) {
-        g->pr_nhot = 0;
-        if (nvec < (1ull << 18) || V >= GRZ_HUB_BASE) {
-            g->pr_hot_known = 1;
-            return GRZ_OK;
-        }
-        const uint32_t dmin = (uint32_t)std::min<uint64_t>(g->E / V + 1, 0xffffffffull);
-        unsigned long long* hist = nullptr;
-        uint32_t* cnt = nullptr;
-        unsigned long long pick[3] = { 0, 0, 0 };
-        int rc = grz_dev_alloc(g, (void**)&hist, sizeof(unsigned long long) * (2 * HOT_BINS + 3));
-        if (!rc) rc = grz_cuda_check(g, cudaMemsetAsync(hist, 0, sizeof(unsigned long long) * (2 * HOT_BINS + 3), st), "memset");
-        if (!rc) {
-            const unsigned grid = (unsigned)std::min<uint64_t>(blocks_for(V), (uint64_t)g->num_sms * 8);
-            k_hot_hist<<<grid, PR_THREADS, 0, st>>>(g->degree, V, dmin, hist); GRZ_COUNT_LAUNCH(g);
-            k_hot_pick<<<1, 32, 0, st>>>(hist, GRZ_PR_HOT_MAX, hist + 2 * HOT_BINS); GRZ_COUNT_LAUNCH(g);
-            rc = grz_cuda_check(g, cudaGetLastError(), "k_hot_pick");
-        }
-        if (!rc) rc = grz_cuda_check(g, cudaMemcpyAsync(pick, hist + 2 * HOT_BINS, sizeof(pick), cudaMemcpyDeviceToHost, st), "D2H");
-        if (!rc) rc = grz_cuda_check(g, cudaStreamSynchronize(st), "hot sources");
-        if (!rc && pick[1] && pick[2] * 10 >= g->E) {
-            rc = grz_dev_alloc(g, (void**)&g->pr_hotmap, sizeof(uint2) * words);
-            if (!rc) rc = grz_dev_alloc(g, (void**)&cnt, sizeof(uint32_t) * words);
-            if (!rc) {
-                k_hot_mark<<<blocks_for(V), PR_THREADS, 0, st>>>(g->degree, V, dmin, (uint32_t)pick[0], g->pr_hotmap, cnt); GRZ_COUNT_LAUNCH(g);
-                rc = grz_cuda_check(g, cudaGetLastError(), "k_hot_mark");
-            }
-            if (!rc) rc = grz_exclusive_sum_u32_on(g, cnt, cnt, words, nullptr, st);
-            if (!rc) {
-                k_hot_base<<<blocks_for(words), PR_THREADS, 0, st>>>(cnt, words, g->pr_hotmap); GRZ_COUNT_LAUNCH(g);
-                rc = grz_cuda_check(g, cudaGetLastError(), "k_hot_base");
-            }
-            for (int i = 0; i < 2 && !rc; ++i) {
-                if (!g->pr_hot[i]) rc = grz_cuda_check(g, cudaMalloc((void**)&g->pr_hot[i], sizeof(pk_t) * (GRZ_PR_HOT_MAX + 2)), "hot props");
-                // the slots past the last stay zero
-                if (!rc) rc = grz_cuda_check(g, cudaMemsetAsync(g->pr_hot[i], 0, sizeof(pk_t) * (GRZ_PR_HOT_MAX + 2), st), "memset");
-            }
-        }
-        grz_dev_free(g, hist);
-        grz_dev_free(g, cnt);
-        if (rc) return rc;
-        if (g->pr_hotmap) g->pr_nhot = (uint32_t)pick[1];
+    g->pr_nhot = 0;
+    if (g->pull.nvec < (1ull << 18) || V >= GRZ_HUB_BASE) {
         g->pr_hot_known = 1;
-        if (!g->pr_nhot) return GRZ_OK;
+        return GRZ_OK;
     }
-    grz_dev_free(g, g->pr_hot_nbr);
-    g->pr_hot_nbr = nullptr;
-    g->pr_hot_of = nullptr;
-    GRZ_TRY(grz_dev_alloc(g, (void**)&g->pr_hot_nbr, sizeof(uint4) * nvec));
-    k_hot_encode<<<blocks_for(nvec), PR_THREADS, 0, st>>>(list, nvec, g->pr_hotmap, g->pr_nhot, g->pr_hot_nbr); GRZ_COUNT_LAUNCH(g);
-    GRZ_CK(g, cudaGetLastError());
-    g->pr_hot_of = list;
+    const uint32_t dmin = (uint32_t)std::min<uint64_t>(g->E / V + 1, 0xffffffffull);
+    unsigned long long* hist = nullptr;
+    uint32_t* cnt = nullptr;
+    unsigned long long pick[3] = { 0, 0, 0 };
+    int rc = grz_dev_alloc(g, (void**)&hist, sizeof(unsigned long long) * (2 * HOT_BINS + 3));
+    if (!rc) rc = grz_cuda_check(g, cudaMemsetAsync(hist, 0, sizeof(unsigned long long) * (2 * HOT_BINS + 3), st), "memset");
+    if (!rc) {
+        const unsigned grid = (unsigned)std::min<uint64_t>(blocks_for(V), (uint64_t)g->num_sms * 8);
+        k_hot_hist<<<grid, PR_THREADS, 0, st>>>(g->degree, V, dmin, hist); GRZ_COUNT_LAUNCH(g);
+        k_hot_pick<<<1, HOT_PICK_T, 0, st>>>(hist, GRZ_PR_HOT_MAX, hist + 2 * HOT_BINS); GRZ_COUNT_LAUNCH(g);
+        rc = grz_cuda_check(g, cudaGetLastError(), "k_hot_pick");
+    }
+    if (!rc) rc = grz_cuda_check(g, cudaMemcpyAsync(pick, hist + 2 * HOT_BINS, sizeof(pick), cudaMemcpyDeviceToHost, st), "D2H");
+    if (!rc) rc = grz_cuda_check(g, cudaStreamSynchronize(st), "hot sources");
+    if (!rc && pick[1] && pick[2] * 10 >= g->E) {
+        rc = grz_dev_alloc(g, (void**)&g->pr_hotmap, sizeof(uint2) * words);
+        if (!rc) rc = grz_dev_alloc(g, (void**)&cnt, sizeof(uint32_t) * words);
+        if (!rc) rc = grz_dev_alloc(g, (void**)&g->pr_hot_vid, sizeof(uint32_t) * pick[1]);
+        if (!rc) {
+            k_hot_mark<<<blocks_for(V), PR_THREADS, 0, st>>>(g->degree, V, dmin, (uint32_t)pick[0], g->pr_hotmap, cnt); GRZ_COUNT_LAUNCH(g);
+            rc = grz_cuda_check(g, cudaGetLastError(), "k_hot_mark");
+        }
+        if (!rc) rc = grz_exclusive_sum_u32_on(g, cnt, cnt, words, nullptr, st);
+        if (!rc) {
+            k_hot_base<<<blocks_for(words), PR_THREADS, 0, st>>>(cnt, words, g->pr_hotmap, g->pr_hot_vid); GRZ_COUNT_LAUNCH(g);
+            rc = grz_cuda_check(g, cudaGetLastError(), "k_hot_base");
+        }
+        for (int i = 0; i < 2 && !rc; ++i) {
+            if (!g->pr_hot[i]) rc = grz_cuda_check(g, cudaMalloc((void**)&g->pr_hot[i], sizeof(pk_t) * (GRZ_PR_HOT_MAX + 2)), "hot props");
+            // the slots past the last stay zero
+            if (!rc) rc = grz_cuda_check(g, cudaMemsetAsync(g->pr_hot[i], 0, sizeof(pk_t) * (GRZ_PR_HOT_MAX + 2), st), "memset");
+        }
+    }
+    grz_dev_free(g, hist);
+    grz_dev_free(g, cnt);
+    if (rc) {
+        grz_dev_free(g, g->pr_hotmap);
+        grz_dev_free(g, g->pr_hot_vid);
+        g->pr_hotmap = nullptr;
+        g->pr_hot_vid = nullptr;
+        return rc;
+    }
+    if (g->pr_hotmap) g->pr_nhot = (uint32_t)pick[1];
+    g->pr_hot_known = 1;
     return GRZ_OK;
+}
+
+// The pull list encoded for the packed gather (source segments are encoded as they are built).
+static int pr_hot_encode(grz_graph* g)
+{
+    if (!g->pr_nhot || g->pr_hot_nbr) return GRZ_OK;
+    GRZ_TRY(grz_dev_alloc(g, (void**)&g->pr_hot_nbr, sizeof(uint4) * g->pull.nvec));
+    k_hot_encode<<<blocks_for(g->pull.nvec), PR_THREADS, 0, g->stream>>>(g->pull.nbr, g->pull.nvec, g->pr_hotmap, g->pr_nhot, g->pr_hot_nbr);
+    GRZ_COUNT_LAUNCH(g);
+    return grz_cuda_check(g, cudaGetLastError(), "k_hot_encode");
 }
 
 static int pr_build_segments(grz_graph* g, uint32_t bits);
 
-// Sources per segment (log2) of the segmented lists, 0 for none: the tuned size, else, when the
-// double props exceed 4x L2 (or `force`), the largest segment whose props are at most 1.25x L2
-// (see grz_pr_prepare); never more than GRZ_PR_MAX_SEGMENTS segments.
+// Sources per segment (log2) of the segmented lists, 0 for none: the tuned size, else by the size
+// of the packed props (8V bytes) against L2; never more than GRZ_PR_MAX_SEGMENTS segments.  GB300
+// (128 MB of L2), ms per iteration unsegmented / with 2^24 / 2^23 sources per segment, and the first
+// grz_pr_init's extra ms for the lists:
+//   hot sources (R-MAT): 2^25 vertices 2.16 / 2.39 / 2.45; 40M 2.78 / 2.50 / 2.58 (+8.1); 50M 2.95 /
+//     2.06 / 2.17 (+6.5); 2^26 7.85 / 5.07 / 5.31 (+13): from 2.75 times L2 on, where the lists pay
+//     for themselves within a run of 8 iterations, in segments of 1.25 times L2
+//   none (uniform): 8.4M 0.59 / - / 0.62; 10M, degree 16 0.89 / - / 0.80, degree 6 0.45 / - / 0.53; 13M
+//     1.65 / - / 1.04 and 0.75 / - / 0.68; 17M 2.71 / 2.81 / 1.45; 30M 7.04 / 4.86 / 3.25; 40M 3.26 /
+//     3.01 / 3.21; 60M 10.2 / 7.37 / 7.74 (+0.8 to +2.6): from 3/4 of L2 on, in segments of 5/8 of
+//     L2 while that gives at most four, else of twice that
+// (`force`: for the CC pull, before the hot sources are known.)
 static uint32_t pr_segment_bits(const grz_graph* g, int force)
 {
     const uint64_t V = g->V;
@@ -1104,9 +1106,14 @@ static uint32_t pr_segment_bits(const grz_graph* g, int force)
     const uint32_t sb = g->tune.pr_segment_bits;
     if (sb >= 8) {
         bits = sb;
-    } else if (sb == 0 && (force || (uint64_t)sizeof(double) * V > 4ull * (uint64_t)g->l2_bytes)) {
-        bits = 8;
-        while ((8ull << (bits + 1)) <= (uint64_t)g->l2_bytes * 5 / 4) ++bits;
+    } else if (sb == 0) {
+        const uint64_t props = (uint64_t)sizeof(pk_t) * V, l2 = (uint64_t)g->l2_bytes;
+        const bool hot = force || g->pr_nhot;
+        if (force || props * 4 > l2 * (hot ? 11 : 3)) {
+            bits = 8;
+            while ((8ull << (bits + 1)) <= l2 * 5 / (hot ? 4 : 8)) ++bits;
+            if (!hot && ((V + (1ull << bits) - 1) >> bits) > 4) ++bits;
+        }
     }
     while (bits && ((V + (1ull << bits) - 1) >> bits) > GRZ_PR_MAX_SEGMENTS) ++bits;
     return bits;
@@ -1147,14 +1154,10 @@ int grz_pr_prepare(grz_graph* g)
     // for a few integer instructions per edge (GB300, a thread per vector, gather per iteration, 16 ->
     // 8 bytes: R-MAT 20 71 -> 63 us, R-MAT 24 1089 -> 938 us, uniform 3M vertices 153 -> 145 us).
     g->pr_pkmode = g->tune.pr_props != 1;
-    // Source segments when even the packed props are far larger than L2 (or when chosen): each
-    // segment's props (8 bytes x 2^bits) mostly stay in L2 while its edges stream, instead of one
-    // random DRAM sector per gathered prop.  Segment props of about the size of L2 are best: on
-    // GB300 at R-MAT 27 (16 iterations) the gather took 23.2 ms unsegmented and 17.8 / 18.1 /
-    // 19.0 / 20.5 ms with 2^24 / 2^23 / 2^22 / 2^21 sources per segment (128 MB of props for
-    // 2^24 against 126 MB of L2); smaller segments add more (segment, destination)
-    // read-modify-writes and partial vectors than they save.  Needs sources in ascending order
-    // along each destination's lanes, which hub encoding breaks.
+    if (!g->pull.nhub && V) GRZ_TRY(pr_hot_choose(g));
+    // Source segments (pr_segment_bits): each segment's props mostly stay in L2 while its edges
+    // stream, instead of one random DRAM sector per gathered prop.  They need sources in ascending
+    // order along each destination's lanes, which hub encoding breaks.
     const uint32_t bits = pr_segment_bits(g, 0);
     g->pr_segmode = 0;
     if (bits && g->pull.nhub == 0 && g->pull.nvec) {
@@ -1169,66 +1172,61 @@ int grz_pr_prepare(grz_graph* g)
         GRZ_CK(g, cudaMemsetAsync(g->pr_pk[0], 0, sizeof(pk_t) * (V + 1), g->stream));
         GRZ_CK(g, cudaMemsetAsync(g->pr_pk[1], 0, sizeof(pk_t) * (V + 1), g->stream));
     }
-    if (g->pr_pkmode && !g->pull.nhub && V)
-        GRZ_TRY(g->pr_segmode ? pr_hot_prepare(g, g->seg_nbr, g->seg_first[g->nseg]) : pr_hot_prepare(g, g->pull.nbr, g->pull.nvec));
+    if (g->pr_pkmode && !g->pr_segmode && !g->pull.nhub && V) GRZ_TRY(pr_hot_encode(g));
     return GRZ_OK;
 }
 
-// Builds the source-segmented pull lists with 2^bits sources per segment (once per lists and bits).
+// Builds the source-segmented pull lists with 2^bits sources per segment (once per lists, bits and
+// encoding: with the hot sources as codes when there are any).
 static int pr_build_segments(grz_graph* g, uint32_t bits)
 {
-    if (g->seg_nbr && g->seg_bits == bits) return GRZ_OK;
+    if (g->seg_nbr && g->seg_bits == bits && g->seg_nhot == g->pr_nhot) return GRZ_OK;
     grz_dev_free(g, g->seg_nbr);
     grz_dev_free(g, g->seg_dst);
     g->seg_nbr = nullptr;
     g->seg_dst = nullptr;
     g->seg_bits = 0;
-    const uint64_t V = g->V;
+    const uint64_t V = g->V, n = g->pull.nvec;
     const uint32_t nseg = (uint32_t)((V + (1ull << bits) - 1) >> bits);
     if (nseg == 0 || nseg > GRZ_PR_MAX_SEGMENTS) return grz_set_error(g, GRZ_ERR_RANGE, "%u source segments (at most %d)", nseg, GRZ_PR_MAX_SEGMENTS);
     cudaStream_t st = g->stream;
-    uint32_t *cnt = nullptr, *tot = nullptr, *nbig = nullptr;
-    SegBig* big = nullptr;
-    const uint64_t ncnt = (uint64_t)nseg * (V + 1);
-    int rc = grz_dev_alloc(g, (void**)&cnt, sizeof(uint32_t) * ncnt);
+    uint32_t *start = nullptr, *off = nullptr, *tot = nullptr;
+    const uint64_t npair = (uint64_t)nseg * (V + 1);
+    int rc = grz_dev_alloc(g, (void**)&start, sizeof(uint32_t) * npair);
+    if (!rc) rc = grz_dev_alloc(g, (void**)&off, sizeof(uint32_t) * npair);
     if (!rc) rc = grz_dev_alloc(g, (void**)&tot, sizeof(uint32_t) * (nseg + 1));
-    if (!rc) rc = grz_cuda_check(g, cudaMemsetAsync(cnt, 0, sizeof(uint32_t) * ncnt, st), "memset");
-    const unsigned grid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(blocks_for(V), (uint64_t)g->num_sms * 8));
+    if (!rc) rc = grz_cuda_check(g, cudaMemsetAsync(start, 0, sizeof(uint32_t) * npair, st), "memset");
+    if (!rc) rc = grz_cuda_check(g, cudaMemsetAsync(off, 0, sizeof(uint32_t) * npair, st), "memset");
     if (!rc) {
-        k_seg_count<<<grid, PR_THREADS, 0, st>>>(g->pull.nbr, g->pull.rowptr, (uint32_t)V, bits, cnt); GRZ_COUNT_LAUNCH(g);
-        rc = grz_cuda_check(g, cudaGetLastError(), "k_seg_count");
+        k_seg_bounds<<<blocks_for(n), PR_THREADS, 0, st>>>(g->pull.nbr, g->pull.shared, g->pull.rowptr, n, V, bits, start, off); GRZ_COUNT_LAUNCH(g);
+        const unsigned grid = (unsigned)std::min<uint64_t>(blocks_for(npair), (uint64_t)g->num_sms * 8);
+        k_seg_sizes<<<grid, PR_THREADS, 0, st>>>(start, off, npair); GRZ_COUNT_LAUNCH(g);
+        rc = grz_cuda_check(g, cudaGetLastError(), "k_seg_bounds");
     }
     for (uint32_t sg = 0; sg < nseg && !rc; ++sg)
-        rc = grz_exclusive_sum_u32_on(g, cnt + (uint64_t)sg * (V + 1), cnt + (uint64_t)sg * (V + 1), V + 1, tot + sg, st);
+        rc = grz_exclusive_sum_u32_on(g, off + (uint64_t)sg * (V + 1), off + (uint64_t)sg * (V + 1), V + 1, tot + sg, st);
     std::vector<uint32_t> th(nseg);
     if (!rc) rc = grz_cuda_check(g, cudaMemcpyAsync(th.data(), tot, sizeof(uint32_t) * nseg, cudaMemcpyDeviceToHost, st), "D2H");
     if (!rc) rc = grz_cuda_check(g, cudaStreamSynchronize(st), "segment counts");
-    uint64_t total = 0, maxn = 0;
+    SegFirst first;
+    uint64_t total = 0;
     if (!rc) {
         for (uint32_t sg = 0; sg < nseg; ++sg) {
-            g->seg_first[sg] = total;
+            g->seg_first[sg] = first.at[sg] = total;
             total += th[sg];
-            maxn = std::max<uint64_t>(maxn, th[sg]);
         }
         g->seg_first[nseg] = total;
         if (total >= 0xffffffffull) rc = grz_set_error(g, GRZ_ERR_RANGE, "segmented lists of %llu vectors", (unsigned long long)total);
     }
     if (!rc) rc = grz_dev_alloc(g, (void**)&g->seg_nbr, sizeof(uint4) * std::max<uint64_t>(total, 1));
     if (!rc) rc = grz_dev_alloc(g, (void**)&g->seg_dst, sizeof(uint32_t) * std::max<uint64_t>(total, 1));
-    // long runs: at most one per SEG_BIG_VECTORS + 1 vectors of a segment
-    if (!rc) rc = grz_dev_alloc(g, (void**)&big, sizeof(SegBig) * (maxn / (SEG_BIG_VECTORS + 1) + 1));
-    if (!rc) rc = grz_dev_alloc(g, (void**)&nbig, sizeof(uint32_t));
-    for (uint32_t sg = 0; sg < nseg && !rc; ++sg) {
-        if (!th[sg]) continue;
-        rc = grz_cuda_check(g, cudaMemsetAsync(nbig, 0, sizeof(uint32_t), st), "memset");
-        if (rc) break;
-        k_seg_write<<<grid, PR_THREADS, 0, st>>>(g->pull.nbr, g->pull.rowptr, (uint32_t)V, bits, sg, cnt + (uint64_t)sg * (V + 1),
-                                                 g->seg_first[sg], g->seg_nbr, g->seg_dst, big, nbig); GRZ_COUNT_LAUNCH(g);
-        k_seg_write_big<<<(unsigned)g->num_sms * 4, PR_THREADS, 0, st>>>(g->pull.nbr, g->pull.rowptr, big, nbig, g->seg_first[sg],
-                                                                        g->seg_nbr, g->seg_dst); GRZ_COUNT_LAUNCH(g);
-        rc = grz_cuda_check(g, cudaGetLastError(), "k_seg_write");
+    if (!rc) {
+        k_seg_emit<<<blocks_for(n), PR_THREADS, 0, st>>>(g->pull.nbr, g->pull.shared, g->pull.rowptr, n, V, bits, start, off, first,
+                                                         g->pr_nhot ? g->pr_hotmap : nullptr, g->pr_nhot,
+                                                         reinterpret_cast<uint32_t*>(g->seg_nbr), g->seg_dst); GRZ_COUNT_LAUNCH(g);
+        rc = grz_cuda_check(g, cudaGetLastError(), "k_seg_emit");
     }
-    for (void* q : { (void*)cnt, (void*)tot, (void*)big, (void*)nbig }) grz_dev_free(g, q);
+    for (void* q : { (void*)start, (void*)off, (void*)tot }) grz_dev_free(g, q);
     if (rc) {
         grz_dev_free(g, g->seg_nbr);
         grz_dev_free(g, g->seg_dst);
@@ -1237,6 +1235,8 @@ static int pr_build_segments(grz_graph* g, uint32_t bits)
         return rc;
     }
     g->seg_bits = bits;
+    g->seg_nhot = g->pr_nhot;
+    g->seg_gen++;
     g->nseg = nseg;
     return GRZ_OK;
 }
@@ -1248,17 +1248,18 @@ int grz_pr_init_state(grz_graph* g, double damping)
     if (rc) return rc;
     g->pr_damping = damping;
     g->pr_cur = 0;
-    g->pr_fx_stale = g->pr_pk_stale = 0;
+    g->pr_fx_stale = g->pr_pkmode;
+    g->pr_pk_stale = g->pr_pk[0] && !g->pr_pkmode;
     g->pr_sum_cur = 0;
     g->pr_iters_done = 0;
-    GRZ_CK(g, cudaMemsetAsync(g->pr_sum, 0, sizeof(u128) * 2 * (blocks_for(g->V) + 1), g->stream));
     GRZ_CK(g, cudaMemsetAsync(g->accum, 0, sizeof(double) * (g->V + 8), g->stream));
-    g->pr_nparts[0] = g->pr_nparts[1] = blocks_for(g->V);
     if (g->V) {
-        k_pr_init<<<blocks_for(g->V), PR_THREADS, 0, g->stream>>>(g->outdeg, g->degree, g->V, g->prop, g->accum, g->pr_fx[0],
-                                                                 g->pr_pkmode ? g->pr_pk[0] : nullptr, g->pr_nhot ? g->pr_hotmap : nullptr,
-                                                                 g->pr_hot[0], g->pr_sum); GRZ_COUNT_LAUNCH(g);
+        const unsigned grid = (unsigned)std::min<uint64_t>(blocks_for(g->V), (uint64_t)g->num_sms * 8);
+        k_pr_init<<<grid, PR_THREADS, 0, g->stream>>>(g->inv_deg, g->degree, g->V, 1.0 / (double)g->V, g->pr_fx[0],
+                                                      g->pr_pkmode ? g->pr_pk[0] : nullptr, g->pr_nhot ? g->pr_hotmap : nullptr,
+                                                      g->pr_hot[0], g->pr_sum); GRZ_COUNT_LAUNCH(g);
         GRZ_CK(g, cudaGetLastError());
+        g->pr_nparts[0] = grid;
     }
     return GRZ_OK;
 }
@@ -1347,7 +1348,6 @@ static int pr_gather_pk(grz_graph* g, const uint4* nbr, const uint32_t* dstv, ui
 static int pr_gather_segments(grz_graph* g, const PRConst& pc0)
 {
     grz_prof_begin(g, GRZ_PROF_PR_GATHER);
-    const uint4* nbr = g->pr_nhot ? g->pr_hot_nbr : g->seg_nbr;
     bool first = true;
     int rc = GRZ_OK;
     for (uint32_t sg = 0; sg < g->nseg && !rc; ++sg) {
@@ -1356,10 +1356,10 @@ static int pr_gather_segments(grz_graph* g, const PRConst& pc0)
         PRConst pc = pc0;
         if (!first) pc.K_out = nullptr;  // the iteration's constant once
         first = false;
-        rc = pr_gather_pk<true>(g, nbr, g->seg_dst, a, b, pc);
+        rc = pr_gather_pk<true>(g, g->seg_nbr, g->seg_dst, a, b, pc);
     }
     // no edges at all: the constant still has to be published
-    if (first && !rc) rc = pr_gather_pk<true>(g, nbr, g->seg_dst, 0, 0, pc0);
+    if (first && !rc) rc = pr_gather_pk<true>(g, g->seg_nbr, g->seg_dst, 0, 0, pc0);
     grz_prof_end(g);
     return rc;
 }
