@@ -576,199 +576,116 @@ __global__ void __launch_bounds__(T) k_bfs_pull(const uint4* __restrict__ nbr, c
 // ---------------------------------------------------------------------------------------------
 // Push: frontier compaction and edge-balanced expansion.
 //
-// The active sources that have out-vectors are compacted in vertex order, each with the offset
+// The active sources that have out-vectors are compacted, each with the offset
 // of its first vector in the concatenation of their vector ranges.  The expansion then splits
 // that concatenation into tiles of PUSH_TILE vectors spread over the grid, so a hub's vectors
 // are spread over many blocks.  tile_first[t] is the frontier entry that owns the first vector
-// of tile t.  Passes: k_fr_count (per block of bitmap words: sources and vectors),
-// k_fr_scan (one block: exclusive scan of the block totals), k_fr_write (frontier entries,
-// their vector offsets and the tile owners), k_push_expand.
+// of tile t.  Passes: k_fr_compact (frontier entries, their vector offsets and the tile owners),
+// k_push_expand.
 
 constexpr uint32_t PUSH_TILE = 1024;
 
-// block-wide exclusive scan of two u32 values; returns the block totals through the references
-__device__ __forceinline__ void block_scan2(uint32_t& a, uint32_t& b, uint32_t& tot_a, uint32_t& tot_b, uint32_t* sa,
-                                            uint32_t* sb)
-{
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    uint32_t xa = a, xb = b;
-    for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t ya = __shfl_up_sync(0xffffffffu, xa, o);
-        const uint32_t yb = __shfl_up_sync(0xffffffffu, xb, o);
-        if (lane >= o) { xa += ya; xb += yb; }
-    }
-    if (lane == 31) { sa[warp] = xa; sb[warp] = xb; }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        uint32_t ra = 0, rb = 0;
-        for (int k = 0; k < T / 32; ++k) {
-            const uint32_t ta = sa[k], tb = sb[k];
-            sa[k] = ra; sb[k] = rb;
-            ra += ta; rb += tb;
-        }
-        sa[T / 32] = ra; sb[T / 32] = rb;
-    }
-    __syncthreads();
-    a = sa[warp] + xa - a;
-    b = sb[warp] + xb - b;
-    tot_a = sa[T / 32];
-    tot_b = sb[T / 32];
-}
+// Each block takes CCHUNK consecutive vertices, each thread one 32-vertex word of the two bitmaps
+// (HasInfo and out-vectors for push; WantsInfo, or the destinations a first pass left open, and
+// in-vectors for the pulls); a block with nothing selected returns after reading its words.  A warp
+// then walks its words with a lane per vertex, so row pointers and entries are read and written
+// coalesced: once to count its vectors, and, after one 64-bit atomic per block has given the block
+// its place (selected vertices in the high half, their vectors in the low half, so the two stay in
+// step), once more to write.  The list is in vertex order inside a block's part only, which is all
+// its readers need: a vertex's vectors stay consecutive and offsets ascend along the list.
+// Before: a count kernel, a one-block scan and a write kernel with 32 vertices per thread.  GB300,
+// whole runs, three kernels -> one: 8 BFS at R-MAT 24 9.67 -> 9.15 ms, a BFS of 1400 levels on a mesh of
+// 250k vertices 33.4 -> 30.6 ms.
+constexpr uint32_t CCHUNK = T * 32;
+constexpr int FR_STEP = 4;  // words whose row pointers are loaded together
 
-// The compaction kernels give each thread CU = 32 consecutive vertices (half a bitmap word) and
-// each block CCHUNK consecutive vertices, so a block needs a single block-wide scan and a block
-// with nothing selected exits after reading its words.  A thread with a selected vertex reads its
-// 33 row pointers with 128-bit loads issued together and works from registers.  Selected: the bit
-// is set in both bitmaps (HasInfo and out-vectors for push; WantsInfo and in-vectors for the BFS
-// pull).
-constexpr int CU = 32;
-constexpr uint32_t CCHUNK = T * CU;
-
-// selection bits of vertices [v0, v0 + CU), v0 a multiple of CU
-__device__ __forceinline__ uint32_t selected_bits(const unsigned long long* __restrict__ bm1,
-                                                  const unsigned long long* __restrict__ bm2, uint64_t v0, uint64_t V)
+// `counters`[2] = vectors, [3] = selected vertices (zero before the launch).
+// frontier[i] = a selected vertex, voff[i] = offset of its first vector among the selected
+// vertices' vectors, vdelta[i] = its first vector's index in the list minus voff[i] (mod 2^32);
+// tile_first[t] for the tiles that start in its range.  `skip` leaves out the first vectors of
+// every selected vertex (each selected one has more).  A zero gate selects nothing (the bitmaps
+// were not written in this phase).
+__global__ void __launch_bounds__(T) k_fr_compact(const unsigned long long* __restrict__ bm1, const unsigned long long* __restrict__ bm2,
+                                                  uint64_t V, const uint32_t* __restrict__ rowptr, uint32_t skip,
+                                                  const uint32_t* __restrict__ gate, uint32_t* __restrict__ counters,
+                                                  uint32_t* __restrict__ frontier, uint32_t* __restrict__ voff,
+                                                  uint32_t* __restrict__ vdelta, uint32_t* __restrict__ tile_first)
 {
-    if (v0 >= V) return 0u;
-    const uint64_t w = v0 >> 6;
-    uint32_t bits = (uint32_t)((bm1[w] & bm2[w]) >> (v0 & 63));
-    if (v0 + CU > V) bits &= (1u << (V - v0)) - 1u;
-    return bits;
-}
-
-// r[0..CU] = rowptr[v0 .. v0 + CU] (entries past V are not read; their bits are clear)
-__device__ __forceinline__ void load_rowptr(const uint32_t* __restrict__ rowptr, uint64_t v0, uint64_t V, uint32_t* r)
-{
-    if (v0 + CU <= V) {
-        const uint4* p = reinterpret_cast<const uint4*>(rowptr + v0);  // v0 * 4 bytes is a multiple of 128
-#pragma unroll
-        for (int q = 0; q < CU / 4; ++q) {
-            const uint4 x = p[q];
-            r[4 * q] = x.x; r[4 * q + 1] = x.y; r[4 * q + 2] = x.z; r[4 * q + 3] = x.w;
-        }
-        r[CU] = rowptr[v0 + CU];
-    } else {
-#pragma unroll
-        for (int j = 0; j <= CU; ++j) r[j] = (v0 + j <= V) ? rowptr[v0 + j] : 0u;
-    }
-}
-
-__global__ void __launch_bounds__(T) k_fr_count(const unsigned long long* __restrict__ bm1,
-                                                const unsigned long long* __restrict__ bm2, uint64_t V,
-                                                const uint32_t* __restrict__ rowptr, uint32_t skip, const uint32_t* __restrict__ gate,
-                                                uint32_t* __restrict__ part_n, uint32_t* __restrict__ part_vec)
-{
-    __shared__ uint32_t sa[T / 32 + 1], sb[T / 32 + 1];
-    // a zero gate selects nothing (the bitmaps were not written in this phase): k_fr_scan then
-    // reports an empty list without reading the partials, and k_fr_write returns at once
+    __shared__ uint32_t sn[T / 32], sv[T / 32];
+    __shared__ unsigned long long s_base;
     if (gate && *gate == 0u) return;
-    const uint64_t v0 = (uint64_t)blockIdx.x * CCHUNK + (uint64_t)threadIdx.x * CU;
-    const uint32_t bits = selected_bits(bm1, bm2, v0, V);
-    if (!__syncthreads_or(bits)) {
-        if (threadIdx.x == 0) { part_n[blockIdx.x] = 0; part_vec[blockIdx.x] = 0; }
-        return;
-    }
-    uint32_t n = __popc(bits), vec = 0;
-    if (bits) {
-        uint32_t r[CU + 1];
-        load_rowptr(rowptr, v0, V, r);
-#pragma unroll
-        for (int j = 0; j < CU; ++j)
-            if ((bits >> j) & 1u) vec += r[j + 1] - r[j] - skip;
-    }
-    uint32_t tn, tv;
-    block_scan2(n, vec, tn, tv, sa, sb);
-    if (threadIdx.x == 0) { part_n[blockIdx.x] = tn; part_vec[blockIdx.x] = tv; }
-}
-
-// one block of SCAN_T threads: exclusive scan of the per-block totals in place (each thread a
-// contiguous segment); counters[0] = selected vertices, counters[2] = their vectors
-constexpr int SCAN_T = 1024;
-
-__global__ void __launch_bounds__(SCAN_T) k_fr_scan(uint32_t* __restrict__ part_n, uint32_t* __restrict__ part_vec, uint32_t nb,
-                                                    uint32_t* __restrict__ counters, const uint32_t* __restrict__ gate)
-{
-    __shared__ uint32_t sa[SCAN_T / 32 + 1], sb[SCAN_T / 32 + 1];
-    if (gate && *gate == 0u) {  // gated off: an empty list (the partials were not written)
-        if (threadIdx.x == 0) { counters[0] = 0; counters[2] = 0; }
-        return;
-    }
-    const uint32_t per = (nb + SCAN_T - 1) / SCAN_T;
-    const uint32_t lo = min(nb, threadIdx.x * per), hi = min(nb, lo + per);
-    uint32_t sn = 0, sv = 0;
-#pragma unroll 8
-    for (uint32_t i = lo; i < hi; ++i) { sn += part_n[i]; sv += part_vec[i]; }
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    uint32_t xa = sn, xb = sv;
-    for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t ya = __shfl_up_sync(0xffffffffu, xa, o);
-        const uint32_t yb = __shfl_up_sync(0xffffffffu, xb, o);
-        if (lane >= o) { xa += ya; xb += yb; }
+    const uint64_t word = (uint64_t)blockIdx.x * T + threadIdx.x;  // bits of vertices [32 word, 32 word + 32)
+    uint32_t bits = 0;
+    if (32 * word < V) bits = reinterpret_cast<const uint32_t*>(bm1)[word] & reinterpret_cast<const uint32_t*>(bm2)[word];
+    if (32 * word + 32 > V && bits) bits &= (1u << (V - 32 * word)) - 1u;
+    if (!__syncthreads_or(bits)) return;
+    const uint32_t vbase = (uint32_t)((uint64_t)blockIdx.x * CCHUNK) + 1024u * warp + lane;  // this lane's vertex of the warp's word 0
+    const unsigned words = __ballot_sync(0xffffffffu, bits != 0);
+    // vectors of this lane's vertices in words j .. j + FR_STEP - 1 (0 if not selected), their first in r0
+    auto rows = [&](int j, uint32_t* r0, uint32_t* cnt) {
+#pragma unroll
+        for (int q = 0; q < FR_STEP; ++q) {
+            const uint32_t v = vbase + 32u * (j + q);
+            r0[q] = cnt[q] = 0;
+            if ((__shfl_sync(0xffffffffu, bits, j + q) >> lane) & 1u) {
+                r0[q] = rowptr[v];
+                cnt[q] = rowptr[v + 1];
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < FR_STEP; ++q)
+            if (cnt[q]) {
+                r0[q] += skip;
+                cnt[q] -= r0[q];
+            }
+    };
+    const uint32_t n = __reduce_add_sync(0xffffffffu, (unsigned)__popc(bits));
+    uint32_t vec = 0;
+    for (int j = 0; j < 32; j += FR_STEP) {
+        if (!((words >> j) & ((1u << FR_STEP) - 1u))) continue;  // warp-uniform
+        uint32_t r0[FR_STEP], cnt[FR_STEP];
+        rows(j, r0, cnt);
+#pragma unroll
+        for (int q = 0; q < FR_STEP; ++q) vec += cnt[q];
     }
-    if (lane == 31) { sa[warp] = xa; sb[warp] = xb; }
+    vec = __reduce_add_sync(0xffffffffu, vec);
+    if (lane == 0) { sn[warp] = n; sv[warp] = vec; }
     __syncthreads();
     if (threadIdx.x == 0) {
-        uint32_t ra = 0, rb = 0;
-        for (int k = 0; k < SCAN_T / 32; ++k) {
-            const uint32_t ta = sa[k], tb = sb[k];
-            sa[k] = ra; sb[k] = rb;
-            ra += ta; rb += tb;
+        uint32_t an = 0, av = 0;
+        for (int w = 0; w < T / 32; ++w) {
+            const uint32_t tn = sn[w], tv = sv[w];
+            sn[w] = an; sv[w] = av;
+            an += tn; av += tv;
         }
-        counters[0] = ra;
-        counters[2] = rb;
+        s_base = atomicAdd(reinterpret_cast<unsigned long long*>(counters + 2), ((unsigned long long)an << 32) | av);
     }
     __syncthreads();
-    uint32_t en = sa[warp] + xa - sn, ev = sb[warp] + xb - sv;
-    for (uint32_t i = lo; i < hi; ++i) {
-        const uint32_t tn = part_n[i], tv = part_vec[i];
-        part_n[i] = en;
-        part_vec[i] = ev;
-        en += tn;
-        ev += tv;
-    }
-}
-
-// frontier[i] = i-th selected vertex (ID order), voff[i] = offset of its first vector among the
-// selected vertices' vectors, vdelta[i] = its first vector's index in the list minus voff[i]
-// (mod 2^32); tile_first[t] for the tiles that start in its range.  voff[count] = total vectors.
-// `skip` leaves out the first vectors of every selected vertex (each selected one has more).
-__global__ void __launch_bounds__(T) k_fr_write(const unsigned long long* __restrict__ bm1,
-                                                const unsigned long long* __restrict__ bm2, uint64_t V,
-                                                const uint32_t* __restrict__ rowptr, uint32_t skip, const uint32_t* __restrict__ base_n,
-                                                const uint32_t* __restrict__ base_vec, const uint32_t* __restrict__ counters,
-                                                uint32_t nb, uint32_t* __restrict__ frontier, uint32_t* __restrict__ voff,
-                                                uint32_t* __restrict__ vdelta, uint32_t* __restrict__ tile_first,
-                                                const uint32_t* __restrict__ gate)
-{
-    __shared__ uint32_t sa[T / 32 + 1], sb[T / 32 + 1];
-    if (gate && *gate == 0u) return;  // gated off: nothing selected
-    if (blockIdx.x == 0 && threadIdx.x == 0) voff[counters[0]] = counters[2];
-    const uint32_t b0 = base_n[blockIdx.x];
-    const uint32_t b1 = blockIdx.x + 1 < nb ? base_n[blockIdx.x + 1] : counters[0];
-    if (b0 == b1) return;  // nothing selected in this block (uniform)
-    const uint64_t v0 = (uint64_t)blockIdx.x * CCHUNK + (uint64_t)threadIdx.x * CU;
-    const uint32_t bits = selected_bits(bm1, bm2, v0, V);
-    uint32_t r[CU + 1];
-    uint32_t n = __popc(bits), vec = 0;
-    if (bits) {
-        load_rowptr(rowptr, v0, V, r);
+    uint32_t pos = (uint32_t)(s_base >> 32) + sn[warp], vo = (uint32_t)s_base + sv[warp];
+    for (int j = 0; j < 32; j += FR_STEP) {
+        if (!((words >> j) & ((1u << FR_STEP) - 1u))) continue;
+        uint32_t r0[FR_STEP], cnt[FR_STEP];
+        rows(j, r0, cnt);
 #pragma unroll
-        for (int j = 0; j < CU; ++j)
-            if ((bits >> j) & 1u) vec += r[j + 1] - r[j] - skip;
-    }
-    uint32_t tn, tv;
-    block_scan2(n, vec, tn, tv, sa, sb);
-    if (!bits) return;
-    uint32_t pos = b0 + n, vo = base_vec[blockIdx.x] + vec;
-#pragma unroll
-    for (int j = 0; j < CU; ++j) {
-        if (!((bits >> j) & 1u)) continue;
-        const uint32_t cnt = r[j + 1] - r[j] - skip;
-        frontier[pos] = (uint32_t)(v0 + j);
-        voff[pos] = vo;
-        vdelta[pos] = r[j] + skip - vo;
-        for (uint64_t t = ((uint64_t)vo + PUSH_TILE - 1) / PUSH_TILE; t * PUSH_TILE < (uint64_t)vo + cnt; ++t) tile_first[t] = pos;
-        ++pos;
-        vo += cnt;
+        for (int q = 0; q < FR_STEP; ++q) {
+            const uint32_t b = __shfl_sync(0xffffffffu, bits, j + q);
+            if (!b) continue;  // warp-uniform
+            uint32_t x = cnt[q];
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+                if (lane >= o) x += y;
+            }
+            if ((b >> lane) & 1u) {
+                const uint32_t p = pos + __popc(b & ((1u << lane) - 1u)), o = vo + x - cnt[q];
+                frontier[p] = vbase + 32u * (j + q);
+                voff[p] = o;
+                vdelta[p] = r0[q] - o;
+                for (uint64_t t = ((uint64_t)o + PUSH_TILE - 1) / PUSH_TILE; t * PUSH_TILE < (uint64_t)o + cnt[q]; ++t) tile_first[t] = p;
+            }
+            pos += __popc(b);
+            vo += __shfl_sync(0xffffffffu, x, 31);
+        }
     }
 }
 
@@ -786,14 +703,14 @@ __global__ void __launch_bounds__(T) k_push_expand(const uint32_t* __restrict__ 
                                                    unsigned long long* __restrict__ chg, uint32_t epoch,
                                                    const uint32_t* __restrict__ epoch_dev)
 {
-    __shared__ uint32_t s_src[PUSH_TILE + 1];
+    __shared__ uint32_t s_src[PUSH_TILE];
     __shared__ uint32_t red32[T / 32];
     uint32_t my_min = INF;  // CC: the smallest label written (cc_prev_min of the next iteration)
-    __shared__ uint32_t s_off[PUSH_TILE + 1];
-    __shared__ uint32_t s_delta[PUSH_TILE + 1];
+    __shared__ uint32_t s_off[PUSH_TILE];
+    __shared__ uint32_t s_delta[PUSH_TILE];
     __shared__ unsigned long long red[T / 32];
     __shared__ bool s_full;  // BFS: the touched list is long enough for the visit to sweep (read per tile)
-    const uint32_t nf = counters[0], total = counters[2];
+    const uint32_t nf = counters[3], total = counters[2];
     const uint32_t ntiles = (total + PUSH_TILE - 1) / PUSH_TILE;
     unsigned long long my_vote = 0;
     for (uint32_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
@@ -802,12 +719,10 @@ __global__ void __launch_bounds__(T) k_push_expand(const uint32_t* __restrict__ 
         const uint32_t tend = min(total, t0 + PUSH_TILE);
         // entries first .. first+nw-1 own every vector of the tile (each owns at least one)
         const uint32_t nw = min(PUSH_TILE, nf - first);
-        for (uint32_t i = threadIdx.x; i <= nw; i += T) {
+        for (uint32_t i = threadIdx.x; i < nw; i += T) {
             s_off[i] = voff[first + i];
-            if (i < nw) {
-                s_src[i] = frontier[first + i];
-                s_delta[i] = vdelta[first + i];
-            }
+            s_src[i] = frontier[first + i];
+            s_delta[i] = vdelta[first + i];
         }
         if (IsBfs && threadIdx.x == 0) s_full = touched_full(ntouched, V);
         __syncthreads();
@@ -884,12 +799,12 @@ __global__ void __launch_bounds__(T) k_bfs_pull_expand(const uint32_t* __restric
                                                        uint32_t nhub, unsigned long long* __restrict__ has_next,
                                                        uint32_t* __restrict__ queue)
 {
-    __shared__ uint32_t s_dst[PUSH_TILE + 1];
-    __shared__ uint32_t s_off[PUSH_TILE + 1];
-    __shared__ uint32_t s_delta[PUSH_TILE + 1];
+    __shared__ uint32_t s_dst[PUSH_TILE];
+    __shared__ uint32_t s_off[PUSH_TILE];
+    __shared__ uint32_t s_delta[PUSH_TILE];
     __shared__ uint32_t s_chunk;
     __shared__ bool s_full;  // the touched list is long enough for the visit to sweep (read per tile)
-    const uint32_t nd = counters[0], total = counters[2];
+    const uint32_t nd = counters[3], total = counters[2];
     const uint32_t ntiles = (total + PUSH_TILE - 1) / PUSH_TILE;
     const int lane = threadIdx.x & 31;
     for (;;) {
@@ -904,12 +819,10 @@ __global__ void __launch_bounds__(T) k_bfs_pull_expand(const uint32_t* __restric
             const uint32_t t0 = tile * PUSH_TILE;
             const uint32_t tend = min(total, t0 + PUSH_TILE);
             const uint32_t nw = min(PUSH_TILE, nd - first);
-            for (uint32_t i = threadIdx.x; i <= nw; i += T) {
+            for (uint32_t i = threadIdx.x; i < nw; i += T) {
                 s_off[i] = voff[first + i];
-                if (i < nw) {
-                    s_dst[i] = dests[first + i];
-                    s_delta[i] = vdelta[first + i];
-                }
+                s_dst[i] = dests[first + i];
+                s_delta[i] = vdelta[first + i];
             }
             if (threadIdx.x == 0) s_full = touched_full(ntouched, V);
             __syncthreads();
@@ -985,14 +898,14 @@ __global__ void __launch_bounds__(T) k_cc_pull_expand(const uint32_t* __restrict
                                                       uint32_t epoch, const uint32_t* __restrict__ epoch_dev,
                                                       uint32_t* __restrict__ queue, unsigned long long* __restrict__ work)
 {
-    __shared__ uint32_t s_dst[PUSH_TILE + 1];
-    __shared__ uint32_t s_off[PUSH_TILE + 1];
-    __shared__ uint32_t s_delta[PUSH_TILE + 1];
+    __shared__ uint32_t s_dst[PUSH_TILE];
+    __shared__ uint32_t s_off[PUSH_TILE];
+    __shared__ uint32_t s_delta[PUSH_TILE];
     __shared__ uint32_t s_chunk;
     __shared__ unsigned long long red[T / 32];
     __shared__ uint32_t red32[T / 32];
     const uint32_t ep = epoch_dev ? *epoch_dev : epoch;
-    const uint32_t nd = counters[0], total = counters[2];
+    const uint32_t nd = counters[3], total = counters[2];
     const uint32_t ntiles = (total + PUSH_TILE - 1) / PUSH_TILE;
     const int lane = threadIdx.x & 31;
     unsigned long long my_vote = 0, my_vecs = 0;
@@ -1014,12 +927,10 @@ __global__ void __launch_bounds__(T) k_cc_pull_expand(const uint32_t* __restrict
             const uint32_t t0 = tile * PUSH_TILE;
             const uint32_t tend = min(total, t0 + PUSH_TILE);
             const uint32_t nw = min(PUSH_TILE, nd - first);
-            for (uint32_t i = threadIdx.x; i <= nw; i += T) {
+            for (uint32_t i = threadIdx.x; i < nw; i += T) {
                 s_off[i] = voff[first + i];
-                if (i < nw) {
-                    s_dst[i] = dests[first + i];
-                    s_delta[i] = vdelta[first + i];
-                }
+                s_dst[i] = dests[first + i];
+                s_delta[i] = vdelta[first + i];
             }
             __syncthreads();
             for (uint32_t base = t0; base < tend; base += T) {  // warp-uniform trip count
@@ -1357,7 +1268,6 @@ static int ensure_frontier_state(grz_graph* g)
     GRZ_CK(g, cudaMalloc((void**)&f.voff, sizeof(uint32_t) * (V + 1)));
     GRZ_CK(g, cudaMalloc((void**)&f.vdelta, sizeof(uint32_t) * (V + 1)));
     GRZ_CK(g, cudaMalloc((void**)&f.tile_first, sizeof(uint32_t) * tiles));
-    GRZ_CK(g, cudaMalloc((void**)&f.fr_part, sizeof(uint32_t) * 2 * (V / CCHUNK + 1)));
     GRZ_CK(g, cudaMalloc((void**)&f.nonempty_pull, sizeof(unsigned long long) * W));
     GRZ_CK(g, cudaMalloc((void**)&f.unres, sizeof(unsigned long long) * W));
     GRZ_CK(g, cudaMalloc((void**)&f.touched, sizeof(uint32_t) * (V + 1)));
@@ -1636,17 +1546,14 @@ static int launch_cc_pull(grz_graph* g, uint64_t first, uint64_t count, const Vo
 }
 
 // Compacts the vertices selected by bm1 & bm2, with their vector ranges in `rowptr`, into
-// fr.frontier / voff / vdelta / tile_first (counts on the device in counters[0], [2]).
+// fr.frontier / voff / vdelta / tile_first (counts on the device in counters[3], [2], which are zero).
 static void compact(grz_graph* g, const unsigned long long* bm1, const unsigned long long* bm2, const uint32_t* rowptr,
                     uint32_t skip, const uint32_t* gate)
 {
     grz_frontier_state& f = g->fr;
-    cudaStream_t st = g->stream;
     const unsigned nb = (unsigned)(g->V / CCHUNK + 1);
-    k_fr_count<<<nb, T, 0, st>>>(bm1, bm2, g->V, rowptr, skip, gate, f.fr_part, f.fr_part + nb); GRZ_COUNT_LAUNCH(g);
-    k_fr_scan<<<1, SCAN_T, 0, st>>>(f.fr_part, f.fr_part + nb, nb, f.counters, gate); GRZ_COUNT_LAUNCH(g);
-    k_fr_write<<<nb, T, 0, st>>>(bm1, bm2, g->V, rowptr, skip, f.fr_part, f.fr_part + nb, f.counters, nb, f.frontier, f.voff,
-                                 f.vdelta, f.tile_first, gate); GRZ_COUNT_LAUNCH(g);
+    k_fr_compact<<<nb, T, 0, g->stream>>>(bm1, bm2, g->V, rowptr, skip, gate, f.counters, f.frontier, f.voff, f.vdelta, f.tile_first);
+    GRZ_COUNT_LAUNCH(g);
 }
 
 // One edge phase on a vector range of the pull (pull=1) or push list.  Leaves the vote of the
@@ -1671,6 +1578,7 @@ static int edge_phase(grz_graph* g, int pull, uint64_t first, uint64_t count)
             if (g->stats_on) {  // the work counted is the reference's: every vector of the wanted destinations
                 compact(g, f.wants, f.nonempty_pull, g->pull.rowptr);
                 GRZ_TRY(grz_stats_count_selected(g, &g->pull, f.frontier, f.counters));
+                GRZ_CK(g, cudaMemsetAsync(f.counters, 0, sizeof(uint32_t) * 8, st));  // the compaction below counts anew
             }
             grz_prof_begin(g, GRZ_PROF_BFS_PULL);
             const uint64_t pgroups = (W + FW - 1) / FW;
@@ -1937,7 +1845,7 @@ void grz_frontier_free(grz_graph* g)
 {
     grz_frontier_state& f = g->fr;
     void* ptrs[] = { f.label, f.level, f.has, f.has_next, f.wants, f.nonempty_push, f.nonempty_pull, f.unres, f.frontier, f.voff, f.vdelta, f.tile_first, f.chg, f.dev_err,
-                     f.fr_part, f.touched, f.cand64, f.cand32,
+                     f.touched, f.cand64, f.cand32,
                      f.counters, f.vote, f.sw_out, f.snap };
     for (void* p : ptrs) cudaFree(p);
     if (f.ev[0]) { cudaEventDestroy(f.ev[0]); cudaEventDestroy(f.ev[1]); }
@@ -2171,9 +2079,9 @@ int grz_frontier_run_graph(grz_graph* g, uint64_t* launches)
     const bool bfs = f.app == GRZ_APP_BREADTH_FIRST_SEARCH;
     // kernels of one pull iteration: BFS scan + visit, or (first pass,) compaction, expand, visit;
     // CC one pull launch, or one per source segment plus the whole-list one
-    const uint64_t per_pull = bfs ? (g->tune.bfs_pull_scan ? 2 : (g->tune.bfs_pull_first ? 6 : 5))
-                                  : (f.run_seg ? cc_segment_launches(g) + 1 : (g->tune.cc_pull_first == 2 ? 6 : (g->tune.cc_pull_first == 3 ? 7 : (g->tune.cc_pull_first == 4 ? 6 : (g->tune.cc_pull_first ? 2 : 1)))));
-    const uint64_t per_push = bfs ? 5 : 4;
+    const uint64_t per_pull = bfs ? (g->tune.bfs_pull_scan ? 2 : (g->tune.bfs_pull_first ? 4 : 3))
+                                  : (f.run_seg ? cc_segment_launches(g) + 1 : (g->tune.cc_pull_first == 2 ? 4 : (g->tune.cc_pull_first == 3 ? 5 : (g->tune.cc_pull_first == 4 ? 4 : (g->tune.cc_pull_first ? 2 : 1)))));
+    const uint64_t per_push = bfs ? 3 : 2;
     uint64_t k = 1 + n + (uint64_t)c.npull * per_pull + (uint64_t)c.npush * per_push + (n % 2);
     g->nlaunch += k;
     if (launches) *launches = k;

@@ -457,11 +457,10 @@ struct grz_frontier_state {
     uint32_t* voff;                  // push: offset of each source's first vector among the frontier's
     uint32_t* vdelta;                // push: first vector index in the list minus voff (mod 2^32)
     uint32_t* tile_first;            // push: frontier entry owning the first vector of each tile
-    uint32_t* fr_part;               // push: per-block source and vector totals (scanned)
     uint32_t* touched;               // BFS destinations reached in this phase
     unsigned long long* cand64;      // BFS pull: (vector index, ~source) per destination
     uint32_t* cand32;                // BFS push: smallest source per destination
-    uint32_t* counters;              // [0] frontier size, [1] touched count
+    uint32_t* counters;              // [1] touched count, [2] vectors and [3] vertices of the compacted list, [5] tile queue, [6], [7] gates
     unsigned long long* vote;        // GRZ_VOTE_SLOTS * GRZ_VOTE_STRIDE
     unsigned long long* chg;         // CC: smallest label written per iteration, tagged (2 words, grz_ccbfs.cu)
     unsigned long long mail_chg[2];  // host copy of the initial chg words (outlives the async copy)

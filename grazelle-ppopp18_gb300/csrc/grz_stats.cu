@@ -36,12 +36,12 @@ __global__ void k_stat_range(const uint4* __restrict__ nbr, uint64_t first, uint
     add_warp(out + 1, e);
 }
 
-// vectors and valid lanes of the compacted selection (counters[0] vertices in `sel`)
+// vectors and valid lanes of the compacted selection (counters[3] vertices in `sel`)
 __global__ void k_stat_selected(const uint32_t* __restrict__ sel, const uint32_t* __restrict__ counters,
                                 const uint32_t* __restrict__ rowptr, const uint4* __restrict__ nbr,
                                 unsigned long long* __restrict__ out)
 {
-    const uint32_t n = counters[0];
+    const uint32_t n = counters[3];
     unsigned long long vec = 0, e = 0;
     for (uint32_t i = blockIdx.x * ST_T + threadIdx.x; i < n; i += gridDim.x * ST_T) {
         const uint32_t v = sel[i];
