@@ -29,12 +29,16 @@
 //     keeps the largest HasInfo source of the lowest-indexed vector that holds one (a 64-bit
 //     atomicMin on (vector index, ~source)); push keeps the smallest HasInfo source (atomicMin).
 //     A vertex's BFS level is the iteration that visits it, so levels are exact by construction.
+#include <cooperative_groups.h>
 #include <string.h>
 
 #include <algorithm>
 #include <type_traits>
 
 #include "grz_internal.cuh"
+#include "grz_switch.cuh"
+
+namespace cg = cooperative_groups;
 
 namespace {
 
@@ -108,6 +112,13 @@ __device__ __forceinline__ void touched_append(bool pred, uint32_t val, uint32_t
     if (lane == leader) base = atomicAdd(count, (uint32_t)__popc(m));
     base = __shfl_sync(0xffffffffu, base, leader);
     if (pred) list[base + __popc(m & ((1u << lane) - 1u))] = val;
+}
+
+__device__ __forceinline__ unsigned long long now_ns()
+{
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+    return t;
 }
 
 struct VoteCfg {
@@ -1165,6 +1176,423 @@ __global__ void __launch_bounds__(T) k_bfs_visit(const uint32_t* __restrict__ to
 }
 
 // ---------------------------------------------------------------------------------------------
+// Small iterations, many per launch.
+//
+// A frontier of a few hundred vertices leaves the chip idle: an iteration of the run graph costs
+// about 21 us in kernel starts whatever its size, and a road network or any long tail has a
+// thousand of them.  One cluster of 16 blocks runs such iterations back to back, with the frontier's
+// vectors listed in its shared memory, until the frontier is empty or too large (GRZ_HOP_VOTE),
+// the policy chooses an engine it does not stand in for, or a bound of the run is reached; the last
+// iteration is left to the decision kernel, as if the engine's kernels had run it.  A cluster,
+// because one SM takes one gather per clock, and a frontier of 10k edges needs four for each.  GB300, BFS of 764 levels on a mesh of 250k
+// vertices (7 kernels per level -> one block -> this): 29 -> 4.0 -> 2.2 ms.
+//
+// An iteration is one pass over the listed vectors and one cluster barrier.  BFS: a destination's
+// candidate is (iteration << 33 | pull << 32 | source), lowered by atomicMin in cand64.  The
+// iteration number makes the candidates of earlier iterations win, so a destination keeps its first
+// iteration and, within it, the smallest source; no visit pass separates the iterations.  The
+// destination whose candidate was empty is new: its vectors are listed for the next iteration, in the
+// shared memory of the block that found it (when a list outgrows one step of its block, the next
+// iteration shares all lists evenly, reading the other blocks').  That source is the push engine's parent.  A pull visits the same
+// destinations (every unvisited one with a frontier source), so a small pull runs the same way, and
+// only the parent differs: the largest frontier source of the first vector that holds one.  Where
+// sources ascend along the list that vector is the smallest frontier source's, found by a binary
+// search once all levels are known (k_hop_visit, k_hop_parents).  CC: labels are lowered in place,
+// as k_push_expand does, and a lowered destination is listed once per iteration (the first to lower
+// its stamp, cand32, to the iteration's); a pull is left to the pull kernels.  Votes, engine choice,
+// iteration numbers and the smallest label written are those of single iterations.  The vertices
+// that were listed are marked in `map`, from which k_hop_visit / k_hop_labels write what outlives the
+// launch (the last frontier's HasInfo* among it) and empty the scratch arrays.
+//
+// What an iteration waits for is a chain of round trips (GB300, clocks: L2 300-450, an atomic 500-850,
+// shared memory of another block 400, cluster barrier 480), so a thread takes one edge, not a
+// vector of four whose branches would wait in turn, and nothing that is not needed is outstanding
+// when the barrier is reached: its release waits for every write to arrive, and with reductions to
+// global memory on their way it takes 2200 clocks instead of 480.  The marks are therefore set by
+// the iteration after, at its start.
+constexpr int HOP_CTAS = 16;
+constexpr int HOP_T = 512;
+constexpr uint32_t HOP_CAP = 8192;  // listed vectors per block: twice an even share
+constexpr uint32_t HOP_STEP = HOP_T / 4;  // vectors a block takes in one step
+constexpr size_t HOP_SMEM = sizeof(uint32_t) * HOP_CAP * 4;  // two lists of vectors and their sources
+
+struct HopIn {
+    const uint4* nbr;                   // push list
+    const uint32_t* rowptr;
+    const uint32_t* degree;
+    uint32_t V;
+    double dV, dE, max_degree;
+    const unsigned long long* wants;    // BFS
+    unsigned long long* cand64;         // BFS: all ~0 before, and again after the kernels that follow
+    uint32_t* cand32;                   // CC: likewise
+    uint32_t* label;                    // CC
+    unsigned long long* map;            // all zero before, and again after the kernels that follow
+    const uint32_t* list;               // the frontier's vertices (ctl->hop_n of them)
+    unsigned long long* vote;
+    unsigned long long* chg;            // CC
+    grz_runctl* ctl;
+    int pulls;                          // small pulls run here too (BFS over ascending lists)
+};
+
+// an iteration's totals
+struct __align__(16) HopPart {
+    uint32_t vote_lo, vote_hi;  // vote = vote_lo + 2^16 vote_hi
+    uint32_t verts;             // vertices of the next frontier
+    uint32_t flags;             // HOP_OVER, HOP_LATE
+    uint32_t min;               // CC: smallest label written
+    uint32_t items;             // vectors the block has listed
+    uint32_t pad[2];
+};
+constexpr uint32_t HOP_OVER = 1u, HOP_LATE = 2u;
+constexpr uint32_t HOP_FIRST = 0x80000000u;  // of a listed source: this vector marks it in `map`
+constexpr uint32_t HOP_NOVEC = 0xffffffffu;  // a vertex without vectors, listed to be marked
+
+// the warp's totals of every lane's x, in all lanes
+__device__ __forceinline__ HopPart hop_reduce(HopPart x)
+{
+    x.vote_lo = __reduce_add_sync(0xffffffffu, x.vote_lo);
+    x.vote_hi = __reduce_add_sync(0xffffffffu, x.vote_hi);
+    x.verts = __reduce_add_sync(0xffffffffu, x.verts);
+    x.flags = __reduce_or_sync(0xffffffffu, x.flags);
+    x.min = __reduce_min_sync(0xffffffffu, x.min);
+    return x;
+}
+
+__device__ __forceinline__ HopPart hop_zero()
+{
+    HopPart x;
+    x.vote_lo = x.vote_hi = x.verts = x.flags = x.items = 0;
+    x.min = INF;
+    return x;
+}
+
+// the cluster's totals of every thread's x, after a cluster barrier; s_block (zeroed) and s_part are not
+// those of the call before.  s_part[r].items = *items of block r.
+__device__ __forceinline__ HopPart hop_exchange(cg::cluster_group& cl, HopPart x, const uint32_t* items, HopPart* s_block, HopPart* s_part)
+{
+    const int lane = threadIdx.x & 31;
+    if (__any_sync(0xffffffffu, x.vote_lo != 0 || x.vote_hi != 0 || x.flags != 0 || x.min != INF)) {
+        x = hop_reduce(x);
+        if (lane == 0) {
+            atomicAdd(&s_block->vote_lo, x.vote_lo & 0xffffu);
+            atomicAdd(&s_block->vote_hi, x.vote_hi + (x.vote_lo >> 16));
+            atomicAdd(&s_block->verts, x.verts);
+            if (x.flags) atomicOr(&s_block->flags, x.flags);
+            if (x.min != INF) atomicMin(&s_block->min, x.min);
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x < HOP_CTAS) {
+        HopPart y = *s_block;
+        y.items = *items;
+        *cl.map_shared_rank(s_part + cl.block_rank(), threadIdx.x) = y;
+    }
+    cl.sync();
+    return hop_reduce(lane < HOP_CTAS ? s_part[lane] : hop_zero());
+}
+
+// (started by the decision kernel when the next iteration's vote is at most GRZ_HOP_VOTE)
+template <bool IsBfs>
+__global__ void __cluster_dims__(HOP_CTAS, 1, 1) __launch_bounds__(HOP_T, 1) k_hop(const HopIn in)
+{
+    extern __shared__ uint32_t s_mem[];
+    __shared__ uint32_t s_items[4];  // vectors listed for an iteration, by its number mod 4
+    __shared__ HopPart s_block[2], s_part[2][HOP_CTAS];
+    __shared__ int s_pull;
+    __shared__ float s_f[NF], s_par[MLP_WARP_FLOATS];
+    cg::cluster_group cl = cg::this_cluster();
+    grz_runctl* const ctl = in.ctl;
+    const int tid = threadIdx.x, lane = tid & 31;
+    const uint32_t rank = cl.block_rank();
+    const uint32_t n0 = ctl->hop_n;
+    if (tid < 4) s_items[tid] = 0;
+    if (tid < 2) s_block[tid] = hop_zero();
+    const uint32_t level0 = ctl->level, max_level = ctl->max_level, mode0 = ctl->engine;
+    const int force = ctl->force;
+    const float* params = ctl->params;
+    const double threshold = ctl->threshold;
+    const unsigned long long t0 = ctl->t0_ns, limit = ctl->limit_ns, unvisited = ctl->unvisited;
+    if (params) mlp_stage(params, s_par, tid, HOP_T);
+    cl.sync();
+    // The starting frontier's vectors, spread over the blocks in runs of at most 32, a full list's over
+    // the next ones: they are fewer than the vote, which is half of what the lists hold.
+    HopPart sum = hop_zero();
+    for (uint32_t i = rank + HOP_CTAS * tid; i < n0; i += HOP_CTAS * HOP_T) {
+        const uint32_t d = in.list[i], r0 = __ldg(in.rowptr + d), n = __ldg(in.rowptr + d + 1) - r0;
+        uint32_t to = (rank + tid) & (HOP_CTAS - 1);
+        for (uint32_t j = 0, tries = 0; j < n && tries < 64u; to = (to + 1) & (HOP_CTAS - 1)) {
+            const uint32_t k = min(32u, n - j);
+            const uint32_t at = atomicAdd(cl.map_shared_rank(&s_items[0], to), k);
+            uint32_t* vec = cl.map_shared_rank(s_mem, to);
+            if (at + k > HOP_CAP) {  // the places no one takes
+                for (uint32_t q = at; q < HOP_CAP; ++q) { vec[q] = HOP_NOVEC; vec[HOP_CAP + q] = 0; }
+                ++tries;
+                continue;
+            }
+            for (uint32_t q = 0; q < k; ++q) { vec[at + q] = r0 + j + q; vec[HOP_CAP + at + q] = d; }
+            j += k;
+        }
+    }
+    cl.sync();  // other blocks have added to this one's list
+    hop_exchange(cl, sum, &s_items[0], &s_block[1], s_part[1]);
+    // lists vertex d's vectors [r0, r0 + n) in this block's list q; false when it is full
+    auto append = [&](int q, int slot, uint32_t d, uint32_t r0, uint32_t n) -> bool {
+        const uint32_t k = max(n, 1u), at = atomicAdd(&s_items[slot], k);
+        uint32_t* vec = s_mem + q * 2 * HOP_CAP;
+        if (at > HOP_CAP || k > HOP_CAP - at) {
+            atomicOr(in.map + (d >> 6), 1ull << (d & 63));
+            for (uint32_t i = at; i < HOP_CAP; ++i) vec[HOP_CAP + i] = 0;  // places no one takes carry no mark
+            return false;
+        }
+        for (uint32_t i = 0; i < k; ++i) {
+            vec[at + i] = n ? r0 + i : HOP_NOVEC;
+            vec[HOP_CAP + at + i] = i == 0 ? d | HOP_FIRST : d;
+        }
+        return true;
+    };
+    uint32_t it = 0, mode = mode0, pulls = 0;     // iterations finished, this one's engine, pulls before it
+    unsigned long long left = unvisited, vote;    // BFS: vertices not visited yet
+    for (;; ++it) {
+        const int p = it & 1, nxt = (it + 1) & 3;
+        const uint32_t level = level0 + it;
+        // this block's share: its own list, or every 16th vector of all lists when one is longer than a step
+        const uint32_t theirs = lane < HOP_CTAS ? min(s_part[p ^ 1][lane].items, HOP_CAP) : 0u;
+        const bool own = __reduce_max_sync(0xffffffffu, theirs) <= HOP_STEP;
+        uint32_t m = __shfl_sync(0xffffffffu, theirs, (int)rank), before = theirs;
+        if (!own) {
+            for (int o = 1; o < HOP_CTAS; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xffffffffu, before, o);
+                if (lane >= o) before += y;  // vectors of the lists up to this lane's
+            }
+            m = __shfl_sync(0xffffffffu, before, HOP_CTAS - 1);
+        }
+        if (tid == 0) {
+            s_items[(it + 2) & 3] = 0;
+            s_block[p ^ 1] = hop_zero();
+        }
+        sum = hop_zero();
+        // a timer read is slow
+        if (rank == 0 && tid == 0 && (it & 15) == 0 && now_ns() - t0 > limit) sum.flags = HOP_LATE;
+        const uint32_t l = tid & 3;  // this thread's lane of its vectors
+        const uint32_t every = own ? 1 : HOP_CTAS, shift = own ? 0 : rank;
+        for (uint32_t k0 = (tid - lane) >> 2; k0 * every < m; k0 += HOP_STEP) {  // warp-uniform
+            uint32_t at = (k0 + (lane >> 2)) * every + shift, from = rank;
+            const bool in_list = at < m;
+            if (!own) {  // the list that holds vector `at` of all
+                from = 0;
+#pragma unroll
+                for (int r = 0; r < HOP_CTAS - 1; ++r) from += at >= __shfl_sync(0xffffffffu, before, r);
+                const uint32_t b = __shfl_sync(0xffffffffu, before, from ? (int)from - 1 : 0);
+                if (from) at -= b;
+            }
+            if (!in_list) continue;
+            const uint32_t* vec = cl.map_shared_rank(s_mem + p * 2 * HOP_CAP, from);
+            const uint32_t us = vec[HOP_CAP + at], v = vec[at], u = us & ~HOP_FIRST;
+            if ((us & HOP_FIRST) && l == 0) atomicOr(in.map + (u >> 6), 1ull << (u & 63));
+            if (v == HOP_NOVEC) continue;
+            const uint32_t d = __ldg(reinterpret_cast<const uint32_t*>(in.nbr) + 4 * (uint64_t)v + l);
+            if (d >= in.V) continue;
+            bool fresh = false;
+            uint32_t r0 = 0, r1 = 0, deg = 0;
+            // the row pointers and degree are loaded while the atomic that decides is on its way
+            if (IsBfs) {
+                const unsigned long long key = ((unsigned long long)level << 33) | ((unsigned long long)mode << 32) | u;
+                const unsigned long long c = __ldcg(in.cand64 + d);
+                const bool w = (__ldg(in.wants + (d >> 6)) >> (d & 63)) & 1ull;
+                if (w && key < c) {
+                    const unsigned long long old = atomicMin(in.cand64 + d, key);
+                    r0 = __ldg(in.rowptr + d);
+                    r1 = __ldg(in.rowptr + d + 1);
+                    deg = __ldg(in.degree + d);
+                    fresh = old == ~0ull;
+                }
+            } else {
+                const uint32_t msg = __ldcg(in.label + u);
+                if (msg < __ldcg(in.label + d)) {
+                    const uint32_t old = atomicMin(in.label + d, msg);
+                    r0 = __ldg(in.rowptr + d);
+                    r1 = __ldg(in.rowptr + d + 1);
+                    deg = __ldg(in.degree + d);
+                    if (msg < old) {
+                        sum.min = min(sum.min, msg);
+                        fresh = atomicMin(in.cand32 + d, ~level) > ~level;
+                    }
+                }
+            }
+            if (fresh) {
+                const unsigned long long x = 1ull + deg + sum.vote_lo;
+                sum.vote_lo = (uint32_t)(x & 0xffffu);
+                sum.vote_hi += (uint32_t)(x >> 16);
+                sum.verts += 1;
+                if (!append(p ^ 1, nxt, d, r0, r1 - r0)) sum.flags |= HOP_OVER;
+            }
+        }
+        sum = hop_exchange(cl, sum, &s_items[nxt], &s_block[p], s_part[p]);
+        // every thread of the cluster takes the same decision from the iteration's totals
+        vote = sum.vote_lo + ((unsigned long long)sum.vote_hi << 16);
+        if (IsBfs) left -= sum.verts;
+        if (vote == 0 || vote > GRZ_HOP_VOTE || sum.flags || level >= max_level) break;
+        int pull;
+        if (force >= 0) {
+            pull = force;
+        } else if (params) {
+            if (tid < 32) {
+                FeatIn fe;
+                fe.V = in.dV;
+                fe.E = in.dE;
+                fe.max_degree = in.max_degree;
+                fe.iter = level + 1;
+                fe.app_bfs = IsBfs;
+                fe.last_engine = (int)mode;
+                if (lane < NF) s_f[lane] = feature(lane, fe, (float)(unsigned long long)sum.verts, IsBfs ? (float)left : 0.f, (float)vote);
+                __syncwarp();
+                const float z = mlp_logit_warp(MlpShared{ s_par }, s_f, lane);
+                if (lane == 0) s_pull = z > 0.f ? 1 : 0;
+            }
+            __syncthreads();
+            pull = s_pull;
+        } else {
+            pull = (double)vote > threshold ? 1 : 0;
+        }
+        if (pull && !in.pulls) break;
+        pulls += mode;
+        mode = (uint32_t)pull;
+    }
+    // the last frontier's marks
+    const uint32_t* last = s_mem + ((it & 1) ^ 1) * 2 * HOP_CAP + HOP_CAP;
+    for (uint32_t i = tid; i < min(s_items[(it + 1) & 3], HOP_CAP); i += HOP_T) {
+        const uint32_t u = last[i];
+        if (u & HOP_FIRST) atomicOr(in.map + ((u & ~HOP_FIRST) >> 6), 1ull << (u & 63));
+    }
+    // iteration `it` is the last: the decision kernel counts it and reads its vote from the slots
+    if (tid == 0 && rank == 0) {
+        const uint32_t level = level0 + it;
+        in.vote[0] = vote;
+        if (!IsBfs && sum.min != INF)
+            atomicMax(in.chg + (level & 1), ((unsigned long long)level << 32) | (unsigned long long)(~sum.min));
+        ctl->level = level;
+        ctl->engine = mode;
+        ctl->npull += pulls;
+        ctl->npush += it - pulls;
+        ctl->hop_pulls = pulls + mode;
+        ctl->hop_levels[0] += it + 1 - pulls - mode;
+        ctl->hop_levels[1] += pulls + mode;
+        ctl->hop_runs += 1;
+    }
+}
+
+// Calls f(word, bits, vertex, whether it is marked) for every nonzero word of `map`, a warp per word, first
+// the lower then the upper 32 vertices (f is called by whole warps); g(word, bits) once after each.
+template <typename F, typename G>
+__device__ __forceinline__ void hop_marked(const unsigned long long* __restrict__ map, uint64_t W, F f, G g)
+{
+    const int lane = threadIdx.x & 31;
+    const uint64_t nwarps = (uint64_t)gridDim.x * (T / 32);
+    for (uint64_t w0 = 32 * ((uint64_t)blockIdx.x * (T / 32) + (threadIdx.x >> 5)); w0 < W; w0 += 32 * nwarps) {
+        const unsigned long long mine = w0 + lane < W ? map[w0 + lane] : 0ull;
+        for (unsigned nz = __ballot_sync(0xffffffffu, mine != 0); nz; nz &= nz - 1) {
+            const int j = __ffs(nz) - 1;
+            const unsigned long long bits = __shfl_sync(0xffffffffu, mine, j);
+            f((uint32_t)(64 * (w0 + j)) + lane, ((bits >> lane) & 1ull) != 0, 0);
+            f((uint32_t)(64 * (w0 + j)) + 32 + lane, ((bits >> (32 + lane)) & 1ull) != 0, 1);
+            if (lane == 0) g(w0 + j, bits);
+        }
+    }
+}
+
+// BFS, after k_hop: levels, WantsInfo and the last frontier's HasInfo* of the marked vertices, and the
+// parents of those that a push visited, whose candidates it empties.  `clear`: no k_hop_parents follows.
+__global__ void __launch_bounds__(T) k_hop_visit(const grz_runctl* __restrict__ ctl, unsigned long long* __restrict__ map, uint64_t W,
+                                                 unsigned long long* __restrict__ cand64, uint32_t* __restrict__ parent,
+                                                 uint32_t* __restrict__ level, unsigned long long* __restrict__ wants,
+                                                 unsigned long long* __restrict__ has_next, int clear)
+{
+    const uint32_t last = ctl->level;
+    unsigned long long in_last = 0ull;
+    hop_marked(
+        map, W,
+        [&](uint32_t d, bool marked, int half) {
+            bool l = false;
+            if (marked) {
+                const unsigned long long c = cand64[d];
+                const uint32_t lv = (uint32_t)(c >> 33);
+                level[d] = lv;
+                l = lv == last;
+                if (!((c >> 32) & 1ull)) {
+                    parent[d] = (uint32_t)c;
+                    cand64[d] = ~0ull;
+                }
+            }
+            const unsigned long long m = __ballot_sync(0xffffffffu, l);
+            in_last = half ? in_last | (m << 32) : m;
+        },
+        [&](uint64_t w, unsigned long long bits) {
+            wants[w] &= ~bits;
+            has_next[w] = in_last;
+            if (clear) map[w] = 0ull;
+        });
+}
+
+// BFS: parents of the marked vertices that a pull visited.  The candidate's source is the smallest in
+// the frontier; its vector is the last one that starts at or below it, and the parent is the largest
+// source there that was visited one iteration earlier.
+__global__ void __launch_bounds__(T) k_hop_parents(const grz_runctl* __restrict__ ctl, unsigned long long* __restrict__ map, uint64_t W,
+                                                   unsigned long long* __restrict__ cand64, uint32_t* __restrict__ parent,
+                                                   const uint32_t* __restrict__ level, uint32_t V, const uint4* __restrict__ nbr,
+                                                   const uint32_t* __restrict__ rowptr, const uint32_t* __restrict__ hub_vid, uint32_t nhub)
+{
+    if (!ctl->hop_pulls) {
+        hop_marked(map, W, [](uint32_t, bool, int) {}, [&](uint64_t w, unsigned long long) { map[w] = 0ull; });
+        return;
+    }
+    hop_marked(
+        map, W,
+        [&](uint32_t d, bool marked, int) {
+            const unsigned long long c = marked ? cand64[d] : ~0ull;
+            if (c == ~0ull) return;  // a push visited it
+            cand64[d] = ~0ull;
+            const uint32_t u = (uint32_t)c, before = (uint32_t)(c >> 33) - 1;
+            uint32_t lo = __ldg(rowptr + d), hi = __ldg(rowptr + d + 1) - 1;
+            while (lo < hi) {
+                const uint32_t mid = lo + (hi - lo + 1) / 2;
+                if (grz_hub_decode(__ldg(&nbr[mid].x), hub_vid, nhub) <= u) lo = mid; else hi = mid - 1;
+            }
+            const uint4 s = __ldg(nbr + lo);
+            const uint32_t id[4] = { grz_hub_decode(s.x, hub_vid, nhub), grz_hub_decode(s.y, hub_vid, nhub),
+                                     grz_hub_decode(s.z, hub_vid, nhub), grz_hub_decode(s.w, hub_vid, nhub) };
+            uint32_t best = u;
+#pragma unroll
+            for (int l = 0; l < 4; ++l)
+                if (id[l] < V && id[l] > best && level[id[l]] == before) best = id[l];
+            parent[d] = best;
+        },
+        [&](uint64_t w, unsigned long long) { map[w] = 0ull; });
+}
+
+// CC, after k_hop: the last frontier's HasInfo*; empties the stamps
+__global__ void __launch_bounds__(T) k_hop_labels(const grz_runctl* __restrict__ ctl, unsigned long long* __restrict__ map, uint64_t W,
+                                                  uint32_t* __restrict__ cand32, unsigned long long* __restrict__ has_next)
+{
+    const uint32_t last = ctl->level;
+    unsigned long long in_last = 0ull;
+    hop_marked(
+        map, W,
+        [&](uint32_t d, bool marked, int half) {
+            bool l = false;
+            if (marked) {
+                l = cand32[d] == ~last;
+                cand32[d] = INF;
+            }
+            const unsigned long long m = __ballot_sync(0xffffffffu, l);
+            in_last = half ? in_last | (m << 32) : m;
+        },
+        [&](uint64_t w, unsigned long long) {
+            has_next[w] = in_last;
+            map[w] = 0ull;
+        });
+}
+
+// ---------------------------------------------------------------------------------------------
 // init / output
 
 // execution_initialize_vertex_prop_cc: (double)id; entry V = +inf.  Four labels per thread with one
@@ -1846,7 +2274,7 @@ void grz_frontier_free(grz_graph* g)
     grz_frontier_state& f = g->fr;
     void* ptrs[] = { f.label, f.level, f.has, f.has_next, f.wants, f.nonempty_push, f.nonempty_pull, f.unres, f.frontier, f.voff, f.vdelta, f.tile_first, f.chg, f.dev_err,
                      f.touched, f.cand64, f.cand32,
-                     f.counters, f.vote, f.sw_out, f.snap };
+                     f.counters, f.vote, f.sw_out, f.snap, f.hop_buf, f.hop_map };
     for (void* p : ptrs) cudaFree(p);
     if (f.ev[0]) { cudaEventDestroy(f.ev[0]); cudaEventDestroy(f.ev[1]); }
     if (f.mail) cudaFreeHost(f.mail);
@@ -1862,11 +2290,11 @@ void grz_frontier_free(grz_graph* g)
 // ---------------------------------------------------------------------------------------------
 // A whole CC/BFS run as one CUDA graph.
 //
-//   k_run_decide (initial: sets pull0/push0)  ->  WHILE (loop) {
-//       IF (pull0) { pull edge phase, even roles }   IF (push0) { push edge phase, even roles }
-//       k_run_decide (next HasInfo = B, clears A; sets pull1/push1, loop)
-//       IF (pull1) { pull edge phase, odd roles }    IF (push1) { push edge phase, odd roles }
-//       k_run_decide (next HasInfo = A, clears B; sets pull0/push0, loop)
+//   k_run_decide (initial: sets engine0)  ->  WHILE (loop) {
+//       SWITCH (engine0) { pull edge phase | push edge phase | k_hop, even roles }
+//       k_run_decide (next HasInfo = B, clears A; sets engine1, loop)
+//       SWITCH (engine1) { the same, odd roles }
+//       k_run_decide (next HasInfo = A, clears B; sets engine0, loop)
 //   }
 //
 // Even iterations read HasInfo from buffer A and write HasInfo* into B; odd ones the reverse,
@@ -1900,16 +2328,99 @@ static int capture_end(grz_graph* g, cudaStream_t cs, cudaGraphNode_t* sink)
     return GRZ_OK;
 }
 
+// a conditional node with `size` bodies (a SWITCH runs the one its handle names, or none)
 static int add_conditional(grz_graph* g, cudaGraph_t graph, const cudaGraphNode_t* deps, size_t ndeps, cudaGraphConditionalHandle h,
-                           cudaGraphConditionalNodeType type, cudaGraphNode_t* node, cudaGraph_t* body)
+                           cudaGraphConditionalNodeType type, unsigned size, cudaGraphNode_t* node, cudaGraph_t* bodies)
 {
     cudaGraphNodeParams p = {};
     p.type = cudaGraphNodeTypeConditional;
     p.conditional.handle = h;
     p.conditional.type = type;
-    p.conditional.size = 1;
+    p.conditional.size = size;
     GRZ_CK(g, cudaGraphAddNode(node, graph, deps, nullptr, ndeps, &p));
-    *body = p.conditional.phGraph_out[0];
+    for (unsigned i = 0; i < size; ++i) bodies[i] = p.conditional.phGraph_out[i];
+    return GRZ_OK;
+}
+
+// whether small pulls go through k_hop as well
+static bool hop_pulls(const grz_graph* g)
+{
+    return g->fr.hop_list && g->fr.app == GRZ_APP_BREADTH_FIRST_SEARCH && g->pull.ascending;
+}
+
+// k_hop and what writes its results, captured as a body of its own
+static int hop_phase(grz_graph* g)
+{
+    grz_frontier_state& f = g->fr;
+    const bool bfs = f.app == GRZ_APP_BREADTH_FIRST_SEARCH;
+    HopIn in;
+    memset(&in, 0, sizeof(in));
+    in.nbr = g->push.nbr;
+    in.rowptr = g->push.rowptr;
+    in.degree = g->degree;
+    in.V = (uint32_t)g->V;
+    in.dV = (double)g->V;
+    in.dE = (double)(g->E ? g->E : 1);
+    in.max_degree = (double)g->max_degree;
+    in.wants = f.wants;
+    in.cand64 = f.cand64;
+    in.cand32 = f.cand32;
+    in.label = f.label;
+    in.map = f.hop_map;
+    in.list = f.hop_list;
+    in.vote = f.vote;
+    in.chg = f.chg;
+    in.ctl = f.ctl;
+    in.pulls = hop_pulls(g);
+    const uint64_t W = words_of(g->V);
+    const unsigned grid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>((W + T - 1) / T, (uint64_t)g->num_sms * 4));
+    if (bfs) {
+        k_hop<true><<<HOP_CTAS, HOP_T, HOP_SMEM, g->stream>>>(in);
+        k_hop_visit<<<grid, T, 0, g->stream>>>(f.ctl, f.hop_map, W, f.cand64, f.label, f.level, f.wants, f.has_next, !in.pulls);
+        if (in.pulls)
+            k_hop_parents<<<grid, T, 0, g->stream>>>(f.ctl, f.hop_map, W, f.cand64, f.label, f.level, (uint32_t)g->V, g->pull.nbr, g->pull.rowptr,
+                                                     g->pull.hub_vid, g->pull.nhub);
+    } else {
+        k_hop<false><<<HOP_CTAS, HOP_T, HOP_SMEM, g->stream>>>(in);
+        k_hop_labels<<<grid, T, 0, g->stream>>>(f.ctl, f.hop_map, W, f.cand32, f.has_next);
+    }
+    return grz_cuda_check(g, cudaGetLastError(), "k_hop");
+}
+
+// Whether a run's small iterations go through k_hop: its frontiers are bounded by the vote, so the
+// vote has to count vertices and out-edges (the default; forced engines included).
+static int hop_prepare(grz_graph* g)
+{
+    grz_frontier_state& f = g->fr;
+    if ((f.flags & (GRZ_FLAG_WITHOUT_COUNT | GRZ_FLAG_WITHOUT_OUTDEG)) || g->V >= 0x80000000ull) {  // (31-bit iteration numbers)
+        f.hop_list = nullptr;
+        return GRZ_OK;
+    }
+    if (!f.hop_buf) {
+        // a cluster of 16 blocks needs the opt-in, and a GPC that can hold it
+        int clusters = 0;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(HOP_CTAS);
+        cfg.blockDim = dim3(HOP_T);
+        cfg.dynamicSmemBytes = HOP_SMEM;
+        cudaLaunchAttribute at = {};
+        at.id = cudaLaunchAttributeClusterDimension;
+        at.val.clusterDim.x = HOP_CTAS;
+        at.val.clusterDim.y = at.val.clusterDim.z = 1;
+        cfg.attrs = &at;
+        cfg.numAttrs = 1;
+        for (const void* k : { (const void*)k_hop<true>, (const void*)k_hop<false> }) {
+            GRZ_CK(g, cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+            GRZ_CK(g, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)HOP_SMEM));
+            GRZ_CK(g, cudaOccupancyMaxActiveClusters(&clusters, k, &cfg));
+            if (clusters < 1) return grz_set_error(g, GRZ_ERR_CUDA, "a cluster of %d blocks does not fit", HOP_CTAS);
+        }
+        const uint64_t W = words_of(g->V);
+        GRZ_CK(g, cudaMalloc((void**)&f.hop_map, sizeof(unsigned long long) * W));
+        GRZ_CK(g, cudaMemsetAsync(f.hop_map, 0, sizeof(unsigned long long) * W, g->stream));
+        GRZ_CK(g, cudaMalloc((void**)&f.hop_buf, sizeof(uint32_t) * GRZ_HOP_VOTE));
+    }
+    f.hop_list = f.hop_buf;
     return GRZ_OK;
 }
 
@@ -1927,48 +2438,41 @@ static int build_run_graph(grz_graph* g)
     GRZ_CK(g, cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking));
     cudaGraph_t top = nullptr;
     int rc = grz_cuda_check(g, cudaGraphCreate(&top, 0), "graph create");
-    // one handle per conditional node: the loop, and pull / push for the even and odd halves
-    cudaGraphConditionalHandle hloop = 0, hpull[2] = { 0, 0 }, hpush[2] = { 0, 0 };
+    // one handle per conditional node: the loop, and the engine of the even and odd halves
+    cudaGraphConditionalHandle hloop = 0, hengine[2] = { 0, 0 };
     if (!rc) rc = grz_cuda_check(g, cudaGraphConditionalHandleCreate(&hloop, top, 1, cudaGraphCondAssignDefault), "handle");
-    for (int p = 0; p < 2 && !rc; ++p) {
-        rc = grz_cuda_check(g, cudaGraphConditionalHandleCreate(&hpull[p], top, 0, cudaGraphCondAssignDefault), "handle");
-        if (!rc) rc = grz_cuda_check(g, cudaGraphConditionalHandleCreate(&hpush[p], top, 0, cudaGraphCondAssignDefault), "handle");
-    }
+    for (int p = 0; p < 2 && !rc; ++p)
+        rc = grz_cuda_check(g, cudaGraphConditionalHandleCreate(&hengine[p], top, GRZ_RUN_NONE, cudaGraphCondAssignDefault), "handle");
     g->stream = cs;
     f.level_dev = &f.ctl->level;
     cudaGraphNode_t n0 = nullptr, wnode = nullptr;
     cudaGraph_t body = nullptr;
     if (!rc) rc = capture_begin(g, cs, top, nullptr, 0);
     if (!rc) {
-        rc = grz_switch_launch_run_decide(g, A, nullptr, 1, hloop, hpull[0], hpush[0]);
+        rc = grz_switch_launch_run_decide(g, A, nullptr, 1, hloop, hengine[0], hop_pulls(g));
         const int rc2 = capture_end(g, cs, &n0);
         if (!rc) rc = rc2;
     }
-    if (!rc) rc = add_conditional(g, top, &n0, 1, hloop, cudaGraphCondTypeWhile, &wnode, &body);
+    if (!rc) rc = add_conditional(g, top, &n0, 1, hloop, cudaGraphCondTypeWhile, 1, &wnode, &body);
     cudaGraphNode_t prev = nullptr;
     for (int parity = 0; parity < 2 && !rc; ++parity) {
         f.has = parity ? B : A;
         f.has_next = parity ? A : B;
-        cudaGraphNode_t npull = nullptr, npush = nullptr, ndec = nullptr;
-        cudaGraph_t bpull = nullptr, bpush = nullptr;
-        rc = add_conditional(g, body, prev ? &prev : nullptr, prev ? 1 : 0, hpull[parity], cudaGraphCondTypeIf, &npull, &bpull);
-        if (!rc) rc = capture_begin(g, cs, bpull, nullptr, 0);
-        if (!rc) {
-            rc = edge_phase(g, 1, 0, g->pull.nvec);
+        cudaGraphNode_t nengine = nullptr, ndec = nullptr;
+        cudaGraph_t engine[3] = { nullptr, nullptr, nullptr };  // GRZ_RUN_PULL, _PUSH, _HOP
+        rc = add_conditional(g, body, prev ? &prev : nullptr, prev ? 1 : 0, hengine[parity], cudaGraphCondTypeSwitch, f.hop_list ? 3 : 2,
+                             &nengine, engine);
+        for (int e = 0; e < (f.hop_list ? 3 : 2) && !rc; ++e) {
+            rc = capture_begin(g, cs, engine[e], nullptr, 0);
+            if (rc) break;
+            rc = e == GRZ_RUN_PULL ? edge_phase(g, 1, 0, g->pull.nvec) : (e == GRZ_RUN_PUSH ? edge_phase(g, 0, 0, g->push.nvec) : hop_phase(g));
             const int rc2 = capture_end(g, cs, nullptr);
             if (!rc) rc = rc2;
         }
-        if (!rc) rc = add_conditional(g, body, &npull, 1, hpush[parity], cudaGraphCondTypeIf, &npush, &bpush);
-        if (!rc) rc = capture_begin(g, cs, bpush, nullptr, 0);
-        if (!rc) {
-            rc = edge_phase(g, 0, 0, g->push.nvec);
-            const int rc2 = capture_end(g, cs, nullptr);
-            if (!rc) rc = rc2;
-        }
-        if (!rc) rc = capture_begin(g, cs, body, &npush, 1);
+        if (!rc) rc = capture_begin(g, cs, body, &nengine, 1);
         if (!rc) {
             // decides the other half's engine
-            rc = grz_switch_launch_run_decide(g, f.has_next, f.has, 0, hloop, hpull[1 - parity], hpush[1 - parity]);
+            rc = grz_switch_launch_run_decide(g, f.has_next, f.has, 0, hloop, hengine[1 - parity], hop_pulls(g));
             const int rc2 = capture_end(g, cs, &ndec);
             if (!rc) rc = rc2;
         }
@@ -2028,6 +2532,7 @@ int grz_frontier_run_graph(grz_graph* g, uint64_t* launches)
         const size_t smem = sizeof(uint32_t) * std::min<uint32_t>(g->tune.cc_cache, g->pull.nhub);
         rc = g->tune.cc_threads == 256 ? cc_pull_config_any<256>(g, smem, &resident)
              : (g->tune.cc_threads == 1024 ? cc_pull_config_any<1024>(g, smem, &resident) : cc_pull_config_any<512>(g, smem, &resident));
+        if (!rc) rc = hop_prepare(g);
         if (!rc) rc = build_run_graph(g);
         if (rc) return rc;
     }
@@ -2054,7 +2559,7 @@ int grz_frontier_run_graph(grz_graph* g, uint64_t* launches)
         f.iter += c.npull + c.npush;
         f.npull += c.npull;
         f.npush += c.npush;
-        if ((c.npull + c.npush) % 2 == 0 && c.npull + c.npush > 0) {
+        if (c.bodies % 2 == 0 && c.bodies > 0) {
             unsigned long long* t = f.has;
             f.has = f.has_next;
             f.has_next = t;
@@ -2070,8 +2575,8 @@ int grz_frontier_run_graph(grz_graph* g, uint64_t* launches)
     f.last_engine = (int)c.last_engine;
     f.next_pull = (int)c.engine;
     memcpy(f.last_features, c.features, sizeof(f.last_features));
-    // iteration k (1-based within the launch) read HasInfo from A when k is odd
-    if (n % 2 == 0 && n > 0) {
+    // iteration k of the loop (1-based within the launch) read HasInfo from A when k is odd
+    if (c.bodies % 2 == 0 && c.bodies > 0) {
         unsigned long long* t = f.has;
         f.has = f.has_next;
         f.has_next = t;
@@ -2082,7 +2587,9 @@ int grz_frontier_run_graph(grz_graph* g, uint64_t* launches)
     const uint64_t per_pull = bfs ? (g->tune.bfs_pull_scan ? 2 : (g->tune.bfs_pull_first ? 4 : 3))
                                   : (f.run_seg ? cc_segment_launches(g) + 1 : (g->tune.cc_pull_first == 2 ? 4 : (g->tune.cc_pull_first == 3 ? 5 : (g->tune.cc_pull_first == 4 ? 4 : (g->tune.cc_pull_first ? 2 : 1)))));
     const uint64_t per_push = bfs ? 3 : 2;
-    uint64_t k = 1 + n + (uint64_t)c.npull * per_pull + (uint64_t)c.npush * per_push + (n % 2);
+    // decisions, iterations by an engine's kernels, and k_hop's launches
+    const uint64_t k = 1 + c.bodies + (uint64_t)(c.npull - c.hop_levels[1]) * per_pull + (uint64_t)(c.npush - c.hop_levels[0]) * per_push +
+                       (uint64_t)c.hop_runs * (2 + hop_pulls(g)) + (c.bodies % 2);
     g->nlaunch += k;
     if (launches) *launches = k;
     return GRZ_OK;

@@ -327,6 +327,7 @@ struct grz_list {
     uint32_t* rowptr;       // uint32[V+1]
     uint32_t* hub_vid;      // pull list: vertex of each hub slot, slots by out-degree, highest first
     uint32_t nhub;
+    int ascending;          // each shared vertex's neighbours ascend (the file order; the API asks for grouping only)
 };
 
 // Hub sources of the pull list.  In power-law graphs a few thousand vertices are the source of
@@ -365,6 +366,16 @@ struct grz_prof;
 // the vote is added into GRZ_VOTE_SLOTS counters, 128 bytes apart (block mod slots)
 #define GRZ_VOTE_SLOTS 64
 #define GRZ_VOTE_STRIDE 16
+
+// Largest vote (frontier vertices and their out-edges) of an iteration that k_hop runs (grz_ccbfs.cu).
+// GB300, a BFS run with 2048 / 8192 / 32768 / 65536: R-MAT of 100k vertices 270 / 238 / 218 / 223 us, R-MAT
+// 24 940 / 939 / 939 / 901 us; 65536 is half of what its lists hold.
+#define GRZ_HOP_VOTE 65536u
+// what the run graph's SWITCH runs next
+#define GRZ_RUN_PULL 0
+#define GRZ_RUN_PUSH 1
+#define GRZ_RUN_HOP 2
+#define GRZ_RUN_NONE 3
 
 // learned switch (grz_switch.cu)
 #define GRZ_MLP_FEATURES 12
@@ -438,6 +449,13 @@ struct grz_runctl {
     double threshold;                // vote threshold (E/5 or V/2)
     int32_t force;                   // 1 pull, 0 push, -1 the policy decides
     float features[GRZ_MLP_FEATURES];
+    // small push iterations run in one launch (k_hop)
+    uint32_t hop_cnt;                // the decision kernel's listing counter (zero between uses)
+    uint32_t hop_n;                  // vertices listed for the iteration about to run (0: not listed)
+    uint32_t hop_pulls;              // pulls among the last k_hop's iterations (BFS)
+    uint32_t hop_levels[2], hop_runs;  // push and pull iterations run by k_hop, and its launches
+    uint32_t bodies;                 // iterations of the graph's loop (k_hop's many count once)
+    unsigned long long unvisited;    // WantsInfo's count at the last decision
 };
 
 // CC / BFS state (grz_ccbfs.cu)
@@ -479,6 +497,9 @@ struct grz_frontier_state {
     cudaEvent_t ev[2];
     // the run as one CUDA graph (WHILE over two iterations with IF nodes per engine)
     grz_runctl* ctl;                 // device
+    uint32_t* hop_buf;               // u32[GRZ_HOP_VOTE]
+    unsigned long long* hop_map;     // vertices k_hop listed (zero between uses)
+    uint32_t* hop_list;              // hop_buf, or null in a run that does not use k_hop
     const uint32_t* level_dev;       // set while capturing: BFS level read from ctl->level
     cudaGraphExec_t run_exec;
     unsigned long long* run_bm[2];   // the HasInfo buffers in the graph's even-iteration roles
@@ -662,7 +683,7 @@ int grz_frontier_digest(grz_graph* g, uint64_t* out3);
 int grz_switch_max_degree(grz_graph* g);
 void grz_switch_policy_ctl(grz_graph* g, grz_runctl* c);
 int grz_switch_launch_run_decide(grz_graph* g, const unsigned long long* next_frontier, unsigned long long* clear_bm, int initial,
-                                 unsigned long long hloop, unsigned long long hpull, unsigned long long hpush);
+                                 unsigned long long hloop, unsigned long long hengine, int hop_pulls);
 // learned switch: features of a state + the policy's decision; frontier = HasInfo of the
 // iteration the decision is for; vote_override = ~0 to read the vote slots
 int grz_switch_decide(grz_graph* g, const unsigned long long* frontier, uint64_t vote_override, uint32_t iter,

@@ -38,7 +38,8 @@ __device__ __forceinline__ uint64_t piece_of(uint64_t s, int lane)
 }
 
 // edge range of each shared vertex: start[s] = its first edge, end[s] = one past its last (both
-// 0 without edges).  flags[0]: not grouped in ascending order, flags[1]: an ID >= V.
+// 0 without edges).  flags[0]: not grouped in ascending order, flags[1]: an ID >= V, flags[2]: the other
+// vertices of a group do not ascend.
 __global__ void k_group_bounds(const uint64_t* __restrict__ pairs, uint64_t E, uint64_t V, int shared_is_dst,
                                uint32_t* __restrict__ start, uint32_t* __restrict__ end, unsigned* __restrict__ flags)
 {
@@ -53,6 +54,7 @@ __global__ void k_group_bounds(const uint64_t* __restrict__ pairs, uint64_t E, u
         const uint64_t sp = pairs[2 * (e - 1) + sh];
         head = sp != s;
         if (sp > s) atomicOr(&flags[0], 1u);
+        if (sp == s && pairs[2 * (e - 1) + (1 - sh)] > nb) atomicOr(&flags[2], 1u);
     }
     if (e + 1 < E) tail = pairs[2 * (e + 1) + sh] != s;
     if (s < V) {
@@ -260,13 +262,13 @@ int grz_build_list(grz_graph* g, grz_list* L, const uint64_t* d_pairs, uint64_t 
         LCK(cudaGetLastError());
         L->vindex_start = L->vindex_end = 0;
     } else {
-        unsigned flags_h[2] = { 0, 0 };
+        unsigned flags_h[3] = { 0, 0, 0 };
         uint64_t ends_h[2] = { 0, 0 };
         const int sh = shared_is_dst ? 1 : 0;
-        LCK(cudaMallocAsync((void**)&flags, 2 * sizeof(unsigned), st));
+        LCK(cudaMallocAsync((void**)&flags, 3 * sizeof(unsigned), st));
         LCK(cudaMallocAsync((void**)&start, sizeof(uint32_t) * (V + 1), st));
         LCK(cudaMallocAsync((void**)&end, sizeof(uint32_t) * (V + 1), st));
-        LCK(cudaMemsetAsync(flags, 0, 2 * sizeof(unsigned), st));
+        LCK(cudaMemsetAsync(flags, 0, 3 * sizeof(unsigned), st));
         LCK(cudaMemsetAsync(start, 0, sizeof(uint32_t) * (V + 1), st));
         LCK(cudaMemsetAsync(end, 0, sizeof(uint32_t) * (V + 1), st));
         k_group_bounds<<<grid_blocks_for(E), BT, 0, st>>>(d_pairs, E, V, shared_is_dst, start, end, flags); GRZ_COUNT_LAUNCH(g);
@@ -277,6 +279,7 @@ int grz_build_list(grz_graph* g, grz_list* L, const uint64_t* d_pairs, uint64_t 
         LCK(cudaStreamSynchronize(st));
         if (flags_h[0]) { rc = grz_set_error(g, GRZ_ERR_UNSORTED, "%s list is not grouped by %s in ascending order", shared_is_dst ? "pull" : "push", shared_is_dst ? "destination" : "source"); goto done; }
         if (flags_h[1]) { rc = grz_set_error(g, GRZ_ERR_RANGE, "%s list holds a vertex ID >= V (%llu)", shared_is_dst ? "pull" : "push", (unsigned long long)V); goto done; }
+        L->ascending = !flags_h[2];
         rc = grz_build_list_from_bounds(g, L, d_pairs, E, shared_is_dst, start, end, ends_h[0], ends_h[1], run_len, g->stream, 0);
     }
 done:

@@ -722,7 +722,6 @@ __global__ void __launch_bounds__(PR_THREADS) k_seg_bounds(const uint4* __restri
     const uint4 x = __ldg(nbr + v);
     const uint32_t id[5] = { x.x, x.y, x.z, x.w, seg_next_src(nbr, (uint32_t)v, r1) };
     const uint32_t pos = 4 * ((uint32_t)v - r0);
-    if (pos == 0) start[(uint64_t)(id[0] >> bits) * (V + 1) + d] = 0;
 #pragma unroll
     for (int l = 0; l < 4; ++l) {
         if (id[l] == GRZ_INVALID_ID) break;
@@ -1122,7 +1121,7 @@ static uint32_t pr_segment_bits(const grz_graph* g, int force)
 int grz_pr_ensure_segments(grz_graph* g, int force)
 {
     const uint32_t bits = pr_segment_bits(g, force);
-    if (!bits || g->pull.nhub || !g->pull.nvec) return GRZ_OK;
+    if (!bits || g->pull.nhub || !g->pull.nvec || !g->pull.ascending) return GRZ_OK;
     return pr_build_segments(g, bits);
 }
 
@@ -1157,10 +1156,10 @@ int grz_pr_prepare(grz_graph* g)
     if (!g->pull.nhub && V) GRZ_TRY(pr_hot_choose(g));
     // Source segments (pr_segment_bits): each segment's props mostly stay in L2 while its edges
     // stream, instead of one random DRAM sector per gathered prop.  They need sources in ascending
-    // order along each destination's lanes, which hub encoding breaks.
+    // order along each destination's lanes: not a hub-encoded list, nor one that is only grouped.
     const uint32_t bits = pr_segment_bits(g, 0);
     g->pr_segmode = 0;
-    if (bits && g->pull.nhub == 0 && g->pull.nvec) {
+    if (bits && g->pull.nhub == 0 && g->pull.nvec && g->pull.ascending) {
         const int rc = pr_build_segments(g, bits);
         if (rc) return rc;
         g->pr_segmode = 1;

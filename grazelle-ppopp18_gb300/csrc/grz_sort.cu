@@ -70,18 +70,21 @@ __global__ void __launch_bounds__(ST) k_ingest(const ulonglong2* __restrict__ ch
 #pragma unroll
     for (int c = 0; c < SI; ++c) s_dst[c * ST + threadIdx.x] = p[c].y;
     __syncthreads();
-    bool bad_order = false, bad_range = false;
+    bool bad_order = false, bad_range = false, bad_minor = false;
 #pragma unroll
     for (int c = 0; c < SI; ++c) {
         const int i = c * ST + threadIdx.x;
-        if (base + i >= n) continue;
         const uint64_t e = e0 + base + i;
         const uint64_t s = p[c].x, d = p[c].y;
+        uint64_t sp = __shfl_up_sync(0xffffffffu, (unsigned long long)s, 1);  // the edge before's source
+        if (base + i >= n) continue;
+        if ((threadIdx.x & 31) == 0) sp = base + i > 0 ? chunk[base + i - 1].x : (e > 0 ? all[e - 1].x : 0ull);
         const uint64_t dp = i > 0 ? s_dst[i - 1] : (e > 0 ? dst_at(e - 1) : d);
         const uint64_t dn = i + 1 < STILE ? s_dst[i + 1] : (e + 1 < E ? dst_at(e + 1) : d);
         keys[e] = (s << 32) | (d & 0xffffffffull);
         if (s >= V || d >= V) bad_range = true;
         if (e > 0 && dp > d) bad_order = true;
+        if (e > 0 && dp == d && sp > s) bad_minor = true;
         const bool head = e == 0 || dp != d;
         const bool tail = e + 1 == E || dn != d;
         if (d < V) {
@@ -93,6 +96,7 @@ __global__ void __launch_bounds__(ST) k_ingest(const ulonglong2* __restrict__ ch
     }
     if (bad_order) atomicOr(&flags[0], 1u);
     if (bad_range) atomicOr(&flags[1], 1u);
+    if (bad_minor) atomicOr(&flags[2], 1u);
     __syncthreads();
     hist[(uint64_t)threadIdx.x * ntiles + blockIdx.x] = cnt[threadIdx.x];
 }
@@ -476,7 +480,7 @@ int grz_ingest_pull_derive(grz_graph* g, const uint64_t* pull, uint64_t E, const
     const uint64_t pcap = E / 4 + std::min<uint64_t>(V, E) + 1;
     unsigned* flags = nullptr;
     uint64_t* seg = nullptr;
-    unsigned flags_h[2] = { 0, 0 };
+    unsigned flags_h[3] = { 0, 0, 0 };
     unsigned long long kends[2] = { 0, 0 };
     uint32_t nv32 = 0;
     uint32_t qends[2] = { 0, 0 };
@@ -515,7 +519,7 @@ int grz_ingest_pull_derive(grz_graph* g, const uint64_t* pull, uint64_t E, const
     IRC(grz_dev_alloc(g, (void**)&start, sizeof(uint32_t) * (V + 1)));
     IRC(grz_dev_alloc(g, (void**)&end, sizeof(uint32_t) * (V + 1)));
     IRC(grz_dev_alloc(g, (void**)&off, sizeof(uint32_t) * (V + 1)));
-    IRC(grz_dev_alloc(g, (void**)&flags, sizeof(unsigned) * 2));
+    IRC(grz_dev_alloc(g, (void**)&flags, sizeof(unsigned) * 3));
     IRC(grz_dev_alloc(g, (void**)&heads, sizeof(uint32_t) * ntiles));
     IRC(grz_dev_alloc(g, (void**)&carry, sizeof(uint32_t) * (nchunks + 1)));
     ICK(cudaMallocAsync((void**)&P->nbr, sizeof(uint4) * pcap, st));
@@ -524,7 +528,7 @@ int grz_ingest_pull_derive(grz_graph* g, const uint64_t* pull, uint64_t E, const
     IRC(grz_alloc_outdegrees(g));  // g->degree zeroed: the running count per source
     ICK(cudaMemsetAsync(start, 0, sizeof(uint32_t) * (V + 1), st));
     ICK(cudaMemsetAsync(end, 0, sizeof(uint32_t) * (V + 1), st));
-    ICK(cudaMemsetAsync(flags, 0, sizeof(unsigned) * 2, st));
+    ICK(cudaMemsetAsync(flags, 0, sizeof(unsigned) * 3, st));
     // 2. per chunk, once it is in: the first pass, its -pull vectors, its sort by source and its
     //    edges' ranks; its slot then takes the chunk nslots further on
     for (uint64_t c = 0; c < nchunks; ++c) {
@@ -582,6 +586,7 @@ int grz_ingest_pull_derive(grz_graph* g, const uint64_t* pull, uint64_t E, const
     ICK(cudaStreamSynchronize(st));
     if (flags_h[0]) { rc = grz_set_error(g, GRZ_ERR_UNSORTED, "pull list is not grouped by destination in ascending order"); goto done; }
     if (flags_h[1]) { rc = grz_set_error(g, GRZ_ERR_RANGE, "pull list holds a vertex ID >= V (%llu)", (unsigned long long)V); goto done; }
+    P->ascending = !flags_h[2];
     Q->nvec = nv32;
     ICK(cudaMallocAsync((void**)&Q->nbr, sizeof(uint4) * Q->nvec, st));
     ICK(cudaMallocAsync((void**)&Q->shared, sizeof(uint32_t) * Q->nvec, st));

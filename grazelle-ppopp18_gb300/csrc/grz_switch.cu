@@ -22,26 +22,12 @@
 #include <algorithm>
 
 #include "grz_internal.cuh"
+#include "grz_switch.cuh"
 #include "../../include/grazelle_gb300.h"
-
-#define NF GRZ_MLP_FEATURES
-#define NH GRZ_MLP_HIDDEN
 
 namespace {
 
 constexpr int T = 256;
-// parameter layout (floats): W1[NH][NF] b1[NH] W2[NH][NH] b2[NH] W3[NH] b3
-constexpr int OFF_W1 = 0;
-constexpr int OFF_B1 = OFF_W1 + NH * NF;
-constexpr int OFF_W2 = OFF_B1 + NH;
-constexpr int OFF_B2 = OFF_W2 + NH * NH;
-constexpr int OFF_W3 = OFF_B2 + NH;
-constexpr int OFF_B3 = OFF_W3 + NH;
-constexpr int NP = OFF_B3 + 1;
-static_assert(NP == GRZ_MLP_PARAMS, "parameter count");
-
-__device__ __forceinline__ float relu(float x) { return x > 0.f ? x : 0.f; }
-
 // forward of one sample: returns the logit (pull faster) and the hidden activations
 __device__ __forceinline__ float mlp_forward(const float* p, const float* x, float* h1, float* h2)
 {
@@ -60,73 +46,9 @@ __device__ __forceinline__ float mlp_forward(const float* p, const float* x, flo
     return z;
 }
 
-// features of the state the next iteration will start from (computed before the frontier swap:
-// has_next is the next HasInfo)
-struct FeatIn {
-    const unsigned long long* frontier;
-    unsigned long long vote_override;  // ~0: read the vote slots
-    const unsigned long long* wants;
-    const unsigned long long* vote_slots;
-    uint64_t words;
-    double V, E, max_degree;
-    uint32_t iter;
-    int app_bfs;
-    int last_engine;
-};
-
 // sw_out layout (u64): [0] vote, [1] decision, [2] |frontier|, [3] |WantsInfo|, [4] block
 // ticket, then NF floats.  Words 2-4 are zero between calls.
 constexpr int SW_U64 = 5;
-
-// MLP forward pass of one sample by one warp, lane j computing hidden unit j.  Same operation
-// order as mlp_forward, so the logit equals grz_mlp_predict's.  f: NF features, h: NH scratch
-// (both shared); every lane returns the logit.
-// One warp, lane j = hidden unit j, the weights in registers: lane j loads its own rows of W1 and
-// W2 straight from global memory (all loads issued together, one L2 round trip), and the hidden
-// activations pass between lanes by shuffles.  The operation order is mlp_forward's, so the
-// logit equals grz_mlp_predict's bit for bit.
-__device__ float mlp_logit_warp(const float* __restrict__ params, const float* f, int lane)
-{
-    float w1[NF], w2[NH];
-#pragma unroll
-    for (int k = 0; k < NF; ++k) w1[k] = __ldg(params + OFF_W1 + lane * NF + k);
-#pragma unroll
-    for (int k = 0; k < NH; ++k) w2[k] = __ldg(params + OFF_W2 + lane * NH + k);
-    const float b1 = __ldg(params + OFF_B1 + lane), b2 = __ldg(params + OFF_B2 + lane);
-    const float w3 = __ldg(params + OFF_W3 + lane), b3 = __ldg(params + OFF_B3);
-    float s = b1;
-#pragma unroll
-    for (int k = 0; k < NF; ++k) s = fmaf(w1[k], f[k], s);
-    const float h1 = relu(s);
-    s = b2;
-#pragma unroll
-    for (int k = 0; k < NH; ++k) s = fmaf(w2[k], __shfl_sync(0xffffffffu, h1, k), s);
-    const float h2 = relu(s);
-    float z = b3;
-#pragma unroll
-    for (int k = 0; k < NH; ++k) z = fmaf(__shfl_sync(0xffffffffu, w3, k), __shfl_sync(0xffffffffu, h2, k), z);
-    return z;
-}
-
-// feature k of the state (lane k computes it)
-__device__ float feature(int k, const FeatIn& in, float F, float U, float vote)
-{
-    const float V = (float)in.V, E = (float)in.E;
-    switch (k) {
-    case 0: return log2f(F + 1.f) / log2f(V + 1.f);
-    case 1: return F / V;
-    case 2: return vote / E;
-    case 3: return log2f(vote + 1.f) / log2f(E + 1.f);
-    case 4: return in.app_bfs ? U / V : 0.f;
-    case 5: return (float)in.iter / 32.f;
-    case 6: return log2f(E / V + 1.f) / 8.f;
-    case 7: return log2f(V) / 32.f;
-    case 8: return log2f((float)in.max_degree + 1.f) / log2f(E + 1.f);
-    case 9: return in.app_bfs ? 1.f : 0.f;
-    case 10: return in.last_engine ? 1.f : 0.f;
-    default: return log2f(F + 1.f) / 32.f;
-    }
-}
 
 // One launch: grid-wide popcounts of the frontier bitmap and (BFS) WantsInfo; the last block
 // to finish then computes the features, the vote (sum of the vote slots) and, with one warp,
@@ -172,7 +94,7 @@ __global__ void __launch_bounds__(T) k_features_decide(FeatIn in, const float* _
     __syncwarp();
     int pull;
     if (use_mlp) {
-        pull = mlp_logit_warp(params, f, lane) > 0.f ? 1 : 0;
+        pull = mlp_logit_warp(MlpGlobal{ params }, f, lane) > 0.f ? 1 : 0;
     } else {
         pull = (double)vote > threshold ? 1 : 0;
     }
@@ -191,7 +113,7 @@ __global__ void __launch_bounds__(T) k_features_decide(FeatIn in, const float* _
 // reference's vertex phase after the pointer swap, source/phase_vertex_cc.asm:37-46).  The
 // last block: the vote (sum of the slots, which it re-zeroes), convergence (vote 0), the
 // iteration bound, the run statistics, the next engine (forced, threshold or MLP), and the
-// graph's conditional handles: hpull / hpush select the next iteration's engine body, hloop
+// graph's conditional handles: hengine selects the next iteration's body, hloop
 // keeps the WHILE node going.  `initial`: the decision before the first iteration, from the
 // starting vote; no statistics, no clearing.
 struct RunIn {
@@ -199,10 +121,12 @@ struct RunIn {
     unsigned long long* vote_slots;     // read and re-zeroed
     unsigned long long* clear_bm;       // old HasInfo (null when initial)
     int initial;
+    uint32_t* hop_list;                 // the next frontier's vertices when its vote is at most GRZ_HOP_VOTE, or null
+    int hop_pulls;                      // small pulls go to k_hop as well
 };
 
 __global__ void __launch_bounds__(T) k_run_decide(RunIn in, grz_runctl* __restrict__ ctl, cudaGraphConditionalHandle hloop,
-                                                  cudaGraphConditionalHandle hpull, cudaGraphConditionalHandle hpush)
+                                                  cudaGraphConditionalHandle hengine)
 {
     __shared__ unsigned s_pf[T / 32], s_pw[T / 32];
     __shared__ bool s_last;
@@ -210,15 +134,43 @@ __global__ void __launch_bounds__(T) k_run_decide(RunIn in, grz_runctl* __restri
     if (!in.initial && !*(volatile uint32_t*)&ctl->running) return;
     const FeatIn& fi = in.feat;
     const float* params = ctl->params;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    // The vote counts every vertex of the next frontier, so a small one means few vertices: those
+    // are listed for the kernel that runs small push iterations (the votes are complete here).
+    bool list = false;
+    if (in.hop_list) {
+        unsigned long long v = ctl->vote;
+        if (!in.initial) {
+            const volatile unsigned long long* slots = in.vote_slots;
+            v = slots[lane * GRZ_VOTE_STRIDE] + slots[(lane + 32) * GRZ_VOTE_STRIDE];
+            for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        }
+        list = v <= GRZ_HOP_VOTE;
+    }
     unsigned pf = 0, pw = 0;
-    for (uint64_t w = (uint64_t)blockIdx.x * T + threadIdx.x; w < fi.words; w += (uint64_t)gridDim.x * T) {
-        pf += __popcll(fi.frontier[w]);
-        if (fi.app_bfs) pw += __popcll(fi.wants[w]);
-        if (in.clear_bm) in.clear_bm[w] = 0ull;
+    for (uint64_t w0 = (uint64_t)blockIdx.x * T + 32 * warp; w0 < fi.words; w0 += (uint64_t)gridDim.x * T) {  // warp-uniform
+        const uint64_t w = w0 + lane;
+        unsigned long long bits = 0ull;
+        if (w < fi.words) {
+            bits = fi.frontier[w];
+            if (fi.app_bfs) pw += __popcll(fi.wants[w]);
+            if (in.clear_bm) in.clear_bm[w] = 0ull;
+        }
+        const unsigned n = __popcll(bits);
+        pf += n;
+        if (list && __any_sync(0xffffffffu, n != 0)) {
+            unsigned x = n, at = 0;
+            for (int o = 1; o < 32; o <<= 1) {
+                const unsigned y = __shfl_up_sync(0xffffffffu, x, o);
+                if (lane >= o) x += y;
+            }
+            if (lane == 31) at = atomicAdd(&ctl->hop_cnt, x);
+            at = __shfl_sync(0xffffffffu, at, 31) + x - n;
+            for (; bits && at < GRZ_HOP_VOTE; bits &= bits - 1) in.hop_list[at++] = (uint32_t)(64 * w) + (uint32_t)(__ffsll((long long)bits) - 1);
+        }
     }
     pf = __reduce_add_sync(0xffffffffu, pf);
     pw = __reduce_add_sync(0xffffffffu, pw);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if (lane == 0) { s_pf[warp] = pf; s_pw[warp] = pw; }
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -270,7 +222,7 @@ __global__ void __launch_bounds__(T) k_run_decide(RunIn in, grz_runctl* __restri
     } else if (!running) {
         pull = 0;  // the loop stops: no next engine to choose
     } else if (params) {
-        pull = mlp_logit_warp(params, f, lane) > 0.f ? 1 : 0;
+        pull = mlp_logit_warp(MlpGlobal{ params }, f, lane) > 0.f ? 1 : 0;
     } else {
         pull = (double)vote > ctl->threshold ? 1 : 0;
     }
@@ -278,7 +230,11 @@ __global__ void __launch_bounds__(T) k_run_decide(RunIn in, grz_runctl* __restri
     if (lane == 0) {
         if (!in.initial) {
             if (ran) ctl->npull += 1; else ctl->npush += 1;
+            ctl->bodies += 1;
         }
+        ctl->hop_n = *(volatile uint32_t*)&ctl->hop_cnt;
+        ctl->hop_cnt = 0;
+        ctl->unvisited = U;
         if (in.initial) ctl->t0_ns = now;
         ctl->vote = vote;
         ctl->running = running;
@@ -289,8 +245,9 @@ __global__ void __launch_bounds__(T) k_run_decide(RunIn in, grz_runctl* __restri
         ctl->cnt_f = 0ull;
         ctl->cnt_u = 0ull;
         ctl->ticket = 0ull;
-        cudaGraphSetConditional(hpull, running && pull ? 1u : 0u);
-        cudaGraphSetConditional(hpush, running && !pull ? 1u : 0u);
+        // a small iteration goes to k_hop (the listing above covers its frontier)
+        const bool hop = list && vote != 0ull && (!pull || in.hop_pulls);
+        cudaGraphSetConditional(hengine, !running ? GRZ_RUN_NONE : (hop ? GRZ_RUN_HOP : (pull ? GRZ_RUN_PULL : GRZ_RUN_PUSH)));
         cudaGraphSetConditional(hloop, running);
     }
 }
@@ -582,7 +539,7 @@ int grz_switch_decide(grz_graph* g, const unsigned long long* frontier, uint64_t
 // Launches k_run_decide on the graph's stream (called while capturing the run graph).  The
 // policy is not captured: the host writes it into the control block before each launch.
 int grz_switch_launch_run_decide(grz_graph* g, const unsigned long long* next_frontier, unsigned long long* clear_bm, int initial,
-                                 unsigned long long hloop, unsigned long long hpull, unsigned long long hpush)
+                                 unsigned long long hloop, unsigned long long hengine, int hop_pulls)
 {
     grz_frontier_state& f = g->fr;
     RunIn in;
@@ -599,8 +556,10 @@ int grz_switch_launch_run_decide(grz_graph* g, const unsigned long long* next_fr
     in.vote_slots = f.vote;
     in.clear_bm = clear_bm;
     in.initial = initial;
+    in.hop_list = f.hop_list;
+    in.hop_pulls = hop_pulls;
     const unsigned grid = (unsigned)std::min<uint64_t>((in.feat.words + T - 1) / T, (uint64_t)g->num_sms * 2);
-    k_run_decide<<<grid, T, 0, g->stream>>>(in, f.ctl, hloop, hpull, hpush);
+    k_run_decide<<<grid, T, 0, g->stream>>>(in, f.ctl, hloop, hengine);
     return grz_cuda_check(g, cudaGetLastError(), "run decision");
 }
 

@@ -1,0 +1,115 @@
+// grz_switch.cuh -- the engine decision's device code: the state's features and the MLP's forward pass
+// of one sample.  Shared by the decision kernels (grz_switch.cu) and the kernel that runs many small
+// push iterations in one launch (grz_ccbfs.cu), so that both choose alike, bit for bit.
+#pragma once
+
+#include "grz_internal.cuh"
+
+#define NF GRZ_MLP_FEATURES
+#define NH GRZ_MLP_HIDDEN
+
+namespace {
+
+// parameter layout (floats): W1[NH][NF] b1[NH] W2[NH][NH] b2[NH] W3[NH] b3
+constexpr int OFF_W1 = 0;
+constexpr int OFF_B1 = OFF_W1 + NH * NF;
+constexpr int OFF_W2 = OFF_B1 + NH;
+constexpr int OFF_B2 = OFF_W2 + NH * NH;
+constexpr int OFF_W3 = OFF_B2 + NH;
+constexpr int OFF_B3 = OFF_W3 + NH;
+constexpr int NP = OFF_B3 + 1;
+static_assert(NP == GRZ_MLP_PARAMS, "parameter count");
+
+__device__ __forceinline__ float relu(float x) { return x > 0.f ? x : 0.f; }
+
+// features of the state the next iteration will start from (computed before the frontier swap:
+// has_next is the next HasInfo)
+struct FeatIn {
+    const unsigned long long* frontier;
+    unsigned long long vote_override;  // ~0: read the vote slots
+    const unsigned long long* wants;
+    const unsigned long long* vote_slots;
+    uint64_t words;
+    double V, E, max_degree;
+    uint32_t iter;
+    int app_bfs;
+    int last_engine;
+};
+
+// MLP forward pass of one sample by one warp, lane j computing hidden unit j.  Same operation
+// order as mlp_forward, so the logit equals grz_mlp_predict's.  f: NF features, h: NH scratch
+// (both shared); every lane returns the logit.
+// One warp, lane j = hidden unit j, the weights in registers: lane j loads its own rows of W1 and
+// W2 straight from global memory (all loads issued together, one L2 round trip), and the hidden
+// activations pass between lanes by shuffles.  The operation order is mlp_forward's, so the
+// logit equals grz_mlp_predict's bit for bit.
+// Weights: from global memory, or staged in shared memory for a warp that decides again and again (lane
+// j's rows as columns: no bank conflicts).
+struct MlpGlobal {
+    const float* p;
+    __device__ __forceinline__ float w1(int lane, int k) const { return __ldg(p + OFF_W1 + lane * NF + k); }
+    __device__ __forceinline__ float w2(int lane, int k) const { return __ldg(p + OFF_W2 + lane * NH + k); }
+    __device__ __forceinline__ float rest(int off) const { return __ldg(p + off); }
+};
+constexpr int MLP_WARP_FLOATS = NP;
+struct MlpShared {
+    const float* p;
+    __device__ __forceinline__ float w1(int lane, int k) const { return p[OFF_W1 + k * NH + lane]; }
+    __device__ __forceinline__ float w2(int lane, int k) const { return p[OFF_W2 + k * NH + lane]; }
+    __device__ __forceinline__ float rest(int off) const { return p[off]; }
+};
+__device__ __forceinline__ void mlp_stage(const float* __restrict__ params, float* s, int tid, int nthreads)
+{
+    for (int i = tid; i < NP; i += nthreads) {
+        int to = i;
+        if (i < OFF_B1) to = OFF_W1 + (i % NF) * NH + i / NF;
+        else if (i >= OFF_W2 && i < OFF_B2) to = OFF_W2 + ((i - OFF_W2) % NH) * NH + (i - OFF_W2) / NH;
+        s[to] = __ldg(params + i);
+    }
+}
+
+template <typename W>
+__device__ __forceinline__ float mlp_logit_warp(const W w, const float* f, int lane)
+{
+    float w1[NF], w2[NH];
+#pragma unroll
+    for (int k = 0; k < NF; ++k) w1[k] = w.w1(lane, k);
+#pragma unroll
+    for (int k = 0; k < NH; ++k) w2[k] = w.w2(lane, k);
+    const float b1 = w.rest(OFF_B1 + lane), b2 = w.rest(OFF_B2 + lane);
+    const float w3 = w.rest(OFF_W3 + lane), b3 = w.rest(OFF_B3);
+    float s = b1;
+#pragma unroll
+    for (int k = 0; k < NF; ++k) s = fmaf(w1[k], f[k], s);
+    const float h1 = relu(s);
+    s = b2;
+#pragma unroll
+    for (int k = 0; k < NH; ++k) s = fmaf(w2[k], __shfl_sync(0xffffffffu, h1, k), s);
+    const float h2 = relu(s);
+    float z = b3;
+#pragma unroll
+    for (int k = 0; k < NH; ++k) z = fmaf(__shfl_sync(0xffffffffu, w3, k), __shfl_sync(0xffffffffu, h2, k), z);
+    return z;
+}
+
+// feature k of the state (lane k computes it)
+__device__ float feature(int k, const FeatIn& in, float F, float U, float vote)
+{
+    const float V = (float)in.V, E = (float)in.E;
+    switch (k) {
+    case 0: return log2f(F + 1.f) / log2f(V + 1.f);
+    case 1: return F / V;
+    case 2: return vote / E;
+    case 3: return log2f(vote + 1.f) / log2f(E + 1.f);
+    case 4: return in.app_bfs ? U / V : 0.f;
+    case 5: return (float)in.iter / 32.f;
+    case 6: return log2f(E / V + 1.f) / 8.f;
+    case 7: return log2f(V) / 32.f;
+    case 8: return log2f((float)in.max_degree + 1.f) / log2f(E + 1.f);
+    case 9: return in.app_bfs ? 1.f : 0.f;
+    case 10: return in.last_engine ? 1.f : 0.f;
+    default: return log2f(F + 1.f) / 32.f;
+    }
+}
+
+}  // namespace
