@@ -1595,46 +1595,54 @@ __global__ void __launch_bounds__(T) k_hop_labels(const grz_runctl* __restrict__
 // ---------------------------------------------------------------------------------------------
 // init / output
 
-// execution_initialize_vertex_prop_cc: (double)id; entry V = +inf.  Four labels per thread with one
-// 16-byte store (the array is 256-byte aligned), the last few one by one.
-__global__ void k_cc_init(uint32_t* __restrict__ label, uint64_t V)
+// The starting state of a run, in one launch: CC labels (execution_initialize_vertex_prop_cc: the ID) or
+// BFS parents and levels (INF, the root's level 0), entry V = +inf; HasInfo and WantsInfo (CC all,
+// execution_cc.c:66-73; BFS the root, and all but the root), HasInfo* empty; the words of cc_prev_min
+// (before iteration 1 every vertex counts as changed, the smallest label being 0); the vote slots; and
+// a graph run's control block (`ctl` not null).  Four vertices per thread with 16-byte stores (the
+// arrays are 256-byte aligned), the last few one by one; bitmap bits at and beyond V stay clear.
+__global__ void __launch_bounds__(T) k_frontier_init(uint32_t* __restrict__ label, uint32_t* __restrict__ level,
+                                                     unsigned long long* __restrict__ has, unsigned long long* __restrict__ wants,
+                                                     unsigned long long* __restrict__ has_next, uint64_t V, uint64_t W, int bfs, uint32_t root,
+                                                     unsigned long long* __restrict__ chg, unsigned* __restrict__ err,
+                                                     unsigned long long* __restrict__ vote, grz_runctl* __restrict__ ctl,
+                                                     const __grid_constant__ grz_runctl c)
 {
     const uint64_t q = (uint64_t)blockIdx.x * T + threadIdx.x;
     const uint64_t v = 4 * q;
-    if (v + 3 < V) {
-        reinterpret_cast<uint4*>(label)[q] = make_uint4((uint32_t)v, (uint32_t)v + 1, (uint32_t)v + 2, (uint32_t)v + 3);
-    } else {
-        for (uint64_t k = v; k <= V && k < v + 4; ++k) label[k] = k < V ? (uint32_t)k : INF;
+    if (v <= V) {
+        uint32_t a[4], b[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            a[j] = bfs || v + j >= V ? INF : (uint32_t)(v + j);
+            b[j] = v + j == root ? 0u : INF;
+        }
+        if (v + 3 <= V) {
+            reinterpret_cast<uint4*>(label)[q] = make_uint4(a[0], a[1], a[2], a[3]);
+            if (bfs) reinterpret_cast<uint4*>(level)[q] = make_uint4(b[0], b[1], b[2], b[3]);
+        } else {
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                if (v + j <= V) {
+                    label[v + j] = a[j];
+                    if (bfs) level[v + j] = b[j];
+                }
+        }
     }
-}
-
-// parent and level of entries [0, V] = INF: four of each per thread with 16-byte stores (the arrays
-// are 256-byte aligned), the last few one by one
-__global__ void k_bfs_init(uint32_t* __restrict__ parent, uint32_t* __restrict__ level, uint64_t V)
-{
-    const uint64_t q = (uint64_t)blockIdx.x * T + threadIdx.x;
-    const uint64_t v = 4 * q;
-    const uint4 inf4 = make_uint4(INF, INF, INF, INF);
-    if (v + 3 <= V) {
-        reinterpret_cast<uint4*>(parent)[q] = inf4;
-        reinterpret_cast<uint4*>(level)[q] = inf4;
-    } else {
-        for (uint64_t u = v; u <= V; ++u) { parent[u] = INF; level[u] = INF; }
+    if (q < W) {
+        const unsigned long long all = 64 * q + 64 <= V ? ~0ull : (64 * q < V ? (1ull << (V - 64 * q)) - 1ull : 0ull);
+        const unsigned long long r = bfs && q == root >> 6 ? 1ull << (root & 63) : 0ull;
+        has[q] = bfs ? r : all;
+        wants[q] = all & ~r;
+        has_next[q] = 0ull;
     }
-}
-
-// bitmaps: `all_ones` sets bits [0, V); bits at and beyond V stay clear
-__global__ void k_bitmap_init(unsigned long long* __restrict__ bm, uint64_t words, uint64_t V, int all_ones)
-{
-    const uint64_t w = (uint64_t)blockIdx.x * T + threadIdx.x;
-    if (w >= words) return;
-    unsigned long long x = 0;
-    if (all_ones) {
-        const uint64_t lo = w * 64;
-        if (lo + 64 <= V) x = ~0ull;
-        else if (lo < V) x = (1ull << (V - lo)) - 1ull;
+    if (q < GRZ_VOTE_SLOTS * GRZ_VOTE_STRIDE) vote[q] = 0ull;
+    if (q == 0) {
+        chg[0] = 0x00000000ffffffffull;
+        chg[1] = 0ull;
+        *err = 0u;
+        if (ctl) *ctl = c;
     }
-    bm[w] = x;
 }
 
 // bitmap of vertices that own at least one vector in a list: a thread per vertex, a warp per
@@ -1656,6 +1664,12 @@ __global__ void k_u32_to_double(const uint32_t* __restrict__ x, uint64_t V, doub
     if (v >= V) return;
     const uint32_t a = x[v];
     out[v] = (bfs && a == INF) ? -1.0 : (double)a;
+}
+
+__global__ void k_levels_out(const uint32_t* __restrict__ level, uint64_t V, int64_t* __restrict__ out)
+{
+    const uint64_t v = (uint64_t)blockIdx.x * T + threadIdx.x;
+    if (v < V) out[v] = level[v] == INF ? -1 : (int64_t)level[v];
 }
 
 }  // namespace
@@ -1738,7 +1752,9 @@ static VoteCfg vote_cfg(const grz_graph* g)
     return vc;
 }
 
-int grz_frontier_init(grz_graph* g, int app, int flags, uint32_t root)
+// Everything of an initialisation but the device state, which frontier_reset writes.  Leaves the
+// starting vote in fr.vote_host, for BFS without the root's out-degree.
+int grz_frontier_prepare(grz_graph* g, int app, int flags, uint32_t root)
 {
     if (!g->outdeg) return grz_set_error(g, GRZ_ERR_STATE, "no graph loaded");
     int rc = ensure_frontier_state(g);
@@ -1747,7 +1763,6 @@ int grz_frontier_init(grz_graph* g, int app, int flags, uint32_t root)
         rc = grz_pr_ensure_segments(g, 1);
         if (rc) return rc;
     }
-    const uint64_t V = g->V, W = words_of(V);
     grz_frontier_state& f = g->fr;
     f.app = app;
     f.flags = flags;
@@ -1757,43 +1772,40 @@ int grz_frontier_init(grz_graph* g, int app, int flags, uint32_t root)
     f.last_engine = 1;
     f.next_pull = 1;
     f.cc_partial = 0;
-    cudaStream_t st = g->stream;
-    GRZ_CK(g, cudaMemsetAsync(f.dev_err, 0, sizeof(unsigned), st));
+    f.vote_host = 0;
     if (app == GRZ_APP_CONNECTED_COMPONENTS) {
-        k_cc_init<<<blocks_for(V / 4 + 1), T, 0, st>>>(f.label, V); GRZ_COUNT_LAUNCH(g);
-        k_bitmap_init<<<blocks_for(W), T, 0, st>>>(f.has, W, V, 1); GRZ_COUNT_LAUNCH(g);      // HasInfo = all (execution_cc.c:66-73)
-        k_bitmap_init<<<blocks_for(W), T, 0, st>>>(f.wants, W, V, 1); GRZ_COUNT_LAUNCH(g);
-        // before iteration 1 every vertex counts as changed, the smallest label being 0 (tag 0)
-        const unsigned long long chg0[2] = { 0x00000000ffffffffull, 0ull };
-        memcpy(f.mail_chg, chg0, sizeof(chg0));
-        GRZ_CK(g, cudaMemcpyAsync(f.chg, f.mail_chg, sizeof(chg0), cudaMemcpyHostToDevice, st));
-        f.vote_host = 0;
         if (!(flags & GRZ_FLAG_WITHOUT_OUTDEG)) f.vote_host += g->E;     // execution_cc.c:106-112
-        if (!(flags & GRZ_FLAG_WITHOUT_COUNT)) f.vote_host += V;
+        if (!(flags & GRZ_FLAG_WITHOUT_COUNT)) f.vote_host += g->V;
     } else {
-        if (root >= V) return grz_set_error(g, GRZ_ERR_ARG, "root %u >= V", root);
-        k_bfs_init<<<blocks_for((V + 1) / 4 + 1), T, 0, st>>>(f.label, f.level, V); GRZ_COUNT_LAUNCH(g);
-        k_bitmap_init<<<blocks_for(W), T, 0, st>>>(f.has, W, V, 0); GRZ_COUNT_LAUNCH(g);
-        k_bitmap_init<<<blocks_for(W), T, 0, st>>>(f.wants, W, V, 1); GRZ_COUNT_LAUNCH(g);
-        const unsigned long long rbit = 1ull << (root & 63);
-        unsigned long long w0 = 0, w1 = 0;
-        GRZ_CK(g, cudaMemcpyAsync(&w1, f.wants + (root >> 6), 8, cudaMemcpyDeviceToHost, st));
-        GRZ_CK(g, cudaStreamSynchronize(st));
-        w0 = rbit;
-        w1 &= ~rbit;
-        GRZ_CK(g, cudaMemcpyAsync(f.has + (root >> 6), &w0, 8, cudaMemcpyHostToDevice, st));
-        GRZ_CK(g, cudaMemcpyAsync(f.wants + (root >> 6), &w1, 8, cudaMemcpyHostToDevice, st));
-        const uint32_t zero = 0;
-        GRZ_CK(g, cudaMemcpyAsync(f.level + root, &zero, 4, cudaMemcpyHostToDevice, st));
-        double od = 0;
-        GRZ_CK(g, cudaMemcpyAsync(&od, g->outdeg + root, 8, cudaMemcpyDeviceToHost, st));
-        GRZ_CK(g, cudaStreamSynchronize(st));
-        f.vote_host = 0;
-        if (!(flags & GRZ_FLAG_WITHOUT_OUTDEG)) f.vote_host += (uint64_t)od;  // execution_bfs.c:132-137
-        if (!(flags & GRZ_FLAG_WITHOUT_COUNT)) f.vote_host += 1;
+        if (root >= g->V) return grz_set_error(g, GRZ_ERR_ARG, "root %u >= V", root);
+        if (!(flags & GRZ_FLAG_WITHOUT_COUNT)) f.vote_host += 1;         // execution_bfs.c:132-137
     }
-    GRZ_CK(g, cudaMemsetAsync(f.has_next, 0, sizeof(unsigned long long) * W, st));
-    GRZ_CK(g, cudaGetLastError());
+    return GRZ_OK;
+}
+
+// the device state of the prepared run; `c`: also a graph run's control block
+static int frontier_reset(grz_graph* g, const grz_runctl* c)
+{
+    grz_frontier_state& f = g->fr;
+    const uint64_t V = g->V, W = words_of(V);
+    const uint64_t n = std::max<uint64_t>(std::max<uint64_t>(V / 4 + 1, W), GRZ_VOTE_SLOTS * GRZ_VOTE_STRIDE);
+    grz_runctl none;
+    memset(&none, 0, sizeof(none));
+    k_frontier_init<<<blocks_for(n), T, 0, g->stream>>>(f.label, f.level, f.has, f.wants, f.has_next, V, W, f.app == GRZ_APP_BREADTH_FIRST_SEARCH,
+                                                        f.root, f.chg, f.dev_err, f.vote, c ? f.ctl : nullptr, c ? *c : none); GRZ_COUNT_LAUNCH(g);
+    return grz_cuda_check(g, cudaGetLastError(), "k_frontier_init");
+}
+
+int grz_frontier_init(grz_graph* g, int app, int flags, uint32_t root)
+{
+    GRZ_TRY(grz_frontier_prepare(g, app, flags, root));
+    GRZ_TRY(frontier_reset(g, nullptr));
+    if (app == GRZ_APP_BREADTH_FIRST_SEARCH && !(flags & GRZ_FLAG_WITHOUT_OUTDEG)) {
+        uint32_t deg = 0;
+        GRZ_CK(g, cudaMemcpyAsync(&deg, g->degree + root, sizeof(deg), cudaMemcpyDeviceToHost, g->stream));
+        GRZ_CK(g, cudaStreamSynchronize(g->stream));
+        g->fr.vote_host += deg;
+    }
     return GRZ_OK;
 }
 
@@ -2250,13 +2262,22 @@ int grz_frontier_digest(grz_graph* g, uint64_t* out3)
     return GRZ_OK;
 }
 
-int grz_frontier_props(grz_graph* g)
+// the props (CC labels, BFS parents) as doubles, into device or mapped host memory
+int grz_frontier_props(grz_graph* g, double* out)
 {
     grz_frontier_state& f = g->fr;
     if (!grz_frontier_live(g)) return grz_set_error(g, GRZ_ERR_STATE, "no CC/BFS result for the loaded graph");
-    k_u32_to_double<<<blocks_for(g->V), T, 0, g->stream>>>(f.label, g->V, g->prop, f.app == GRZ_APP_BREADTH_FIRST_SEARCH); GRZ_COUNT_LAUNCH(g);
+    k_u32_to_double<<<blocks_for(g->V), T, 0, g->stream>>>(f.label, g->V, out, f.app == GRZ_APP_BREADTH_FIRST_SEARCH); GRZ_COUNT_LAUNCH(g);
     GRZ_CK(g, cudaGetLastError());
     return GRZ_OK;
+}
+
+// the BFS levels (-1 unreached) as int64, into device or mapped host memory
+int grz_frontier_levels(grz_graph* g, int64_t* out)
+{
+    if (!g->V) return GRZ_OK;
+    k_levels_out<<<blocks_for(g->V), T, 0, g->stream>>>(g->fr.level, g->V, out); GRZ_COUNT_LAUNCH(g);
+    return grz_cuda_check(g, cudaGetLastError(), "k_levels_out");
 }
 
 void grz_frontier_park(grz_graph* g)
@@ -2499,7 +2520,7 @@ static int build_run_graph(grz_graph* g)
     return GRZ_OK;
 }
 
-// Before grz_frontier_init: puts the HasInfo buffers back in the roles the cached graph has.
+// Before a graph run: puts the HasInfo buffers back in the roles the cached graph has.
 void grz_frontier_run_prepare(grz_graph* g)
 {
     grz_frontier_state& f = g->fr;
@@ -2509,9 +2530,10 @@ void grz_frontier_run_prepare(grz_graph* g)
     }
 }
 
-// Runs the initialised CC/BFS state to convergence with one graph launch.  *launches: kernels
-// the graph ran.
-int grz_frontier_run_graph(grz_graph* g, uint64_t* launches)
+// Runs the prepared CC/BFS state (grz_frontier_prepare) to convergence: one kernel for the starting state
+// and the control block, and one graph launch.  `started` is recorded between the two.  *launches:
+// kernels the graph ran.
+int grz_frontier_run_graph(grz_graph* g, cudaEvent_t started, uint64_t* launches)
 {
     grz_frontier_state& f = g->fr;
     if (!grz_frontier_live(g)) return grz_set_error(g, GRZ_ERR_STATE, "frontier state not initialised for the loaded graph");
@@ -2542,13 +2564,14 @@ int grz_frontier_run_graph(grz_graph* g, uint64_t* launches)
     c.level = f.iter + 1;
     c.last_engine = (uint32_t)f.last_engine;
     c.vote = f.vote_host;
+    const bool bfs = f.app == GRZ_APP_BREADTH_FIRST_SEARCH;
+    if (bfs && !(f.flags & GRZ_FLAG_WITHOUT_OUTDEG)) c.root_degree = g->degree + f.root;
     const uint64_t max_it = g->tune.run_max_iterations ? g->tune.run_max_iterations : std::min<uint64_t>(g->V + 2, 0xfffffff0ull);
     c.max_level = (uint32_t)std::min<uint64_t>(max_it + f.iter, 0xfffffff0ull);
     c.limit_ns = g->tune.run_limit_us ? (unsigned long long)g->tune.run_limit_us * 1000ull : 300ull * 1000000000ull;
     grz_switch_policy_ctl(g, &c);
-    memcpy(f.mail, &c, sizeof(c));
-    GRZ_CK(g, cudaMemcpyAsync(f.ctl, f.mail, sizeof(c), cudaMemcpyHostToDevice, g->stream));
-    GRZ_CK(g, cudaMemsetAsync(f.vote, 0, sizeof(unsigned long long) * GRZ_VOTE_SLOTS * GRZ_VOTE_STRIDE, g->stream));
+    GRZ_TRY(frontier_reset(g, &c));
+    GRZ_CK(g, cudaEventRecord(started, g->stream));
     GRZ_CK(g, cudaGraphLaunch(f.run_exec, g->stream));
     GRZ_CK(g, cudaMemcpyAsync(f.mail, f.ctl, sizeof(c), cudaMemcpyDeviceToHost, g->stream));
     GRZ_CK(g, cudaStreamSynchronize(g->stream));
@@ -2581,7 +2604,6 @@ int grz_frontier_run_graph(grz_graph* g, uint64_t* launches)
         f.has = f.has_next;
         f.has_next = t;
     }
-    const bool bfs = f.app == GRZ_APP_BREADTH_FIRST_SEARCH;
     // kernels of one pull iteration: BFS scan + visit, or (first pass,) compaction, expand, visit;
     // CC one pull launch, or one per source segment plus the whole-list one
     const uint64_t per_pull = bfs ? (g->tune.bfs_pull_scan ? 2 : (g->tune.bfs_pull_first ? 4 : 3))

@@ -447,6 +447,7 @@ struct grz_runctl {
     // the engine policy, read at run time so that one captured graph serves every policy
     const float* params;             // MLP parameters (learned policy) or null
     double threshold;                // vote threshold (E/5 or V/2)
+    const uint32_t* root_degree;     // BFS: the starting vote counts the root's out-edges (null: not)
     int32_t force;                   // 1 pull, 0 push, -1 the policy decides
     float features[GRZ_MLP_FEATURES];
     // small push iterations run in one launch (k_hop)
@@ -481,7 +482,6 @@ struct grz_frontier_state {
     uint32_t* counters;              // [1] touched count, [2] vectors and [3] vertices of the compacted list, [5] tile queue, [6], [7] gates
     unsigned long long* vote;        // GRZ_VOTE_SLOTS * GRZ_VOTE_STRIDE
     unsigned long long* chg;         // CC: smallest label written per iteration, tagged (2 words, grz_ccbfs.cu)
-    unsigned long long mail_chg[2];  // host copy of the initial chg words (outlives the async copy)
     int cc_partial;                  // a phases.h pull covered part of the list: no converged-destination skip
     unsigned* dev_err;               // set by an edge phase whose bounded wait gave up
     // engine policy
@@ -586,6 +586,7 @@ struct grz_graph {
     uint32_t max_degree;
     int max_degree_known;
     grz_frontier_state fr;
+    cudaEvent_t run_ev[2];  // around a CC/BFS run, made on first use
     grz_prof* prof;       // kernel timing (null unless enabled)
     unsigned long long nlaunch;  // kernels launched by this graph (grz_launch_count)
     grz_tuning tune;
@@ -667,13 +668,15 @@ int grz_scratch(grz_graph* g, size_t bytes, void** out);
 
 // CC / BFS (grz_ccbfs.cu)
 int grz_frontier_init(grz_graph* g, int app, int flags, uint32_t root);
+int grz_frontier_prepare(grz_graph* g, int app, int flags, uint32_t root);
 int grz_frontier_step(grz_graph* g, int engine, int* engine_out, uint64_t* vote_out);
 int grz_frontier_vertex_phase(grz_graph* g, uint64_t first, uint64_t count);
-int grz_frontier_props(grz_graph* g);
+int grz_frontier_props(grz_graph* g, double* out);
+int grz_frontier_levels(grz_graph* g, int64_t* out);
 int grz_engine_threshold(const grz_graph* g, uint64_t vote);
 int grz_read_vote(grz_graph* g, uint64_t* out);
 int grz_frontier_mail(grz_graph* g);
-int grz_frontier_run_graph(grz_graph* g, uint64_t* launches);
+int grz_frontier_run_graph(grz_graph* g, cudaEvent_t started, uint64_t* launches);
 int grz_frontier_check_waits(grz_graph* g);
 // builds the source-segmented pull lists by the size rule of grz_pr_init (grz_pr.cu); `force`:
 // also below the size threshold, with the tuned or the default segment size

@@ -815,7 +815,7 @@ __global__ void k_pr_vertex(const double* __restrict__ accum, const double* __re
 // the accumulators' clearing (a division per vertex, props also written as doubles and in fixed point
 // -> now): V = 2^26 1.94 -> 0.70 ms, 2^20 52 -> 20 us.
 __global__ void __launch_bounds__(PR_THREADS, 8) k_pr_init(const double* __restrict__ inv_deg, const uint32_t* __restrict__ degree, uint64_t V,
-                                                           double c, u128* __restrict__ prop_fx, pk_t* __restrict__ prop_pk,
+                                                           double c, double* __restrict__ accum, u128* __restrict__ prop_fx, pk_t* __restrict__ prop_pk,
                                                            const uint2* __restrict__ hotmap, pk_t* __restrict__ hot, u128* __restrict__ part0)
 {
     __shared__ u128 red[PR_THREADS / 32];
@@ -835,8 +835,10 @@ __global__ void __launch_bounds__(PR_THREADS, 8) k_pr_init(const double* __restr
             pf = fx_from_double(p);
             prop_fx[v] = pf;
         }
+        accum[v] = 0.0;
         s = u128_add(s, u128_mul32(pf, deg));
     }
+    if (blockIdx.x == 0 && threadIdx.x < 8) accum[V + threadIdx.x] = 0.0;
     s = block_reduce_u128(s, red);
     if (threadIdx.x == 0) part0[blockIdx.x] = s;
 }
@@ -1251,10 +1253,9 @@ int grz_pr_init_state(grz_graph* g, double damping)
     g->pr_pk_stale = g->pr_pk[0] && !g->pr_pkmode;
     g->pr_sum_cur = 0;
     g->pr_iters_done = 0;
-    GRZ_CK(g, cudaMemsetAsync(g->accum, 0, sizeof(double) * (g->V + 8), g->stream));
     if (g->V) {
         const unsigned grid = (unsigned)std::min<uint64_t>(blocks_for(g->V), (uint64_t)g->num_sms * 8);
-        k_pr_init<<<grid, PR_THREADS, 0, g->stream>>>(g->inv_deg, g->degree, g->V, 1.0 / (double)g->V, g->pr_fx[0],
+        k_pr_init<<<grid, PR_THREADS, 0, g->stream>>>(g->inv_deg, g->degree, g->V, 1.0 / (double)g->V, g->accum, g->pr_fx[0],
                                                       g->pr_pkmode ? g->pr_pk[0] : nullptr, g->pr_nhot ? g->pr_hotmap : nullptr,
                                                       g->pr_hot[0], g->pr_sum); GRZ_COUNT_LAUNCH(g);
         GRZ_CK(g, cudaGetLastError());
@@ -1569,14 +1570,14 @@ int grz_pr_vertex(grz_graph* g, uint64_t first, uint64_t count, double S)
     return GRZ_OK;
 }
 
-// reference-format props (double) from the current fixed-point props
-int grz_pr_props_to_double(grz_graph* g)
+// reference-format props (double) from the current fixed-point props, into device or mapped host memory
+int grz_pr_props_to_double(grz_graph* g, double* out)
 {
     if (g->V == 0) return GRZ_OK;
     if (g->pr_fx_stale) {
-        k_pk_unpack<<<blocks_for(g->V), PR_THREADS, 0, g->stream>>>(g->pr_pk[g->pr_cur], g->V, nullptr, g->prop); GRZ_COUNT_LAUNCH(g);
+        k_pk_unpack<<<blocks_for(g->V), PR_THREADS, 0, g->stream>>>(g->pr_pk[g->pr_cur], g->V, nullptr, out); GRZ_COUNT_LAUNCH(g);
     } else {
-        k_fx_to_double<<<blocks_for(g->V), PR_THREADS, 0, g->stream>>>(g->pr_fx[g->pr_cur], g->V, g->prop); GRZ_COUNT_LAUNCH(g);
+        k_fx_to_double<<<blocks_for(g->V), PR_THREADS, 0, g->stream>>>(g->pr_fx[g->pr_cur], g->V, out); GRZ_COUNT_LAUNCH(g);
     }
     GRZ_CK(g, cudaGetLastError());
     return GRZ_OK;

@@ -138,8 +138,9 @@ __global__ void __launch_bounds__(T) k_run_decide(RunIn in, grz_runctl* __restri
     // The vote counts every vertex of the next frontier, so a small one means few vertices: those
     // are listed for the kernel that runs small push iterations (the votes are complete here).
     bool list = false;
+    const unsigned long long root_edges = in.initial && ctl->root_degree ? *ctl->root_degree : 0ull;
     if (in.hop_list) {
-        unsigned long long v = ctl->vote;
+        unsigned long long v = ctl->vote + root_edges;
         if (!in.initial) {
             const volatile unsigned long long* slots = in.vote_slots;
             v = slots[lane * GRZ_VOTE_STRIDE] + slots[(lane + 32) * GRZ_VOTE_STRIDE];
@@ -186,7 +187,7 @@ __global__ void __launch_bounds__(T) k_run_decide(RunIn in, grz_runctl* __restri
     __threadfence();
     const unsigned long long F = *(volatile unsigned long long*)&ctl->cnt_f;
     const unsigned long long U = *(volatile unsigned long long*)&ctl->cnt_u;
-    unsigned long long vote = ctl->vote;  // initial: the starting vote, written by the host
+    unsigned long long vote = ctl->vote + root_edges;  // initial: the starting vote, the host's part and the root's
     if (!in.initial) {
         unsigned long long* a = in.vote_slots + lane * GRZ_VOTE_STRIDE;
         unsigned long long* b = in.vote_slots + (lane + 32) * GRZ_VOTE_STRIDE;
