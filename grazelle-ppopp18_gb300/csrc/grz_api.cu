@@ -18,9 +18,7 @@
 
 // grz_pr.cu
 int grz_pr_init_state(grz_graph* g, double damping);
-int grz_pr_fused_iteration(grz_graph* g, int write_double_props);
-int grz_pr_use_persistent(const grz_graph* g);
-int grz_pr_persistent_iterations(grz_graph* g, uint32_t iters);
+int grz_pr_iterations(grz_graph* g, uint32_t iterations);
 int grz_pr_props_to_double(grz_graph* g, double* out);
 
 int grz_set_error(grz_graph* g, int code, const char* fmt, ...)
@@ -719,12 +717,7 @@ extern "C" int grz_pr_iterate(grz_graph* g, uint32_t iterations)
     if (!g) return GRZ_ERR_ARG;
     if (!grz_pr_live(g)) return grz_set_error(g, GRZ_ERR_STATE, "grz_pr_init not called since the graph was loaded");
     GRZ_CK(g, cudaSetDevice(g->device));
-    if (grz_pr_use_persistent(g)) return grz_pr_persistent_iterations(g, iterations);
-    for (uint32_t i = 0; i < iterations; ++i) {
-        int rc = grz_pr_fused_iteration(g, 0);
-        if (rc) return rc;
-    }
-    return GRZ_OK;
+    return grz_pr_iterations(g, iterations);
 }
 
 extern "C" int grz_pr_time_iterations(grz_graph* g, uint32_t iterations, float* ms_out)
@@ -736,9 +729,7 @@ extern "C" int grz_pr_time_iterations(grz_graph* g, uint32_t iterations, float* 
     GRZ_CK(g, cudaEventCreate(&e1));
     int rc = GRZ_OK;
     cudaEventRecord(e0, g->stream);
-    if (grz_pr_use_persistent(g)) rc = grz_pr_persistent_iterations(g, iterations);
-    else
-        for (uint32_t i = 0; i < iterations && rc == GRZ_OK; ++i) rc = grz_pr_fused_iteration(g, 0);
+    rc = grz_pr_iterations(g, iterations);
     cudaEventRecord(e1, g->stream);
     if (rc == GRZ_OK) rc = grz_cuda_check(g, cudaEventSynchronize(e1), "event sync");
     if (rc == GRZ_OK) cudaEventElapsedTime(ms_out, e0, e1);

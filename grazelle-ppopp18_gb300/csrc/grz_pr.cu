@@ -25,12 +25,15 @@
 //   * The vertex formula is fma(acc, d, G*d + (1-d)/V) times a precomputed 1/deg'.  It stays
 //     within a few roundings of the reference's ((acc + G)*d + (1-d)/V) / deg': two FP64 ops
 //     per vertex instead of three plus a division, on a part whose FP64 rate is low.
+#include <cooperative_groups.h>
 #include <string.h>
 
 #include <algorithm>
 #include <vector>
 
 #include "grz_internal.cuh"
+
+namespace cg = cooperative_groups;
 
 namespace {
 
@@ -288,6 +291,50 @@ __device__ __forceinline__ u128 u128_shfl(u128 v, int src)
     return r;
 }
 
+// Sums a warp's group of vectors by destination.  k, v0..v3: the destinations and sums of the lane's four
+// consecutive vectors (GRZ_INVALID_ID past the range).  carry, ckey: the sum so far of the
+// destination that the group before left open.  after: the destination after lane `last`'s vectors,
+// the group's last ones.  put(destination, sum): a destination that ends in this group; open(...):
+// one that goes on past the range, whose last group this is (`ends`).
+template <typename Put, typename Open>
+__device__ __forceinline__ void pk_group(uint4 k, u128 v0, u128 v1, u128 v2, u128 v3, uint32_t after, bool ends, int last, u128& carry,
+                                         uint32_t& ckey, Put put, Open open)
+{
+    const int lane = threadIdx.x & 31;
+    uint32_t kp = __shfl_up_sync(0xffffffffu, k.w, 1), kn = __shfl_down_sync(0xffffffffu, k.x, 1);
+    if (lane == 0) kp = ckey;
+    if (lane == last) kn = after;
+    // the thread's vectors: the first destination's sum if it ends here (`head`), destinations that
+    // start and end here (put at once), and the last destination's sum (`cur`)
+    u128 cur = v0, head = u128_zero();
+    bool closed = false;
+    if (k.y == k.x) cur = u128_add(cur, v1);
+    else { head = cur; closed = true; cur = v1; }
+    if (k.z == k.y) cur = u128_add(cur, v2);
+    else { if (closed) put(k.y, cur); else { head = cur; closed = true; } cur = v2; }
+    if (k.w == k.z) cur = u128_add(cur, v3);
+    else { if (closed) put(k.z, cur); else { head = cur; closed = true; } cur = v3; }
+    if (lane == 0 && !closed && kp == k.x) cur = u128_add(cur, carry);
+    // segmented inclusive scan of `cur` over the threads
+    const unsigned heads = __ballot_sync(0xffffffffu, lane == 0 || closed || kp != k.x);
+    const int segstart = 31 - __clz(heads & (0xffffffffu >> (31 - lane)));
+    const int maxlen = __reduce_max_sync(0xffffffffu, (unsigned)(lane - segstart + 1));
+    for (int off = 1; off < maxlen; off <<= 1) {
+        const u128 o = u128_shfl_up(cur, off);
+        if (lane - off >= segstart) cur = u128_add(cur, o);
+    }
+    u128 before = u128_shfl_up(cur, 1);
+    if (lane == 0) before = carry;
+    if (closed) {
+        if (kp == k.x) head = u128_add(head, before);
+        put(k.x, head);
+    }
+    if (k.w != kn) put(k.w, cur);
+    carry = u128_shfl(cur, 31);
+    ckey = __shfl_sync(0xffffffffu, k.w, 31);
+    if (ends && lane == last && k.w == kn && k.w != GRZ_INVALID_ID) open(k.w, cur);
+}
+
 // The vectors [first, end) of a list whose first vector is at a multiple of 16 bytes of `dstv`.
 // `base` is `first` rounded down to a multiple of 4 (vectors before `first` count as empty), so that
 // the wide loads are aligned; ranges are [base + w * per, base + (w + 1) * per), per a multiple of 4.
@@ -386,41 +433,9 @@ __global__ void __launch_bounds__(PK_THREADS, 1) k_pr_gather_pk(const uint4* __r
             v3 = u128_add(u128_add(pk_to_fx(p[4]), pk_to_fx(p[5])), u128_add(pk_to_fx(p[6]), pk_to_fx(p[7])));
         }
         const uint32_t after = __shfl_sync(0xffffffffu, nk.x, 0);
-        uint32_t kp = __shfl_up_sync(0xffffffffu, k.w, 1), kn = __shfl_down_sync(0xffffffffu, k.x, 1);
-        if (lane == 0) kp = ckey;
         const bool ends = v + PK_GROUP >= hi;  // the range's last group: its last vectors may not fill the warp
-        const int last = ends ? (int)((hi - (uint32_t)v + 3) / 4) - 1 : 31;
-        if (lane == last) kn = after;
-        // the thread's vectors: the first destination's sum if it ends here (`head`), destinations
-        // that start and end here (stored at once), and the last destination's sum (`cur`)
-        u128 cur = v0, head = u128_zero();
-        bool closed = false;
-        if (k.y == k.x) cur = u128_add(cur, v1);
-        else { head = cur; closed = true; cur = v1; }
-        if (k.z == k.y) cur = u128_add(cur, v2);
-        else { if (closed) put(k.y, cur); else { head = cur; closed = true; } cur = v2; }
-        if (k.w == k.z) cur = u128_add(cur, v3);
-        else { if (closed) put(k.z, cur); else { head = cur; closed = true; } cur = v3; }
-        if (lane == 0 && !closed && kp == k.x) cur = u128_add(cur, carry);
-        // segmented inclusive scan of `cur` over the threads
-        const unsigned heads = __ballot_sync(0xffffffffu, lane == 0 || closed || kp != k.x);
-        const int segstart = 31 - __clz(heads & (0xffffffffu >> (31 - lane)));
-        const int maxlen = __reduce_max_sync(0xffffffffu, (unsigned)(lane - segstart + 1));
-        for (int off = 1; off < maxlen; off <<= 1) {
-            const u128 o = u128_shfl_up(cur, off);
-            if (lane - off >= segstart) cur = u128_add(cur, o);
-        }
-        u128 before = u128_shfl_up(cur, 1);
-        if (lane == 0) before = carry;
-        if (closed) {
-            if (kp == k.x) head = u128_add(head, before);
-            put(k.x, head);
-        }
-        if (k.w != kn) put(k.w, cur);
-        carry = u128_shfl(cur, 31);
-        ckey = __shfl_sync(0xffffffffu, k.w, 31);
-        // the destination goes on in the next range
-        if (ends && lane == last && k.w == kn && k.w != GRZ_INVALID_ID) u128_atomic_add(rowacc + k.w, cur);
+        pk_group(k, v0, v1, v2, v3, after, ends, ends ? (int)((hi - (uint32_t)v + 3) / 4) - 1 : 31, carry, ckey, put,
+                 [&](uint32_t key, u128 x) { u128_atomic_add(rowacc + key, x); });
     }
 }
 
@@ -668,6 +683,169 @@ __global__ void __launch_bounds__(PR_THREADS, MINB) k_pr_persistent(const PRPers
         sc ^= 1;
         nparts = nb;
     }
+}
+
+// ---------------------------------------------------------------------------------------------
+// All iterations of a small graph in one launch.
+//
+// Two kernels per iteration cost about 10 us in starts however small the graph.  Here one cluster of 16
+// blocks runs every iteration.  Each block owns a range of vertices (an even share of vectors and
+// vertices) with their vectors, and holds a copy of all packed props in shared memory, so a gather is
+// a shared-memory read.  It sums its vectors as k_pr_gather_pk does, computes its vertices' new props
+// and writes them into every block's copy of the next iteration's props, with its part of the next S;
+// one cluster barrier ends the iteration.  Sums and formulas are those of the two kernels, bit for bit.
+// Bounds: V at most PS_MAX_V (two copies of the props, 128 KB) and PS_MAX_VEC vectors; a block's vectors
+// past PS_CAP, when a few destinations hold most of the list, are read from memory each time.  GB300,
+// R-MAT of 4096 vertices and 61k edges, 16 iterations: SMALLUS.
+constexpr int PS_CTAS = 16;
+constexpr int PS_T = 512;
+constexpr uint32_t PS_MAX_V = 8192;
+constexpr uint32_t PS_MAX_VEC = 49152;
+constexpr uint32_t PS_CAP = PS_MAX_VEC / 8;      // vectors a block keeps in shared memory (10 bytes each)
+constexpr uint32_t PS_ACC = PS_MAX_V / 8 + 32;   // its accumulators
+
+struct PRSmall {
+    const uint4* nbr;
+    const uint32_t* rowptr;
+    uint32_t V, nvec;
+    const double* inv_deg;
+    const uint32_t* degree;
+    const pk_t* props;       // in: V + 1 (the last one zero)
+    pk_t* props_out;
+    const u128* part_in;     // partials of S
+    uint32_t nparts;
+    u128* part_out;          // the last S
+    double damping, c, nverts;
+    uint32_t iters;
+};
+
+constexpr size_t ps_smem(uint32_t V) { return sizeof(pk_t) * 2 * (V + 2) + sizeof(u128) * PS_ACC + (sizeof(ushort4) + sizeof(uint16_t)) * PS_CAP; }
+
+__global__ void __cluster_dims__(PS_CTAS, 1, 1) __launch_bounds__(PS_T, 1) k_pr_small(const PRSmall q)
+{
+    extern __shared__ __align__(16) unsigned char s_raw[];
+    __shared__ u128 s_red[PS_T / 32], s_part[2][PS_CTAS];
+    __shared__ uint32_t s_v[2];
+    cg::cluster_group cl = cg::this_cluster();
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const uint32_t rank = cl.block_rank(), V = q.V;
+    u128* const s_acc = reinterpret_cast<u128*>(s_raw);
+    pk_t* const s_prop = reinterpret_cast<pk_t*>(s_raw + sizeof(u128) * PS_ACC);
+    const uint32_t pstride = V + 2;  // entry V is zero: empty lanes gather it
+    ushort4* const s_vec = reinterpret_cast<ushort4*>(s_prop + 2 * pstride);
+    uint16_t* const s_dst = reinterpret_cast<uint16_t*>(s_vec + PS_CAP);
+    // This block's vertices: those whose weight, rowptr[v] * V + v * nvec, lies in its share.  All vectors
+    // together weigh as much as all vertices, so a block has at most twice an even share of either
+    // (and the vectors of its last destination).
+    if (tid < 2) {
+        const uint64_t total = 2ull * q.nvec * V, want = total * (rank + tid) / PS_CTAS;
+        uint32_t lo = 0, hi = V;
+        while (lo < hi) {
+            const uint32_t mid = (lo + hi) / 2;
+            if ((uint64_t)__ldg(q.rowptr + mid) * V + (uint64_t)mid * q.nvec < want) lo = mid + 1; else hi = mid;
+        }
+        s_v[tid] = rank + tid == PS_CTAS ? V : lo;
+    }
+    for (uint32_t i = tid; i < V; i += PS_T) s_prop[i] = q.props[i];
+    if (tid < 4) s_prop[(tid & 1) * pstride + V + (tid >> 1)] = 0ull;
+    for (uint32_t i = tid; i < PS_ACC; i += PS_T) s_acc[i] = u128_zero();
+    __syncthreads();
+    const uint32_t v0 = s_v[0], nv = s_v[1] - v0;
+    const uint32_t r0 = __ldg(q.rowptr + v0), m = __ldg(q.rowptr + v0 + nv) - r0;
+    auto id16 = [&](uint32_t id) { return (unsigned short)min(id, V); };
+    for (uint32_t i = tid; i < min(m, PS_CAP); i += PS_T) {
+        const uint4 x = __ldg(q.nbr + r0 + i);
+        s_vec[i] = make_ushort4(id16(x.x), id16(x.y), id16(x.z), id16(x.w));
+    }
+    for (uint32_t i = tid; i < nv; i += PS_T)
+        for (uint32_t r = __ldg(q.rowptr + v0 + i) - r0, e = __ldg(q.rowptr + v0 + i + 1) - r0; r < e && r < PS_CAP; ++r) s_dst[r] = (uint16_t)i;
+    // destination (from v0) of vector i past the kept ones
+    auto dst_of = [&](uint32_t i) -> uint32_t {
+        if (i < PS_CAP) return s_dst[i];
+        uint32_t lo = 0, hi = nv - 1;  // last vertex whose vectors start at or before i
+        while (lo < hi) {
+            const uint32_t mid = (lo + hi + 1) / 2;
+            if (__ldg(q.rowptr + v0 + mid) - r0 <= i) lo = mid; else hi = mid - 1;
+        }
+        return lo;
+    };
+    // S of the first iteration, summed by every block
+    u128 S = u128_zero();
+    for (uint32_t b = lane; b < q.nparts; b += 32) S = u128_add(S, q.part_in[b]);
+    for (int o = 16; o > 0; o >>= 1) S = u128_add(S, u128_shfl_down(S, o));
+    S = u128_shfl(S, 0);
+    cl.sync();
+    const uint32_t per = ((m + PS_T / 32 - 1) / (PS_T / 32) + 3) & ~3u;
+    const uint32_t lo = min(m, warp * per), hi = min(m, lo + per);
+    const uint32_t kbefore = lo > 0 && lo < hi ? dst_of(lo - 1) : GRZ_INVALID_ID - 1;
+    const uint32_t after = hi < m ? dst_of(hi) : GRZ_INVALID_ID;
+    for (uint32_t it = 0; it < q.iters; ++it) {
+        const pk_t* prop = s_prop + (it & 1) * pstride;
+        const uint32_t next = ((it & 1) ^ 1) * pstride;
+        const double K = __fma_rn((1.0 - fx_to_double(S)) / q.nverts, q.damping, q.c);
+        // gather
+        u128 carry = u128_zero();
+        uint32_t ckey = GRZ_INVALID_ID - 1;
+        auto put = [&](uint32_t key, u128 x) {
+            if (key == GRZ_INVALID_ID) return;
+            if (key != kbefore) s_acc[key] = x;
+            else u128_atomic_add(s_acc + key, x);
+        };
+        for (uint32_t v = lo; v < hi; v += PK_GROUP) {  // warp-uniform
+            uint32_t k[4];
+            u128 x[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const uint32_t i = v + 4 * lane + j;
+                k[j] = GRZ_INVALID_ID;
+                x[j] = u128_zero();
+                if (i < hi) {
+                    k[j] = dst_of(i);
+                    ushort4 s;
+                    if (i < PS_CAP) {
+                        s = s_vec[i];
+                    } else {
+                        const uint4 y = __ldg(q.nbr + r0 + i);
+                        s = make_ushort4(id16(y.x), id16(y.y), id16(y.z), id16(y.w));
+                    }
+                    x[j] = u128_add(u128_add(pk_to_fx(prop[s.x]), pk_to_fx(prop[s.y])), u128_add(pk_to_fx(prop[s.z]), pk_to_fx(prop[s.w])));
+                }
+            }
+            const bool ends = v + PK_GROUP >= hi;
+            uint32_t next_key = after;
+            if (!ends) next_key = dst_of(v + PK_GROUP);
+            pk_group(make_uint4(k[0], k[1], k[2], k[3]), x[0], x[1], x[2], x[3], next_key, ends, ends ? (int)((hi - v + 3) / 4) - 1 : 31, carry, ckey,
+                     put, [&](uint32_t key, u128 y) { u128_atomic_add(s_acc + key, y); });
+        }
+        __syncthreads();
+        // apply, to every block's copy
+        u128 s = u128_zero();
+        for (uint32_t i = tid; i < nv; i += PS_T) {
+            const u128 a = s_acc[i];
+            s_acc[i] = u128_zero();
+            const double p = __dmul_rn(__fma_rn(fx_to_double(a), q.damping, K), __ldg(q.inv_deg + v0 + i));
+            const pk_t w = pk_from_double(p);
+#pragma unroll
+            for (int r = 0; r < PS_CTAS; ++r) *cl.map_shared_rank(s_prop + next + v0 + i, r) = w;
+            s = u128_add(s, u128_mul32(pk_to_fx(w), __ldg(q.degree + v0 + i)));
+        }
+        for (int o = 16; o > 0; o >>= 1) s = u128_add(s, u128_shfl_down(s, o));
+        if (lane == 0) s_red[warp] = s;
+        __syncthreads();
+        if (warp == 0) {
+            s = lane < PS_T / 32 ? s_red[lane] : u128_zero();
+            for (int o = 8; o > 0; o >>= 1) s = u128_add(s, u128_shfl_down(s, o));
+            s = u128_shfl(s, 0);
+            if (lane < PS_CTAS) *cl.map_shared_rank(&s_part[it & 1][rank], lane) = s;
+        }
+        cl.sync();
+        S = lane < PS_CTAS ? s_part[it & 1][lane] : u128_zero();
+        for (int o = 8; o > 0; o >>= 1) S = u128_add(S, u128_shfl_down(S, o));
+        S = u128_shfl(S, 0);
+    }
+    const pk_t* prop = s_prop + (q.iters & 1) * pstride;
+    for (uint32_t i = tid; i < nv; i += PS_T) q.props_out[v0 + i] = prop[v0 + i];
+    if (tid == 0 && rank == 0) *q.part_out = S;
 }
 
 // bit j of word t: vertex 32t + j has pull vectors in two or more of the gather's ranges of `per`
@@ -1529,6 +1707,60 @@ int grz_pr_persistent_iterations(grz_graph* g, uint32_t iters)
     }
     g->pr_rowacc_stale = 1;
     g->pr_iters_done += iters;
+    return GRZ_OK;
+}
+
+// Whether a graph's iterations run in one cluster (k_pr_small): packed props of a small graph, unless a
+// form or grid of the two kernels is asked for, or their times.
+static bool pr_use_small(const grz_graph* g)
+{
+    return g->pr_pkmode && !g->pr_segmode && !g->pull.nhub && !g->pr_nhot && g->tune.pr_persistent == 0 && g->tune.pr_grid == 0 &&
+           !(g->prof && g->prof->on) && g->V && g->V <= PS_MAX_V && g->pull.nvec <= PS_MAX_VEC;
+}
+
+static int pr_small_iterations(grz_graph* g, uint32_t iters)
+{
+    static bool configured[64] = {};
+    if (g->device < 0 || g->device >= 64 || !configured[g->device]) {
+        GRZ_CK(g, cudaFuncSetAttribute(k_pr_small, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+        GRZ_CK(g, cudaFuncSetAttribute(k_pr_small, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ps_smem(PS_MAX_V)));
+        if (g->device >= 0 && g->device < 64) configured[g->device] = true;
+    }
+    GRZ_TRY(pr_sync_pk(g));
+    const uint32_t stride = blocks_for(g->V) + 1;
+    const int k = g->pr_sum_cur, cur = g->pr_cur ^ (int)(iters & 1);
+    PRSmall q;
+    q.nbr = g->pull.nbr;
+    q.rowptr = g->pull.rowptr;
+    q.V = (uint32_t)g->V;
+    q.nvec = (uint32_t)g->pull.nvec;
+    q.inv_deg = g->inv_deg;
+    q.degree = g->degree;
+    q.props = g->pr_pk[g->pr_cur];
+    q.props_out = g->pr_pk[cur];
+    q.part_in = g->pr_sum + (size_t)k * stride;
+    q.nparts = g->pr_nparts[k];
+    q.part_out = g->pr_sum + (size_t)(k ^ 1) * stride;
+    q.damping = g->pr_damping;
+    q.nverts = (double)g->V;
+    q.c = (1.0 - g->pr_damping) / q.nverts;
+    q.iters = iters;
+    k_pr_small<<<PS_CTAS, PS_T, ps_smem((uint32_t)g->V), g->stream>>>(q); GRZ_COUNT_LAUNCH(g);
+    GRZ_CK(g, cudaGetLastError());
+    g->pr_cur = cur;
+    g->pr_sum_cur = k ^ 1;
+    g->pr_nparts[k ^ 1] = 1;
+    g->pr_fx_stale = 1;
+    g->pr_iters_done += iters;
+    return GRZ_OK;
+}
+
+// `iterations` PageRank iterations in the form that suits the graph
+int grz_pr_iterations(grz_graph* g, uint32_t iterations)
+{
+    if (grz_pr_use_persistent(g)) return grz_pr_persistent_iterations(g, iterations);
+    if (iterations && pr_use_small(g)) return pr_small_iterations(g, iterations);
+    for (uint32_t i = 0; i < iterations; ++i) GRZ_TRY(grz_pr_fused_iteration(g, 0));
     return GRZ_OK;
 }
 

@@ -103,3 +103,48 @@ def test_segments_follow_the_hot_choice():
         p = G.pagerank(6, damping=0.85)
         np.testing.assert_array_equal(G.connected_components(), lab)
     np.testing.assert_array_equal(p, pagerank(g, pr_props=1, pr_segment_bits=1))
+
+
+@pytest.mark.parametrize("V,degree", [(1, 0), (2, 1), (15, 2), (16, 3), (33, 0.5), (1000, 4), (4096, 16), (8191, 5), (8192, 20), (8193, 5)])
+def test_small_graphs_in_one_launch(V, degree):
+    """Graphs small enough for the one-cluster form, and just too large: the same props after any split
+    of the iterations, with the two-kernel form in between, and as the general gather."""
+    from grazelle import graphgen as gg
+    from grazelle.engine import Graph
+    if degree and V > 2:
+        g = gg.erdos_renyi(V, degree, seed=V)
+    else:
+        g = gg.EdgeList(V, np.arange(V - 1, dtype=np.uint64)[:degree], np.arange(1, V, dtype=np.uint64)[:degree])
+    ref = pagerank(g, 7, pr_props=1)
+    with Graph(0) as G:
+        G.load_pairs(V, g.pull_order().pairs())
+        for split in ((7,), (1, 6), (2, 5), (3, 1, 3)):
+            G.pr_init(0.85)
+            for n in split:
+                G.pr_iterate(n)
+            np.testing.assert_array_equal(G.props(), ref, err_msg=str(split))
+        G.pr_init(0.85).pr_iterate(3)
+        G.tune(pr_persistent=1)
+        G.pr_iterate(2)
+        G.tune(pr_persistent=0)
+        G.pr_iterate(2)
+        np.testing.assert_array_equal(G.props(), ref)
+        G.load_pairs(V, g.pull_order().pairs())
+        np.testing.assert_array_equal(G.pagerank(7, damping=0.85), ref)
+
+
+@pytest.mark.parametrize("hub_edges", [600, 4000, 8000])
+def test_small_graph_with_most_edges_at_few_destinations(hub_edges):
+    """Destinations whose vectors outgrow a block's share, and its shared memory."""
+    from grazelle import graphgen as gg
+    V = 8100
+    rng = np.random.RandomState(3)
+    src, dst = [], []
+    for hub in (5, 6, 7, 8, 4000, 8099):
+        s = rng.permutation(V - 1)[:hub_edges]
+        src.append(s + (s >= hub))
+        dst.append(np.full(hub_edges, hub))
+    src.append(np.arange(20))
+    dst.append(np.arange(20) + 100)
+    g = gg.EdgeList(V, np.concatenate(src).astype(np.uint64), np.concatenate(dst).astype(np.uint64))
+    np.testing.assert_array_equal(pagerank(g, 9), pagerank(g, 9, pr_props=1))
