@@ -322,6 +322,7 @@ extern "C" void grz_graph_destroy(grz_graph* g)
     if (g->stats_dev) cudaFree(g->stats_dev);
     if (g->prof_work) cudaFree(g->prof_work);
     if (g->pr_bar) cudaFree(g->pr_bar);
+    if (g->pr_small_parts) cudaFree(g->pr_small_parts);
     if (g->pr_bar_host) cudaFreeHost(g->pr_bar_host);
     if (g->copy_stream) {
         cudaStreamDestroy(g->copy_stream);

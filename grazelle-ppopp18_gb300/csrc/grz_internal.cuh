@@ -551,6 +551,7 @@ struct grz_graph {
     uint32_t seg_nhot;    // hot sources encoded
     uint32_t seg_gen;     // builds so far (a captured run names one of them)
     int pr_segmode;       // fused iterations gather segment by segment
+    u128* pr_small_parts; // parts of S of the blocks that run a small graph's iterations
     void* pr_bar;         // grid barrier and phase timer of the persistent PageRank kernel (device)
     void* pr_bar_host;    // pinned read-back of its error word and phase times
     unsigned long long* pr_pk[2];  // u64[V+1]: the props packed (pk_to_fx), gathered instead of pr_fx in pr_pkmode

@@ -691,106 +691,128 @@ __global__ void __launch_bounds__(PR_THREADS, MINB) k_pr_persistent(const PRPers
 // Two kernels per iteration cost about 10 us in starts however small the graph.  Here one cluster of 16
 // blocks runs every iteration.  Each block owns a range of vertices (an even share of vectors and
 // vertices) with their vectors, and holds a copy of all packed props in shared memory, so a gather is
-// a shared-memory read.  It sums its vectors as k_pr_gather_pk does, computes its vertices' new props
-// and writes them into every block's copy of the next iteration's props, with its part of the next S;
-// one cluster barrier ends the iteration.  Sums and formulas are those of the two kernels, bit for bit.
-// Bounds: V at most PS_MAX_V (two copies of the props, 128 KB) and PS_MAX_VEC vectors; a block's vectors
-// past PS_CAP, when a few destinations hold most of the list, are read from memory each time.  GB300,
-// R-MAT of 4096 vertices and 61k edges, 16 iterations: SMALLUS.
+// a shared-memory read.  It sums its vectors as k_pr_gather_pk does, a contiguous range per warp; the
+// destinations cut by the ranges are pieced together by the thread that owns the vertex, which knows
+// the pieces from the start (no atomics: a 64-bit one on shared memory is a loop).  It writes its
+// vertices' new props and its part of the next S to memory; one cluster barrier ends the iteration,
+// and every block copies all new props, which is 1900 clocks for 32 KB.  (Writing them into the other
+// blocks' shared memory instead took 4800: it moves 7 bytes per clock.)  Sums and formulas are those
+// of the two kernels, bit for bit.  A block's vectors past PS_CAP, when a few destinations hold most of
+// the list, are read from memory each time.  The bounds (PS_MAX_V, PS_MAX_VEC) lie where the two kernels
+// overtake it.  GB300, us per iteration (16 in a launch), two kernels / this: 1000 vertices and 20k edges
+// 6.2 / 4.6, R-MAT of 4096 and 53k 7.3 / 5.3, of 4096 and 65k 7.2 / 6.9, uniform 6000 and 72k 6.9 / 5.9;
+// past the bounds, uniform 8192 and 49k 5.8 / 6.0, R-MAT of 8192 and 111k 6.5 / 7.8, 12000 and 48k 5.9 / 6.8.
 constexpr int PS_CTAS = 16;
 constexpr int PS_T = 512;
-constexpr uint32_t PS_MAX_V = 8192;
-constexpr uint32_t PS_MAX_VEC = 49152;
-constexpr uint32_t PS_CAP = PS_MAX_VEC / 8;      // vectors a block keeps in shared memory (10 bytes each)
-constexpr uint32_t PS_ACC = PS_MAX_V / 8 + 32;   // its accumulators
+constexpr int PS_WARPS = PS_T / 32;
+constexpr uint32_t PS_MAX_V = 6144;
+constexpr uint32_t PS_MAX_VEC = 24576;
+constexpr uint32_t PS_CAP = PS_MAX_VEC / 8;  // vectors a block keeps in shared memory: twice an even share
+// a block's vertices: at most twice an even share, PS_OWN per thread
+constexpr uint32_t PS_ACC = PS_MAX_V / 8 + 32;
+constexpr int PS_OWN = (PS_ACC + PS_T - 1) / PS_T;
 
 struct PRSmall {
     const uint4* nbr;
+    const uint32_t* dstv;
     const uint32_t* rowptr;
     uint32_t V, nvec;
     const double* inv_deg;
     const uint32_t* degree;
-    const pk_t* props;       // in: V + 1 (the last one zero)
-    pk_t* props_out;
+    pk_t* props0;            // in; after an even number of iterations, out (entry V is zero)
+    pk_t* props1;            // after an odd number
     const u128* part_in;     // partials of S
     uint32_t nparts;
+    u128* parts;             // [2][PS_CTAS]: each block's part of S, by iteration parity
     u128* part_out;          // the last S
     double damping, c, nverts;
     uint32_t iters;
 };
 
-constexpr size_t ps_smem(uint32_t V) { return sizeof(pk_t) * 2 * (V + 2) + sizeof(u128) * PS_ACC + (sizeof(ushort4) + sizeof(uint16_t)) * PS_CAP; }
+constexpr size_t ps_smem(uint32_t V)
+{
+    return sizeof(u128) * PS_ACC + sizeof(pk_t) * ((V + 2) & ~1u) + (sizeof(ushort4) + sizeof(uint16_t)) * PS_CAP;
+}
 
 __global__ void __cluster_dims__(PS_CTAS, 1, 1) __launch_bounds__(PS_T, 1) k_pr_small(const PRSmall q)
 {
     extern __shared__ __align__(16) unsigned char s_raw[];
-    __shared__ u128 s_red[PS_T / 32], s_part[2][PS_CTAS];
-    __shared__ uint32_t s_v[2];
+    __shared__ u128 s_red[PS_WARPS], s_piece[2 * PS_WARPS];
+    __shared__ uint32_t s_v[2], s_cut[2 * PS_WARPS];
+    __shared__ double s_K;
     cg::cluster_group cl = cg::this_cluster();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t rank = cl.block_rank(), V = q.V;
     u128* const s_acc = reinterpret_cast<u128*>(s_raw);
     pk_t* const s_prop = reinterpret_cast<pk_t*>(s_raw + sizeof(u128) * PS_ACC);
-    const uint32_t pstride = V + 2;  // entry V is zero: empty lanes gather it
-    ushort4* const s_vec = reinterpret_cast<ushort4*>(s_prop + 2 * pstride);
+    ushort4* const s_vec = reinterpret_cast<ushort4*>(s_prop + ((V + 2) & ~1u));
     uint16_t* const s_dst = reinterpret_cast<uint16_t*>(s_vec + PS_CAP);
     // This block's vertices: those whose weight, rowptr[v] * V + v * nvec, lies in its share.  All vectors
     // together weigh as much as all vertices, so a block has at most twice an even share of either
-    // (and the vectors of its last destination).
-    if (tid < 2) {
-        const uint64_t total = 2ull * q.nvec * V, want = total * (rank + tid) / PS_CTAS;
-        uint32_t lo = 0, hi = V;
-        while (lo < hi) {
-            const uint32_t mid = (lo + hi) / 2;
-            if ((uint64_t)__ldg(q.rowptr + mid) * V + (uint64_t)mid * q.nvec < want) lo = mid + 1; else hi = mid;
+    // (and the vectors of its last destination).  The first vertex at or past each end, by all threads.
+    const uint64_t total = 2ull * q.nvec * V;
+    if (tid < 2) s_v[tid] = V;
+    __syncthreads();
+    for (uint32_t v = tid; v < V; v += PS_T) {
+        const uint64_t w = (uint64_t)__ldg(q.rowptr + v) * V + (uint64_t)v * q.nvec;
+        const uint64_t before = v ? (uint64_t)__ldg(q.rowptr + v - 1) * V + (uint64_t)(v - 1) * q.nvec : 0;
+#pragma unroll
+        for (uint32_t e = 0; e < 2; ++e) {
+            const uint64_t want = total * (rank + e) / PS_CTAS;
+            if (rank + e < PS_CTAS && w >= want && (v == 0 || before < want)) s_v[e] = v;
         }
-        s_v[tid] = rank + tid == PS_CTAS ? V : lo;
+        s_prop[v] = q.props0[v];
     }
-    for (uint32_t i = tid; i < V; i += PS_T) s_prop[i] = q.props[i];
-    if (tid < 4) s_prop[(tid & 1) * pstride + V + (tid >> 1)] = 0ull;
+    if (tid == 0) s_prop[V] = 0ull;  // empty lanes gather it
     for (uint32_t i = tid; i < PS_ACC; i += PS_T) s_acc[i] = u128_zero();
+    if (tid < 2 * PS_WARPS) s_cut[tid] = GRZ_INVALID_ID;
     __syncthreads();
     const uint32_t v0 = s_v[0], nv = s_v[1] - v0;
     const uint32_t r0 = __ldg(q.rowptr + v0), m = __ldg(q.rowptr + v0 + nv) - r0;
-    auto id16 = [&](uint32_t id) { return (unsigned short)min(id, V); };
-    for (uint32_t i = tid; i < min(m, PS_CAP); i += PS_T) {
+    auto vec_of = [&](uint32_t i) -> ushort4 {
         const uint4 x = __ldg(q.nbr + r0 + i);
-        s_vec[i] = make_ushort4(id16(x.x), id16(x.y), id16(x.z), id16(x.w));
-    }
-    for (uint32_t i = tid; i < nv; i += PS_T)
-        for (uint32_t r = __ldg(q.rowptr + v0 + i) - r0, e = __ldg(q.rowptr + v0 + i + 1) - r0; r < e && r < PS_CAP; ++r) s_dst[r] = (uint16_t)i;
-    // destination (from v0) of vector i past the kept ones
-    auto dst_of = [&](uint32_t i) -> uint32_t {
-        if (i < PS_CAP) return s_dst[i];
-        uint32_t lo = 0, hi = nv - 1;  // last vertex whose vectors start at or before i
-        while (lo < hi) {
-            const uint32_t mid = (lo + hi + 1) / 2;
-            if (__ldg(q.rowptr + v0 + mid) - r0 <= i) lo = mid; else hi = mid - 1;
-        }
-        return lo;
+        return make_ushort4((unsigned short)min(x.x, V), (unsigned short)min(x.y, V), (unsigned short)min(x.z, V), (unsigned short)min(x.w, V));
     };
-    // S of the first iteration, summed by every block
+    for (uint32_t i = tid; i < min(m, PS_CAP); i += PS_T) {
+        s_vec[i] = vec_of(i);
+        s_dst[i] = (uint16_t)(__ldg(q.dstv + r0 + i) - v0);
+    }
+    // S of the first iteration, summed by every warp
     u128 S = u128_zero();
     for (uint32_t b = lane; b < q.nparts; b += 32) S = u128_add(S, q.part_in[b]);
     for (int o = 16; o > 0; o >>= 1) S = u128_add(S, u128_shfl_down(S, o));
     S = u128_shfl(S, 0);
-    cl.sync();
-    const uint32_t per = ((m + PS_T / 32 - 1) / (PS_T / 32) + 3) & ~3u;
+    __syncthreads();
+    auto dst_of = [&](uint32_t i) -> uint32_t { return i < PS_CAP ? s_dst[i] : __ldg(q.dstv + r0 + i) - v0; };
+    const uint32_t per = ((m + PS_WARPS - 1) / PS_WARPS + 3) & ~3u;
     const uint32_t lo = min(m, warp * per), hi = min(m, lo + per);
+    // the destinations cut by the start and the end of the warp's range: their pieces are s_piece[warp]
+    // and s_piece[PS_WARPS + warp] (one that fills the whole range is a piece at the end)
     const uint32_t kbefore = lo > 0 && lo < hi ? dst_of(lo - 1) : GRZ_INVALID_ID - 1;
-    const uint32_t after = hi < m ? dst_of(hi) : GRZ_INVALID_ID;
+    const uint32_t after = lo < hi && hi < m ? dst_of(hi) : GRZ_INVALID_ID;
+    if (lane == 0 && lo < hi) {
+        const uint32_t first = dst_of(lo), last = dst_of(hi - 1);
+        if (last == after) s_cut[PS_WARPS + warp] = last;
+        if (first == kbefore && !(first == last && last == after)) s_cut[warp] = first;
+    }
+    __syncthreads();
+    // of each vertex this thread owns: its pieces, 1/deg' and degree (a cluster barrier empties L1)
+    uint32_t pieces[PS_OWN], deg[PS_OWN];
+    double inv[PS_OWN];
+#pragma unroll
+    for (int j = 0; j < PS_OWN; ++j) {
+        const uint32_t i = tid + j * PS_T;
+        inv[j] = i < nv ? __ldg(q.inv_deg + v0 + i) : 0.0;
+        deg[j] = i < nv ? __ldg(q.degree + v0 + i) : 0u;
+        pieces[j] = 0;
+        for (int k = 0; k < 2 * PS_WARPS; ++k)
+            if (s_cut[k] == (uint32_t)(tid + j * PS_T)) pieces[j] |= 1u << k;
+    }
     for (uint32_t it = 0; it < q.iters; ++it) {
-        const pk_t* prop = s_prop + (it & 1) * pstride;
-        const uint32_t next = ((it & 1) ^ 1) * pstride;
-        const double K = __fma_rn((1.0 - fx_to_double(S)) / q.nverts, q.damping, q.c);
-        // gather
+        // one thread: 512 FP64 divisions would take 3500 clocks of the SM's two FP64 lanes
+        if (tid == PS_T - 1) s_K = __fma_rn((1.0 - fx_to_double(S)) / q.nverts, q.damping, q.c);
         u128 carry = u128_zero();
         uint32_t ckey = GRZ_INVALID_ID - 1;
-        auto put = [&](uint32_t key, u128 x) {
-            if (key == GRZ_INVALID_ID) return;
-            if (key != kbefore) s_acc[key] = x;
-            else u128_atomic_add(s_acc + key, x);
-        };
         for (uint32_t v = lo; v < hi; v += PK_GROUP) {  // warp-uniform
             uint32_t k[4];
             u128 x[4];
@@ -801,50 +823,60 @@ __global__ void __cluster_dims__(PS_CTAS, 1, 1) __launch_bounds__(PS_T, 1) k_pr_
                 x[j] = u128_zero();
                 if (i < hi) {
                     k[j] = dst_of(i);
-                    ushort4 s;
-                    if (i < PS_CAP) {
-                        s = s_vec[i];
-                    } else {
-                        const uint4 y = __ldg(q.nbr + r0 + i);
-                        s = make_ushort4(id16(y.x), id16(y.y), id16(y.z), id16(y.w));
-                    }
-                    x[j] = u128_add(u128_add(pk_to_fx(prop[s.x]), pk_to_fx(prop[s.y])), u128_add(pk_to_fx(prop[s.z]), pk_to_fx(prop[s.w])));
+                    const ushort4 s = i < PS_CAP ? s_vec[i] : vec_of(i);
+                    x[j] = u128_add(u128_add(pk_to_fx(s_prop[s.x]), pk_to_fx(s_prop[s.y])), u128_add(pk_to_fx(s_prop[s.z]), pk_to_fx(s_prop[s.w])));
                 }
             }
             const bool ends = v + PK_GROUP >= hi;
-            uint32_t next_key = after;
-            if (!ends) next_key = dst_of(v + PK_GROUP);
-            pk_group(make_uint4(k[0], k[1], k[2], k[3]), x[0], x[1], x[2], x[3], next_key, ends, ends ? (int)((hi - v + 3) / 4) - 1 : 31, carry, ckey,
-                     put, [&](uint32_t key, u128 y) { u128_atomic_add(s_acc + key, y); });
+            pk_group(
+                make_uint4(k[0], k[1], k[2], k[3]), x[0], x[1], x[2], x[3], ends ? after : dst_of(v + PK_GROUP), ends,
+                ends ? (int)((hi - v + 3) / 4) - 1 : 31, carry, ckey,
+                [&](uint32_t key, u128 y) {
+                    if (key == GRZ_INVALID_ID) return;
+                    if (key != kbefore) s_acc[key] = y;
+                    else s_piece[warp] = y;
+                },
+                [&](uint32_t, u128 y) { s_piece[PS_WARPS + warp] = y; });
         }
         __syncthreads();
-        // apply, to every block's copy
+        const double K = s_K;
+        pk_t* const out = it & 1 ? q.props0 : q.props1;
         u128 s = u128_zero();
-        for (uint32_t i = tid; i < nv; i += PS_T) {
-            const u128 a = s_acc[i];
-            s_acc[i] = u128_zero();
-            const double p = __dmul_rn(__fma_rn(fx_to_double(a), q.damping, K), __ldg(q.inv_deg + v0 + i));
-            const pk_t w = pk_from_double(p);
 #pragma unroll
-            for (int r = 0; r < PS_CTAS; ++r) *cl.map_shared_rank(s_prop + next + v0 + i, r) = w;
-            s = u128_add(s, u128_mul32(pk_to_fx(w), __ldg(q.degree + v0 + i)));
+        for (int j = 0; j < PS_OWN; ++j) {
+            const uint32_t i = tid + j * PS_T;
+            if (i < nv) {
+                u128 a = s_acc[i];
+                for (uint32_t k = pieces[j]; k; k &= k - 1) a = u128_add(a, s_piece[__ffs(k) - 1]);
+                const double p = __dmul_rn(__fma_rn(fx_to_double(a), q.damping, K), inv[j]);
+                const pk_t w = pk_from_double(p);
+                __stcg(out + v0 + i, w);
+                s = u128_add(s, u128_mul32(pk_to_fx(w), deg[j]));
+            }
         }
         for (int o = 16; o > 0; o >>= 1) s = u128_add(s, u128_shfl_down(s, o));
         if (lane == 0) s_red[warp] = s;
         __syncthreads();
+        u128* const parts = q.parts + (it & 1) * PS_CTAS;
         if (warp == 0) {
-            s = lane < PS_T / 32 ? s_red[lane] : u128_zero();
+            s = lane < PS_WARPS ? s_red[lane] : u128_zero();
             for (int o = 8; o > 0; o >>= 1) s = u128_add(s, u128_shfl_down(s, o));
-            s = u128_shfl(s, 0);
-            if (lane < PS_CTAS) *cl.map_shared_rank(&s_part[it & 1][rank], lane) = s;
+            if (lane == 0) __stcg(reinterpret_cast<ulonglong2*>(parts + rank), make_ulonglong2(s.lo, s.hi));
         }
         cl.sync();
-        S = lane < PS_CTAS ? s_part[it & 1][lane] : u128_zero();
+        // all new props (this block's gathers of the old ones are done) and S
+        for (uint32_t v = 2 * tid; v < V; v += 2 * PS_T)  // (entry V is zero)
+            *reinterpret_cast<ulonglong2*>(s_prop + v) = __ldcg(reinterpret_cast<const ulonglong2*>(out + v));
+        S = u128_zero();
+        if (lane < PS_CTAS) {
+            const ulonglong2 x = __ldcg(reinterpret_cast<const ulonglong2*>(parts + lane));
+            S.lo = x.x;
+            S.hi = x.y;
+        }
         for (int o = 8; o > 0; o >>= 1) S = u128_add(S, u128_shfl_down(S, o));
         S = u128_shfl(S, 0);
+        __syncthreads();
     }
-    const pk_t* prop = s_prop + (q.iters & 1) * pstride;
-    for (uint32_t i = tid; i < nv; i += PS_T) q.props_out[v0 + i] = prop[v0 + i];
     if (tid == 0 && rank == 0) *q.part_out = S;
 }
 
@@ -1726,6 +1758,7 @@ static int pr_small_iterations(grz_graph* g, uint32_t iters)
         GRZ_CK(g, cudaFuncSetAttribute(k_pr_small, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ps_smem(PS_MAX_V)));
         if (g->device >= 0 && g->device < 64) configured[g->device] = true;
     }
+    if (!g->pr_small_parts) GRZ_CK(g, cudaMalloc((void**)&g->pr_small_parts, sizeof(u128) * 2 * PS_CTAS));
     GRZ_TRY(pr_sync_pk(g));
     const uint32_t stride = blocks_for(g->V) + 1;
     const int k = g->pr_sum_cur, cur = g->pr_cur ^ (int)(iters & 1);
@@ -1736,8 +1769,10 @@ static int pr_small_iterations(grz_graph* g, uint32_t iters)
     q.nvec = (uint32_t)g->pull.nvec;
     q.inv_deg = g->inv_deg;
     q.degree = g->degree;
-    q.props = g->pr_pk[g->pr_cur];
-    q.props_out = g->pr_pk[cur];
+    q.dstv = g->pull.shared;
+    q.props0 = g->pr_pk[g->pr_cur];
+    q.props1 = g->pr_pk[g->pr_cur ^ 1];
+    q.parts = g->pr_small_parts;
     q.part_in = g->pr_sum + (size_t)k * stride;
     q.nparts = g->pr_nparts[k];
     q.part_out = g->pr_sum + (size_t)(k ^ 1) * stride;

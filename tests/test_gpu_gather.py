@@ -105,7 +105,7 @@ def test_segments_follow_the_hot_choice():
     np.testing.assert_array_equal(p, pagerank(g, pr_props=1, pr_segment_bits=1))
 
 
-@pytest.mark.parametrize("V,degree", [(1, 0), (2, 1), (15, 2), (16, 3), (33, 0.5), (1000, 4), (4096, 16), (8191, 5), (8192, 20), (8193, 5)])
+@pytest.mark.parametrize("V,degree", [(1, 0), (2, 1), (15, 2), (16, 3), (33, 0.5), (1000, 4), (4096, 16), (6143, 5), (6144, 13), (6145, 5)])
 def test_small_graphs_in_one_launch(V, degree):
     """Graphs small enough for the one-cluster form, and just too large: the same props after any split
     of the iterations, with the two-kernel form in between, and as the general gather."""
@@ -133,14 +133,14 @@ def test_small_graphs_in_one_launch(V, degree):
         np.testing.assert_array_equal(G.pagerank(7, damping=0.85), ref)
 
 
-@pytest.mark.parametrize("hub_edges", [600, 4000, 8000])
+@pytest.mark.parametrize("hub_edges", [600, 4000, 6000])
 def test_small_graph_with_most_edges_at_few_destinations(hub_edges):
     """Destinations whose vectors outgrow a block's share, and its shared memory."""
     from grazelle import graphgen as gg
-    V = 8100
+    V = 6100
     rng = np.random.RandomState(3)
     src, dst = [], []
-    for hub in (5, 6, 7, 8, 4000, 8099):
+    for hub in (5, 6, 7, 8, 9, 4000, 6099):
         s = rng.permutation(V - 1)[:hub_edges]
         src.append(s + (s >= hub))
         dst.append(np.full(hub_edges, hub))
