@@ -115,10 +115,9 @@ static void free_graph_data(grz_graph* g, uint64_t next_V = ~0ull)
         // the PageRank arrays are sized by V alone: kept, and refilled at the next grz_pr_init
         g->pr_lists_changed = 1;
     } else {
-        void* plain[] = { g->pr_fx[0], g->pr_fx[1], g->pr_sum, g->pr_K, g->pr_rowacc, g->pr_cut, g->pr_pk[0], g->pr_pk[1], g->pr_hot[0], g->pr_hot[1] };
+        void* plain[] = { g->pr_fx[0], g->pr_fx[1], g->pr_sum, g->pr_K, g->pr_rowacc, g->pr_cut, g->pr_pk[0], g->pr_pk[1] };
         for (void* p : plain) cudaFree(p);
         g->pr_pk[0] = g->pr_pk[1] = nullptr;
-        g->pr_hot[0] = g->pr_hot[1] = nullptr;
         g->pr_fx[0] = g->pr_fx[1] = nullptr; g->pr_sum = nullptr; g->pr_K = nullptr; g->pr_rowacc = nullptr;
         g->pr_cut = nullptr;
     }
@@ -136,6 +135,9 @@ static void free_graph_data(grz_graph* g, uint64_t next_V = ~0ull)
     g->pr_hot_nbr = nullptr;
     grz_dev_free(g, g->pr_hot_vid);
     g->pr_hot_vid = nullptr;
+    grz_dev_free(g, g->pr_hot[0]);
+    grz_dev_free(g, g->pr_hot[1]);
+    g->pr_hot[0] = g->pr_hot[1] = nullptr;
     g->pr_hotmap = nullptr;
     g->pr_nhot = 0;
     g->pr_hot_known = 0;

@@ -1051,7 +1051,7 @@ __global__ void k_pr_vertex(const double* __restrict__ accum, const double* __re
 // counts and up to 100k at 360 others (checked against the division on the CPU), at 3 FP64
 // operations instead of a division's; the grid strides, with one partial of S_0 per block.  GB300, with
 // the accumulators' clearing (a division per vertex, props also written as doubles and in fixed point
-// -> now): V = 2^26 1.94 -> 0.70 ms, 2^20 52 -> 20 us.
+// -> now): V = 2^24 512 -> 171 us, 2^20 52 -> 24 us.
 __global__ void __launch_bounds__(PR_THREADS, 8) k_pr_init(const double* __restrict__ inv_deg, const uint32_t* __restrict__ degree, uint64_t V,
                                                            double c, double* __restrict__ accum, u128* __restrict__ prop_fx, pk_t* __restrict__ prop_pk,
                                                            const uint2* __restrict__ hotmap, pk_t* __restrict__ hot, u128* __restrict__ part0)
@@ -1254,8 +1254,11 @@ static int pr_cut_for(grz_graph* g, uint32_t per)
 
 // Chooses the hot sources of the loaded lists.  Once per loaded lists; one read-back.  Worth it
 // when the hot sources are at least a tenth of the edges: with 1% (a uniform graph) the gather is no
-// faster, with 20% (R-MAT 24) it is 13% faster, with 52% (R-MAT 20) 20-30%.  Lists below 2^18
-// vectors stay as they are: their props fit L1.
+// faster, with 20% (R-MAT 24) it is 13% faster, with 52% (R-MAT 20) 20-30%.  Lists below 2^21
+// vectors stay as they are: their props are mostly L1 hits and the table's copy is not for free (GB300,
+// R-MAT, us per iteration without / with the table: 0.5M vectors 13.6 / 15.3, 1.05M 18.7 / 20.0, 2.1M
+// 33.7 / 30.3; choosing and encoding take 120 us there).
+constexpr uint64_t PR_HOT_MIN_VECTORS = 1ull << 21;
 static int pr_hot_choose(grz_graph* g)
 {
     const uint64_t V = g->V;
@@ -1263,7 +1266,7 @@ static int pr_hot_choose(grz_graph* g)
     cudaStream_t st = g->stream;
     const uint64_t words = (V + 31) / 32;
     g->pr_nhot = 0;
-    if (g->pull.nvec < (1ull << 18) || V >= GRZ_HUB_BASE) {
+    if (g->pull.nvec < PR_HOT_MIN_VECTORS || V >= GRZ_HUB_BASE) {
         g->pr_hot_known = 1;
         return GRZ_OK;
     }
@@ -1295,7 +1298,7 @@ static int pr_hot_choose(grz_graph* g)
             rc = grz_cuda_check(g, cudaGetLastError(), "k_hot_base");
         }
         for (int i = 0; i < 2 && !rc; ++i) {
-            if (!g->pr_hot[i]) rc = grz_cuda_check(g, cudaMalloc((void**)&g->pr_hot[i], sizeof(pk_t) * (GRZ_PR_HOT_MAX + 2)), "hot props");
+            rc = grz_dev_alloc(g, (void**)&g->pr_hot[i], sizeof(pk_t) * (GRZ_PR_HOT_MAX + 2));
             // the slots past the last stay zero
             if (!rc) rc = grz_cuda_check(g, cudaMemsetAsync(g->pr_hot[i], 0, sizeof(pk_t) * (GRZ_PR_HOT_MAX + 2), st), "memset");
         }
@@ -1303,10 +1306,10 @@ static int pr_hot_choose(grz_graph* g)
     grz_dev_free(g, hist);
     grz_dev_free(g, cnt);
     if (rc) {
-        grz_dev_free(g, g->pr_hotmap);
-        grz_dev_free(g, g->pr_hot_vid);
+        for (void* p : { (void*)g->pr_hotmap, (void*)g->pr_hot_vid, (void*)g->pr_hot[0], (void*)g->pr_hot[1] }) grz_dev_free(g, p);
         g->pr_hotmap = nullptr;
         g->pr_hot_vid = nullptr;
+        g->pr_hot[0] = g->pr_hot[1] = nullptr;
         return rc;
     }
     if (g->pr_hotmap) g->pr_nhot = (uint32_t)pick[1];

@@ -49,13 +49,13 @@ def test_one_destination_of_every_length(vectors):
 
 @pytest.mark.parametrize("seg", [1, 12, 14])
 def test_hot_sources(seg):
-    """A power-law graph large enough for the hot table (2^18 vectors and more), unsegmented and in
+    """A power-law graph large enough for the hot table (2^21 vectors and more), unsegmented and in
     segments: grids of any size, a reload with the same V, the phase API and CC on the encoded
     segments."""
     import ctypes as C
     from grazelle import graphgen as gg, native
     from grazelle.engine import Graph
-    g, h = gg.rmat(17, 16, seed=81), gg.rmat(17, 16, seed=82)
+    g, h = gg.rmat(18, 44, seed=81), gg.rmat(18, 44, seed=82)
     V = g.num_vertices
     pull, push = g.pull_order().pairs(), g.push_order().pairs()
     ref, ref_h = pagerank(g, pr_props=1, pr_segment_bits=1), pagerank(h, pr_props=1, pr_segment_bits=1)
@@ -93,7 +93,7 @@ def test_segments_follow_the_hot_choice():
     and a CC run captured on the first build reads the second."""
     from grazelle import graphgen as gg
     from grazelle.engine import Graph
-    g = gg.rmat(17, 16, seed=83)
+    g = gg.rmat(18, 44, seed=83)
     pull, push = g.pull_order().pairs(), g.push_order().pairs()
     with Graph(0) as G:
         G.tune(cc_pull_first=0, cc_segments=2, pr_segment_bits=13)
