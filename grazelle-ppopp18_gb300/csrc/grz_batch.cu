@@ -15,20 +15,18 @@
 //     the vertices of the graphs before it, and the union is loaded as one grz_graph.  Kernels
 //     never need to know where one graph ends; only the per-graph sums S do.
 //   * Up to GRZ_BATCH_K (8) instances per graph share one pass over the edges.  Props are stored
-//     [vertex][instance] in 4.124 fixed point (the apply converts each prop once), so the 8 lanes
-//     that serve one vector's instances read one aligned 128-byte row per source: the random
-//     gather costs one line for 8 instances instead of 8 lines, and no conversion per edge.
-//   * PPR gather: a warp owns a tile of 32 vectors and walks it 4 vectors x 8 instances at a
-//     time.  Lane (vector, instance) sums its four sources exactly; a shuffle scan over the 4
-//     vectors and a carried running sum complete each destination inside the warp, with no
-//     shared memory and no barrier.  Destinations complete inside the tile are stored, the (at
-//     most two) cut by the tile edge are added with exact u128 atomics.  Sums are exact, so
-//     results do not depend on the launch shape.
-//   * PPR apply: thread per (vertex, instance); it reads S of its graph and instance (summed
-//     exactly by the previous apply as sum deg(u) * prop(u)), writes the new props and clears
-//     the accumulators.  The next S is summed in registers per graph, then per block in shared
-//     memory, and reaches global memory with one atomic per block, graph and instance (one
-//     cache line per graph would otherwise take an atomic from every 32 vertices).
+//     [vertex][instance] packed in 8 bytes (pk_to_fx), so the 8 lanes that serve one vector's
+//     instances read one aligned 64-byte row per source: the random gather costs one line for 8
+//     instances instead of 8 lines.
+//   * PPR iteration: one kernel gathers and applies.  S only enters at the seed and is the sum of
+//     deg(u) * prop(u) of the props being gathered, so it is known before the iteration, and a
+//     destination whose sum is complete gets its new prop at once: the accumulators of the
+//     destinations that one slot sums alone never reach memory.  A warp is 4 slots of 8 lanes (lane =
+//     8 * slot + instance), and each slot walks a contiguous range of vectors, two at a time.  The
+//     destinations that the ranges cut are added with exact u128 atomics and finished by a second,
+//     small kernel, which also serves the seeds without in-edges (every other vertex without
+//     in-edges keeps a prop of zero).  The next S is summed in registers per graph, then per block
+//     in shared memory.  Sums are exact, so results do not depend on the launch shape.
 //   * Multi-source BFS: bit-parallel, 8 roots per graph.  visited / frontier are one byte per
 //     vertex (bit i = instance i).  Pull: a vector's new bits are the OR of its sources'
 //     frontier bytes, reduced per destination within the warp, minus the visited bits; the
@@ -48,20 +46,14 @@
 namespace {
 
 constexpr int K = GRZ_BATCH_K;  // instances per graph (8)
-constexpr int GT = 256;         // threads per block: 32 vectors (or vertices) x 8 instances
-constexpr int TV = GT / K;      // vectors per gather tile
+constexpr int GT = 256;         // threads per block
+constexpr int MIN_V = 32;       // vertices of the smallest graph
 constexpr uint32_t NONE = 0xffffffffu;
 constexpr int MAX_GRAPHS = 1024;
 
-__device__ __forceinline__ u128 shfl_up_u128(u128 v, int off)
-{
-    u128 r;
-    r.lo = __shfl_up_sync(0xffffffffu, v.lo, off);
-    r.hi = __shfl_up_sync(0xffffffffu, v.hi, off);
-    return r;
-}
+typedef unsigned long long pk_t;  // a packed prop (pk_to_fx)
 
-// graph of union vertex v (voff: G+1 ascending offsets in shared memory)
+// graph of union vertex v (voff: G+1 ascending offsets)
 __device__ __forceinline__ uint32_t graph_of(const uint32_t* voff, uint32_t G, uint32_t v)
 {
     uint32_t lo = 0, hi = G - 1;
@@ -73,233 +65,285 @@ __device__ __forceinline__ uint32_t graph_of(const uint32_t* voff, uint32_t G, u
 }
 
 // initial PPR state: prop = one-hot(seed) / deg'; S = deg(seed) * prop(seed) per (graph, instance).
-// The props are 4.124 fixed point (prop) or the doubles they are the exact conversions of (propd).
+// The props and ranks are zero elsewhere (and in the buffer the first iteration writes).
 __global__ void k_ppr_init(const uint32_t* __restrict__ seeds, uint32_t G, const double* __restrict__ inv_deg,
-                           const uint32_t* __restrict__ degree, u128* __restrict__ prop, double* __restrict__ propd,
-                           u128* __restrict__ S)
+                           const uint32_t* __restrict__ degree, pk_t* __restrict__ prop, u128* __restrict__ S, u128* __restrict__ S_next)
 {
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= G * K) return;
     const uint32_t s = seeds[t];
-    const uint32_t i = t % K;
     u128 v = u128_zero();
     if (s != NONE) {
-        const u128 p = fx_from_double(inv_deg[s]);
-        if (propd) propd[(uint64_t)s * K + i] = inv_deg[s];
-        else prop[(uint64_t)s * K + i] = p;
-        v = u128_mul32(p, degree[s]);
+        const pk_t w = pk_from_double(inv_deg[s]);
+        prop[(uint64_t)s * K + t % K] = w;
+        v = u128_mul32(pk_to_fx(w), degree[s]);
     }
     S[t] = v;
+    S_next[t] = u128_zero();
 }
 
-__device__ __forceinline__ u128 ldg_u128(const u128* p)
+// what finishing a destination needs
+struct PprApply {
+    const double* inv_deg;
+    const uint32_t* degree;
+    const uint32_t* voff;    // [G + 1]
+    uint32_t G;
+    const uint32_t* seeds;   // [G][K]
+    double damping;
+    const u128* S;           // [G][K]: sum of deg * prop of the props being gathered
+    u128* S_next;            // the same of the props being written
+    pk_t* prop_out;          // [vertex][K]
+    double* rank_out;        // last iteration, or null
+};
+
+// d * (1 - S) + (1 - d): the seed's teleport and dangling mass
+__device__ __forceinline__ double ppr_teleport(const PprApply& ap, uint32_t g, int inst)
 {
-    const ulonglong2 q = __ldg(reinterpret_cast<const ulonglong2*>(p));
-    u128 r;
-    r.lo = q.x;
-    r.hi = q.y;
-    return r;
+    const double S = fx_to_double(ap.S[g * K + inst]);
+    return __dadd_rn(__dmul_rn(ap.damping, 1.0 - S), 1.0 - ap.damping);
 }
 
-// edge-pull of all instances (see the file comment).  Warp-level tiles of TV = 32 vectors,
-// persistent over the grid's warps.  A warp walks its tile in 8 steps of 4 vectors x 8 instances
-// (lane = 8 * slot + instance): it sums each lane's four sources exactly, scans the step's 4
-// vectors per instance (keys ascend, so equal keys form one run), and carries the open
-// destination's running sum into the next step.  A destination whose vectors all lie in the
-// tile is stored once by the lane of its last vector; one cut by the tile edge is added with
-// exact u128 atomics.  Block 0 first clears S_next for the apply that follows.
-constexpr int GSTEPS = TV / 4;  // steps of 4 vectors per tile
-constexpr int GCHUNK = 2;       // steps whose loads are issued together
-// 6 blocks per SM: occupancy beats deeper per-warp load batches (GB300 sweep over steps per
-// chunk 1-8 and 4-8 blocks per SM: 99.8 ms per 256-instance run here, 102-163 ms elsewhere)
-constexpr int GATHER_RESIDENT = 6;
-
-// a gathered prop in fixed point: read as such, or converted (exactly) from the double it came from
-__device__ __forceinline__ u128 ld_prop(const u128* p) { return ldg_u128(p); }
-__device__ __forceinline__ u128 ld_prop(const double* p) { return fx_from_double(__ldg(p)); }
-
-__device__ __forceinline__ u128 shfl_u128(u128 v, int src)
+// rank' = fma(accum, d, [v == seed] * teleport) and prop' = rank' / deg' of one vertex and instance;
+// returns deg * prop'.  Two FP64 operations: the FP64 pipe is the narrowest of the chip (one warp
+// instruction in 16 clocks per SM).
+__device__ __forceinline__ u128 ppr_finish(const PprApply& ap, uint32_t v, int inst, u128 x, double teleport)
 {
-    u128 r;
-    r.lo = __shfl_sync(0xffffffffu, v.lo, src);
-    r.hi = __shfl_sync(0xffffffffu, v.hi, src);
-    return r;
-}
-
-template <typename P>
-__global__ void __launch_bounds__(GT, GATHER_RESIDENT) k_ppr_gather(const uint4* __restrict__ nbr, const uint32_t* __restrict__ dstv,
-                                                   uint64_t nvec, uint32_t V, const P* __restrict__ prop,
-                                                   u128* __restrict__ rowacc, u128* __restrict__ S_next, uint32_t nS)
-{
-    if (blockIdx.x == 0)
-        for (uint32_t k = threadIdx.x; k < nS; k += GT) S_next[k] = u128_zero();
-    const int lane = threadIdx.x & 31;
-    const int q = lane / K, inst = lane % K;
-    const uint64_t ntiles = (nvec + TV - 1) / TV;
-    const uint64_t nwarps = (uint64_t)gridDim.x * (GT / 32);
-    for (uint64_t tile = (uint64_t)blockIdx.x * (GT / 32) + (threadIdx.x >> 5); tile < ntiles; tile += nwarps) {
-        const uint64_t v0 = tile * TV;
-        // the tile's 32 keys, one per lane (NONE past the list), and the keys either side of it
-        const uint32_t kall = v0 + lane < nvec ? __ldcs(dstv + v0 + lane) : NONE;
-        const uint32_t kbefore = v0 > 0 ? __ldg(dstv + v0 - 1) : NONE - 1;
-        const uint32_t kafter = v0 + TV < nvec ? __ldg(dstv + v0 + TV) : NONE - 1;
-        u128 carry = u128_zero();
-        uint32_t ckey = NONE - 1;  // destination of the open run carried from the previous step
-#pragma unroll
-        for (int h = 0; h < GSTEPS; h += GCHUNK) {
-            u128 val[GCHUNK];
-#pragma unroll
-            for (int j = 0; j < GCHUNK; ++j) {
-                const uint64_t v = v0 + (uint64_t)(h + j) * 4 + q;
-                val[j] = u128_zero();
-                if (v < nvec) {
-                    const uint4 sv = __ldg(nbr + v);
-                    const uint32_t ids[4] = { sv.x, sv.y, sv.z, sv.w };
-#pragma unroll
-                    for (int l = 0; l < 4; ++l)
-                        if (ids[l] < V) val[j] = u128_add(val[j], ld_prop(prop + (uint64_t)ids[l] * K + inst));
-                }
-            }
-#pragma unroll
-            for (int j = 0; j < GCHUNK; ++j) {
-                const int pos = (h + j) * 4 + q;  // vector of this lane within the tile
-                u128 x = val[j];
-                const uint32_t k = __shfl_sync(0xffffffffu, kall, pos);
-#pragma unroll
-                for (int off = 1; off < 4; off <<= 1) {
-                    const u128 o = shfl_up_u128(x, off * K);
-                    const uint32_t ko = __shfl_sync(0xffffffffu, kall, pos >= off ? pos - off : 0);
-                    if (q >= off && ko == k) x = u128_add(x, o);
-                }
-                if (k == ckey) x = u128_add(x, carry);
-                const uint32_t kn_in = __shfl_sync(0xffffffffu, kall, (pos + 1) & (TV - 1));  // every lane shuffles
-                const uint32_t kn = pos + 1 < TV ? kn_in : kafter;
-                const bool tail = kn != k;
-                if (k != NONE && (tail || pos == TV - 1)) {
-                    u128* dst = rowacc + (uint64_t)k * K + inst;
-                    if (tail && k != kbefore) *dst = x;                // every vector of k is in this tile
-                    else if (x.lo | x.hi) u128_atomic_add(dst, x);     // cut by the tile edge
-                }
-                carry = shfl_u128(x, 3 * K + inst);
-                ckey = __shfl_sync(0xffffffffu, k, 3 * K + inst);
-            }
-        }
-    }
+    const double rank = __fma_rn(fx_to_double(x), ap.damping, teleport);
+    // rounding can leave 1 - S below zero at damping 1; props are taken without sign (fx_from_double)
+    const pk_t w = pk_from_double(fabs(__dmul_rn(rank, __ldg(ap.inv_deg + v))));
+    ap.prop_out[(uint64_t)v * K + inst] = w;
+    if (ap.rank_out) ap.rank_out[(uint64_t)v * K + inst] = rank;
+    return u128_mul32(pk_to_fx(w), __ldg(ap.degree + v));
 }
 
 constexpr int APPLY_SLOTS = 64;  // graphs whose next S a block sums in shared memory (beyond: global atomics)
-#ifndef GRZ_PPR_APPLY_U
-#define GRZ_PPR_APPLY_U 1
-#endif
-#ifndef GRZ_PPR_APPLY_MINB
-#define GRZ_PPR_APPLY_MINB 8
-#endif
-// Tiles whose accumulators a thread loads before it stores anything, and resident apply blocks
-// per SM.  GB300 sweep (256 PPR x 20 iterations on the 32-graph batch): 8 tiles at 3 blocks per SM
-// (80 registers) 100.9 ms, 4 at 4 95.3 ms, 2 at 6 91.5 ms, 1 at 8 (32 registers) 89.7 ms: the
-// apply wants every warp slot more than loads in flight per thread.
-constexpr int APPLY_U = GRZ_PPR_APPLY_U;
+constexpr uint32_t PQ = 16;      // ring of the complete sums a warp holds: 3 left over and 8 of a step at most
+constexpr int PPR_RESIDENT = 4;  // blocks per SM the launch bounds fit
 
-// bit j of word t: vertex 32t + j has pull vectors in two or more gather tiles, so its
-// accumulator is summed with atomics and the apply must clear it.  Every other accumulator is
-// either stored whole by each gather or never written (no in-edges), and needs no clearing.
-__global__ void k_ppr_cutbits(const uint32_t* __restrict__ rowptr, uint32_t V, uint32_t* __restrict__ cut)
+// Ranges of the slots: bnd[4 w + s] is the first vector of slot s of warp w (a multiple of 4), bnd[4 nwarps]
+// = nvec.  The warps' ranges are equal in PPR_WV per vector + PPR_WD per vertex up to their destinations, about
+// the instructions k_ppr_step has for each; a warp's slots have the same number of vectors.  All ranges run at
+// once, so the longest sets the time: 8-graph batch of 1.04M vertices, 8 instances x 20 iterations, ranges of
+// equal vectors 4.46 ms, weights 4:5 3.49, 2:3 3.56, 4:7 3.65 ms.
+constexpr uint32_t PPR_WV = 4, PPR_WD = 5;
+
+__global__ void k_ppr_bounds(const uint32_t* __restrict__ dstv, uint32_t nvec, uint32_t V, uint32_t nwarps, uint32_t* __restrict__ bnd)
 {
-    const uint32_t v = blockIdx.x * blockDim.x + threadIdx.x;
-    bool c = false;
-    if (v < V) {
-        const uint32_t r0 = rowptr[v], r1 = rowptr[v + 1];
-        c = r1 > r0 && r0 / TV != (r1 - 1) / TV;
+    const uint32_t w = blockIdx.x * blockDim.x + threadIdx.x;
+    if (w > nwarps) return;
+    const uint64_t total = (uint64_t)PPR_WV * nvec + (uint64_t)PPR_WD * V;
+    uint32_t at[2];
+    for (int e = 0; e < 2; ++e) {
+        const uint64_t goal = total * (w + e) / nwarps;
+        uint32_t lo = 0, hi = (nvec + 3) / 4;  // in groups of 4 vectors
+        while (lo < hi) {
+            const uint32_t mid = (lo + hi) / 2;
+            if ((uint64_t)PPR_WV * 4 * mid + (uint64_t)PPR_WD * dstv[4 * mid] < goal) lo = mid + 1;
+            else hi = mid;
+        }
+        at[e] = w + e >= nwarps ? (nvec + 3) / 4 : lo;
     }
-    const unsigned m = __ballot_sync(0xffffffffu, c);
-    if ((threadIdx.x & 31) == 0 && v < V) cut[v / 32] = m;
+    const uint32_t q = (at[1] - at[0] + 3) / 4;
+    for (uint32_t s = 0; s < 4 && w < nwarps; ++s) bnd[4 * w + s] = min(4 * min(at[0] + s * q, at[1]), nvec);
+    if (w == nwarps) bnd[4 * w] = nvec;
 }
 
-__device__ __forceinline__ void s_flush(u128* s_part, u128* S_next, uint32_t g, int inst, u128 x)
+// cut[r]: the destination that the start of range r cuts, once per destination; NONE elsewhere
+__global__ void k_ppr_cuts(const uint32_t* __restrict__ dstv, const uint32_t* __restrict__ bnd, uint32_t nranges, uint32_t* __restrict__ cut)
 {
-    if ((x.lo | x.hi) == 0) return;
-    if (g < (uint32_t)APPLY_SLOTS) u128_atomic_add(s_part + g * K + inst, x);
-    else u128_atomic_add(S_next + (uint64_t)g * K + inst, x);
+    const uint32_t r = blockIdx.x * blockDim.x + threadIdx.x;
+    if (r >= nranges) return;
+    const uint32_t lo = bnd[r];
+    uint32_t v = NONE;
+    if (lo > 0 && lo < bnd[r + 1] && dstv[lo - 1] == dstv[lo]) {
+        v = dstv[lo];
+        uint32_t p = r;  // the range before that is not empty
+        while (bnd[p] == lo) --p;
+        if (bnd[p] > 0 && dstv[bnd[p] - 1] == v) v = NONE;
+    }
+    cut[r] = v;
 }
 
-// vertex phase of all instances; thread per (vertex, instance).  The grid strides over tiles of
-// 32 vertices (all blocks on one moving front of the arrays), APPLY_U tiles at a time: their
-// accumulators are loaded first, then the tiles are finished in order.
-__global__ void __launch_bounds__(GT, GRZ_PPR_APPLY_MINB) k_ppr_apply(u128* __restrict__ rowacc, const uint32_t* __restrict__ cut,
-                                                     const double* __restrict__ inv_deg,
-                                                     const uint32_t* __restrict__ degree, uint32_t V,
-                                                     const uint32_t* __restrict__ voff_g, uint32_t G,
-                                                     const uint32_t* __restrict__ seeds, double damping,
-                                                     const u128* __restrict__ S_cur, u128* __restrict__ S_next,
-                                                     u128* __restrict__ prop_out, double* __restrict__ propd_out,
-                                                     double* __restrict__ rank_out)
+// pk_to_fx of a prop of at least 2^-60 (s < 64), or zero
+__device__ __forceinline__ u128 pk_to_fx_near(pk_t w)
+{
+    const uint32_t s = (uint32_t)w & 63u;
+    const pk_t x = w & ~127ull;
+    u128 r;
+    r.hi = x >> s;
+    r.lo = shl64_clamp(x, 64u - s);
+    return r;
+}
+
+// block sums of the next S in shared memory
+__device__ __forceinline__ void ppr_add_S(u128* s_part, const PprApply& ap, uint32_t g, int inst, u128 m)
+{
+    if ((m.lo | m.hi) == 0) return;
+    if (g < (uint32_t)APPLY_SLOTS) u128_atomic_add(s_part + g * K + inst, m);
+    else u128_atomic_add(ap.S_next + (uint64_t)g * K + inst, m);
+}
+
+__device__ __forceinline__ void ppr_flush_S(const u128* s_part, uint32_t nslots, const PprApply& ap)
+{
+    __syncthreads();
+    for (uint32_t k = threadIdx.x; k < nslots; k += GT) {
+        const u128 y = s_part[k];
+        if (y.lo | y.hi) u128_atomic_add(ap.S_next + k, y);
+    }
+}
+
+// One PPR iteration but for the cut destinations (see the file comment).  Block 0 clears S_clear for the
+// iteration after.  prop row V is zero: empty lanes gather it.
+//
+// Bound by the ALU pipe (shifts, logic and additions of the 128-bit sums: 53% of its peak over the whole
+// launch, memory below 35%).  So the slots walk ranges of their own, which needs no scan across lanes (a scan
+// over the slots: 722 instructions per 16 vectors and 206 us, without 535 and 160 us); props of 2^-60 and
+// more, nearly all, are unpacked by a shorter form when all of a warp's are; and complete sums wait in shared
+// memory to be finished four at a time with all lanes, for FP64 instructions cost the same for one lane.
+//
+// GB300, 8 graphs of 1.04M vertices and 10.5M edges in all, 8 instances, us per iteration: a gather of
+// 16-byte fixed-point rows and an apply over all vertices 224; this and k_ppr_rest 175.  32 graphs of 245M
+// edges, 20 iterations: 89.9 ms and 71.8 ms.
+__global__ void __launch_bounds__(GT, PPR_RESIDENT) k_ppr_step(const uint4* __restrict__ nbr, const uint32_t* __restrict__ dstv,
+                                                              const uint32_t* __restrict__ bnd, uint32_t nvec, uint32_t V,
+                                                              const pk_t* __restrict__ prop, u128* __restrict__ rowacc,
+                                                              u128* __restrict__ S_clear, const PprApply ap)
 {
     __shared__ uint32_t voff[MAX_GRAPHS + 1];
     __shared__ u128 s_part[APPLY_SLOTS * K];
-    const uint32_t nslots = (G < (uint32_t)APPLY_SLOTS ? G : (uint32_t)APPLY_SLOTS) * K;
-    for (uint32_t k = threadIdx.x; k <= G; k += GT) voff[k] = voff_g[k];
+    __shared__ u128 s_sum[GT / 32][PQ * K];
+    __shared__ uint32_t s_vid[GT / 32][PQ];
+    u128* const qsum = s_sum[threadIdx.x >> 5];
+    uint32_t* const qvid = s_vid[threadIdx.x >> 5];
+    const uint32_t nslots = (ap.G < (uint32_t)APPLY_SLOTS ? ap.G : (uint32_t)APPLY_SLOTS) * K;
+    for (uint32_t k = threadIdx.x; k <= ap.G; k += GT) voff[k] = ap.voff[k];
+    for (uint32_t k = threadIdx.x; k < nslots; k += GT) s_part[k] = u128_zero();
+    if (blockIdx.x == 0)
+        for (uint32_t k = threadIdx.x; k < ap.G * K; k += GT) S_clear[k] = u128_zero();
+    __syncthreads();
+    const int lane = threadIdx.x & 31;
+    const int slot = lane / K, inst = lane % K;
+    const uint32_t below = (1u << (slot * K)) - 1u;
+    const uint32_t range = 4 * ((threadIdx.x >> 5) * gridDim.x + blockIdx.x) + slot;
+    const uint32_t lo = __ldg(bnd + range), hi = __ldg(bnd + range + 1);
+    const uint32_t steps = __reduce_max_sync(0xffffffffu, (hi - lo + 1) / 2);
+    const uint32_t kbefore = lo > 0 && lo < hi ? __ldg(dstv + lo - 1) : NONE - 1;
+    const uint32_t kafter = lo < hi && hi < nvec ? __ldg(dstv + hi) : NONE;
+    // the graph of the destinations this lane is finishing
+    uint32_t g = 0, gbeg = 0, gend = 0, seed = NONE;
+    double teleport = 0.0;
+    u128 acc = u128_zero();
+    auto finish = [&](uint32_t v, u128 x) {
+        if (v < gbeg || v >= gend) {
+            ppr_add_S(s_part, ap, g, inst, acc);
+            acc = u128_zero();
+            g = graph_of(voff, ap.G, v);
+            gbeg = voff[g];
+            gend = voff[g + 1];
+            seed = ap.seeds[g * K + inst];
+            teleport = seed != NONE ? ppr_teleport(ap, g, inst) : 0.0;
+        }
+        if (seed != NONE) acc = u128_add(acc, ppr_finish(ap, v, inst, x, v == seed ? teleport : 0.0));
+    };
+    auto cut = [&](uint32_t v, u128 x) {  // a part of a destination that other ranges share
+        if (x.lo | x.hi) u128_atomic_add(rowacc + (uint64_t)v * K + inst, x);
+    };
+    const pk_t* const row = prop + inst;
+    uint32_t ids[8];
+    uint2 nk;
+    auto load = [&](uint32_t v) {  // the slot's two vectors from v on, the same in its 8 lanes
+        uint4 x = make_uint4(NONE, NONE, NONE, NONE), y = x;
+        nk = make_uint2(NONE, NONE);
+        if (v + 1 < hi) {
+            x = __ldg(nbr + v);
+            y = __ldg(nbr + v + 1);
+            nk = __ldg(reinterpret_cast<const uint2*>(dstv + v));
+        } else if (v < hi) {
+            x = __ldg(nbr + v);
+            nk.x = __ldg(dstv + v);
+        }
+        ids[0] = x.x; ids[1] = x.y; ids[2] = x.z; ids[3] = x.w;
+        ids[4] = y.x; ids[5] = y.y; ids[6] = y.z; ids[7] = y.w;
+    };
+    load(lo);
+    u128 sum = u128_zero();     // of the destination being read
+    uint32_t qh = 0, nq = 0;    // complete sums waiting
+    for (uint32_t i = 0, v = lo; i < steps; ++i, v += 2) {
+        const uint2 k = nk;
+        u128 x[2];
+        pk_t p[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) p[j] = __ldg(row + (uint64_t)min(ids[j], V) * K);
+        load(v + 2);
+        const uint32_t far = (uint32_t)(p[0] | p[1] | p[2] | p[3] | p[4] | p[5] | p[6] | p[7]) & 64u;
+        if (!__any_sync(0xffffffffu, far)) {
+#pragma unroll
+            for (int j = 0; j < 2; ++j)
+                x[j] = u128_add(u128_add(pk_to_fx_near(p[4 * j]), pk_to_fx_near(p[4 * j + 1])),
+                                u128_add(pk_to_fx_near(p[4 * j + 2]), pk_to_fx_near(p[4 * j + 3])));
+        } else {
+#pragma unroll
+            for (int j = 0; j < 2; ++j)
+                x[j] = u128_add(u128_add(pk_to_fx(p[4 * j]), pk_to_fx(p[4 * j + 1])), u128_add(pk_to_fx(p[4 * j + 2]), pk_to_fx(p[4 * j + 3])));
+        }
+        const uint32_t key[3] = {k.x, k.y, v + 2 < hi ? nk.x : kafter};
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            sum = u128_add(sum, x[j]);
+            const bool ends = key[j] != key[j + 1] && key[j] != NONE;
+            const bool whole = ends && key[j] != kbefore;
+            const uint32_t m = __ballot_sync(0xffffffffu, whole) & 0x01010101u;
+            if (ends) {
+                if (whole) {
+                    const uint32_t at = (qh + nq + __popc(m & below)) % PQ;
+                    qsum[at * K + inst] = sum;
+                    if (inst == 0) qvid[at] = key[j];
+                } else {
+                    cut(key[j], sum);
+                }
+                sum = u128_zero();
+            }
+            nq += __popc(m);
+        }
+        __syncwarp();
+        for (; nq >= 4; nq -= 4, qh += 4) finish(qvid[(qh + slot) % PQ], qsum[(qh + slot) % PQ * K + inst]);
+        __syncwarp();
+    }
+    if ((uint32_t)slot < nq) finish(qvid[(qh + slot) % PQ], qsum[(qh + slot) % PQ * K + inst]);
+    if (kafter != NONE) cut(kafter, sum);  // nothing is left of a destination that ended
+    ppr_add_S(s_part, ap, g, inst, acc);
+    ppr_flush_S(s_part, nslots, ap);
+}
+
+// The rest of an iteration: the cut destinations, whose accumulators are emptied, and the seeds without
+// in-edges.
+__global__ void __launch_bounds__(GT) k_ppr_rest(const uint32_t* __restrict__ cuts, uint32_t nranges, const uint32_t* __restrict__ rowptr,
+                                                 u128* __restrict__ rowacc, const PprApply ap)
+{
+    __shared__ u128 s_part[APPLY_SLOTS * K];
+    const uint32_t nslots = (ap.G < (uint32_t)APPLY_SLOTS ? ap.G : (uint32_t)APPLY_SLOTS) * K;
     for (uint32_t k = threadIdx.x; k < nslots; k += GT) s_part[k] = u128_zero();
     __syncthreads();
-    const uint64_t ntiles = ((uint64_t)V + TV - 1) / TV;
-    const int inst = threadIdx.x % K, lv = threadIdx.x / K;
-    // per-thread state of the graph of its current vertex (vertices ascend); the seed's teleport
-    // term d * (1 - S) + (1 - d) is computed once per graph
-    uint32_t g = 0, gend = 0, seed = NONE;
-    double cseed = 0.0;
-    u128 acc = u128_zero();
-    for (uint64_t tile = blockIdx.x; tile < ntiles; tile += (uint64_t)APPLY_U * gridDim.x) {
-        u128 a[APPLY_U];
-        uint32_t cw[APPLY_U];
-#pragma unroll
-        for (int j = 0; j < APPLY_U; ++j) {
-            const uint64_t t = tile + (uint64_t)j * gridDim.x;
-            const uint64_t v = t * TV + lv;
-            a[j] = u128_zero();
-            cw[j] = 0;
-            if (v < V) {
-                const ulonglong2 q = *(reinterpret_cast<const ulonglong2*>(rowacc) + v * K + inst);
-                a[j].lo = q.x;
-                a[j].hi = q.y;
-                cw[j] = __ldg(cut + t);
-            }
+    const uint32_t t = blockIdx.x * GT + threadIdx.x, item = t / K;
+    const int inst = t % K;
+    uint32_t v = NONE;
+    u128 x = u128_zero();
+    if (item < nranges) {
+        v = __ldg(cuts + item);
+        if (v != NONE) {
+            u128* a = rowacc + (uint64_t)v * K + inst;
+            x = *a;
+            *a = u128_zero();
         }
-#pragma unroll
-        for (int j = 0; j < APPLY_U; ++j) {
-            const uint64_t v64 = (tile + (uint64_t)j * gridDim.x) * TV + lv;
-            if (v64 >= V) break;
-            const uint32_t v = (uint32_t)v64;
-            if (v >= gend) {
-                s_flush(s_part, S_next, g, inst, acc);
-                acc = u128_zero();
-                g = graph_of(voff, G, v);
-                gend = voff[g + 1];
-                seed = seeds[g * K + inst];
-                const double S = fx_to_double(S_cur[g * K + inst]);
-                cseed = __dadd_rn(__dmul_rn(damping, 1.0 - S), 1.0 - damping);
-            }
-            const uint64_t idx = (uint64_t)v * K + inst;
-            const bool mass = (a[j].lo | a[j].hi) != 0;
-            if (mass && ((cw[j] >> lv) & 1u)) rowacc[idx] = u128_zero();
-            // rank' = fma(accum, d, [v == seed] * teleport); zero without mass (most vertices early on)
-            double rank = 0.0, pd = 0.0;
-            u128 p = u128_zero();
-            if (seed != NONE && (mass || v == seed)) {
-                rank = __fma_rn(fx_to_double(a[j]), damping, v == seed ? cseed : 0.0);
-                pd = __dmul_rn(rank, __ldg(inv_deg + v));
-                p = fx_from_double(pd);
-                if (p.lo | p.hi) acc = u128_add(acc, u128_mul32(p, __ldg(degree + v)));
-            }
-            if (propd_out) propd_out[idx] = pd;  // the gather converts it to p
-            else *(reinterpret_cast<ulonglong2*>(prop_out) + idx) = make_ulonglong2(p.lo, p.hi);
-            if (rank_out) rank_out[idx] = rank;
-        }
+    } else if (item - nranges < ap.G) {
+        v = ap.seeds[(item - nranges) * K + inst];
+        if (v != NONE && __ldg(rowptr + v + 1) > __ldg(rowptr + v)) v = NONE;
     }
-    s_flush(s_part, S_next, g, inst, acc);
-    __syncthreads();
-    for (uint32_t k = threadIdx.x; k < nslots; k += GT) {
-        const u128 x = s_part[k];
-        if (x.lo | x.hi) u128_atomic_add(S_next + k, x);
+    if (v != NONE) {
+        const uint32_t g = graph_of(ap.voff, ap.G, v), seed = ap.seeds[g * K + inst];
+        if (seed != NONE) ppr_add_S(s_part, ap, g, inst, ppr_finish(ap, v, inst, x, v == seed ? ppr_teleport(ap, g, inst) : 0.0));
     }
+    ppr_flush_S(s_part, nslots, ap);
 }
 
 // ----------------------------------------------------------------------------------------------
@@ -433,18 +477,16 @@ struct grz_batch {
     uint32_t* d_voff;
     uint32_t* d_seeds;                   // [G][K] union vertex IDs or NONE
     // PPR
-    u128* prop[2];                       // [vertex][instance] 4.124 fixed point
-    double* propd[2];                    // the same props as the doubles they convert from exactly
-    int ppr_props;                       // tuning: 0 or 1 fixed point, 2 doubles
-    int ppr_dmode;                       // the captured loop gathers propd
+    pk_t* prop[2];                       // [V + 1][instance], packed; row V zero
+    int ppr_props;                       // tuning, kept for callers: the props are packed whatever it says
     double* rank;
-    u128* rowacc;
-    uint32_t* cut;                       // [V/32] accumulators the apply clears (k_ppr_cutbits)
-    u128* S[2];
+    u128* rowacc;                        // [V][instance]: sums of the cut destinations, zero between iterations
+    uint32_t* ppr_bnd;                   // ranges of k_ppr_step (k_ppr_bounds) and the destinations they cut
+    uint32_t* ppr_cut;
+    u128* S[3];                          // of the props gathered, written, and of the iteration after
     cudaGraphExec_t ppr_exec;
     uint32_t ppr_iters;
     double ppr_damping;
-    int ppr_final;                        // which prop buffer the last replay wrote
     // BFS
     uint8_t* visited;
     uint8_t* frontier;
@@ -458,7 +500,6 @@ struct grz_batch {
     cudaGraphExec_t run_exec;
     uint32_t run_iters;
     double run_damping;
-    int run_dmode;
     unsigned long long* stamps;          // PPR start / end, BFS start / end (%globaltimer, written inside the graph)
     int ppr_blocks, bfs_blocks;          // resident blocks per SM of the persistent kernels
     void* mail;                          // pinned host read-back
@@ -504,16 +545,15 @@ extern "C" int grz_batch_create(grz_batch** out, int device, void* stream)
 
 static void free_state(grz_batch* b)
 {
-    void* p[] = { b->d_voff, b->d_seeds, b->d_roots, b->stamps, b->prop[0], b->prop[1], b->propd[0], b->propd[1], b->rank, b->rowacc, b->cut, b->S[0], b->S[1],
+    void* p[] = { b->d_voff, b->d_seeds, b->d_roots, b->stamps, b->prop[0], b->prop[1], b->rank, b->rowacc, b->ppr_bnd, b->ppr_cut, b->S[0], b->S[1], b->S[2],
                   b->visited, b->frontier, b->next_words, b->level, b->ctl, b->iter };
     for (void* x : p) cudaFree(x);
     b->d_voff = b->d_seeds = b->d_roots = nullptr;
     b->stamps = nullptr;
     b->prop[0] = b->prop[1] = nullptr;
-    b->propd[0] = b->propd[1] = nullptr;
     b->rank = nullptr;
-    b->rowacc = b->S[0] = b->S[1] = nullptr;
-    b->cut = nullptr;
+    b->rowacc = b->S[0] = b->S[1] = b->S[2] = nullptr;
+    b->ppr_bnd = b->ppr_cut = nullptr;
     b->visited = b->frontier = nullptr;
     b->next_words = nullptr;
     b->level = nullptr;
@@ -544,7 +584,7 @@ extern "C" int grz_batch_add_graph(grz_batch* b, uint64_t V, uint64_t E, const u
 {
     if (!b || V == 0 || (E > 0 && !pull_pairs)) return GRZ_ERR_ARG;
     if (b->voff.size() > MAX_GRAPHS) return bset(b, GRZ_ERR_RANGE, "too many graphs");
-    if (V < TV) return bset(b, GRZ_ERR_RANGE, "a batched graph needs at least 32 vertices");
+    if (V < MIN_V) return bset(b, GRZ_ERR_RANGE, "a batched graph needs at least 32 vertices");
     const uint64_t base = b->voff.back();
     if (base + V >= GRZ_HUB_BASE) return bset(b, GRZ_ERR_RANGE, "the union exceeds 2^31 vertices");
     std::vector<uint64_t> p(2 * E);
@@ -614,52 +654,64 @@ static int upload_seeds(grz_batch* b, const uint32_t* local, uint32_t k, uint32_
     return GRZ_OK;
 }
 
-// Enqueues the fixed-length PPR loop (gather + apply per iteration) on cs, which is capturing.
-// Returns the prop buffer the last iteration wrote.
-static int enqueue_ppr_chain(grz_batch* b, cudaStream_t cs, uint32_t iterations, double damping, int dmode, const uint32_t* seeds,
-                             int* final_cur)
+// blocks of k_ppr_step: a step of 16 vectors per warp at least
+static unsigned ppr_grid(const grz_batch* b)
 {
-    grz_graph* u = b->u;
-    const uint32_t V = (uint32_t)u->V, G = (uint32_t)b->Vg.size();
-    // the gather's unit is a warp tile of TV vectors; blocks beyond residency would only queue
-    int gres = 0;
-    const cudaError_t oe = dmode ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&gres, k_ppr_gather<double>, GT, 0)
-                                 : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&gres, k_ppr_gather<u128>, GT, 0);
-    if (oe != cudaSuccess || gres < 1) {
-        cudaGetLastError();
-        gres = 1;
-    }
-    const uint64_t gtiles = (u->pull.nvec + TV - 1) / TV;
-    const unsigned ggrid = persistent_grid(b, (gtiles + GT / 32 - 1) / (GT / 32), std::min(b->ppr_blocks, gres));
-    // GRZ_PPR_APPLY_MINB blocks per SM fit the apply's registers
-    const unsigned agrid = persistent_grid(b, (V + TV - 1) / TV, std::min(b->ppr_blocks, GRZ_PPR_APPLY_MINB));
-    int cur = 0;
-    for (uint32_t it = 0; it < iterations; ++it) {
-        if (dmode)
-            k_ppr_gather<<<ggrid, GT, 0, cs>>>(u->pull.nbr, u->pull.shared, u->pull.nvec, V, b->propd[cur], b->rowacc, b->S[cur ^ 1], G * K);
-        else
-            k_ppr_gather<<<ggrid, GT, 0, cs>>>(u->pull.nbr, u->pull.shared, u->pull.nvec, V, b->prop[cur], b->rowacc, b->S[cur ^ 1], G * K);
-        k_ppr_apply<<<agrid, GT, 0, cs>>>(b->rowacc, b->cut, u->inv_deg, u->degree, V, b->d_voff, G, seeds, damping, b->S[cur],
-                                         b->S[cur ^ 1], b->prop[cur ^ 1], dmode ? b->propd[cur ^ 1] : nullptr,
-                                         it + 1 == iterations ? b->rank : nullptr);
-        cur ^= 1;
-        const int rc = bck(b, cudaGetLastError(), "ppr launch");
-        if (rc) return rc;
-    }
-    *final_cur = cur;
-    return GRZ_OK;
+    const uint64_t steps = (b->u->pull.nvec + 15) / 16;
+    return persistent_grid(b, (steps + GT / 32 - 1) / (GT / 32), std::min(b->ppr_blocks, PPR_RESIDENT));
 }
 
-// the fixed-length PPR iteration loop as one CUDA graph (gather + apply per iteration)
-static int build_ppr_graph(grz_batch* b, uint32_t iterations, double damping, int dmode)
+// the ranges of k_ppr_step, before its graph is captured: a graph's launches have the grid of its capture,
+// and a change of ppr_blocks drops the captured graphs
+static int ppr_ranges(grz_batch* b)
+{
+    grz_graph* u = b->u;
+    const uint32_t nwarps = ppr_grid(b) * (GT / 32), nranges = 4 * nwarps;
+    k_ppr_bounds<<<nwarps / 256 + 1, 256, 0, b->stream>>>(u->pull.shared, (uint32_t)u->pull.nvec, (uint32_t)u->V, nwarps, b->ppr_bnd);
+    k_ppr_cuts<<<(nranges + 255) / 256, 256, 0, b->stream>>>(u->pull.shared, b->ppr_bnd, nranges, b->ppr_cut);
+    return bck(b, cudaGetLastError(), "ppr ranges");
+}
+
+// Enqueues the PPR's initial state and its fixed-length loop (k_ppr_step, k_ppr_rest per iteration) on cs.
+static int enqueue_ppr(grz_batch* b, cudaStream_t cs, uint32_t iterations, double damping)
+{
+    grz_graph* u = b->u;
+    const uint32_t V = (uint32_t)u->V, G = (uint32_t)b->Vg.size(), nvec = (uint32_t)u->pull.nvec;
+    for (pk_t* p : b->prop) BCK(b, cudaMemsetAsync(p, 0, sizeof(pk_t) * (uint64_t)V * K, cs));
+    BCK(b, cudaMemsetAsync(b->rank, 0, sizeof(double) * (uint64_t)V * K, cs));
+    k_ppr_init<<<(G * K + 255) / 256, 256, 0, cs>>>(b->d_seeds, G, u->inv_deg, u->degree, b->prop[0], b->S[0], b->S[1]);
+    const unsigned grid = ppr_grid(b);
+    const uint32_t nranges = 4 * grid * (GT / 32);
+    PprApply ap;
+    ap.inv_deg = u->inv_deg;
+    ap.degree = u->degree;
+    ap.voff = b->d_voff;
+    ap.G = G;
+    ap.seeds = b->d_seeds;
+    ap.damping = damping;
+    for (uint32_t it = 0; it < iterations; ++it) {
+        ap.S = b->S[it % 3];
+        ap.S_next = b->S[(it + 1) % 3];
+        ap.prop_out = b->prop[(it & 1) ^ 1];
+        ap.rank_out = it + 1 == iterations ? b->rank : nullptr;
+        k_ppr_step<<<grid, GT, 0, cs>>>(u->pull.nbr, u->pull.shared, b->ppr_bnd, nvec, V, b->prop[it & 1], b->rowacc, b->S[(it + 2) % 3],
+                                       ap);
+        k_ppr_rest<<<(unsigned)(((uint64_t)(nranges + G) * K + GT - 1) / GT), GT, 0, cs>>>(b->ppr_cut, nranges, u->pull.rowptr, b->rowacc, ap);
+    }
+    return bck(b, cudaGetLastError(), "ppr launch");
+}
+
+// a PPR run as one CUDA graph
+static int build_ppr_graph(grz_batch* b, uint32_t iterations, double damping)
 {
     if (b->ppr_exec) { cudaGraphExecDestroy(b->ppr_exec); b->ppr_exec = nullptr; }
+    const int rr = ppr_ranges(b);
+    if (rr) return rr;
     cudaStream_t cs = nullptr;
     BCK(b, cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking));
     cudaGraph_t graph = nullptr;
-    int cur = 0;
     int rc = bck(b, cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal), "begin capture");
-    if (!rc) rc = enqueue_ppr_chain(b, cs, iterations, damping, dmode, b->d_seeds, &cur);
+    if (!rc) rc = enqueue_ppr(b, cs, iterations, damping);
     const cudaError_t e = cudaStreamEndCapture(cs, &graph);
     if (!rc) rc = bck(b, e, "end capture");
     if (!rc) rc = bck(b, cudaGraphInstantiate(&b->ppr_exec, graph, 0), "instantiate");
@@ -668,33 +720,26 @@ static int build_ppr_graph(grz_batch* b, uint32_t iterations, double damping, in
     if (rc) { b->ppr_exec = nullptr; return rc; }
     b->ppr_iters = iterations;
     b->ppr_damping = damping;
-    b->ppr_final = cur;
-    b->ppr_dmode = dmode;
     return GRZ_OK;
 }
 
-// the PPR state (props, ranks, accumulators, straddle bits), allocated on first use
-static int ppr_alloc(grz_batch* b, int dmode)
+// the PPR state (props, ranks, accumulators), allocated on first use
+static int ppr_alloc(grz_batch* b)
 {
-    grz_graph* u = b->u;
-    const uint64_t V = u->V;
+    const uint64_t V = b->u->V;
     const uint32_t G = (uint32_t)b->Vg.size();
-    if (!b->prop[0]) {
-        BCK(b, cudaMalloc((void**)&b->prop[0], sizeof(u128) * V * K));
-        BCK(b, cudaMalloc((void**)&b->prop[1], sizeof(u128) * V * K));
-        BCK(b, cudaMalloc((void**)&b->rank, sizeof(double) * V * K));
-        BCK(b, cudaMalloc((void**)&b->rowacc, sizeof(u128) * (V + 1) * K));
-        BCK(b, cudaMalloc((void**)&b->S[0], sizeof(u128) * G * K));
-        BCK(b, cudaMalloc((void**)&b->S[1], sizeof(u128) * G * K));
-        BCK(b, cudaMemsetAsync(b->rowacc, 0, sizeof(u128) * (V + 1) * K, b->stream));
-        BCK(b, cudaMalloc((void**)&b->cut, sizeof(uint32_t) * ((V + 31) / 32)));
-        k_ppr_cutbits<<<(unsigned)((V + 255) / 256), 256, 0, b->stream>>>(u->pull.rowptr, (uint32_t)V, b->cut);
-        BCK(b, cudaGetLastError());
+    if (b->prop[0]) return GRZ_OK;
+    for (pk_t*& p : b->prop) {
+        BCK(b, cudaMalloc((void**)&p, sizeof(pk_t) * (V + 1) * K));
+        BCK(b, cudaMemsetAsync(p + V * K, 0, sizeof(pk_t) * K, b->stream));
     }
-    if (dmode && !b->propd[0]) {
-        BCK(b, cudaMalloc((void**)&b->propd[0], sizeof(double) * V * K));
-        BCK(b, cudaMalloc((void**)&b->propd[1], sizeof(double) * V * K));
-    }
+    BCK(b, cudaMalloc((void**)&b->rank, sizeof(double) * V * K));
+    BCK(b, cudaMalloc((void**)&b->rowacc, sizeof(u128) * V * K));
+    const uint64_t max_ranges = 4ull * (GT / 32) * b->u->num_sms * PPR_RESIDENT;
+    BCK(b, cudaMalloc((void**)&b->ppr_bnd, sizeof(uint32_t) * (max_ranges + 1)));
+    BCK(b, cudaMalloc((void**)&b->ppr_cut, sizeof(uint32_t) * max_ranges));
+    for (u128*& x : b->S) BCK(b, cudaMalloc((void**)&x, sizeof(u128) * G * K));
+    BCK(b, cudaMemsetAsync(b->rowacc, 0, sizeof(u128) * V * K, b->stream));
     return GRZ_OK;
 }
 
@@ -708,20 +753,12 @@ extern "C" int grz_batch_ppr(grz_batch* b, const uint32_t* seeds, uint32_t k, ui
     BCK(b, cudaSetDevice(b->device));
     grz_graph* u = b->u;
     const uint64_t V = u->V;
-    const uint32_t G = (uint32_t)b->Vg.size();
-    // Doubles gathered instead of 16-byte fixed point only when chosen: each row of a source's 8
-    // instances is 64 bytes instead of 128, and the gather converts each double exactly to the
-    // fixed point the apply would have stored, so the sums and results are the same bit for bit.
-    // The gather is bound by L1TEX and instructions, not DRAM, so the conversions cost more than
-    // the halved rows save: GB300, the 32-graph batch (1.9 GB of fixed-point rows, 15x L2), 256
-    // instances x 20 iterations: 101 ms fixed point, 155 ms doubles.
-    const int dmode = b->ppr_props == 2;
-    int rc = ppr_alloc(b, dmode);
+    int rc = ppr_alloc(b);
     if (rc) return rc;
     rc = upload_seeds(b, seeds, k);
     if (rc) return rc;
-    if (!b->ppr_exec || b->ppr_iters != iterations || b->ppr_damping != damping || b->ppr_dmode != dmode) {
-        rc = build_ppr_graph(b, iterations, damping, dmode);
+    if (!b->ppr_exec || b->ppr_iters != iterations || b->ppr_damping != damping) {
+        rc = build_ppr_graph(b, iterations, damping);
         if (rc) return rc;
     }
     cudaEvent_t e0, e1;
@@ -729,13 +766,6 @@ extern "C" int grz_batch_ppr(grz_batch* b, const uint32_t* seeds, uint32_t k, ui
     BCK(b, cudaEventCreate(&e1));
     cudaStream_t st = b->stream;
     rc = bck(b, cudaEventRecord(e0, st), "event");
-    if (!rc && dmode) rc = bck(b, cudaMemsetAsync(b->propd[0], 0, sizeof(double) * V * K, st), "memset");
-    if (!rc && !dmode) rc = bck(b, cudaMemsetAsync(b->prop[0], 0, sizeof(u128) * V * K, st), "memset");
-    if (!rc) {
-        k_ppr_init<<<(G * K + 255) / 256, 256, 0, st>>>(b->d_seeds, G, u->inv_deg, u->degree, b->prop[0], dmode ? b->propd[0] : nullptr,
-                                                        b->S[0]);
-        rc = bck(b, cudaGetLastError(), "ppr init");
-    }
     if (!rc) rc = bck(b, cudaGraphLaunch(b->ppr_exec, st), "graph launch");
     if (!rc) rc = bck(b, cudaEventRecord(e1, st), "event");
     if (!rc && ranks_out) {
@@ -846,10 +876,12 @@ static int end_capture_sink(grz_batch* b, cudaStream_t cs, cudaGraphNode_t* sink
 // PPR and multi-source BFS as one CUDA graph with two independent branches, each from its initial
 // state to its results: branch 1 the PPR loop (d_seeds), branch 2 the BFS loop (d_roots).  Event
 // records at both ends of each branch time them inside the one launch.
-static int build_run_graph(grz_batch* b, uint32_t iterations, double damping, int dmode)
+static int build_run_graph(grz_batch* b, uint32_t iterations, double damping)
 {
     if (b->run_exec) { cudaGraphExecDestroy(b->run_exec); b->run_exec = nullptr; }
     if (!b->stamps) BCK(b, cudaMalloc((void**)&b->stamps, 4 * sizeof(unsigned long long)));
+    const int rr = ppr_ranges(b);
+    if (rr) return rr;
     grz_graph* u = b->u;
     const uint64_t V = u->V;
     const uint64_t Vw = (V + 3) / 4 * 4;
@@ -858,17 +890,11 @@ static int build_run_graph(grz_batch* b, uint32_t iterations, double damping, in
     BCK(b, cudaGraphCreate(&top, 0));
     cudaStream_t cs = nullptr;
     int rc = bck(b, cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking), "stream");
-    int cur = 0;
     // branch 1: PPR
     if (!rc) rc = bck(b, cudaStreamBeginCaptureToGraph(cs, top, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal), "capture");
     if (!rc) {
         k_stamp<<<1, 1, 0, cs>>>(b->stamps + 0);
-        if (dmode) cudaMemsetAsync(b->propd[0], 0, sizeof(double) * V * K, cs);
-        else cudaMemsetAsync(b->prop[0], 0, sizeof(u128) * V * K, cs);
-        k_ppr_init<<<(G * K + 255) / 256, 256, 0, cs>>>(b->d_seeds, G, u->inv_deg, u->degree, b->prop[0], dmode ? b->propd[0] : nullptr,
-                                                        b->S[0]);
-        rc = bck(b, cudaGetLastError(), "ppr init");
-        if (!rc) rc = enqueue_ppr_chain(b, cs, iterations, damping, dmode, b->d_seeds, &cur);
+        rc = enqueue_ppr(b, cs, iterations, damping);
         k_stamp<<<1, 1, 0, cs>>>(b->stamps + 1);
         const int rc2 = end_capture_sink(b, cs, nullptr);
         if (!rc) rc = rc2;
@@ -902,8 +928,6 @@ static int build_run_graph(grz_batch* b, uint32_t iterations, double damping, in
     if (rc) { b->run_exec = nullptr; return rc; }
     b->run_iters = iterations;
     b->run_damping = damping;
-    b->run_dmode = dmode;
-    b->ppr_final = cur;
     return GRZ_OK;
 }
 
@@ -987,14 +1011,13 @@ extern "C" int grz_batch_run(grz_batch* b, const uint32_t* seeds, uint32_t k, ui
     BCK(b, cudaSetDevice(b->device));
     grz_graph* u = b->u;
     const uint64_t V = u->V;
-    const int dmode = b->ppr_props == 2;
-    int rc = ppr_alloc(b, dmode);
+    int rc = ppr_alloc(b);
     if (!rc) rc = bfs_alloc(b);
     if (!rc) rc = upload_seeds(b, seeds, k, b->d_seeds);
     if (!rc) rc = upload_seeds(b, roots, kb, b->d_roots);
     if (rc) return rc;
-    if (!b->run_exec || b->run_iters != iterations || b->run_damping != damping || b->run_dmode != dmode) {
-        rc = build_run_graph(b, iterations, damping, dmode);
+    if (!b->run_exec || b->run_iters != iterations || b->run_damping != damping) {
+        rc = build_run_graph(b, iterations, damping);
         if (rc) return rc;
     }
     cudaStream_t st = b->stream;
@@ -1051,8 +1074,8 @@ extern "C" int grz_batch_tune_set(grz_batch* b, int param, int64_t value)
 {
     if (!b) return GRZ_ERR_ARG;
     if (param == GRZ_BATCH_TUNE_PPR_PROPS) {
-        if (value < 0 || value > 2) return bset(b, GRZ_ERR_RANGE, "PPR props must be 0 (by size), 1 (fixed point) or 2 (doubles)");
-        b->ppr_props = (int)value;  // the next run captures its loop again if the mode changes
+        if (value < 0 || value > 2) return bset(b, GRZ_ERR_RANGE, "PPR props must be 0, 1 or 2");
+        b->ppr_props = (int)value;
         return GRZ_OK;
     }
     if (value < 1 || value > 32) return bset(b, GRZ_ERR_RANGE, "blocks per SM must be 1..32");

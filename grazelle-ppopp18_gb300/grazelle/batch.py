@@ -104,8 +104,8 @@ class Batch:
         return split(ranks), split(levels), sp, sb, tot.value
 
     def tune(self, ppr_blocks: int | None = None, bfs_blocks: int | None = None, ppr_props: int | None = None):
-        """Resident blocks per SM of the persistent batch kernels, and the props the PPR gather
-        reads (0 or 1 fixed point, 2 doubles); results never depend on them."""
+        """Resident blocks per SM of the persistent batch kernels (results never depend on them);
+        `ppr_props` (0, 1 or 2) is kept but has no effect: the PPR gather reads packed props."""
         for p, v in ((native.BATCH_TUNE_PPR_BLOCKS, ppr_blocks), (native.BATCH_TUNE_BFS_BLOCKS, bfs_blocks),
                      (native.BATCH_TUNE_PPR_PROPS, ppr_props)):
             if v is not None:

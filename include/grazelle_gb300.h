@@ -203,10 +203,10 @@ int grz_batch_run(grz_batch* b, const uint32_t* seeds, uint32_t k, uint32_t iter
                   uint32_t kb, double* ranks_out, int32_t* levels_out, grz_run_stats_t* ppr_stats, grz_run_stats_t* bfs_stats,
                   float* total_ms);
 /* kernel shapes of a batch (results never depend on them): resident blocks per SM of the
- * persistent PPR gather / apply and multi-source BFS pull kernels, 1..32 (default 8) */
+ * persistent PPR and multi-source BFS pull kernels, 1..32 (default 8; the PPR kernel has at most 4) */
 #define GRZ_BATCH_TUNE_PPR_BLOCKS 0
 #define GRZ_BATCH_TUNE_BFS_BLOCKS 1
-#define GRZ_BATCH_TUNE_PPR_PROPS 2   /* props the PPR gather reads: 0 (default) or 1 = 16-byte fixed point, 2 = 8-byte doubles converted on the gather (measured slower: the gather is not DRAM-bound); results identical */
+#define GRZ_BATCH_TUNE_PPR_PROPS 2   /* 0, 1 or 2; kept, but without effect: the PPR gather reads packed 8-byte props */
 int grz_batch_tune_set(grz_batch* b, int param, int64_t value);
 int grz_batch_tune_get(const grz_batch* b, int param, int64_t* value);
 unsigned long long grz_batch_launch_count(const grz_batch* b);
