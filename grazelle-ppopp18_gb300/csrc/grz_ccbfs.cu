@@ -1010,7 +1010,12 @@ __global__ void __launch_bounds__(T) k_cc_pull_expand(const uint32_t* __restrict
 // (k_bfs_pull_expand, then k_bfs_visit) reads the rest of its vectors.  A warp owns FW whole
 // bitmap words (64 destinations each; lane l of slot q holds destination 64 w0 + 32 q + l), so
 // it writes their WantsInfo, HasInfo* and unres words without atomics, and the first-vector
-// loads of its 2 FW slots are issued together.
+// loads of its 2 FW slots are issued together.  Where at most 32 of the 64 FW destinations are
+// wanted, each lane takes one of them instead (late pulls: bound by instructions spent on empty
+// slots).  GB300, R-MAT of 2^24 vertices, the pulls of one run: 156, 65 and 42 us with slots only,
+// 154, 45 and 22 us so.  The first is near what its row pointers, first vectors, degrees, parents and
+// levels take at the memory's rate (106 us); probing the frontier bits in two or four steps, loading a
+// word ahead, and 1 or 4 words per warp gave nothing.
 
 __global__ void __launch_bounds__(T, GRZ_BFS_MINB) k_bfs_pull_first(unsigned long long* __restrict__ wants,
                                                       const unsigned long long* __restrict__ nonempty,
@@ -1024,8 +1029,11 @@ __global__ void __launch_bounds__(T, GRZ_BFS_MINB) k_bfs_pull_first(unsigned lon
                                                       unsigned long long* __restrict__ vote)
 {
     __shared__ unsigned long long red[T / 32];
+    __shared__ uint8_t s_bit[T / 32][32];
     constexpr int Q = 2 * FW;
     const int lane = threadIdx.x & 31;
+    uint8_t* const bit_at = s_bit[threadIdx.x >> 5];
+    const uint32_t below = (1u << lane) - 1u;
     const uint32_t iter = iter_dev ? *iter_dev : iter_host;
     unsigned long long my_vote = 0;
     // the largest frontier source of vector `vec`, or INF without one
@@ -1039,57 +1047,91 @@ __global__ void __launch_bounds__(T, GRZ_BFS_MINB) k_bfs_pull_first(unsigned lon
         // lanes ascend by source: the largest frontier source is the last lane with one
         return in[3] ? ids[3] : in[2] ? ids[2] : in[1] ? ids[1] : in[0] ? ids[0] : INF;
     };
+    auto visit = [&](uint32_t v, uint32_t p) {
+        parent[v] = p;
+        level[v] = iter;
+        my_vote += vc.of(v);
+    };
     const uint64_t nwarps = (uint64_t)gridDim.x * (T / 32);
     for (uint64_t w0 = ((uint64_t)blockIdx.x * (T / 32) + (threadIdx.x >> 5)) * FW; w0 < W; w0 += nwarps * FW) {  // warp-uniform
-        unsigned long long sel[FW];
+        // bit `lane` of word q: destination 64 w0 + 32 q + lane (words past the bitmap are empty)
+        uint32_t sel[Q], total = 0;
 #pragma unroll
-        for (int f = 0; f < FW; ++f) sel[f] = w0 + f < W ? wants[w0 + f] & nonempty[w0 + f] : 0ull;
-        uint32_t r0[Q], n[Q];
-#pragma unroll
-        for (int q = 0; q < Q; ++q) {
-            const uint64_t v = 64 * w0 + 32 * (uint64_t)q + lane;
-            n[q] = 0;
-            if (v < V && ((sel[q >> 1] >> (32 * (q & 1) + lane)) & 1ull)) {
-                r0[q] = rowptr[v];
-                n[q] = rowptr[v + 1] - r0[q];
-            }
+        for (int f = 0; f < FW; ++f) {
+            const unsigned long long x = w0 + f < W ? wants[w0 + f] & nonempty[w0 + f] : 0ull;
+            sel[2 * f] = (uint32_t)x;
+            sel[2 * f + 1] = (uint32_t)(x >> 32);
+            total += __popcll(x);
         }
-        uint32_t p[Q];
+        uint32_t hn[Q], un[Q];
 #pragma unroll
-        for (int q = 0; q < Q; ++q) p[q] = n[q] ? vec_best(r0[q]) : INF;
+        for (int q = 0; q < Q; ++q) hn[q] = un[q] = 0u;
+        if (total > 32) {
+            uint32_t r0[Q], n[Q], p[Q];
 #pragma unroll
-        for (int q = 0; q < Q; ++q) {
-            const uint32_t m = min(n[q], first_n);
-            for (uint32_t j = 1; j < m && p[q] == INF; ++j) p[q] = vec_best(r0[q] + j);
-        }
-        unsigned long long un[FW], hn[FW];
-#pragma unroll
-        for (int f = 0; f < FW; ++f) un[f] = hn[f] = 0ull;
-#pragma unroll
-        for (int q = 0; q < Q; ++q) {
-            const uint32_t v = (uint32_t)(64 * w0 + 32 * (uint64_t)q + lane);
-            const bool hit = p[q] != INF;
-            if (hit) {
-                parent[v] = p[q];
-                level[v] = iter;
-                my_vote += vc.of(v);
+            for (int q = 0; q < Q; ++q) {
+                const uint64_t v = 64 * w0 + 32 * (uint64_t)q + lane;
+                n[q] = 0;
+                if ((sel[q] >> lane) & 1u) {
+                    r0[q] = rowptr[v];
+                    n[q] = rowptr[v + 1] - r0[q];
+                }
             }
-            const unsigned mh = __ballot_sync(0xffffffffu, hit);
-            const unsigned mu = __ballot_sync(0xffffffffu, !hit && n[q] > first_n);
-            hn[q >> 1] |= (unsigned long long)mh << (32 * (q & 1));
-            un[q >> 1] |= (unsigned long long)mu << (32 * (q & 1));
+#pragma unroll
+            for (int q = 0; q < Q; ++q) p[q] = n[q] ? vec_best(r0[q]) : INF;
+#pragma unroll
+            for (int q = 0; q < Q; ++q) {
+                const uint32_t m = min(n[q], first_n);
+                for (uint32_t j = 1; j < m && p[q] == INF; ++j) p[q] = vec_best(r0[q] + j);
+            }
+#pragma unroll
+            for (int q = 0; q < Q; ++q) {
+                const bool hit = p[q] != INF;
+                if (hit) visit((uint32_t)(64 * w0 + 32 * (uint64_t)q + lane), p[q]);
+                hn[q] = __ballot_sync(0xffffffffu, hit);
+                un[q] = __ballot_sync(0xffffffffu, !hit && n[q] > first_n);
+            }
+        } else if (total) {
+            // few: lane i takes the i-th
+            uint32_t base = 0;
+#pragma unroll
+            for (int q = 0; q < Q; ++q) {
+                if ((sel[q] >> lane) & 1u) bit_at[base + __popc(sel[q] & below)] = (uint8_t)(32 * q + lane);
+                base += __popc(sel[q]);
+            }
+            __syncwarp();
+            uint32_t bit = 0, p = INF, n = 0;
+            if (lane < total) {
+                bit = bit_at[lane];
+                const uint32_t v = (uint32_t)(64 * w0) + bit, r0 = rowptr[v];
+                n = rowptr[v + 1] - r0;
+                const uint32_t m = min(n, first_n);
+                for (uint32_t j = 0; j < m && p == INF; ++j) p = vec_best(r0 + j);
+                if (p != INF) visit(v, p);
+            }
+            const bool hit = p != INF, open = !hit && n > first_n;
+            if (__any_sync(0xffffffffu, hit || open)) {
+#pragma unroll
+                for (int q = 0; q < Q; ++q) {
+                    const uint32_t m = (int)(bit >> 5) == q ? 1u << (bit & 31u) : 0u;
+                    hn[q] = __reduce_or_sync(0xffffffffu, hit ? m : 0u);
+                    un[q] = __reduce_or_sync(0xffffffffu, open ? m : 0u);
+                }
+            }
         }
         if (lane == 0) {
 #pragma unroll
             for (int f = 0; f < FW; ++f) {
                 if (w0 + f >= W) break;
-                unres[w0 + f] = un[f];
-                if (hn[f]) {
-                    has_next[w0 + f] |= hn[f];
-                    wants[w0 + f] &= ~hn[f];
+                const unsigned long long h = (unsigned long long)hn[2 * f + 1] << 32 | hn[2 * f];
+                unres[w0 + f] = (unsigned long long)un[2 * f + 1] << 32 | un[2 * f];
+                if (h) {
+                    has_next[w0 + f] |= h;
+                    wants[w0 + f] &= ~h;
                 }
             }
         }
+        __syncwarp();
     }
     my_vote = block_sum_u64(my_vote, red);
     if (threadIdx.x == 0) vote_add(vote, my_vote);

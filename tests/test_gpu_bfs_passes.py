@@ -1,0 +1,80 @@
+"""BFS passes at the edges of their forms, compared exactly.
+
+The first-vector pull takes 128 destinations per warp, one per lane slot or, when at most 32 are wanted,
+packed: against the pull without that pass (bfs_pull_first 0), for groups of 0 to 128 wanted
+destinations.  The push appends up to 128 first touches per warp at once and stops when the visit will
+sweep: a pushed vertex's parent is the smallest of its frontier sources, whatever the order.
+"""
+import numpy as np
+import pytest
+
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+COUNTS = [0, 1, 2, 31, 32, 33, 64, 127, 128]
+
+
+def groups(seed):
+    """groups of 128 vertices, of which COUNTS[i] have in-edges: 1 to 12 of them, from anywhere"""
+    from grazelle import graphgen as gg
+    rng = np.random.RandomState(seed)
+    V = 128 * len(COUNTS) * 4 + 37
+    src, dst = [], []
+    for i in range(V // 128):
+        for v in 128 * i + rng.permutation(128)[:COUNTS[i % len(COUNTS)]]:
+            n = rng.choice([1, 4, 5, 12])
+            src += list(rng.randint(0, V, n))
+            dst += [v] * n
+    src += [0] * 50
+    dst += list(rng.randint(0, V, 50))
+    e = np.unique(np.stack([dst, src], 1), axis=0)
+    return gg.EdgeList(V, e[:, 1].astype(np.uint64), e[:, 0].astype(np.uint64))
+
+
+@pytest.mark.parametrize("hubs", [0, 16])
+@pytest.mark.parametrize("first", [1, 2])
+def test_pull_first_densities(first, hubs):
+    from grazelle import native
+    from grazelle.engine import Graph
+    for seed in (1, 2):
+        g = groups(seed)
+        pull, push = g.pull_order().pairs(), g.push_order().pairs()
+        with Graph(0) as A, Graph(0) as B:
+            A.tune(bfs_pull_first=first, hubs=hubs)
+            B.tune(bfs_pull_first=0)
+            for G in (A, B):
+                G.load_pairs(g.num_vertices, pull, push)
+            for r in (0, int(g.src[5]), g.num_vertices - 1):
+                for flags in (native.FORCE_PULL, native.FORCE_PULL | native.FLAG_HOST_LOOP, 0):
+                    (pa, la), (pb, lb) = A.bfs(r, flags), B.bfs(r, flags)
+                    np.testing.assert_array_equal(la, lb)
+                    np.testing.assert_array_equal(pa, pb)
+                np.testing.assert_array_equal(la, O.bfs_levels(push, g.num_vertices, r))
+
+
+@pytest.mark.parametrize("n,mid,fan", [(300, 3, 40), (70000, 300, 300), (70000, 2, 60000), (1000000, 5000, 700)])
+def test_push_parents(n, mid, fan):
+    """0 -> `mid` vertices -> `fan` random vertices each (many of them shared, in one vector too) -> 0"""
+    from grazelle import graphgen as gg, native
+    from grazelle.engine import Graph
+    rng = np.random.RandomState(n % 1000 + mid)
+    m = 1 + np.arange(mid)
+    src = np.concatenate([np.zeros(mid, dtype=np.int64), np.repeat(m, fan), np.arange(mid + 1, n)])
+    dst = np.concatenate([m, rng.randint(0, n, mid * fan), np.zeros(n - mid - 1, dtype=np.int64)])
+    e = np.unique(src * n + dst)
+    src, dst = e // n, e % n
+    g = gg.EdgeList(n, src.astype(np.uint64), dst.astype(np.uint64))
+    with Graph(0) as G:
+        G.load_pairs(n, g.pull_order().pairs(), g.push_order().pairs())
+        for flags in (native.FORCE_PUSH, native.FORCE_PUSH | native.FLAG_HOST_LOOP):
+            par, lv = G.bfs(0, flags)
+            tree = lv[src] + 1 == lv[dst]
+            tree &= lv[src] >= 0
+            ref = np.full(n, n, dtype=np.int64)
+            np.minimum.at(ref, dst[tree], src[tree])
+            seen = lv > 0
+            np.testing.assert_array_equal(par[seen].astype(np.int64), ref[seen])
+            assert lv[0] == 0 and (lv[m] == 1).all() and seen.sum() == (ref < n).sum()
+        lab = G.connected_components(native.FORCE_PUSH)
+        np.testing.assert_array_equal(lab, G.connected_components(native.FORCE_PULL))
