@@ -114,6 +114,30 @@ __device__ __forceinline__ void touched_append(bool pred, uint32_t val, uint32_t
     if (pred) list[base + __popc(m & ((1u << lane) - 1u))] = val;
 }
 
+// the same for four values per lane, in one atomicAdd
+__device__ __forceinline__ void touched_append4(const bool (&pred)[4], const uint32_t (&val)[4], uint32_t* __restrict__ list,
+                                                uint32_t* __restrict__ count, bool full)
+{
+    if (full) return;
+    unsigned m[4];
+    uint32_t n = 0;
+#pragma unroll
+    for (int l = 0; l < 4; ++l) {
+        m[l] = __ballot_sync(0xffffffffu, pred[l]);
+        n += __popc(m[l]);
+    }
+    if (!n) return;
+    const uint32_t lane = threadIdx.x & 31;
+    uint32_t base = 0;
+    if (lane == 0) base = atomicAdd(count, n);
+    base = __shfl_sync(0xffffffffu, base, 0);
+#pragma unroll
+    for (int l = 0; l < 4; ++l) {
+        if (pred[l]) list[base + __popc(m[l] & ((1u << lane) - 1u))] = val[l];
+        base += __popc(m[l]);
+    }
+}
+
 __device__ __forceinline__ unsigned long long now_ns()
 {
     unsigned long long t;
@@ -593,8 +617,12 @@ __global__ void __launch_bounds__(T) k_bfs_pull(const uint4* __restrict__ nbr, c
 // are spread over many blocks.  tile_first[t] is the frontier entry that owns the first vector
 // of tile t.  Passes: k_fr_compact (frontier entries, their vector offsets and the tile owners),
 // k_push_expand.
+//
+// A tile is one vector per thread: a long tile's vectors would wait for each other, and small frontiers
+// would leave most of the chip idle.  GB300, tiles of 1024, 512 and 256 vectors: the pushes of 8 BFS runs
+// on an R-MAT graph of 2^24 vertices 815, 743 and 687 us, CC of 4096 vertices 148, 140 and 136 us.
 
-constexpr uint32_t PUSH_TILE = 1024;
+constexpr uint32_t PUSH_TILE = T;
 
 // Each block takes CCHUNK consecutive vertices, each thread one 32-vertex word of the two bitmaps
 // (HasInfo and out-vectors for push; WantsInfo, or the destinations a first pass left open, and
@@ -687,12 +715,21 @@ __global__ void __launch_bounds__(T) k_fr_compact(const unsigned long long* __re
                 const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
                 if (lane >= o) x += y;
             }
+            const uint32_t p = pos + __popc(b & ((1u << lane) - 1u)), o = vo + x - cnt[q];
+            uint32_t t0 = 0, t1 = 0;  // tiles whose first vector is the entry's
             if ((b >> lane) & 1u) {
-                const uint32_t p = pos + __popc(b & ((1u << lane) - 1u)), o = vo + x - cnt[q];
                 frontier[p] = vbase + 32u * (j + q);
                 voff[p] = o;
                 vdelta[p] = r0[q] - o;
-                for (uint64_t t = ((uint64_t)o + PUSH_TILE - 1) / PUSH_TILE; t * PUSH_TILE < (uint64_t)o + cnt[q]; ++t) tile_first[t] = p;
+                t0 = (uint32_t)(((uint64_t)o + PUSH_TILE - 1) / PUSH_TILE);
+                t1 = (uint32_t)(((uint64_t)o + cnt[q] + PUSH_TILE - 1) / PUSH_TILE);
+                if (t1 - t0 <= 4)
+                    for (; t0 < t1; ++t0) tile_first[t0] = p;
+            }
+            for (unsigned hubs = __ballot_sync(0xffffffffu, t0 < t1); hubs; hubs &= hubs - 1) {  // the warp writes a hub's
+                const int h = __ffs(hubs) - 1;
+                const uint32_t hp = __shfl_sync(0xffffffffu, p, h), h1 = __shfl_sync(0xffffffffu, t1, h);
+                for (uint32_t t = __shfl_sync(0xffffffffu, t0, h) + lane; t < h1; t += 32) tile_first[t] = hp;
             }
             pos += __popc(b);
             vo += __shfl_sync(0xffffffffu, x, 31);
@@ -703,6 +740,10 @@ __global__ void __launch_bounds__(T) k_fr_compact(const unsigned long long* __re
 // Expand the compacted frontier, one tile of PUSH_TILE vectors at a time (grid-stride over
 // tiles; the totals stay on the device).  The tile's owners are staged in shared memory and
 // each vector finds its owner by a binary search there.
+// Bound by the latency of the random loads and atomics, so those of a vector's four destinations are
+// issued together, and the touched list's counter, one address for the whole chip, gets one add per warp
+// and vector and is looked at again each time.  GB300, R-MAT of 2^24 vertices, the largest push of a run
+// (with tiles of 1024 vectors before): 422 us one destination after the other, 177 us so.
 template <bool IsBfs>
 __global__ void __launch_bounds__(T) k_push_expand(const uint32_t* __restrict__ frontier, const uint32_t* __restrict__ voff,
                                                    const uint32_t* __restrict__ vdelta, const uint32_t* __restrict__ tile_first,
@@ -720,7 +761,6 @@ __global__ void __launch_bounds__(T) k_push_expand(const uint32_t* __restrict__ 
     __shared__ uint32_t s_off[PUSH_TILE];
     __shared__ uint32_t s_delta[PUSH_TILE];
     __shared__ unsigned long long red[T / 32];
-    __shared__ bool s_full;  // BFS: the touched list is long enough for the visit to sweep (read per tile)
     const uint32_t nf = counters[3], total = counters[2];
     const uint32_t ntiles = (total + PUSH_TILE - 1) / PUSH_TILE;
     unsigned long long my_vote = 0;
@@ -735,7 +775,6 @@ __global__ void __launch_bounds__(T) k_push_expand(const uint32_t* __restrict__ 
             s_src[i] = frontier[first + i];
             s_delta[i] = vdelta[first + i];
         }
-        if (IsBfs && threadIdx.x == 0) s_full = touched_full(ntouched, V);
         __syncthreads();
         for (uint32_t base = t0; base < tend; base += T) {  // warp-uniform trip count
             const uint32_t gv = base + threadIdx.x;
@@ -752,30 +791,40 @@ __global__ void __launch_bounds__(T) k_push_expand(const uint32_t* __restrict__ 
                 s = __ldcs(nbr + (uint32_t)(gv + s_delta[lo]));
             }
             const uint32_t ids[4] = { s.x, s.y, s.z, s.w };
+            // the loads, then the atomics, of the four destinations together
+            bool ok[4];
+            uint32_t old[4];
             if (IsBfs) {
+                const bool full = touched_full(ntouched, V);
+#pragma unroll
+                for (int l = 0; l < 4; ++l) ok[l] = ids[l] < V && bit_of(wants, ids[l]);
+#pragma unroll
+                for (int l = 0; l < 4; ++l) old[l] = ok[l] ? cand32[ids[l]] : 0u;
+#pragma unroll
+                for (int l = 0; l < 4; ++l) old[l] = u < old[l] ? atomicMin(cand32 + ids[l], u) : 0u;
 #pragma unroll
                 for (int l = 0; l < 4; ++l) {
-                    const uint32_t d = ids[l];
-                    bool first_touch = false;
-                    if (d < V && bit_of(wants, d) && u < cand32[d]) {
-                        first_touch = atomicMin(cand32 + d, u) == INF;
-                        if (first_touch) atomicOr(has_next + (d >> 6), 1ull << (d & 63));
-                    }
-                    touched_append(first_touch, d, touched, ntouched, s_full);
+                    ok[l] = old[l] == INF;  // the first touch
+                    if (ok[l]) atomicOr(has_next + (ids[l] >> 6), 1ull << (ids[l] & 63));
                 }
+                touched_append4(ok, ids, touched, ntouched, __shfl_sync(0xffffffffu, full, 0));
             } else if (live) {
                 const uint32_t msg = label[u];
 #pragma unroll
+                for (int l = 0; l < 4; ++l) old[l] = ids[l] < V ? label[ids[l]] : 0u;
+#pragma unroll
+                for (int l = 0; l < 4; ++l) old[l] = msg < old[l] ? atomicMin(label + ids[l], msg) : 0u;
+#pragma unroll
                 for (int l = 0; l < 4; ++l) {
-                    const uint32_t d = ids[l];
-                    if (d < V && msg < label[d]) {
-                        const uint32_t old = atomicMin(label + d, msg);
-                        if (msg < old) {
-                            my_min = min(my_min, msg);
-                            if (bit_set_first(has_next, d)) my_vote += vc.of(d);
-                        }
+                    ok[l] = msg < old[l];
+                    if (ok[l]) {
+                        my_min = min(my_min, msg);
+                        ok[l] = bit_set_first(has_next, ids[l]);
                     }
                 }
+#pragma unroll
+                for (int l = 0; l < 4; ++l)
+                    if (ok[l]) my_vote += vc.of(ids[l]);
             }
         }
         __syncthreads();
@@ -792,13 +841,13 @@ __global__ void __launch_bounds__(T) k_push_expand(const uint32_t* __restrict__ 
 // concatenation, so the per-destination minimum candidate (the reference's parent rule, as in
 // k_bfs_pull) is reduced within the warp before one atomicMin.
 // Early exit: the candidate is (first vector with a frontier source, ~largest such source), so
-// once a destination has a candidate, its later vectors cannot win.  Blocks take runs of
-// PULL_CHUNK consecutive tiles from a queue (balanced, and a long destination's tiles are
-// processed roughly in order), and a vector past its destination's first LONG_RUN vectors is
+// once a destination has a candidate, its later vectors cannot win.  Blocks take their first tile
+// by number and the next from a queue, asked for while the tile before is worked on (balanced, and a long
+// destination's tiles are processed roughly in order; runs of 2, 4 and 8 tiles: CC of 4096 vertices 136,
+// 139 and 149 us, single ones 124), and a vector past its destination's first LONG_RUN vectors is
 // skipped (no neighbour or frontier reads) when the candidate already names an earlier vector.
 // In R-MAT the sources of a destination ascend and the hubs have small IDs, so a long
 // destination next to a frontier hub stops after its first vectors.
-constexpr uint32_t PULL_CHUNK = 2;  // GB300 sweep of 2-16 (queue of runs): 2 keeps small pulls cheapest
 constexpr uint32_t LONG_RUN = 32;
 
 __global__ void __launch_bounds__(T) k_bfs_pull_expand(const uint32_t* __restrict__ dests, const uint32_t* __restrict__ voff,
@@ -813,85 +862,81 @@ __global__ void __launch_bounds__(T) k_bfs_pull_expand(const uint32_t* __restric
     __shared__ uint32_t s_dst[PUSH_TILE];
     __shared__ uint32_t s_off[PUSH_TILE];
     __shared__ uint32_t s_delta[PUSH_TILE];
-    __shared__ uint32_t s_chunk;
+    __shared__ uint32_t s_tile;
     __shared__ bool s_full;  // the touched list is long enough for the visit to sweep (read per tile)
     const uint32_t nd = counters[3], total = counters[2];
     const uint32_t ntiles = (total + PUSH_TILE - 1) / PUSH_TILE;
     const int lane = threadIdx.x & 31;
-    for (;;) {
-        if (threadIdx.x == 0) s_chunk = atomicAdd(queue, 1u);
-        __syncthreads();
-        const uint32_t chunk = s_chunk;
-        __syncthreads();  // every thread has read s_chunk before it is replaced
-        if ((uint64_t)chunk * PULL_CHUNK >= ntiles) break;
-        const uint32_t chunk_end = min(ntiles, (chunk + 1) * PULL_CHUNK);
-        for (uint32_t tile = chunk * PULL_CHUNK; tile < chunk_end; ++tile) {
-            const uint32_t first = tile_first[tile];
-            const uint32_t t0 = tile * PUSH_TILE;
-            const uint32_t tend = min(total, t0 + PUSH_TILE);
-            const uint32_t nw = min(PUSH_TILE, nd - first);
-            for (uint32_t i = threadIdx.x; i < nw; i += T) {
-                s_off[i] = voff[first + i];
-                s_dst[i] = dests[first + i];
-                s_delta[i] = vdelta[first + i];
-            }
-            if (threadIdx.x == 0) s_full = touched_full(ntouched, V);
-            __syncthreads();
-            for (uint32_t base = t0; base < tend; base += T) {  // warp-uniform trip count
-                const uint32_t gv = base + threadIdx.x;
-                uint32_t key = INF;
-                unsigned long long k = ~0ull;
-                if (gv < tend) {
-                    int lo = 0, hi = (int)nw - 1;  // last entry with s_off <= gv
-                    while (lo < hi) {
-                        const int mid = (lo + hi + 1) >> 1;
-                        if (s_off[mid] <= gv) lo = mid; else hi = mid - 1;
-                    }
-                    key = s_dst[lo];
-                    const uint32_t vec = gv + s_delta[lo];
-                    bool skip = false;
-                    if (gv >= s_off[lo] + LONG_RUN) {
-                        const unsigned long long c = __ldcg(cand + key);  // atomics of other blocks land in L2
-                        skip = c != ~0ull && (uint32_t)(c >> 32) < vec;
-                    }
-                    if (!skip) {
-                        const uint4 s = __ldcs(nbr + vec);
-                        const uint32_t ids[4] = { grz_hub_decode(s.x, hub_vid, nhub), grz_hub_decode(s.y, hub_vid, nhub),
-                                                  grz_hub_decode(s.z, hub_vid, nhub), grz_hub_decode(s.w, hub_vid, nhub) };
-                        uint32_t best = 0;
-                        bool any = false;
-    #pragma unroll
-                        for (int l = 0; l < 4; ++l) {
-                            const uint32_t id = ids[l];
-                            if (id < V && bit_of(has, id)) {
-                                best = any ? max(best, id) : id;
-                                any = true;
-                            }
-                        }
-                        if (any) k = ((unsigned long long)vec << 32) | (unsigned long long)(~best);
-                    }
-                }
-                if (!__any_sync(0xffffffffu, k != ~0ull)) continue;  // no frontier source in the warp's vectors
-                const uint32_t prevkey = __shfl_up_sync(0xffffffffu, key, 1);
-                const uint32_t nextkey = __shfl_down_sync(0xffffffffu, key, 1);
-                const bool head = lane == 0 || key != prevkey;
-                const bool tail = lane == 31 || key != nextkey;
-                const unsigned heads = __ballot_sync(0xffffffffu, head);
-                const int segstart = 31 - __clz(heads & (0xffffffffu >> (31 - lane)));
-                const int maxlen = __reduce_max_sync(0xffffffffu, (unsigned)(lane - segstart + 1));
-                for (int off = 1; off < maxlen; off <<= 1) {
-                    const unsigned long long o = __shfl_up_sync(0xffffffffu, k, off);
-                    if (lane - off >= segstart) k = min(k, o);
-                }
-                bool first_touch = false;
-                if (tail && k != ~0ull && k < cand[key]) {
-                    first_touch = atomicMin(cand + key, k) == ~0ull;
-                    if (first_touch) atomicOr(has_next + (key >> 6), 1ull << (key & 63));
-                }
-                touched_append(first_touch, key, touched, ntouched, s_full);
-            }
-            __syncthreads();
+    for (uint32_t tile = blockIdx.x; tile < ntiles; tile = s_tile) {
+        uint32_t next = 0;
+        if (threadIdx.x == 0) next = atomicAdd(queue, 1u) + gridDim.x;
+        const uint32_t first = tile_first[tile];
+        const uint32_t t0 = tile * PUSH_TILE;
+        const uint32_t tend = min(total, t0 + PUSH_TILE);
+        const uint32_t nw = min(PUSH_TILE, nd - first);
+        for (uint32_t i = threadIdx.x; i < nw; i += T) {
+            s_off[i] = voff[first + i];
+            s_dst[i] = dests[first + i];
+            s_delta[i] = vdelta[first + i];
         }
+        if (threadIdx.x == 0) s_full = touched_full(ntouched, V);
+        __syncthreads();
+        for (uint32_t base = t0; base < tend; base += T) {  // warp-uniform trip count
+            const uint32_t gv = base + threadIdx.x;
+            uint32_t key = INF;
+            unsigned long long k = ~0ull;
+            if (gv < tend) {
+                int lo = 0, hi = (int)nw - 1;  // last entry with s_off <= gv
+                while (lo < hi) {
+                    const int mid = (lo + hi + 1) >> 1;
+                    if (s_off[mid] <= gv) lo = mid; else hi = mid - 1;
+                }
+                key = s_dst[lo];
+                const uint32_t vec = gv + s_delta[lo];
+                bool skip = false;
+                if (gv >= s_off[lo] + LONG_RUN) {
+                    const unsigned long long c = __ldcg(cand + key);  // atomics of other blocks land in L2
+                    skip = c != ~0ull && (uint32_t)(c >> 32) < vec;
+                }
+                if (!skip) {
+                    const uint4 s = __ldcs(nbr + vec);
+                    const uint32_t ids[4] = { grz_hub_decode(s.x, hub_vid, nhub), grz_hub_decode(s.y, hub_vid, nhub),
+                                              grz_hub_decode(s.z, hub_vid, nhub), grz_hub_decode(s.w, hub_vid, nhub) };
+                    uint32_t best = 0;
+                    bool any = false;
+#pragma unroll
+                    for (int l = 0; l < 4; ++l) {
+                        const uint32_t id = ids[l];
+                        if (id < V && bit_of(has, id)) {
+                            best = any ? max(best, id) : id;
+                            any = true;
+                        }
+                    }
+                    if (any) k = ((unsigned long long)vec << 32) | (unsigned long long)(~best);
+                }
+            }
+            if (!__any_sync(0xffffffffu, k != ~0ull)) continue;  // no frontier source in the warp's vectors
+            const uint32_t prevkey = __shfl_up_sync(0xffffffffu, key, 1);
+            const uint32_t nextkey = __shfl_down_sync(0xffffffffu, key, 1);
+            const bool head = lane == 0 || key != prevkey;
+            const bool tail = lane == 31 || key != nextkey;
+            const unsigned heads = __ballot_sync(0xffffffffu, head);
+            const int segstart = 31 - __clz(heads & (0xffffffffu >> (31 - lane)));
+            const int maxlen = __reduce_max_sync(0xffffffffu, (unsigned)(lane - segstart + 1));
+            for (int off = 1; off < maxlen; off <<= 1) {
+                const unsigned long long o = __shfl_up_sync(0xffffffffu, k, off);
+                if (lane - off >= segstart) k = min(k, o);
+            }
+            bool first_touch = false;
+            if (tail && k != ~0ull && k < cand[key]) {
+                first_touch = atomicMin(cand + key, k) == ~0ull;
+                if (first_touch) atomicOr(has_next + (key >> 6), 1ull << (key & 63));
+            }
+            touched_append(first_touch, key, touched, ntouched, s_full);
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) s_tile = next;
+        __syncthreads();
     }
 }
 
@@ -912,7 +957,7 @@ __global__ void __launch_bounds__(T) k_cc_pull_expand(const uint32_t* __restrict
     __shared__ uint32_t s_dst[PUSH_TILE];
     __shared__ uint32_t s_off[PUSH_TILE];
     __shared__ uint32_t s_delta[PUSH_TILE];
-    __shared__ uint32_t s_chunk;
+    __shared__ uint32_t s_tile;
     __shared__ unsigned long long red[T / 32];
     __shared__ uint32_t red32[T / 32];
     const uint32_t ep = epoch_dev ? *epoch_dev : epoch;
@@ -926,63 +971,59 @@ __global__ void __launch_bounds__(T) k_cc_pull_expand(const uint32_t* __restrict
         const uint32_t id = sl < nhub ? __ldg(hub_vid + sl) : min(xl, V);
         return ld_label(label + id);
     };
-    for (;;) {
-        if (threadIdx.x == 0) s_chunk = atomicAdd(queue, 1u);
-        __syncthreads();
-        const uint32_t chunk = s_chunk;
-        __syncthreads();  // every thread has read s_chunk before it is replaced
-        if ((uint64_t)chunk * PULL_CHUNK >= ntiles) break;
-        const uint32_t chunk_end = min(ntiles, (chunk + 1) * PULL_CHUNK);
-        for (uint32_t tile = chunk * PULL_CHUNK; tile < chunk_end; ++tile) {
-            const uint32_t first = tile_first[tile];
-            const uint32_t t0 = tile * PUSH_TILE;
-            const uint32_t tend = min(total, t0 + PUSH_TILE);
-            const uint32_t nw = min(PUSH_TILE, nd - first);
-            for (uint32_t i = threadIdx.x; i < nw; i += T) {
-                s_off[i] = voff[first + i];
-                s_dst[i] = dests[first + i];
-                s_delta[i] = vdelta[first + i];
-            }
-            __syncthreads();
-            for (uint32_t base = t0; base < tend; base += T) {  // warp-uniform trip count
-                const uint32_t gv = base + threadIdx.x;
-                uint32_t key = INF, m = INF;
-                if (gv < tend) {
-                    int lo = 0, hi = (int)nw - 1;  // last entry with s_off <= gv
-                    while (lo < hi) {
-                        const int mid = (lo + hi + 1) >> 1;
-                        if (s_off[mid] <= gv) lo = mid; else hi = mid - 1;
-                    }
-                    key = s_dst[lo];
-                    if (ld_label(label + key) != 0) {
-                        ++my_vecs;
-                        const uint4 sv = ld_stream(nbr + (uint32_t)(gv + s_delta[lo]));
-                        m = fetch(sv.x);
-                        if (m != 0) m = min(m, min(min(fetch(sv.y), fetch(sv.z)), fetch(sv.w)));
-                    }
-                }
-                if (!__any_sync(0xffffffffu, m != INF)) continue;
-                const uint32_t prevkey = __shfl_up_sync(0xffffffffu, key, 1);
-                const uint32_t nextkey = __shfl_down_sync(0xffffffffu, key, 1);
-                const bool head = lane == 0 || key != prevkey;
-                const bool tail = lane == 31 || key != nextkey;
-                const unsigned heads = __ballot_sync(0xffffffffu, head);
-                const int segstart = 31 - __clz(heads & (0xffffffffu >> (31 - lane)));
-                const int maxlen = __reduce_max_sync(0xffffffffu, (unsigned)(lane - segstart + 1));
-                for (int off = 1; off < maxlen; off <<= 1) {
-                    const uint32_t o = __shfl_up_sync(0xffffffffu, m, off);
-                    if (lane - off >= segstart) m = min(m, o);
-                }
-                if (tail && m != INF && m < ld_label(label + key)) {
-                    const uint32_t old = atomicMin(label + key, m);
-                    if (m < old) {
-                        my_min = min(my_min, m);
-                        if (bit_set_first(has_next, key)) my_vote += vc.of(key);
-                    }
-                }
-            }
-            __syncthreads();
+    for (uint32_t tile = blockIdx.x; tile < ntiles; tile = s_tile) {
+        uint32_t next = 0;
+        if (threadIdx.x == 0) next = atomicAdd(queue, 1u) + gridDim.x;
+        const uint32_t first = tile_first[tile];
+        const uint32_t t0 = tile * PUSH_TILE;
+        const uint32_t tend = min(total, t0 + PUSH_TILE);
+        const uint32_t nw = min(PUSH_TILE, nd - first);
+        for (uint32_t i = threadIdx.x; i < nw; i += T) {
+            s_off[i] = voff[first + i];
+            s_dst[i] = dests[first + i];
+            s_delta[i] = vdelta[first + i];
         }
+        __syncthreads();
+        for (uint32_t base = t0; base < tend; base += T) {  // warp-uniform trip count
+            const uint32_t gv = base + threadIdx.x;
+            uint32_t key = INF, m = INF;
+            if (gv < tend) {
+                int lo = 0, hi = (int)nw - 1;  // last entry with s_off <= gv
+                while (lo < hi) {
+                    const int mid = (lo + hi + 1) >> 1;
+                    if (s_off[mid] <= gv) lo = mid; else hi = mid - 1;
+                }
+                key = s_dst[lo];
+                if (ld_label(label + key) != 0) {
+                    ++my_vecs;
+                    const uint4 sv = ld_stream(nbr + (uint32_t)(gv + s_delta[lo]));
+                    m = fetch(sv.x);
+                    if (m != 0) m = min(m, min(min(fetch(sv.y), fetch(sv.z)), fetch(sv.w)));
+                }
+            }
+            if (!__any_sync(0xffffffffu, m != INF)) continue;
+            const uint32_t prevkey = __shfl_up_sync(0xffffffffu, key, 1);
+            const uint32_t nextkey = __shfl_down_sync(0xffffffffu, key, 1);
+            const bool head = lane == 0 || key != prevkey;
+            const bool tail = lane == 31 || key != nextkey;
+            const unsigned heads = __ballot_sync(0xffffffffu, head);
+            const int segstart = 31 - __clz(heads & (0xffffffffu >> (31 - lane)));
+            const int maxlen = __reduce_max_sync(0xffffffffu, (unsigned)(lane - segstart + 1));
+            for (int off = 1; off < maxlen; off <<= 1) {
+                const uint32_t o = __shfl_up_sync(0xffffffffu, m, off);
+                if (lane - off >= segstart) m = min(m, o);
+            }
+            if (tail && m != INF && m < ld_label(label + key)) {
+                const uint32_t old = atomicMin(label + key, m);
+                if (m < old) {
+                    my_min = min(my_min, m);
+                    if (bit_set_first(has_next, key)) my_vote += vc.of(key);
+                }
+            }
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) s_tile = next;
+        __syncthreads();
     }
     my_vote = block_sum_u64(my_vote, red);
     if (threadIdx.x == 0) vote_add(vote, my_vote);
