@@ -465,6 +465,7 @@ struct grz_frontier_state {
     uint32_t* voff;                  // push: offset of each source's first vector among the frontier's
     uint32_t* vdelta;                // push: first vector index in the list minus voff (mod 2^32)
     uint32_t* tile_first;            // push: frontier entry owning the first vector of each tile
+    unsigned long long* digest;      // u64[4] k_digest's sums and arrivals, zero between calls
     uint32_t* touched;               // BFS destinations reached in this phase
     unsigned long long* cand64;      // BFS pull: (vector index, ~source) per destination
     uint32_t* cand32;                // BFS push: smallest source per destination

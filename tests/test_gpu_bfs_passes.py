@@ -78,3 +78,29 @@ def test_push_parents(n, mid, fan):
             assert lv[0] == 0 and (lv[m] == 1).all() and seen.sum() == (ref < n).sum()
         lab = G.connected_components(native.FORCE_PUSH)
         np.testing.assert_array_equal(lab, G.connected_components(native.FORCE_PULL))
+
+
+@pytest.mark.parametrize("n", [2, 3, 5, 1023, 1026, 300001])
+def test_digest(n):
+    """four vertices per thread, the last n % 4 by themselves; again after other sums"""
+    from grazelle import graphgen as gg
+    from grazelle.engine import Graph
+    rng = np.random.RandomState(n)
+    src, dst = rng.randint(0, n, 2 * n), rng.randint(0, n, 2 * n)
+    src[0], dst[0] = 0, n - 1
+    g = gg.EdgeList(n, src.astype(np.uint64), dst.astype(np.uint64))
+    deg = g.out_degrees().astype(np.int64)
+    odd = (np.arange(n, dtype=np.uint64) * np.uint64(0x9E3779B97F4A7C15)) | np.uint64(1)
+
+    def ref(x, reached, degrees):
+        h = int(np.sum((x.astype(np.uint64) + np.uint64(1)) * odd, dtype=np.uint64))
+        return int(reached.sum()), int(degrees[reached].sum()), h
+
+    with Graph(0) as G:
+        G.load_pairs(n, g.pull_order().pairs(), g.push_order().pairs())
+        for r in (0, n - 1, 0):
+            lv = G.bfs(r)[1]
+            for _ in range(2):
+                assert G.digest() == ref(np.where(lv < 0, 0xffffffff, lv), lv >= 0, deg)
+        lab = G.connected_components()
+        assert G.digest() == ref(lab, lab == np.arange(n), 0 * deg)
