@@ -624,7 +624,7 @@ __global__ void __launch_bounds__(T) k_bfs_pull(const uint4* __restrict__ nbr, c
 
 constexpr uint32_t PUSH_TILE = T;
 
-// Each block takes CCHUNK consecutive vertices, each thread one 32-vertex word of the two bitmaps
+// Each warp takes WORDS consecutive 32-vertex words of the two bitmaps, one per lane
 // (HasInfo and out-vectors for push; WantsInfo, or the destinations a first pass left open, and
 // in-vectors for the pulls); a block with nothing selected returns after reading its words.  A warp
 // then walks its words with a lane per vertex, so row pointers and entries are read and written
@@ -635,7 +635,11 @@ constexpr uint32_t PUSH_TILE = T;
 // Before: a count kernel, a one-block scan and a write kernel with 32 vertices per thread.  GB300,
 // whole runs, three kernels -> one: 8 BFS at R-MAT 24 9.67 -> 9.15 ms, a BFS of 1400 levels on a mesh of
 // 250k vertices 33.4 -> 30.6 ms.
-constexpr uint32_t CCHUNK = T * 32;
+// Words of a warp: its passes over them are a chain of loads, FR_STEP words at a time, so a graph that would
+// give few blocks takes fewer words per warp (GB300, 4096 vertices: 32 words 8 to 13 us, 4 words FRCUS); with
+// more blocks the adds to the one counter cost more than the chain.
+constexpr int FR_WORDS = 32, FR_WORDS_SMALL = 4;
+constexpr uint64_t FR_SMALL_V = 1ull << 19;
 constexpr int FR_STEP = 4;  // words whose row pointers are loaded together
 
 // `counters`[2] = vectors, [3] = selected vertices (zero before the launch).
@@ -644,6 +648,7 @@ constexpr int FR_STEP = 4;  // words whose row pointers are loaded together
 // tile_first[t] for the tiles that start in its range.  `skip` leaves out the first vectors of
 // every selected vertex (each selected one has more).  A zero gate selects nothing (the bitmaps
 // were not written in this phase).
+template <int WORDS>
 __global__ void __launch_bounds__(T) k_fr_compact(const unsigned long long* __restrict__ bm1, const unsigned long long* __restrict__ bm2,
                                                   uint64_t V, const uint32_t* __restrict__ rowptr, uint32_t skip,
                                                   const uint32_t* __restrict__ gate, uint32_t* __restrict__ counters,
@@ -654,12 +659,12 @@ __global__ void __launch_bounds__(T) k_fr_compact(const unsigned long long* __re
     __shared__ unsigned long long s_base;
     if (gate && *gate == 0u) return;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const uint64_t word = (uint64_t)blockIdx.x * T + threadIdx.x;  // bits of vertices [32 word, 32 word + 32)
+    const uint64_t first = ((uint64_t)blockIdx.x * (T / 32) + warp) * WORDS, word = first + lane;  // bits of vertices [32 word, 32 word + 32)
     uint32_t bits = 0;
-    if (32 * word < V) bits = reinterpret_cast<const uint32_t*>(bm1)[word] & reinterpret_cast<const uint32_t*>(bm2)[word];
+    if (lane < WORDS && 32 * word < V) bits = reinterpret_cast<const uint32_t*>(bm1)[word] & reinterpret_cast<const uint32_t*>(bm2)[word];
     if (32 * word + 32 > V && bits) bits &= (1u << (V - 32 * word)) - 1u;
     if (!__syncthreads_or(bits)) return;
-    const uint32_t vbase = (uint32_t)((uint64_t)blockIdx.x * CCHUNK) + 1024u * warp + lane;  // this lane's vertex of the warp's word 0
+    const uint32_t vbase = (uint32_t)(32 * first) + lane;  // this lane's vertex of the warp's word 0
     const unsigned words = __ballot_sync(0xffffffffu, bits != 0);
     // vectors of this lane's vertices in words j .. j + FR_STEP - 1 (0 if not selected), their first in r0
     auto rows = [&](int j, uint32_t* r0, uint32_t* cnt) {
@@ -681,7 +686,7 @@ __global__ void __launch_bounds__(T) k_fr_compact(const unsigned long long* __re
     };
     const uint32_t n = __reduce_add_sync(0xffffffffu, (unsigned)__popc(bits));
     uint32_t vec = 0;
-    for (int j = 0; j < 32; j += FR_STEP) {
+    for (int j = 0; j < WORDS; j += FR_STEP) {
         if (!((words >> j) & ((1u << FR_STEP) - 1u))) continue;  // warp-uniform
         uint32_t r0[FR_STEP], cnt[FR_STEP];
         rows(j, r0, cnt);
@@ -702,7 +707,7 @@ __global__ void __launch_bounds__(T) k_fr_compact(const unsigned long long* __re
     }
     __syncthreads();
     uint32_t pos = (uint32_t)(s_base >> 32) + sn[warp], vo = (uint32_t)s_base + sv[warp];
-    for (int j = 0; j < 32; j += FR_STEP) {
+    for (int j = 0; j < WORDS; j += FR_STEP) {
         if (!((words >> j) & ((1u << FR_STEP) - 1u))) continue;
         uint32_t r0[FR_STEP], cnt[FR_STEP];
         rows(j, r0, cnt);
@@ -1952,6 +1957,12 @@ static int cc_pull_config_any(grz_graph* g, size_t smem, int* resident)
     return g->tune.pull_staging ? cc_pull_config<BT, true>(g, smem, resident) : cc_pull_config<BT, false>(g, smem, resident);
 }
 
+// blocks of the kernels that go through compacted vectors by tiles (their number is on the device)
+static unsigned tile_grid(const grz_graph* g, const grz_list& l)
+{
+    return (unsigned)std::min<uint64_t>(l.nvec / PUSH_TILE + 1, (uint64_t)g->num_sms * 8);
+}
+
 // Compacts the vertices selected by bm1 & bm2 (defined below)
 static void compact(grz_graph* g, const unsigned long long* bm1, const unsigned long long* bm2, const uint32_t* rowptr,
                     uint32_t skip = 0, const uint32_t* gate = nullptr);
@@ -1997,7 +2008,7 @@ static int launch_cc_pull_bt(grz_graph* g, uint64_t first, uint64_t count, const
             work = g->prof_work;
         }
         auto expand = [&]() {
-            k_cc_pull_expand<<<(unsigned)g->num_sms * 8, T, 0, g->stream>>>(f.frontier, f.voff, f.vdelta, f.tile_first, f.counters,
+            k_cc_pull_expand<<<tile_grid(g, g->pull), T, 0, g->stream>>>(f.frontier, f.voff, f.vdelta, f.tile_first, f.counters,
                                                                            g->pull.nbr, (uint32_t)g->V, f.label, g->pull.hub_vid,
                                                                            g->pull.nhub, f.has_next, vc, f.vote, f.chg, f.iter,
                                                                            f.level_dev, f.counters + 5, work); GRZ_COUNT_LAUNCH(g);
@@ -2076,8 +2087,10 @@ static void compact(grz_graph* g, const unsigned long long* bm1, const unsigned 
                     uint32_t skip, const uint32_t* gate)
 {
     grz_frontier_state& f = g->fr;
-    const unsigned nb = (unsigned)(g->V / CCHUNK + 1);
-    k_fr_compact<<<nb, T, 0, g->stream>>>(bm1, bm2, g->V, rowptr, skip, gate, f.counters, f.frontier, f.voff, f.vdelta, f.tile_first);
+    const int words = g->V < FR_SMALL_V ? FR_WORDS_SMALL : FR_WORDS;
+    const unsigned nb = (unsigned)(g->V / ((uint64_t)T * words) + 1);
+    (words == FR_WORDS ? k_fr_compact<FR_WORDS> : k_fr_compact<FR_WORDS_SMALL>)<<<nb, T, 0, g->stream>>>(
+        bm1, bm2, g->V, rowptr, skip, gate, f.counters, f.frontier, f.voff, f.vdelta, f.tile_first);
     GRZ_COUNT_LAUNCH(g);
 }
 
@@ -2091,7 +2104,8 @@ static int edge_phase(grz_graph* g, int pull, uint64_t first, uint64_t count)
     cudaStream_t st = g->stream;
     const VoteCfg vc = vote_cfg(g);
     const bool bfs = f.app == GRZ_APP_BREADTH_FIRST_SEARCH;
-    GRZ_CK(g, cudaMemsetAsync(f.counters, 0, sizeof(uint32_t) * 8, st));
+    // in a captured run the decision before the phase cleared the counters
+    if (!f.level_dev) GRZ_CK(g, cudaMemsetAsync(f.counters, 0, sizeof(uint32_t) * 8, st));
     if (pull) {
         if (!g->pull.nbr) return grz_set_error(g, GRZ_ERR_STATE, "pull list not loaded");
         if (count == 0) return GRZ_OK;
@@ -2113,7 +2127,7 @@ static int edge_phase(grz_graph* g, int pull, uint64_t first, uint64_t count)
                                                   g->pull.hub_vid, g->pull.nhub, f.has_next, f.unres, first_n, f.label, f.level,
                                                   f.iter, f.level_dev, vc, f.vote); GRZ_COUNT_LAUNCH(g);
             compact(g, f.unres, f.unres, g->pull.rowptr, first_n);
-            k_bfs_pull_expand<<<(unsigned)g->num_sms * 8, T, 0, st>>>(f.frontier, f.voff, f.vdelta, f.tile_first, f.counters,
+            k_bfs_pull_expand<<<tile_grid(g, g->pull), T, 0, st>>>(f.frontier, f.voff, f.vdelta, f.tile_first, f.counters,
                                                                      g->pull.nbr, V, f.has, f.cand64, f.touched, f.counters + 1,
                                                                      g->pull.hub_vid, g->pull.nhub, f.has_next, f.counters + 5); GRZ_COUNT_LAUNCH(g);
         } else if (compacted) {
@@ -2123,7 +2137,7 @@ static int edge_phase(grz_graph* g, int pull, uint64_t first, uint64_t count)
             grz_prof_end(g);
             GRZ_TRY(grz_stats_count_selected(g, &g->pull, f.frontier, f.counters));
             grz_prof_begin(g, GRZ_PROF_BFS_PULL);
-            k_bfs_pull_expand<<<(unsigned)g->num_sms * 8, T, 0, st>>>(f.frontier, f.voff, f.vdelta, f.tile_first, f.counters,
+            k_bfs_pull_expand<<<tile_grid(g, g->pull), T, 0, st>>>(f.frontier, f.voff, f.vdelta, f.tile_first, f.counters,
                                                                      g->pull.nbr, V, f.has, f.cand64, f.touched, f.counters + 1,
                                                                      g->pull.hub_vid, g->pull.nhub, f.has_next, f.counters + 5); GRZ_COUNT_LAUNCH(g);
         } else {
@@ -2152,7 +2166,7 @@ static int edge_phase(grz_graph* g, int pull, uint64_t first, uint64_t count)
         grz_prof_end(g);
         GRZ_TRY(grz_stats_count_selected(g, &g->push, f.frontier, f.counters));
         grz_prof_begin(g, bfs ? GRZ_PROF_BFS_PUSH : GRZ_PROF_CC_PUSH);
-        const unsigned grid = (unsigned)g->num_sms * 8;
+        const unsigned grid = tile_grid(g, g->push);
         if (bfs) {
             k_push_expand<true><<<grid, T, 0, st>>>(f.frontier, f.voff, f.vdelta, f.tile_first, f.counters, g->push.nbr, V, f.label,
                                                     f.has_next, f.wants, f.cand32, f.touched, f.counters + 1, vc, f.vote,

@@ -116,10 +116,13 @@ __global__ void __launch_bounds__(T) k_features_decide(FeatIn in, const float* _
 // graph's conditional handles: hengine selects the next iteration's body, hloop
 // keeps the WHILE node going.  `initial`: the decision before the first iteration, from the
 // starting vote; no statistics, no clearing.
+constexpr int DECIDE_U = 4;  // words a thread loads together: one step for up to 20M vertices
+
 struct RunIn {
     FeatIn feat;                        // frontier = the next HasInfo
     unsigned long long* vote_slots;     // read and re-zeroed
     unsigned long long* clear_bm;       // old HasInfo (null when initial)
+    uint32_t* counters;                 // u32[8] of the next edge phase, cleared
     int initial;
     uint32_t* hop_list;                 // the next frontier's vertices when its vote is at most GRZ_HOP_VOTE, or null
     int hop_pulls;                      // small pulls go to k_hop as well
@@ -149,25 +152,33 @@ __global__ void __launch_bounds__(T) k_run_decide(RunIn in, grz_runctl* __restri
         list = v <= GRZ_HOP_VOTE;
     }
     unsigned pf = 0, pw = 0;
-    for (uint64_t w0 = (uint64_t)blockIdx.x * T + 32 * warp; w0 < fi.words; w0 += (uint64_t)gridDim.x * T) {  // warp-uniform
-        const uint64_t w = w0 + lane;
-        unsigned long long bits = 0ull;
-        if (w < fi.words) {
-            bits = fi.frontier[w];
-            if (fi.app_bfs) pw += __popcll(fi.wants[w]);
-            if (in.clear_bm) in.clear_bm[w] = 0ull;
+    const uint64_t stride = (uint64_t)gridDim.x * T;
+    for (uint64_t w0 = (uint64_t)blockIdx.x * T + 32 * warp; w0 < fi.words; w0 += DECIDE_U * stride) {  // warp-uniform
+        unsigned long long word[DECIDE_U], open[DECIDE_U];
+#pragma unroll
+        for (int u = 0; u < DECIDE_U; ++u) {
+            const uint64_t w = w0 + u * stride + lane;
+            word[u] = w < fi.words ? fi.frontier[w] : 0ull;
+            open[u] = fi.app_bfs && w < fi.words ? fi.wants[w] : 0ull;
         }
-        const unsigned n = __popcll(bits);
-        pf += n;
-        if (list && __any_sync(0xffffffffu, n != 0)) {
-            unsigned x = n, at = 0;
-            for (int o = 1; o < 32; o <<= 1) {
-                const unsigned y = __shfl_up_sync(0xffffffffu, x, o);
-                if (lane >= o) x += y;
+#pragma unroll
+        for (int u = 0; u < DECIDE_U; ++u) {
+            const uint64_t w = w0 + u * stride + lane;
+            if (in.clear_bm && w < fi.words) in.clear_bm[w] = 0ull;
+            unsigned long long bits = word[u];
+            const unsigned n = __popcll(bits);
+            pf += n;
+            pw += __popcll(open[u]);
+            if (list && __any_sync(0xffffffffu, n != 0)) {
+                unsigned x = n, at = 0;
+                for (int o = 1; o < 32; o <<= 1) {
+                    const unsigned y = __shfl_up_sync(0xffffffffu, x, o);
+                    if (lane >= o) x += y;
+                }
+                if (lane == 31) at = atomicAdd(&ctl->hop_cnt, x);
+                at = __shfl_sync(0xffffffffu, at, 31) + x - n;
+                for (; bits && at < GRZ_HOP_VOTE; bits &= bits - 1) in.hop_list[at++] = (uint32_t)(64 * w) + (uint32_t)(__ffsll((long long)bits) - 1);
             }
-            if (lane == 31) at = atomicAdd(&ctl->hop_cnt, x);
-            at = __shfl_sync(0xffffffffu, at, 31) + x - n;
-            for (; bits && at < GRZ_HOP_VOTE; bits &= bits - 1) in.hop_list[at++] = (uint32_t)(64 * w) + (uint32_t)(__ffsll((long long)bits) - 1);
         }
     }
     pf = __reduce_add_sync(0xffffffffu, pf);
@@ -228,6 +239,7 @@ __global__ void __launch_bounds__(T) k_run_decide(RunIn in, grz_runctl* __restri
         pull = (double)vote > ctl->threshold ? 1 : 0;
     }
     if (lane < NF) ctl->features[lane] = f[lane];
+    if (lane < 8) in.counters[lane] = 0;
     if (lane == 0) {
         if (!in.initial) {
             if (ran) ctl->npull += 1; else ctl->npush += 1;
@@ -556,6 +568,7 @@ int grz_switch_launch_run_decide(grz_graph* g, const unsigned long long* next_fr
     in.feat.app_bfs = f.app == GRZ_APP_BREADTH_FIRST_SEARCH;
     in.vote_slots = f.vote;
     in.clear_bm = clear_bm;
+    in.counters = f.counters;
     in.initial = initial;
     in.hop_list = f.hop_list;
     in.hop_pulls = hop_pulls;
