@@ -1569,21 +1569,43 @@ __global__ void __cluster_dims__(HOP_CTAS, 1, 1) __launch_bounds__(HOP_T, 1) k_h
     }
 }
 
-// Calls f(word, bits, vertex, whether it is marked) for every nonzero word of `map`, a warp per word, first
-// the lower then the upper 32 vertices (f is called by whole warps); g(word, bits) once after each.
-template <typename F, typename G>
-__device__ __forceinline__ void hop_marked(const unsigned long long* __restrict__ map, uint64_t W, F f, G g)
+// Calls f(vertex, whether it is marked, load(vertex) if it is, half) for the vertices of every nonzero word
+// of `map`, a warp per word, first the lower then the upper 32 vertices (f is called by whole warps);
+// g(word, bits) once after each.  A warp looks at `span` words and takes HOP_WORDS nonzero ones at a time,
+// whose vertices it loads for first: one after the other, each a trip to memory, they took a run that had
+// marked most of 100k vertices 27.6 us, so 4.4 us.  A map of few words is spread over more warps (4 words
+// each; a large one is nearly empty, and 32 words are one load).
+constexpr int HOP_WORDS = 4;
+constexpr uint64_t HOP_SPAN_W = 1u << 15;
+__host__ __device__ constexpr int hop_span(uint64_t W) { return W < HOP_SPAN_W ? HOP_WORDS : 32; }
+template <typename C, typename F, typename G>
+__device__ __forceinline__ void hop_marked(const unsigned long long* __restrict__ map, uint64_t W, C load, F f, G g)
 {
-    const int lane = threadIdx.x & 31;
+    const int lane = threadIdx.x & 31, span = hop_span(W);
     const uint64_t nwarps = (uint64_t)gridDim.x * (T / 32);
-    for (uint64_t w0 = 32 * ((uint64_t)blockIdx.x * (T / 32) + (threadIdx.x >> 5)); w0 < W; w0 += 32 * nwarps) {
-        const unsigned long long mine = w0 + lane < W ? map[w0 + lane] : 0ull;
-        for (unsigned nz = __ballot_sync(0xffffffffu, mine != 0); nz; nz &= nz - 1) {
-            const int j = __ffs(nz) - 1;
-            const unsigned long long bits = __shfl_sync(0xffffffffu, mine, j);
-            f((uint32_t)(64 * (w0 + j)) + lane, ((bits >> lane) & 1ull) != 0, 0);
-            f((uint32_t)(64 * (w0 + j)) + 32 + lane, ((bits >> (32 + lane)) & 1ull) != 0, 1);
-            if (lane == 0) g(w0 + j, bits);
+    for (uint64_t w0 = span * ((uint64_t)blockIdx.x * (T / 32) + (threadIdx.x >> 5)); w0 < W; w0 += span * nwarps) {
+        const unsigned long long mine = lane < span && w0 + lane < W ? map[w0 + lane] : 0ull;
+        unsigned nz = __ballot_sync(0xffffffffu, mine != 0);
+        while (nz) {  // warp-uniform
+            unsigned long long bits[HOP_WORDS], c[2 * HOP_WORDS];
+            uint32_t at[HOP_WORDS];
+#pragma unroll
+            for (int j = 0; j < HOP_WORDS; ++j) {
+                const int i = nz ? __ffs(nz) - 1 : 0;
+                bits[j] = __shfl_sync(0xffffffffu, mine, i);
+                if (!nz) bits[j] = 0ull;
+                at[j] = (uint32_t)(w0 + i);
+                nz &= nz - 1;
+            }
+#pragma unroll
+            for (int j = 0; j < 2 * HOP_WORDS; ++j)
+                c[j] = (bits[j / 2] >> (32 * (j & 1) + lane)) & 1ull ? load(64 * at[j / 2] + 32 * (j & 1) + lane) : 0ull;
+#pragma unroll
+            for (int j = 0; j < 2 * HOP_WORDS; ++j) {
+                if (!bits[j / 2]) break;
+                f(64 * at[j / 2] + 32 * (j & 1) + lane, ((bits[j / 2] >> (32 * (j & 1) + lane)) & 1ull) != 0, c[j], j & 1);
+                if ((j & 1) && lane == 0) g(at[j / 2], bits[j / 2]);
+            }
         }
     }
 }
@@ -1598,11 +1620,10 @@ __global__ void __launch_bounds__(T) k_hop_visit(const grz_runctl* __restrict__ 
     const uint32_t last = ctl->level;
     unsigned long long in_last = 0ull;
     hop_marked(
-        map, W,
-        [&](uint32_t d, bool marked, int half) {
+        map, W, [&](uint32_t d) { return cand64[d]; },
+        [&](uint32_t d, bool marked, unsigned long long c, int half) {
             bool l = false;
             if (marked) {
-                const unsigned long long c = cand64[d];
                 const uint32_t lv = (uint32_t)(c >> 33);
                 level[d] = lv;
                 l = lv == last;
@@ -1630,14 +1651,14 @@ __global__ void __launch_bounds__(T) k_hop_parents(const grz_runctl* __restrict_
                                                    const uint32_t* __restrict__ rowptr, const uint32_t* __restrict__ hub_vid, uint32_t nhub)
 {
     if (!ctl->hop_pulls) {
-        hop_marked(map, W, [](uint32_t, bool, int) {}, [&](uint64_t w, unsigned long long) { map[w] = 0ull; });
+        hop_marked(map, W, [](uint32_t) { return 0ull; }, [](uint32_t, bool, unsigned long long, int) {},
+                   [&](uint64_t w, unsigned long long) { map[w] = 0ull; });
         return;
     }
     hop_marked(
-        map, W,
-        [&](uint32_t d, bool marked, int) {
-            const unsigned long long c = marked ? cand64[d] : ~0ull;
-            if (c == ~0ull) return;  // a push visited it
+        map, W, [&](uint32_t d) { return cand64[d]; },
+        [&](uint32_t d, bool marked, unsigned long long c, int) {
+            if (!marked || c == ~0ull) return;  // a push visited it
             cand64[d] = ~0ull;
             const uint32_t u = (uint32_t)c, before = (uint32_t)(c >> 33) - 1;
             uint32_t lo = __ldg(rowptr + d), hi = __ldg(rowptr + d + 1) - 1;
@@ -1664,11 +1685,11 @@ __global__ void __launch_bounds__(T) k_hop_labels(const grz_runctl* __restrict__
     const uint32_t last = ctl->level;
     unsigned long long in_last = 0ull;
     hop_marked(
-        map, W,
-        [&](uint32_t d, bool marked, int half) {
+        map, W, [&](uint32_t d) { return (unsigned long long)cand32[d]; },
+        [&](uint32_t d, bool marked, unsigned long long c, int half) {
             bool l = false;
             if (marked) {
-                l = cand32[d] == ~last;
+                l = (uint32_t)c == ~last;
                 cand32[d] = INF;
             }
             const unsigned long long m = __ballot_sync(0xffffffffu, l);
@@ -2510,7 +2531,7 @@ static int hop_phase(grz_graph* g)
     in.ctl = f.ctl;
     in.pulls = hop_pulls(g);
     const uint64_t W = words_of(g->V);
-    const unsigned grid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>((W + T - 1) / T, (uint64_t)g->num_sms * 4));
+    const unsigned grid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(W / (hop_span(W) * (T / 32)) + 1, (uint64_t)g->num_sms * 8));
     if (bfs) {
         k_hop<true><<<HOP_CTAS, HOP_T, HOP_SMEM, g->stream>>>(in);
         k_hop_visit<<<grid, T, 0, g->stream>>>(f.ctl, f.hop_map, W, f.cand64, f.label, f.level, f.wants, f.has_next, !in.pulls);
