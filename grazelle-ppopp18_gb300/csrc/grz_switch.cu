@@ -134,23 +134,35 @@ __global__ void __launch_bounds__(T) k_run_decide(RunIn in, grz_runctl* __restri
     __shared__ unsigned s_pf[T / 32], s_pw[T / 32];
     __shared__ bool s_last;
     __shared__ float f[NF];
-    if (!in.initial && !*(volatile uint32_t*)&ctl->running) return;
     const FeatIn& fi = in.feat;
-    const float* params = ctl->params;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    // Everything the decision will need is loaded here, one trip to memory together with the bitmaps: any
+    // block may be the last, whose first warp decides, and only that writes any of it, after all have read.
+    const uint32_t goes_on = ctl->running;
+    const float* const params = ctl->params;
+    const unsigned long long start_vote = ctl->vote;
+    const uint32_t* const root_degree = in.initial ? ctl->root_degree : nullptr;
+    uint32_t level = ctl->level, last_engine = ctl->last_engine;
+    const uint32_t ran = ctl->engine, max_level = ctl->max_level;
+    const int force = ctl->force;
+    const unsigned long long t0_ns = ctl->t0_ns, limit_ns = ctl->limit_ns;
+    const double threshold = ctl->threshold;
+    unsigned long long vote = 0;
+    if (!in.initial) {
+        const volatile unsigned long long* slots = in.vote_slots;
+        vote = slots[lane * GRZ_VOTE_STRIDE] + slots[(lane + 32) * GRZ_VOTE_STRIDE];
+    }
+    if (!in.initial && !goes_on) return;
+    MlpLane mlp;
+    if (warp == 0 && params) mlp.load(MlpGlobal{ params }, lane);
+    if (in.initial) {  // the starting vote, the host's part and the root's
+        vote = start_vote + (root_degree ? *root_degree : 0u);
+    } else {
+        for (int o = 16; o > 0; o >>= 1) vote += __shfl_xor_sync(0xffffffffu, vote, o);
+    }
     // The vote counts every vertex of the next frontier, so a small one means few vertices: those
     // are listed for the kernel that runs small push iterations (the votes are complete here).
-    bool list = false;
-    const unsigned long long root_edges = in.initial && ctl->root_degree ? *ctl->root_degree : 0ull;
-    if (in.hop_list) {
-        unsigned long long v = ctl->vote + root_edges;
-        if (!in.initial) {
-            const volatile unsigned long long* slots = in.vote_slots;
-            v = slots[lane * GRZ_VOTE_STRIDE] + slots[(lane + 32) * GRZ_VOTE_STRIDE];
-            for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-        }
-        list = v <= GRZ_HOP_VOTE;
-    }
+    const bool list = in.hop_list && vote <= GRZ_HOP_VOTE;
     unsigned pf = 0, pw = 0;
     const uint64_t stride = (uint64_t)gridDim.x * T;
     for (uint64_t w0 = (uint64_t)blockIdx.x * T + 32 * warp; w0 < fi.words; w0 += DECIDE_U * stride) {  // warp-uniform
@@ -185,32 +197,29 @@ __global__ void __launch_bounds__(T) k_run_decide(RunIn in, grz_runctl* __restri
     pw = __reduce_add_sync(0xffffffffu, pw);
     if (lane == 0) { s_pf[warp] = pf; s_pw[warp] = pw; }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        unsigned long long bf = 0, bw = 0;
-        for (int i = 0; i < T / 32; ++i) { bf += s_pf[i]; bw += s_pw[i]; }
-        if (bf) atomicAdd(&ctl->cnt_f, bf);
-        if (bw) atomicAdd(&ctl->cnt_u, bw);
+    unsigned long long F = 0, U = 0;
+    if (gridDim.x == 1) {
+        if (warp != 0) return;
+        for (int i = 0; i < T / 32; ++i) { F += s_pf[i]; U += s_pw[i]; }
+    } else {
+        if (threadIdx.x == 0) {
+            unsigned long long bf = 0, bw = 0;
+            for (int i = 0; i < T / 32; ++i) { bf += s_pf[i]; bw += s_pw[i]; }
+            if (bf) atomicAdd(&ctl->cnt_f, bf);
+            if (bw) atomicAdd(&ctl->cnt_u, bw);
+            __threadfence();
+            s_last = atomicAdd(&ctl->ticket, 1ull) == (unsigned long long)(gridDim.x - 1);
+        }
+        __syncthreads();
+        if (!s_last || warp != 0) return;
         __threadfence();
-        s_last = atomicAdd(&ctl->ticket, 1ull) == (unsigned long long)(gridDim.x - 1);
+        F = *(volatile unsigned long long*)&ctl->cnt_f;
+        U = *(volatile unsigned long long*)&ctl->cnt_u;
     }
-    __syncthreads();
-    if (!s_last || warp != 0) return;
-    __threadfence();
-    const unsigned long long F = *(volatile unsigned long long*)&ctl->cnt_f;
-    const unsigned long long U = *(volatile unsigned long long*)&ctl->cnt_u;
-    unsigned long long vote = ctl->vote + root_edges;  // initial: the starting vote, the host's part and the root's
     if (!in.initial) {
-        unsigned long long* a = in.vote_slots + lane * GRZ_VOTE_STRIDE;
-        unsigned long long* b = in.vote_slots + (lane + 32) * GRZ_VOTE_STRIDE;
-        unsigned long long vs = *(volatile unsigned long long*)a + *(volatile unsigned long long*)b;
-        *a = 0ull;
-        *b = 0ull;
-        for (int o = 16; o > 0; o >>= 1) vs += __shfl_down_sync(0xffffffffu, vs, o);
-        vote = __shfl_sync(0xffffffffu, vs, 0);
+        in.vote_slots[lane * GRZ_VOTE_STRIDE] = 0ull;
+        in.vote_slots[(lane + 32) * GRZ_VOTE_STRIDE] = 0ull;
     }
-    uint32_t level = ctl->level;
-    const uint32_t ran = ctl->engine;
-    uint32_t last_engine = ctl->last_engine;
     uint32_t running = 1, overrun = 0;
     unsigned long long now;
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
@@ -219,8 +228,8 @@ __global__ void __launch_bounds__(T) k_run_decide(RunIn in, grz_runctl* __restri
         running = vote != 0ull;
         if (running) {
             ++level;
-            if (level > ctl->max_level) { running = 0; overrun = 1; }
-            if (now - ctl->t0_ns > ctl->limit_ns) { running = 0; overrun = 2; }
+            if (level > max_level) { running = 0; overrun = 1; }
+            if (now - t0_ns > limit_ns) { running = 0; overrun = 2; }
         }
     }
     FeatIn fe = fi;
@@ -229,14 +238,14 @@ __global__ void __launch_bounds__(T) k_run_decide(RunIn in, grz_runctl* __restri
     if (lane < NF) f[lane] = feature(lane, fe, (float)F, (float)U, (float)vote);
     __syncwarp();
     int pull;
-    if (ctl->force >= 0) {
-        pull = ctl->force;
+    if (force >= 0) {
+        pull = force;
     } else if (!running) {
         pull = 0;  // the loop stops: no next engine to choose
     } else if (params) {
-        pull = mlp_logit_warp(MlpGlobal{ params }, f, lane) > 0.f ? 1 : 0;
+        pull = mlp.logit(f) > 0.f ? 1 : 0;
     } else {
-        pull = (double)vote > ctl->threshold ? 1 : 0;
+        pull = (double)vote > threshold ? 1 : 0;
     }
     if (lane < NF) ctl->features[lane] = f[lane];
     if (lane < 8) in.counters[lane] = 0;

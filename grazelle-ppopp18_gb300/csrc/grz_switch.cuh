@@ -68,28 +68,44 @@ __device__ __forceinline__ void mlp_stage(const float* __restrict__ params, floa
     }
 }
 
+// a lane's share of the weights, so that they can be loaded long before the features are known
+struct MlpLane {
+    float w1[NF], w2[NH], b1, b2, w3, b3;
+    template <typename W>
+    __device__ __forceinline__ void load(const W w, int lane)
+    {
+#pragma unroll
+        for (int k = 0; k < NF; ++k) w1[k] = w.w1(lane, k);
+#pragma unroll
+        for (int k = 0; k < NH; ++k) w2[k] = w.w2(lane, k);
+        b1 = w.rest(OFF_B1 + lane);
+        b2 = w.rest(OFF_B2 + lane);
+        w3 = w.rest(OFF_W3 + lane);
+        b3 = w.rest(OFF_B3);
+    }
+    __device__ __forceinline__ float logit(const float* f) const
+    {
+        float s = b1;
+#pragma unroll
+        for (int k = 0; k < NF; ++k) s = fmaf(w1[k], f[k], s);
+        const float h1 = relu(s);
+        s = b2;
+#pragma unroll
+        for (int k = 0; k < NH; ++k) s = fmaf(w2[k], __shfl_sync(0xffffffffu, h1, k), s);
+        const float h2 = relu(s);
+        float z = b3;
+#pragma unroll
+        for (int k = 0; k < NH; ++k) z = fmaf(__shfl_sync(0xffffffffu, w3, k), __shfl_sync(0xffffffffu, h2, k), z);
+        return z;
+    }
+};
+
 template <typename W>
 __device__ __forceinline__ float mlp_logit_warp(const W w, const float* f, int lane)
 {
-    float w1[NF], w2[NH];
-#pragma unroll
-    for (int k = 0; k < NF; ++k) w1[k] = w.w1(lane, k);
-#pragma unroll
-    for (int k = 0; k < NH; ++k) w2[k] = w.w2(lane, k);
-    const float b1 = w.rest(OFF_B1 + lane), b2 = w.rest(OFF_B2 + lane);
-    const float w3 = w.rest(OFF_W3 + lane), b3 = w.rest(OFF_B3);
-    float s = b1;
-#pragma unroll
-    for (int k = 0; k < NF; ++k) s = fmaf(w1[k], f[k], s);
-    const float h1 = relu(s);
-    s = b2;
-#pragma unroll
-    for (int k = 0; k < NH; ++k) s = fmaf(w2[k], __shfl_sync(0xffffffffu, h1, k), s);
-    const float h2 = relu(s);
-    float z = b3;
-#pragma unroll
-    for (int k = 0; k < NH; ++k) z = fmaf(__shfl_sync(0xffffffffu, w3, k), __shfl_sync(0xffffffffu, h2, k), z);
-    return z;
+    MlpLane m;
+    m.load(w, lane);
+    return m.logit(f);
 }
 
 // feature k of the state (lane k computes it)
