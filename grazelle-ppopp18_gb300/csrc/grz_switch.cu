@@ -116,7 +116,10 @@ __global__ void __launch_bounds__(T) k_features_decide(FeatIn in, const float* _
 // graph's conditional handles: hengine selects the next iteration's body, hloop
 // keeps the WHILE node going.  `initial`: the decision before the first iteration, from the
 // starting vote; no statistics, no clearing.
-constexpr int DECIDE_U = 4;  // words a thread loads together: one step for up to 20M vertices
+// Words a thread loads together, with a block per SM: one step for up to 20M vertices.  More blocks queue at
+// the counters (GB300, a BFS run on 2^24 vertices, 1 word with 8 blocks per SM 817 us, 2 with 4 772, 4 with 2
+// 733, 8 with 1 732).
+constexpr int DECIDE_U = 8;
 
 struct RunIn {
     FeatIn feat;                        // frontier = the next HasInfo
@@ -581,7 +584,7 @@ int grz_switch_launch_run_decide(grz_graph* g, const unsigned long long* next_fr
     in.initial = initial;
     in.hop_list = f.hop_list;
     in.hop_pulls = hop_pulls;
-    const unsigned grid = (unsigned)std::min<uint64_t>((in.feat.words + T - 1) / T, (uint64_t)g->num_sms * 2);
+    const unsigned grid = (unsigned)std::min<uint64_t>((in.feat.words + T - 1) / T, (uint64_t)g->num_sms);
     k_run_decide<<<grid, T, 0, g->stream>>>(in, f.ctl, hloop, hengine);
     return grz_cuda_check(g, cudaGetLastError(), "run decision");
 }
