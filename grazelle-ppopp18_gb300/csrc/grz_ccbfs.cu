@@ -1183,6 +1183,48 @@ __global__ void __launch_bounds__(T, GRZ_BFS_MINB) k_bfs_pull_first(unsigned lon
     if (threadIdx.x == 0) vote_add(vote, my_vote);
 }
 
+// Calls f(vertex, whether it is marked, load(vertex) if it is, half) for the vertices of every nonzero word
+// word(i), i < W, a warp per word, first the lower then the upper 32 vertices (f is called by whole warps);
+// g(word, bits) once after each.  A warp looks at `span` words and takes MARK_WORDS nonzero ones at a time,
+// whose vertices it loads for first (one after the other, each a trip to memory, the pass after a run of
+// small iterations that had marked most of 100k vertices took 27.6 us, so 4.4 us; 2 words keep more warps
+// resident than 4).  A map of few words is spread over more warps; a large one is nearly empty, and 32 words
+// are one load.
+constexpr int MARK_WORDS = 2;
+constexpr uint64_t MARK_SPAN_W = 1u << 15;
+__host__ __device__ constexpr int mark_span(uint64_t W) { return W < MARK_SPAN_W ? 4 : 32; }
+template <typename M, typename C, typename F, typename G>
+__device__ __forceinline__ void for_marked(M word, uint64_t W, C load, F f, G g)
+{
+    const int lane = threadIdx.x & 31, span = mark_span(W);
+    const uint64_t nwarps = (uint64_t)gridDim.x * (T / 32);
+    for (uint64_t w0 = span * ((uint64_t)blockIdx.x * (T / 32) + (threadIdx.x >> 5)); w0 < W; w0 += span * nwarps) {
+        const unsigned long long mine = lane < span && w0 + lane < W ? word(w0 + lane) : 0ull;
+        unsigned nz = __ballot_sync(0xffffffffu, mine != 0);
+        while (nz) {  // warp-uniform
+            unsigned long long bits[MARK_WORDS], c[2 * MARK_WORDS];
+            uint32_t at[MARK_WORDS];
+#pragma unroll
+            for (int j = 0; j < MARK_WORDS; ++j) {
+                const int i = nz ? __ffs(nz) - 1 : 0;
+                bits[j] = __shfl_sync(0xffffffffu, mine, i);
+                if (!nz) bits[j] = 0ull;
+                at[j] = (uint32_t)(w0 + i);
+                nz &= nz - 1;
+            }
+#pragma unroll
+            for (int j = 0; j < 2 * MARK_WORDS; ++j)
+                c[j] = (bits[j / 2] >> (32 * (j & 1) + lane)) & 1ull ? load(64 * at[j / 2] + 32 * (j & 1) + lane) : 0ull;
+#pragma unroll
+            for (int j = 0; j < 2 * MARK_WORDS; ++j) {
+                if (!bits[j / 2]) break;
+                f(64 * at[j / 2] + 32 * (j & 1) + lane, ((bits[j / 2] >> (32 * (j & 1) + lane)) & 1ull) != 0, c[j], j & 1);
+                if ((j & 1) && lane == 0) g(at[j / 2], bits[j / 2]);
+            }
+        }
+    }
+}
+
 // BFS: visit the touched destinations (pull: decode the winning (vector, source) key; push: the
 // smallest source), in one pass over the touched list
 template <bool FromPull>
@@ -1218,46 +1260,25 @@ __global__ void __launch_bounds__(T) k_bfs_visit(const uint32_t* __restrict__ to
             atomicAnd(wants + (d >> 6), ~(1ull << (d & 63)));
         }
     } else {
-        // many: every vertex, in ID order, 4 per thread per step with the loads of the 4 issued
-        // together (coalesced, no per-thread dependence chains).  A vertex was touched in this
-        // call when its HasInfo* bit is set (at first touch) and its WantsInfo bit still is (a
-        // caller's earlier vector range of this iteration visited and cleared its own).  Each
-        // vertex is read and written by one thread only, so cand and degree go through the
-        // read-only path.
-        constexpr int U = 4;
-        const uint32_t lane = threadIdx.x & 31;
-        for (uint64_t base = (uint64_t)blockIdx.x * T * U; base < V; base += (uint64_t)gridDim.x * T * U) {  // warp-uniform
-            uint32_t d[U];
-            bool hit[U];
-#pragma unroll
-            for (int j = 0; j < U; ++j) {
-                d[j] = (uint32_t)(base + (uint64_t)j * T + threadIdx.x);
-                hit[j] = d[j] < V && (((has_next[d[j] >> 6] & wants[d[j] >> 6]) >> (d[j] & 63)) & 1ull);
-            }
-            uint32_t p[U], deg[U];
-#pragma unroll
-            for (int j = 0; j < U; ++j) {
-                if (hit[j]) {
-                    p[j] = FromPull ? ~(uint32_t)(__ldg(cand64 + d[j]) & 0xffffffffull) : __ldg(cand32 + d[j]);
-                    deg[j] = __ldg(vc.degree + d[j]);
-                }
-            }
-#pragma unroll
-            for (int j = 0; j < U; ++j) {
-                if (hit[j]) {
-                    if (FromPull) cand64[d[j]] = ~0ull; else cand32[d[j]] = INF;
-                    parent[d[j]] = p[j];
-                    level[d[j]] = iter;
-                    my_vote += (vc.without_count ? 0ull : 1ull) + (vc.without_outdeg ? 0ull : (unsigned long long)deg[j]);
-                }
-                // the warp's 32 vertices lie in one 64-bit word: one atomicAnd clears their WantsInfo bits
-                const unsigned m = __ballot_sync(0xffffffffu, hit[j]);
-                if (m && lane == (uint32_t)(__ffs(m) - 1)) {
-                    const uint32_t d0 = d[j] - lane;
-                    atomicAnd(wants + (d0 >> 6), ~((unsigned long long)m << (d0 & 63)));
-                }
-            }
-        }
+        // many: every word of vertices.  A vertex was touched in this call when its HasInfo* bit is set
+        // (at first touch) and its WantsInfo bit still is (a caller's earlier vector range of this
+        // iteration visited and cleared its own).  Its candidate and out-degree are loaded together.
+        // GB300, R-MAT of 2^24 vertices, a run's large visit until the next kernel starts: 37.8 us with a look
+        // at every vertex, 26.9 us over the nonzero words.
+        for_marked(
+            [&](uint64_t w) { return has_next[w] & wants[w]; }, (uint64_t)V / 64 + 1,
+            [&](uint32_t d) {
+                const uint32_t p = FromPull ? ~(uint32_t)cand64[d] : cand32[d];
+                return (unsigned long long)(vc.without_outdeg ? 0u : vc.degree[d]) << 32 | p;
+            },
+            [&](uint32_t d, bool marked, unsigned long long c, int) {
+                if (!marked) return;
+                if (FromPull) cand64[d] = ~0ull; else cand32[d] = INF;
+                parent[d] = (uint32_t)c;
+                level[d] = iter;
+                my_vote += (vc.without_count ? 0ull : 1ull) + (c >> 32);
+            },
+            [&](uint64_t w, unsigned long long bits) { wants[w] &= ~bits; });
     }
     my_vote = block_sum_u64(my_vote, red);
     if (threadIdx.x == 0) vote_add(vote, my_vote);
@@ -1569,47 +1590,6 @@ __global__ void __cluster_dims__(HOP_CTAS, 1, 1) __launch_bounds__(HOP_T, 1) k_h
     }
 }
 
-// Calls f(vertex, whether it is marked, load(vertex) if it is, half) for the vertices of every nonzero word
-// of `map`, a warp per word, first the lower then the upper 32 vertices (f is called by whole warps);
-// g(word, bits) once after each.  A warp looks at `span` words and takes HOP_WORDS nonzero ones at a time,
-// whose vertices it loads for first: one after the other, each a trip to memory, they took a run that had
-// marked most of 100k vertices 27.6 us, so 4.4 us.  A map of few words is spread over more warps (4 words
-// each; a large one is nearly empty, and 32 words are one load).
-constexpr int HOP_WORDS = 4;
-constexpr uint64_t HOP_SPAN_W = 1u << 15;
-__host__ __device__ constexpr int hop_span(uint64_t W) { return W < HOP_SPAN_W ? HOP_WORDS : 32; }
-template <typename C, typename F, typename G>
-__device__ __forceinline__ void hop_marked(const unsigned long long* __restrict__ map, uint64_t W, C load, F f, G g)
-{
-    const int lane = threadIdx.x & 31, span = hop_span(W);
-    const uint64_t nwarps = (uint64_t)gridDim.x * (T / 32);
-    for (uint64_t w0 = span * ((uint64_t)blockIdx.x * (T / 32) + (threadIdx.x >> 5)); w0 < W; w0 += span * nwarps) {
-        const unsigned long long mine = lane < span && w0 + lane < W ? map[w0 + lane] : 0ull;
-        unsigned nz = __ballot_sync(0xffffffffu, mine != 0);
-        while (nz) {  // warp-uniform
-            unsigned long long bits[HOP_WORDS], c[2 * HOP_WORDS];
-            uint32_t at[HOP_WORDS];
-#pragma unroll
-            for (int j = 0; j < HOP_WORDS; ++j) {
-                const int i = nz ? __ffs(nz) - 1 : 0;
-                bits[j] = __shfl_sync(0xffffffffu, mine, i);
-                if (!nz) bits[j] = 0ull;
-                at[j] = (uint32_t)(w0 + i);
-                nz &= nz - 1;
-            }
-#pragma unroll
-            for (int j = 0; j < 2 * HOP_WORDS; ++j)
-                c[j] = (bits[j / 2] >> (32 * (j & 1) + lane)) & 1ull ? load(64 * at[j / 2] + 32 * (j & 1) + lane) : 0ull;
-#pragma unroll
-            for (int j = 0; j < 2 * HOP_WORDS; ++j) {
-                if (!bits[j / 2]) break;
-                f(64 * at[j / 2] + 32 * (j & 1) + lane, ((bits[j / 2] >> (32 * (j & 1) + lane)) & 1ull) != 0, c[j], j & 1);
-                if ((j & 1) && lane == 0) g(at[j / 2], bits[j / 2]);
-            }
-        }
-    }
-}
-
 // BFS, after k_hop: levels, WantsInfo and the last frontier's HasInfo* of the marked vertices, and the
 // parents of those that a push visited, whose candidates it empties.  `clear`: no k_hop_parents follows.
 __global__ void __launch_bounds__(T) k_hop_visit(const grz_runctl* __restrict__ ctl, unsigned long long* __restrict__ map, uint64_t W,
@@ -1619,8 +1599,8 @@ __global__ void __launch_bounds__(T) k_hop_visit(const grz_runctl* __restrict__ 
 {
     const uint32_t last = ctl->level;
     unsigned long long in_last = 0ull;
-    hop_marked(
-        map, W, [&](uint32_t d) { return cand64[d]; },
+    for_marked(
+        [&](uint64_t w) { return map[w]; }, W, [&](uint32_t d) { return cand64[d]; },
         [&](uint32_t d, bool marked, unsigned long long c, int half) {
             bool l = false;
             if (marked) {
@@ -1651,12 +1631,12 @@ __global__ void __launch_bounds__(T) k_hop_parents(const grz_runctl* __restrict_
                                                    const uint32_t* __restrict__ rowptr, const uint32_t* __restrict__ hub_vid, uint32_t nhub)
 {
     if (!ctl->hop_pulls) {
-        hop_marked(map, W, [](uint32_t) { return 0ull; }, [](uint32_t, bool, unsigned long long, int) {},
+        for_marked([&](uint64_t w) { return map[w]; }, W, [](uint32_t) { return 0ull; }, [](uint32_t, bool, unsigned long long, int) {},
                    [&](uint64_t w, unsigned long long) { map[w] = 0ull; });
         return;
     }
-    hop_marked(
-        map, W, [&](uint32_t d) { return cand64[d]; },
+    for_marked(
+        [&](uint64_t w) { return map[w]; }, W, [&](uint32_t d) { return cand64[d]; },
         [&](uint32_t d, bool marked, unsigned long long c, int) {
             if (!marked || c == ~0ull) return;  // a push visited it
             cand64[d] = ~0ull;
@@ -1684,8 +1664,8 @@ __global__ void __launch_bounds__(T) k_hop_labels(const grz_runctl* __restrict__
 {
     const uint32_t last = ctl->level;
     unsigned long long in_last = 0ull;
-    hop_marked(
-        map, W, [&](uint32_t d) { return (unsigned long long)cand32[d]; },
+    for_marked(
+        [&](uint64_t w) { return map[w]; }, W, [&](uint32_t d) { return (unsigned long long)cand32[d]; },
         [&](uint32_t d, bool marked, unsigned long long c, int half) {
             bool l = false;
             if (marked) {
@@ -2531,7 +2511,7 @@ static int hop_phase(grz_graph* g)
     in.ctl = f.ctl;
     in.pulls = hop_pulls(g);
     const uint64_t W = words_of(g->V);
-    const unsigned grid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(W / (hop_span(W) * (T / 32)) + 1, (uint64_t)g->num_sms * 8));
+    const unsigned grid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(W / (mark_span(W) * (T / 32)) + 1, (uint64_t)g->num_sms * 8));
     if (bfs) {
         k_hop<true><<<HOP_CTAS, HOP_T, HOP_SMEM, g->stream>>>(in);
         k_hop_visit<<<grid, T, 0, g->stream>>>(f.ctl, f.hop_map, W, f.cand64, f.label, f.level, f.wants, f.has_next, !in.pulls);
