@@ -1401,6 +1401,10 @@ __device__ __forceinline__ HopPart hop_exchange(cg::cluster_group& cl, HopPart x
 }
 
 // (started by the decision kernel when the next iteration's vote is at most GRZ_HOP_VOTE)
+// Vectors of a vertex that its lane lists by itself; its warp lists more.  A hub's thousands of vectors listed
+// by one lane held up all 16 blocks: GB300, first small iterations of a BFS on 2^24 R-MAT vertices 58 -> 10 us.
+constexpr uint32_t HOP_NARROW = 4;
+
 template <bool IsBfs>
 __global__ void __cluster_dims__(HOP_CTAS, 1, 1) __launch_bounds__(HOP_T, 1) k_hop(const HopIn in)
 {
@@ -1444,20 +1448,32 @@ __global__ void __cluster_dims__(HOP_CTAS, 1, 1) __launch_bounds__(HOP_T, 1) k_h
     }
     cl.sync();  // other blocks have added to this one's list
     hop_exchange(cl, sum, &s_items[0], &s_block[1], s_part[1]);
-    // lists vertex d's vectors [r0, r0 + n) in this block's list q; false when it is full
-    auto append = [&](int q, int slot, uint32_t d, uint32_t r0, uint32_t n) -> bool {
-        const uint32_t k = max(n, 1u), at = atomicAdd(&s_items[slot], k);
+    // lists the vectors [r0, r0 + n) of the lanes' vertices d that are `fresh` in this block's list q (by
+    // whole warps, which share the writing of long ranges); false for those that it has no room for
+    auto append = [&](int q, int slot, bool fresh, uint32_t d, uint32_t r0, uint32_t n) -> bool {
+        const uint32_t k = fresh ? max(n, 1u) : 0u, at = fresh ? atomicAdd(&s_items[slot], k) : 0u;
         uint32_t* vec = s_mem + q * 2 * HOP_CAP;
-        if (at > HOP_CAP || k > HOP_CAP - at) {
+        const bool fits = at <= HOP_CAP && k <= HOP_CAP - at;
+        if (fresh && !fits) {
             atomicOr(in.map + (d >> 6), 1ull << (d & 63));
             for (uint32_t i = at; i < HOP_CAP; ++i) vec[HOP_CAP + i] = 0;  // places no one takes carry no mark
-            return false;
         }
-        for (uint32_t i = 0; i < k; ++i) {
-            vec[at + i] = n ? r0 + i : HOP_NOVEC;
-            vec[HOP_CAP + at + i] = i == 0 ? d | HOP_FIRST : d;
+        const bool wide = fresh && fits && k > HOP_NARROW;
+        if (fresh && fits && !wide)
+            for (uint32_t i = 0; i < k; ++i) {
+                vec[at + i] = n ? r0 + i : HOP_NOVEC;
+                vec[HOP_CAP + at + i] = i == 0 ? d | HOP_FIRST : d;
+            }
+        for (unsigned todo = __ballot_sync(0xffffffffu, wide); todo; todo &= todo - 1) {
+            const int h = __ffs(todo) - 1;
+            const uint32_t hk = __shfl_sync(0xffffffffu, k, h), ha = __shfl_sync(0xffffffffu, at, h);
+            const uint32_t hr = __shfl_sync(0xffffffffu, r0, h), hd = __shfl_sync(0xffffffffu, d, h);
+            for (uint32_t i = lane; i < hk; i += 32) {
+                vec[ha + i] = hr + i;
+                vec[HOP_CAP + ha + i] = i == 0 ? hd | HOP_FIRST : hd;
+            }
         }
-        return true;
+        return fits;
     };
     uint32_t it = 0, mode = mode0, pulls = 0;     // iterations finished, this one's engine, pulls before it
     unsigned long long left = unvisited, vote;    // BFS: vertices not visited yet
@@ -1494,37 +1510,40 @@ __global__ void __cluster_dims__(HOP_CTAS, 1, 1) __launch_bounds__(HOP_T, 1) k_h
                 const uint32_t b = __shfl_sync(0xffffffffu, before, from ? (int)from - 1 : 0);
                 if (from) at -= b;
             }
-            if (!in_list) continue;
-            const uint32_t* vec = cl.map_shared_rank(s_mem + p * 2 * HOP_CAP, from);
-            const uint32_t us = vec[HOP_CAP + at], v = vec[at], u = us & ~HOP_FIRST;
-            if ((us & HOP_FIRST) && l == 0) atomicOr(in.map + (u >> 6), 1ull << (u & 63));
-            if (v == HOP_NOVEC) continue;
-            const uint32_t d = __ldg(reinterpret_cast<const uint32_t*>(in.nbr) + 4 * (uint64_t)v + l);
-            if (d >= in.V) continue;
+            uint32_t u = 0, d = INF;
+            if (in_list) {
+                const uint32_t* vec = cl.map_shared_rank(s_mem + p * 2 * HOP_CAP, from);
+                const uint32_t us = vec[HOP_CAP + at], v = vec[at];
+                u = us & ~HOP_FIRST;
+                if ((us & HOP_FIRST) && l == 0) atomicOr(in.map + (u >> 6), 1ull << (u & 63));
+                if (v != HOP_NOVEC) d = __ldg(reinterpret_cast<const uint32_t*>(in.nbr) + 4 * (uint64_t)v + l);
+            }
             bool fresh = false;
             uint32_t r0 = 0, r1 = 0, deg = 0;
             // the row pointers and degree are loaded while the atomic that decides is on its way
-            if (IsBfs) {
-                const unsigned long long key = ((unsigned long long)level << 33) | ((unsigned long long)mode << 32) | u;
-                const unsigned long long c = __ldcg(in.cand64 + d);
-                const bool w = (__ldg(in.wants + (d >> 6)) >> (d & 63)) & 1ull;
-                if (w && key < c) {
-                    const unsigned long long old = atomicMin(in.cand64 + d, key);
-                    r0 = __ldg(in.rowptr + d);
-                    r1 = __ldg(in.rowptr + d + 1);
-                    deg = __ldg(in.degree + d);
-                    fresh = old == ~0ull;
-                }
-            } else {
-                const uint32_t msg = __ldcg(in.label + u);
-                if (msg < __ldcg(in.label + d)) {
-                    const uint32_t old = atomicMin(in.label + d, msg);
-                    r0 = __ldg(in.rowptr + d);
-                    r1 = __ldg(in.rowptr + d + 1);
-                    deg = __ldg(in.degree + d);
-                    if (msg < old) {
-                        sum.min = min(sum.min, msg);
-                        fresh = atomicMin(in.cand32 + d, ~level) > ~level;
+            if (d < in.V) {
+                if (IsBfs) {
+                    const unsigned long long key = ((unsigned long long)level << 33) | ((unsigned long long)mode << 32) | u;
+                    const unsigned long long c = __ldcg(in.cand64 + d);
+                    const bool w = (__ldg(in.wants + (d >> 6)) >> (d & 63)) & 1ull;
+                    if (w && key < c) {
+                        const unsigned long long old = atomicMin(in.cand64 + d, key);
+                        r0 = __ldg(in.rowptr + d);
+                        r1 = __ldg(in.rowptr + d + 1);
+                        deg = __ldg(in.degree + d);
+                        fresh = old == ~0ull;
+                    }
+                } else {
+                    const uint32_t msg = __ldcg(in.label + u);
+                    if (msg < __ldcg(in.label + d)) {
+                        const uint32_t old = atomicMin(in.label + d, msg);
+                        r0 = __ldg(in.rowptr + d);
+                        r1 = __ldg(in.rowptr + d + 1);
+                        deg = __ldg(in.degree + d);
+                        if (msg < old) {
+                            sum.min = min(sum.min, msg);
+                            fresh = atomicMin(in.cand32 + d, ~level) > ~level;
+                        }
                     }
                 }
             }
@@ -1533,8 +1552,8 @@ __global__ void __cluster_dims__(HOP_CTAS, 1, 1) __launch_bounds__(HOP_T, 1) k_h
                 sum.vote_lo = (uint32_t)(x & 0xffffu);
                 sum.vote_hi += (uint32_t)(x >> 16);
                 sum.verts += 1;
-                if (!append(p ^ 1, nxt, d, r0, r1 - r0)) sum.flags |= HOP_OVER;
             }
+            if (__any_sync(0xffffffffu, fresh) && !append(p ^ 1, nxt, fresh, d, r0, r1 - r0) && fresh) sum.flags |= HOP_OVER;
         }
         sum = hop_exchange(cl, sum, &s_items[nxt], &s_block[p], s_part[p]);
         // every thread of the cluster takes the same decision from the iteration's totals
