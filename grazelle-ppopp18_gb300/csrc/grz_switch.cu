@@ -126,6 +126,7 @@ struct RunIn {
     unsigned long long* vote_slots;     // read and re-zeroed
     unsigned long long* clear_bm;       // old HasInfo (null when initial)
     uint32_t* counters;                 // u32[8] of the next edge phase, cleared
+    uint32_t* mail;                     // page-locked host memory: the control block, when the run ends
     int initial;
     uint32_t* hop_list;                 // the next frontier's vertices when its vote is at most GRZ_HOP_VOTE, or null
     int hop_pulls;                      // small pulls go to k_hop as well
@@ -275,6 +276,11 @@ __global__ void __launch_bounds__(T) k_run_decide(RunIn in, grz_runctl* __restri
         cudaGraphSetConditional(hengine, !running ? GRZ_RUN_NONE : (hop ? GRZ_RUN_HOP : (pull ? GRZ_RUN_PULL : GRZ_RUN_PUSH)));
         cudaGraphSetConditional(hloop, running);
     }
+    if (running) return;
+    __syncwarp();
+    static_assert(sizeof(grz_runctl) % 4 == 0, "copied by words");
+    const volatile uint32_t* const words = (const volatile uint32_t*)ctl;
+    for (uint32_t i = lane; i < sizeof(grz_runctl) / 4; i += 32) in.mail[i] = words[i];
 }
 
 // Forward + backward of weighted binary cross-entropy on logits, one thread per sample.  Each
@@ -581,6 +587,7 @@ int grz_switch_launch_run_decide(grz_graph* g, const unsigned long long* next_fr
     in.vote_slots = f.vote;
     in.clear_bm = clear_bm;
     in.counters = f.counters;
+    in.mail = (uint32_t*)f.mail;
     in.initial = initial;
     in.hop_list = f.hop_list;
     in.hop_pulls = hop_pulls;
