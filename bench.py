@@ -1044,7 +1044,7 @@ def main():
     ap.add_argument("--tune", action="append", default=[], metavar="KNOB=VALUE",
                     help="kernel-shape knob applied before the load (grazelle.engine.Graph.tune), e.g. pull_staging=1; repeatable")
     ap.add_argument("--pr-props", type=int, default=0, choices=[0, 1, 2],
-                    help="props the PageRank gather reads: 0 by size, 1 fixed point, 2 doubles (results identical)")
+                    help="props the PageRank gather reads: 0 or 2 packed in 8 bytes, 1 16-byte fixed point (results identical)")
     ap.add_argument("--directed", action="store_true", help="CC/BFS on the directed R-MAT (no symmetrisation), as the scale-27 stress configuration")
     a = ap.parse_args()
     if a.warmup < 3:

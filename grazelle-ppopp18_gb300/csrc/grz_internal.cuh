@@ -485,7 +485,7 @@ struct grz_frontier_state {
     float last_edge_ms;              // edge-phase time of the last step when timing is on
     int time_edges;
     cudaEvent_t ev[2];
-    // the run as one CUDA graph (WHILE over two iterations with IF nodes per engine)
+    // the run as one CUDA graph (WHILE over two iterations with a SWITCH over the engines)
     grz_runctl* ctl;                 // device
     uint32_t* hop_buf;               // u32[GRZ_HOP_VOTE]
     unsigned long long* hop_map;     // vertices k_hop listed (zero between uses)
