@@ -769,17 +769,33 @@ __global__ void __launch_bounds__(T) k_push_expand(const uint32_t* __restrict__ 
     const uint32_t nf = counters[3], total = counters[2];
     const uint32_t ntiles = (total + PUSH_TILE - 1) / PUSH_TILE;
     unsigned long long my_vote = 0;
+    // a tile has at most as many owners as threads: each thread holds one of the next tile's, loaded while
+    // this tile is expanded (GB300, 8 BFS by pushes alone on 2^24 vertices 16.56 -> 16.36 ms)
+    static_assert(PUSH_TILE == T, "one owner per thread");
+    uint32_t first = blockIdx.x < ntiles ? tile_first[blockIdx.x] : nf;
+    uint32_t after = (uint64_t)blockIdx.x + gridDim.x < ntiles ? tile_first[blockIdx.x + gridDim.x] : nf;
+    uint32_t n_off = 0, n_src = 0, n_delta = 0;
+    auto owners = [&](uint32_t from) {
+        if (threadIdx.x < nf - from) {
+            n_off = voff[from + threadIdx.x];
+            n_src = frontier[from + threadIdx.x];
+            n_delta = vdelta[from + threadIdx.x];
+        }
+    };
+    owners(first);
     for (uint32_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-        const uint32_t first = tile_first[tile];
         const uint32_t t0 = tile * PUSH_TILE;
         const uint32_t tend = min(total, t0 + PUSH_TILE);
         // entries first .. first+nw-1 own every vector of the tile (each owns at least one)
         const uint32_t nw = min(PUSH_TILE, nf - first);
-        for (uint32_t i = threadIdx.x; i < nw; i += T) {
-            s_off[i] = voff[first + i];
-            s_src[i] = frontier[first + i];
-            s_delta[i] = vdelta[first + i];
+        if (threadIdx.x < nw) {
+            s_off[threadIdx.x] = n_off;
+            s_src[threadIdx.x] = n_src;
+            s_delta[threadIdx.x] = n_delta;
         }
+        first = after;
+        owners(first);
+        after = (uint64_t)tile + 2ull * gridDim.x < ntiles ? tile_first[tile + 2 * gridDim.x] : nf;
         __syncthreads();
         for (uint32_t base = t0; base < tend; base += T) {  // warp-uniform trip count
             const uint32_t gv = base + threadIdx.x;
