@@ -1279,7 +1279,7 @@ static int pr_hot_choose(grz_graph* g)
     if (!rc) {
         const unsigned grid = (unsigned)std::min<uint64_t>(blocks_for(V), (uint64_t)g->num_sms * 8);
         k_hot_hist<<<grid, PR_THREADS, 0, st>>>(g->degree, V, dmin, hist); GRZ_COUNT_LAUNCH(g);
-        k_hot_pick<<<1, HOT_PICK_T, 0, st>>>(hist, GRZ_PR_HOT_MAX, hist + 2 * HOT_BINS); GRZ_COUNT_LAUNCH(g);
+        k_hot_pick<<<1, HOT_PICK_T, 0, st>>>(hist, V < GRZ_PR_HOT_MAX_V ? GRZ_PR_HOT_MAX : GRZ_PR_HOT_FEW, hist + 2 * HOT_BINS); GRZ_COUNT_LAUNCH(g);
         rc = grz_cuda_check(g, cudaGetLastError(), "k_hot_pick");
     }
     if (!rc) rc = grz_cuda_check(g, cudaMemcpyAsync(pick, hist + 2 * HOT_BINS, sizeof(pick), cudaMemcpyDeviceToHost, st), "D2H");
