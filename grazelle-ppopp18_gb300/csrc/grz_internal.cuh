@@ -329,14 +329,14 @@ struct grz_list {
 #define GRZ_PR_MAX_SEGMENTS 256
 
 // Hot sources of the PageRank gather, at most: 12000 packed props are 96 KB of shared memory, the largest
-// table that fits the 100 KB carveout and so leaves L1 the rest, 20000 are 160 KB.  With the hot sources gone,
-// hardly a gather hits L1 (3% at R-MAT 20), so on graphs whose other props are few enough the larger table
-// wins; on larger ones the misses in flight need the room.  GB300, gather per iteration with 768 threads, 12000 /
-// 16000 / 20000 slots, R-MAT: 2^19 vertices 27.6 / 26.7 / 26.7 us, 2^20 47.7 / 47.0 / 46.1, 1.5M and 9M edges
-// 30.4 / 29.7 / 29.6, 2^21 88.0 / 87.8 / 88.9, 2^22 176.5 / 176.1 / 185, 2^24 826 / 906 / 906.  (Fewer: R-MAT 20
-// 46.7 / 44.5 us, R-MAT 24 848 / 807 with 4000 / 7800.)
+// table that fits the 100 KB carveout and so leaves L1 the rest, 20000 are 160 KB.  With the hot sources gone
+// and the other gathers going past L1, the larger table wins until the props outgrow L2, whose misses in
+// flight need the room; the largest, 26000, loses everywhere.  GB300, gather per iteration with 768 threads,
+// 12000 / 16000 / 20000 / 26000 slots, R-MAT: 2^20 vertices 47.4 / 45.3 / 44.9 / 63.8 us, 2^21 87.1 / 85.2 /
+// 84.1 / 90.3, 2^22 174.5 / 174.5 / 169.7 / 203.7, 2^23 198 / 199.5 / 196.6 / 516, 2^24 765 / 811 / 812 / 952,
+// 2^26 in segments 4471 / 4475 / 5078 / 5059.
 #define GRZ_PR_HOT_FEW 12000u
-#define GRZ_PR_HOT_MAX_V (3u << 19)  // vertices from which on a graph has GRZ_PR_HOT_FEW
+#define GRZ_PR_HOT_MAX_V (3u << 22)  // vertices from which on a graph has GRZ_PR_HOT_FEW
 #define GRZ_PR_HOT_MAX 20000u
 
 #define GRZ_BATCH_K 8  // instances per graph of a batch (grz_batch.cu)

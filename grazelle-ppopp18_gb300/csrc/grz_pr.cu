@@ -278,7 +278,10 @@ __global__ void __launch_bounds__(PR_THREADS, PR_GATHER_MIN_BLOCKS) k_pr_gather(
 // its width.  So what helps is fewer gathers through L1 and fewer instructions around them:
 //   * HOT: the props of up to GRZ_PR_HOT_MAX sources of the highest out-degrees are copied into
 //     shared memory when the block starts, and lanes that name one
-//     (GRZ_HUB_BASE + slot in the encoded list) read them there.
+//     (GRZ_HUB_BASE + slot in the encoded list) read them there.  The other gathers of a whole list then
+//     hardly hit L1 (3% at R-MAT 20) and go past it (GB300, through L1 / past it: R-MAT of 2^21 vertices 88 /
+//     84 us, 2^24 828 / 765; in segments 4449 / 4471 at 2^26, and without a table 146 / 286 on a uniform
+//     graph: those stay).
 //   * A thread owns four consecutive vectors (two 32-byte loads and one of four destinations, the
 //     next group's issued before this one's sums): it joins vectors of one destination in registers,
 //     so the u128 scan over the warp runs once per 128 vectors, not once per 32.
@@ -428,7 +431,7 @@ __global__ void __launch_bounds__(PK_THREADS, 1) k_pr_gather_pk(const uint4* __r
     auto get = [&](uint32_t id) -> pk_t {
         if (HOT) {
             if ((int)id < 0) return s_hot[id & (GRZ_HUB_BASE - 1)];
-            return __ldg(props + id);
+            return ADD ? __ldg(props + id) : __ldcg(props + id);
         }
         return __ldg(props + min(id, V));  // entry V is zero
     };
