@@ -115,10 +115,13 @@ static void free_graph_data(grz_graph* g, uint64_t next_V = ~0ull)
         // the PageRank arrays are sized by V alone: kept, and refilled at the next grz_pr_init
         g->pr_lists_changed = 1;
     } else {
-        void* plain[] = { g->pr_fx[0], g->pr_fx[1], g->pr_sum, g->pr_K, g->pr_rowacc, g->pr_cut, g->pr_pk[0], g->pr_pk[1] };
-        for (void* p : plain) cudaFree(p);
+        cudaFree(g->pr_fx[0]);  // and with it the arrays after it (grz_pr_prepare)
+        if (g->pr_pk_own)
+            for (void* p : { (void*)g->pr_pk[0], (void*)g->pr_pk[1] }) cudaFree(p);
+        g->pr_pk_own = 0;
         g->pr_pk[0] = g->pr_pk[1] = nullptr;
         g->pr_fx[0] = g->pr_fx[1] = nullptr; g->pr_sum = nullptr; g->pr_K = nullptr; g->pr_rowacc = nullptr;
+        g->pr_small_parts = nullptr;
         g->pr_cut = nullptr;
     }
     grz_dev_free(g, g->seg_nbr);
@@ -324,7 +327,6 @@ extern "C" void grz_graph_destroy(grz_graph* g)
     if (g->stats_dev) cudaFree(g->stats_dev);
     if (g->prof_work) cudaFree(g->prof_work);
     if (g->pr_bar) cudaFree(g->pr_bar);
-    if (g->pr_small_parts) cudaFree(g->pr_small_parts);
     if (g->pr_bar_host) cudaFreeHost(g->pr_bar_host);
     if (g->copy_stream) {
         cudaStreamDestroy(g->copy_stream);

@@ -550,6 +550,7 @@ struct grz_graph {
     void* pr_bar;         // grid barrier and phase timer of the persistent PageRank kernel (device)
     void* pr_bar_host;    // pinned read-back of its error word and phase times
     unsigned long long* pr_pk[2];  // u64[V+1]: the props packed (pk_to_fx), gathered instead of pr_fx in pr_pkmode
+    int pr_pk_own;        // pr_pk was allocated by itself, not with the other arrays
     int pr_pkmode;        // fused iterations gather pr_pk
     int pr_fx_stale;      // pr_fx[pr_cur] is behind pr_pk[pr_cur]
     int pr_pk_stale;      // pr_pk[pr_cur] is behind pr_fx[pr_cur]
