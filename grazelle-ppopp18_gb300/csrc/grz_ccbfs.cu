@@ -1658,8 +1658,9 @@ __global__ void __launch_bounds__(T) k_hop_visit(const grz_runctl* __restrict__ 
 }
 
 // BFS: parents of the marked vertices that a pull visited.  The candidate's source is the smallest in
-// the frontier; its vector is the last one that starts at or below it, and the parent is the largest
-// source there that was visited one iteration earlier.
+// the frontier; its vector is the last one that starts below it, or, when that one ends before it, the
+// next (repeated edges can fill the end of one vector and the start of the next: the first that holds
+// the source counts).  The parent is the largest source there that was visited one iteration earlier.
 __global__ void __launch_bounds__(T) k_hop_parents(const grz_runctl* __restrict__ ctl, unsigned long long* __restrict__ map, uint64_t W,
                                                    unsigned long long* __restrict__ cand64, uint32_t* __restrict__ parent,
                                                    const uint32_t* __restrict__ level, uint32_t V, const uint4* __restrict__ nbr,
@@ -1677,13 +1678,21 @@ __global__ void __launch_bounds__(T) k_hop_parents(const grz_runctl* __restrict_
             cand64[d] = ~0ull;
             const uint32_t u = (uint32_t)c, before = (uint32_t)(c >> 33) - 1;
             uint32_t lo = __ldg(rowptr + d), hi = __ldg(rowptr + d + 1) - 1;
+            const uint32_t last = hi;
             while (lo < hi) {
                 const uint32_t mid = lo + (hi - lo + 1) / 2;
-                if (grz_hub_decode(__ldg(&nbr[mid].x), hub_vid, nhub) <= u) lo = mid; else hi = mid - 1;
+                if (grz_hub_decode(__ldg(&nbr[mid].x), hub_vid, nhub) < u) lo = mid; else hi = mid - 1;
             }
-            const uint4 s = __ldg(nbr + lo);
-            const uint32_t id[4] = { grz_hub_decode(s.x, hub_vid, nhub), grz_hub_decode(s.y, hub_vid, nhub),
-                                     grz_hub_decode(s.z, hub_vid, nhub), grz_hub_decode(s.w, hub_vid, nhub) };
+            uint32_t id[4];
+            auto sources = [&](uint32_t vec) {
+                const uint4 s = __ldg(nbr + vec);
+                id[0] = grz_hub_decode(s.x, hub_vid, nhub);
+                id[1] = grz_hub_decode(s.y, hub_vid, nhub);
+                id[2] = grz_hub_decode(s.z, hub_vid, nhub);
+                id[3] = grz_hub_decode(s.w, hub_vid, nhub);
+            };
+            sources(lo);
+            if (lo < last && id[3] < u) sources(lo + 1);  // (a vector before the last is full)
             uint32_t best = u;
 #pragma unroll
             for (int l = 0; l < 4; ++l)

@@ -132,3 +132,46 @@ def test_lists_grouped_but_not_ascending(derive):
                 np.testing.assert_array_equal(lv, A.bfs(r, flags)[1])
         np.testing.assert_array_equal(B.connected_components(), A.connected_components())
         np.testing.assert_array_equal(B.pagerank(5), A.pagerank(5))
+
+
+def _repeated(V, seed):
+    """Edges drawn with replacement from few sources: every list holds runs of the same neighbour, across
+    the ends of vectors too.  And the smallest such list, 10 11 12 15 | 15 16 17 18
+    into the last vertex, with 15 and 16 behind the vertex before it."""
+    rng = np.random.RandomState(seed)
+    n = 12 * V
+    src, dst = rng.randint(0, V, size=n) // 3 * 3 % V, rng.randint(0, V, size=n)
+    first = np.array([0, 1, 2, 5, 5, 6, 7, 8]) + 10
+    keep = (src != dst) & (dst != V - 1) & (src != V - 1)
+    src = np.concatenate([src[keep], first, np.full(2, V - 2), np.full(3, 4)])
+    dst = np.concatenate([dst[keep], np.full(8, V - 1), [15, 16], [V - 2] * 3])
+    return _edges(V, src, dst)
+
+
+@pytest.mark.parametrize("V", [60, 700, 4000])
+@pytest.mark.parametrize("hubs", [0, 16])
+def test_parents_over_repeated_edges(V, hubs):
+    """A repeated in-edge may end one vector and begin the next: the first vector that holds a frontier
+    source decides the parent, whatever runs the pull."""
+    from grazelle import native, switch
+    from grazelle.engine import Graph
+    g = _repeated(V, V)
+    pull, push = g.pull_order().pairs(), g.push_order().pairs()
+    L = O.layout(V, pull, push)
+    with Graph(0) as G:
+        G.tune(hubs=hubs)
+        G.load_pairs(V, pull, push)
+        net = switch.pretrained(0)
+        for learned in (False, True):
+            G.set_policy(native.POLICY_LEARNED if learned else native.POLICY_THRESHOLD, net if learned else None)
+            for flags in (0, native.FORCE_PULL, native.FORCE_PUSH):
+                for r in (0, 4, V // 2, V - 2):
+                    what = "learned %s flags %d root %d" % (learned, flags, r)
+                    par, lv = G.bfs(r, flags)
+                    par2, lv2 = G.bfs(r, flags | native.FLAG_HOST_LOOP)
+                    np.testing.assert_array_equal(lv, lv2, err_msg=what)
+                    np.testing.assert_array_equal(par, par2, err_msg=what)
+        G.set_policy(native.POLICY_THRESHOLD)
+        for flags in (0, native.FORCE_PULL, native.FORCE_PUSH):
+            np.testing.assert_array_equal(G.bfs(0, flags)[0], O.bfs(L, flags)[0], err_msg="flags %d" % flags)
+        assert G.bfs(V - 2, native.FORCE_PULL)[0][V - 1] == 15  # of the first vector, 10 11 12 15
