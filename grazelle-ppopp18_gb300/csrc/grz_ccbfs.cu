@@ -1103,11 +1103,11 @@ __global__ void __launch_bounds__(T, GRZ_BFS_MINB) k_bfs_pull_first(unsigned lon
         const uint4 s = __ldcs(nbr + vec);
         const uint32_t ids[4] = { grz_hub_decode(s.x, hub_vid, nhub), grz_hub_decode(s.y, hub_vid, nhub),
                                   grz_hub_decode(s.z, hub_vid, nhub), grz_hub_decode(s.w, hub_vid, nhub) };
-        bool in[4];
+        uint32_t best = 0;  // source + 1 (the sources of a list that is only grouped come in any order)
 #pragma unroll
-        for (int l = 0; l < 4; ++l) in[l] = ids[l] < V && bit_of(has, ids[l]);
-        // lanes ascend by source: the largest frontier source is the last lane with one
-        return in[3] ? ids[3] : in[2] ? ids[2] : in[1] ? ids[1] : in[0] ? ids[0] : INF;
+        for (int l = 0; l < 4; ++l)
+            if (ids[l] < V && bit_of(has, ids[l])) best = max(best, ids[l] + 1);
+        return best - 1;
     };
     auto visit = [&](uint32_t v, uint32_t p) {
         parent[v] = p;

@@ -104,3 +104,36 @@ def test_digest(n):
                 assert G.digest() == ref(np.where(lv < 0, 0xffffffff, lv), lv >= 0, deg)
         lab = G.connected_components()
         assert G.digest() == ref(lab, lab == np.arange(n), 0 * deg)
+
+
+@pytest.mark.parametrize("first_n", [1, 2, 5])
+@pytest.mark.parametrize("hubs", [0, 64])
+def test_first_pass_over_sources_in_any_order(first_n, hubs):
+    """Lists need only be grouped by destination.  The parent is the largest frontier source of the first
+    vector that holds one, wherever in the vector it stands: the early-exit pass, the compacted pull, the
+    scan and a restatement of the rule agree."""
+    from grazelle import graphgen as gg, native
+    from grazelle.engine import Graph
+    g = gg.rmat(12, 8, seed=12)
+    V, pull = g.num_vertices, g.pull_order()
+    o = np.lexsort((np.random.RandomState(2).rand(g.num_edges), pull.dst))
+    src, dst = pull.src[o].astype(np.int64), pull.dst[o].astype(np.int64)
+    start = np.searchsorted(dst, np.arange(V + 1))
+    with Graph(0) as G:
+        G.tune(hubs=hubs)
+        G.load_pairs(V, gg.EdgeList(V, src.astype(np.uint64), dst.astype(np.uint64)).pairs(), g.push_order().pairs())
+        for r in (0, 9):
+            found = []
+            for form in ({"bfs_pull_first": first_n}, {"bfs_pull_first": 0}, {"bfs_pull_scan": 1}):
+                G.tune(bfs_pull_first=first_n, bfs_pull_scan=0).tune(**form)
+                found.append(G.bfs(r, native.FORCE_PULL))
+            levels = found[0][1]
+            rule = np.full(V, -1.0)
+            for v in np.flatnonzero(levels > 0):
+                s = src[start[v]:start[v + 1]]
+                hit = np.flatnonzero(levels[s] == levels[v] - 1)
+                first = s[hit[0] // 4 * 4:hit[0] // 4 * 4 + 4]
+                rule[v] = first[levels[first] == levels[v] - 1].max()
+            for par, lv in found:
+                np.testing.assert_array_equal(lv, levels)
+                np.testing.assert_array_equal(par, rule)
