@@ -365,12 +365,12 @@ static const void* pinned_device_view(const void* p)
     return at.type == cudaMemoryTypeHost ? at.devicePointer : nullptr;
 }
 
-// The device's address of the n bytes at host pointer p when all of them are page-locked and mapped, or
-// null.  A kernel that writes results there saves the copy and its pass over device memory: GB300,
-// reading back 2^24 CC labels 758 -> 706 us, 4096 14 -> 11.6 us.
+// The device's address of the n bytes at host pointer p when all of them are page-locked and mapped, and
+// aligned for the 8-byte values that kernels store, or null.  A kernel that writes results there saves the
+// copy and its pass over device memory: GB300, reading back 2^24 CC labels 758 -> 706 us, 4096 14 -> 11.6 us.
 static void* mapped_view(void* p, size_t n)
 {
-    if (!n) return nullptr;
+    if (!n || ((uintptr_t)p & 7)) return nullptr;
     const char* first = (const char*)pinned_device_view(p);
     if (!first) return nullptr;
     const char* last = (const char*)pinned_device_view((const char*)p + n - 1);
@@ -748,7 +748,7 @@ extern "C" int grz_read_props(grz_graph* g, double* host, uint64_t cap)
     if (!g || !host) return GRZ_ERR_ARG;
     if (cap < g->V) return grz_set_error(g, GRZ_ERR_ARG, "capacity below V");
     GRZ_CK(g, cudaSetDevice(g->device));
-    // page-locked memory is written by the converting kernel itself; other memory gets a copy
+    // aligned page-locked memory is written by the converting kernel itself; other memory gets a copy
     double* direct = (double*)mapped_view(host, sizeof(double) * g->V);
     double* out = direct ? direct : g->prop;
     if (g->app == GRZ_APP_PAGERANK && g->pr_fx[0]) {
