@@ -1103,10 +1103,13 @@ __global__ void __launch_bounds__(T, GRZ_BFS_MINB) k_bfs_pull_first(unsigned lon
         const uint4 s = __ldcs(nbr + vec);
         const uint32_t ids[4] = { grz_hub_decode(s.x, hub_vid, nhub), grz_hub_decode(s.y, hub_vid, nhub),
                                   grz_hub_decode(s.z, hub_vid, nhub), grz_hub_decode(s.w, hub_vid, nhub) };
-        uint32_t best = 0;  // source + 1 (the sources of a list that is only grouped come in any order)
+        bool in[4];
 #pragma unroll
-        for (int l = 0; l < 4; ++l)
-            if (ids[l] < V && bit_of(has, ids[l])) best = max(best, ids[l] + 1);
+        for (int l = 0; l < 4; ++l) in[l] = ids[l] < V && bit_of(has, ids[l]);
+        // (the sources of a list that is only grouped come in any order)
+        uint32_t best = 0;  // source + 1
+#pragma unroll
+        for (int l = 0; l < 4; ++l) best = max(best, in[l] ? ids[l] + 1 : 0u);
         return best - 1;
     };
     auto visit = [&](uint32_t v, uint32_t p) {
