@@ -42,10 +42,20 @@ constexpr int PR_THREADS = 256;
 // The gathers and applies of grz_pr_iterate start while the kernel before them ends (programmatic
 // dependent launch): pdl_start lets the next kernel of the stream begin, pdl_wait holds until the one
 // before has completed and its writes are visible.  What a kernel reads before pdl_wait (the lists,
-// the degrees) no kernel of the chain writes.  GB300, us per iteration, plain launches -> these: R-MAT of 4096
+// the degrees) no kernel of the chain writes.  What the chain does write (props, hot table, sums,
+// accumulators, the iteration's constant) comes through the coherent path and through pointers taken
+// after the wait (after_wait): the read-only path asks for data that stays the same for the whole kernel, and
+// a load through a pointer known before may be moved above the wait.  GB300, us per iteration, plain launches -> these: R-MAT of 4096
 // vertices 10.3 -> 7.3, of 50k 12.4 -> 9.8, of 2^20 59 -> 56.
 __device__ __forceinline__ void pdl_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+template <typename T>
+__device__ __forceinline__ T* after_wait(T* p)
+{
+    asm volatile("" : "+l"(p) : : "memory");
+    return p;
+}
 
 template <typename... P, typename... A>
 cudaError_t pdl_launch(void (*kernel)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t stream, A... args)
@@ -83,6 +93,14 @@ __device__ __forceinline__ u128 ld_fx(const u128* p, uint32_t i)
 typedef unsigned long long pk_t;
 __device__ __forceinline__ u128 ld_prop(const u128* p, uint32_t i) { return ld_fx(p, i); }
 __device__ __forceinline__ u128 ld_prop(const pk_t* p, uint32_t i) { return pk_to_fx(__ldg(p + i)); }
+
+// a packed prop through the coherent path, L1-cached (nothing writes the props while they are read)
+__device__ __forceinline__ pk_t ld_l1(const pk_t* p)
+{
+    pk_t x;
+    asm("ld.global.u64 %0, [%1];" : "=l"(x) : "l"(p));
+    return x;
+}
 
 // The same through the coherent path (ld.global, L1-cached): for the persistent kernel, whose
 // apply phase rewrites the props that a later gather phase of the same launch reads, which the
@@ -368,9 +386,8 @@ __device__ __forceinline__ void pk_group(uint4 k, u128 v0, u128 v1, u128 v2, u12
 template <bool HOT, bool ADD>
 __global__ void __launch_bounds__(PK_THREADS, 1) k_pr_gather_pk(const uint4* __restrict__ nbr, const uint32_t* __restrict__ dstv,
                                                                 uint32_t first, uint32_t end, uint32_t per,
-                                                                const pk_t* __restrict__ props, uint32_t V,
-                                                                const pk_t* __restrict__ hot, uint32_t nhot,
-                                                                u128* __restrict__ rowacc, const PRConst pc)
+                                                                const pk_t* props, uint32_t V, const pk_t* hot, uint32_t nhot,
+                                                                u128* rowacc, const PRConst pc)
 {
     extern __shared__ __align__(16) pk_t s_hot[];
     const int lane = threadIdx.x & 31;
@@ -411,19 +428,23 @@ __global__ void __launch_bounds__(PK_THREADS, 1) k_pr_gather_pk(const uint4* __r
         if (lo > first) kbefore = __ldg(dstv + lo - 1);
     }
     pdl_wait();
+    props = after_wait(props);
+    hot = after_wait(hot);
+    rowacc = after_wait(rowacc);
     if (HOT) {
         // 16 bytes per thread and step, all steps' loads in flight (the table ends in zeros)
         const uint32_t n16 = (nhot + 2) / 2;
 #pragma unroll
         for (uint32_t j = 0; j < (GRZ_PR_HOT_MAX / 2 + PK_THREADS) / PK_THREADS; ++j) {
             const uint32_t i = j * PK_THREADS + threadIdx.x;
-            if (i < n16) reinterpret_cast<ulonglong2*>(s_hot)[i] = __ldg(reinterpret_cast<const ulonglong2*>(hot) + i);
+            if (i < n16) reinterpret_cast<ulonglong2*>(s_hot)[i] = __ldcg(reinterpret_cast<const ulonglong2*>(hot) + i);
         }
     }
     // the iteration's constant (pr_publish_K), by the warp of the last range, which is usually empty
     if (pc.K_out && wid == nwarps - 1) {
         u128 S = u128_zero();
-        for (uint32_t b = lane; b < pc.nparts; b += 32) S = u128_add(S, pc.part_in[b]);
+        const u128* const part_in = after_wait(pc.part_in);
+        for (uint32_t b = lane; b < pc.nparts; b += 32) S = u128_add(S, part_in[b]);
         for (int o = 16; o > 0; o >>= 1) S = u128_add(S, u128_shfl_down(S, o));
         if (lane == 0) *pc.K_out = __fma_rn((1.0 - fx_to_double(S)) / pc.nverts, pc.damping, pc.c);
     }
@@ -431,9 +452,9 @@ __global__ void __launch_bounds__(PK_THREADS, 1) k_pr_gather_pk(const uint4* __r
     auto get = [&](uint32_t id) -> pk_t {
         if (HOT) {
             if ((int)id < 0) return s_hot[id & (GRZ_HUB_BASE - 1)];
-            return ADD ? __ldg(props + id) : __ldcg(props + id);
+            return ADD ? ld_l1(props + id) : __ldcg(props + id);
         }
-        return __ldg(props + min(id, V));  // entry V is zero
+        return ld_l1(props + min(id, V));  // entry V is zero
     };
     auto put = [&](uint32_t key, u128 v) {
         if (key == GRZ_INVALID_ID) return;
@@ -516,7 +537,7 @@ __device__ __forceinline__ void hot_put(const uint2* __restrict__ hotmap, pk_t* 
 // thread loaded before any is stored; returns the block's partial of S' (valid in thread 0;
 // every thread of the block must call it)
 template <int U>
-__device__ __forceinline__ u128 pr_apply_range(u128* __restrict__ rowacc, const uint32_t* __restrict__ cut, bool clear_all,
+__device__ __forceinline__ u128 pr_apply_range(u128* rowacc, const uint32_t* __restrict__ cut, bool clear_all,
                                                const double* __restrict__ inv_deg, const uint32_t* __restrict__ degree, uint64_t V,
                                                double sK, double damping, u128* __restrict__ prop_fx, pk_t* __restrict__ prop_pk,
                                                double* __restrict__ prop_out, const uint2* __restrict__ hotmap, pk_t* __restrict__ hot,
@@ -564,10 +585,10 @@ __device__ __forceinline__ u128 pr_apply_range(u128* __restrict__ rowacc, const 
     return block_reduce_u128(s, red);
 }
 
-__global__ void __launch_bounds__(PR_THREADS, PR_APPLY_RESIDENT) k_pr_apply(u128* __restrict__ rowacc, const uint32_t* __restrict__ cut,
+__global__ void __launch_bounds__(PR_THREADS, PR_APPLY_RESIDENT) k_pr_apply(u128* rowacc, const uint32_t* __restrict__ cut,
                                                                             int clear_all, const double* __restrict__ inv_deg,
                                                                             const uint32_t* __restrict__ degree, uint64_t V,
-                                                                            const double* __restrict__ Kp, u128* __restrict__ part_out,
+                                                                            const double* Kp, u128* __restrict__ part_out,
                                                                             double damping, u128* __restrict__ prop_fx,
                                                                             pk_t* __restrict__ prop_pk, double* __restrict__ prop_out,
                                                                             const uint2* __restrict__ hotmap, pk_t* __restrict__ hot)
@@ -575,7 +596,7 @@ __global__ void __launch_bounds__(PR_THREADS, PR_APPLY_RESIDENT) k_pr_apply(u128
     __shared__ u128 red[PR_THREADS / 32];
     pdl_start();
     pdl_wait();
-    const u128 s = pr_apply_range<PR_APPLY_U>(rowacc, cut, clear_all != 0, inv_deg, degree, V, *Kp, damping, prop_fx, prop_pk, prop_out, hotmap, hot, blockIdx.x,
+    const u128 s = pr_apply_range<PR_APPLY_U>(after_wait(rowacc), cut, clear_all != 0, inv_deg, degree, V, *after_wait(Kp), damping, prop_fx, prop_pk, prop_out, hotmap, hot, blockIdx.x,
                                   gridDim.x, red);
     if (threadIdx.x == 0) part_out[blockIdx.x] = s;  // summed by the next gather kernel's block 0
 }
