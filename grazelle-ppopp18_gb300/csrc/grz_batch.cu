@@ -109,8 +109,8 @@ __device__ __forceinline__ double ppr_teleport(const PprApply& ap, uint32_t g, i
 __device__ __forceinline__ u128 ppr_finish(const PprApply& ap, uint32_t v, int inst, u128 x, double teleport)
 {
     const double rank = __fma_rn(fx_to_double(x), ap.damping, teleport);
-    // rounding can leave 1 - S below zero at damping 1; props are taken without sign (fx_from_double)
-    const pk_t w = pk_from_double(fabs(__dmul_rn(rank, __ldg(ap.inv_deg + v))));
+    // (rounding can leave 1 - S below zero at damping 1; props are taken without sign)
+    const pk_t w = pk_from_double(__dmul_rn(rank, __ldg(ap.inv_deg + v)));
     ap.prop_out[(uint64_t)v * K + inst] = w;
     if (ap.rank_out) ap.rank_out[(uint64_t)v * K + inst] = rank;
     return u128_mul32(pk_to_fx(w), __ldg(ap.degree + v));

@@ -161,11 +161,11 @@ __device__ __forceinline__ u128 pk_to_fx(unsigned long long w)
     r.lo = shl64_clamp(x, 64u - s) | shr64_clamp(x, s - 64u);  // one of the two is 0 unless s = 64 (both are x)
     return r;
 }
-// the packed form of fx_from_double(x), x in [0, 8)
+// the packed form of fx_from_double(x), |x| < 8 (without the sign, as there)
 __device__ __forceinline__ unsigned long long pk_from_double(double x)
 {
     const unsigned long long b = (unsigned long long)__double_as_longlong(x);
-    const int t = (int)(b >> 52) - 1022 + GRZ_FX_FRAC;  // leading bit's index + 1
+    const int t = (int)((b >> 52) & 0x7ff) - 1022 + GRZ_FX_FRAC;  // leading bit's index + 1
     if (t < 1) return 0ull;
     unsigned long long m = (b << 11) | 0x8000000000000000ull;
     if (t < 53) m &= ~0ull << (64 - t);  // bits below 2^-124 are cut off, as in fx_from_double

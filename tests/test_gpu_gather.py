@@ -148,3 +148,24 @@ def test_small_graph_with_most_edges_at_few_destinations(hub_edges):
     dst.append(np.arange(20) + 100)
     g = gg.EdgeList(V, np.concatenate(src).astype(np.uint64), np.concatenate(dst).astype(np.uint64))
     np.testing.assert_array_equal(pagerank(g, 9), pagerank(g, 9, pr_props=1))
+
+
+@pytest.mark.parametrize("V", [300, 5017, 30011])
+def test_negative_constant_at_damping_one(V):
+    """At damping 1 the sum of ranks can round above 1, and a vertex without in-edges then gets a negative
+    prop, which every form takes without its sign.  Every vertex has 5 out-edges, and for these V the sum of
+    V * 5 * ((1 / V) / 5) in doubles is 1 + 2^-52; vertex 0 has no in-edges."""
+    from grazelle import graphgen as gg
+    from grazelle.engine import Graph
+    rng = np.random.RandomState(V)
+    g = gg.EdgeList(V, np.repeat(np.arange(V), 5).astype(np.uint64), rng.randint(1, V, size=5 * V).astype(np.uint64))
+    found = []
+    for tune in ({"pr_props": 1}, {}, {"pr_persistent": 1}, {"pr_segment_bits": 9}):
+        with Graph(0) as G:
+            G.tune(**tune)
+            G.load_pairs(V, g.pull_order().pairs())
+            G.pr_init(1.0)
+            found.append(np.stack([G.pr_iterate(n).props() for n in (1, 1, 3)]))
+    np.testing.assert_allclose(found[0][0, 0], 2.0 ** -52 / V / 5, rtol=1e-12)
+    for other in found[1:]:
+        np.testing.assert_array_equal(other, found[0])
