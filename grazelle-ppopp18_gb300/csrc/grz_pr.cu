@@ -1664,6 +1664,7 @@ int grz_pr_fused_iteration(grz_graph* g, int write_double_props)
     int rc = g->pr_pkmode ? pr_sync_pk(g) : pr_sync_fx(g);
     if (rc) return rc;
     if (g->pr_segmode) {
+        GRZ_TRY(grz_pr_rowacc_clean(g));  // (unsegmented iterations came before)
         rc = pr_gather_segments(g, pc);
     } else if (packed) {
         rc = pr_cut_for(g, pr_gather_pk_range(n, pr_gather_pk_grid(g, n)));
@@ -1690,7 +1691,7 @@ int grz_pr_fused_iteration(grz_graph* g, int write_double_props)
     GRZ_CK(g, ae);
     g->pr_nparts[k ^ 1] = (uint32_t)agrid;
     g->pr_fx_stale = g->pr_pkmode;  // the new props are only in pr_pk
-    g->pr_rowacc_stale = 1;
+    g->pr_rowacc_stale = !g->pr_segmode;  // the apply of segmented iterations clears all
     g->pr_cur ^= 1;
     g->pr_sum_cur = k ^ 1;
     g->pr_iters_done++;

@@ -169,3 +169,21 @@ def test_negative_constant_at_damping_one(V):
     np.testing.assert_allclose(found[0][0, 0], 2.0 ** -52 / V / 5, rtol=1e-12)
     for other in found[1:]:
         np.testing.assert_array_equal(other, found[0])
+
+
+@pytest.mark.parametrize("V,degree", [(500, 6), (20011, 9)])
+@pytest.mark.parametrize("before", [{}, {"pr_props": 1}, {"pr_persistent": 1}, {"pr_persistent": 2}])
+def test_segmented_after_unsegmented(V, degree, before):
+    """A loaded graph whose iterations become segmented, and back: the segmented gather adds into the
+    accumulators, so nothing of the iterations before may be left in them."""
+    from grazelle import graphgen as gg
+    from grazelle.engine import Graph
+    g = gg.erdos_renyi(V, degree, seed=V)
+    ref = pagerank(g, 6, pr_props=1)
+    with Graph(0) as G:
+        G.load_pairs(V, g.pull_order().pairs())
+        for seg in (1, 9, 1, 9, 9):
+            G.tune(pr_segment_bits=seg, pr_props=0, pr_persistent=0)
+            if seg == 1:
+                G.tune(**before)
+            np.testing.assert_array_equal(G.pagerank(6, damping=0.85), ref, err_msg="segment bits %d" % seg)
