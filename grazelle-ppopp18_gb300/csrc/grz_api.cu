@@ -72,6 +72,26 @@ void grz_dev_free(grz_graph* g, void* p)
     if (p) cudaFreeAsync(p, g->stream);
 }
 
+bool grz_clusters_fit(const void* kernel, int ctas, int threads, size_t smem)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(ctas);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cudaLaunchAttribute at = {};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = ctas;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    int clusters = 0;
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg);
+    if (e != cudaSuccess) cudaGetLastError();
+    return e == cudaSuccess && clusters > 0;
+}
+
 // keeps the memory freed into the device's default pool for reuse, once per device
 static int pool_setup(int device)
 {
@@ -952,6 +972,10 @@ extern "C" int grz_tune_set(grz_graph* g, int param, int64_t value)
             return grz_set_error(g, GRZ_ERR_ARG, "PageRank segment bits must be 0 (by size), 1 (none) or 8..31");
         g->tune.pr_segment_bits = (uint32_t)value;  // from the next grz_pr_init
         return GRZ_OK;
+    case GRZ_TUNE_WITHHOLD:
+        if (value > GRZ_WITHHOLD_CLUSTERS) return grz_set_error(g, GRZ_ERR_ARG, "unknown thing to withhold");
+        g->tune.withhold = (uint32_t)value;
+        return GRZ_OK;
     case GRZ_TUNE_RUN_LIMIT_US:
         if (value > 3600000000ll) return grz_set_error(g, GRZ_ERR_RANGE, "run time bound above one hour");
         g->tune.run_limit_us = (uint32_t)value;
@@ -983,6 +1007,7 @@ extern "C" int grz_tune_get(const grz_graph* g, int param, int64_t* value)
     case GRZ_TUNE_CC_SEGMENTS: *value = g->tune.cc_segments; return GRZ_OK;
     case GRZ_TUNE_BFS_PULL_FIRST: *value = g->tune.bfs_pull_first; return GRZ_OK;
     case GRZ_TUNE_CC_PULL_FIRST: *value = g->tune.cc_pull_first; return GRZ_OK;
+    case GRZ_TUNE_WITHHOLD: *value = g->tune.withhold; return GRZ_OK;
     case GRZ_TUNE_HUBS_LOADED: *value = g->pull.nhub; return GRZ_OK;
     default: return GRZ_ERR_ARG;
     }

@@ -2574,38 +2574,37 @@ static int hop_phase(grz_graph* g)
     return grz_cuda_check(g, cudaGetLastError(), "k_hop");
 }
 
+static bool hop_fits(const grz_graph* g)
+{
+    static int known[64] = {};  // per device: 1 fits, 2 does not
+    if (g->device < 0 || g->device >= 64 || (g->tune.withhold & GRZ_WITHHOLD_CLUSTERS)) return false;
+    if (!known[g->device])
+        known[g->device] = grz_clusters_fit((const void*)k_hop<true>, HOP_CTAS, HOP_T, HOP_SMEM) &&
+                           grz_clusters_fit((const void*)k_hop<false>, HOP_CTAS, HOP_T, HOP_SMEM) ? 1 : 2;
+    return known[g->device] == 1;
+}
+
 // Whether a run's small iterations go through k_hop: its frontiers are bounded by the vote, so the
-// vote has to count vertices and out-edges (the default; forced engines included).
+// vote has to count vertices and out-edges (the default; forced engines included).  Where its cluster does
+// not fit (a cluster of 16 blocks needs the opt-in, and a GPC that can hold it) or its memory cannot be had,
+// the engines' kernels run every iteration.
 static int hop_prepare(grz_graph* g)
 {
     grz_frontier_state& f = g->fr;
-    if ((f.flags & (GRZ_FLAG_WITHOUT_COUNT | GRZ_FLAG_WITHOUT_OUTDEG)) || g->V >= 0x80000000ull) {  // (31-bit iteration numbers)
-        f.hop_list = nullptr;
-        return GRZ_OK;
-    }
+    f.hop_list = nullptr;
+    if ((f.flags & (GRZ_FLAG_WITHOUT_COUNT | GRZ_FLAG_WITHOUT_OUTDEG)) || g->V >= 0x80000000ull) return GRZ_OK;  // (31-bit iteration numbers)
+    if (!hop_fits(g)) return GRZ_OK;
     if (!f.hop_buf) {
-        // a cluster of 16 blocks needs the opt-in, and a GPC that can hold it
-        int clusters = 0;
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(HOP_CTAS);
-        cfg.blockDim = dim3(HOP_T);
-        cfg.dynamicSmemBytes = HOP_SMEM;
-        cudaLaunchAttribute at = {};
-        at.id = cudaLaunchAttributeClusterDimension;
-        at.val.clusterDim.x = HOP_CTAS;
-        at.val.clusterDim.y = at.val.clusterDim.z = 1;
-        cfg.attrs = &at;
-        cfg.numAttrs = 1;
-        for (const void* k : { (const void*)k_hop<true>, (const void*)k_hop<false> }) {
-            GRZ_CK(g, cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-            GRZ_CK(g, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)HOP_SMEM));
-            GRZ_CK(g, cudaOccupancyMaxActiveClusters(&clusters, k, &cfg));
-            if (clusters < 1) return grz_set_error(g, GRZ_ERR_CUDA, "a cluster of %d blocks does not fit", HOP_CTAS);
-        }
         const uint64_t W = words_of(g->V);
-        GRZ_CK(g, cudaMalloc((void**)&f.hop_map, sizeof(unsigned long long) * W));
+        cudaError_t e = cudaMalloc((void**)&f.hop_map, sizeof(unsigned long long) * W);
+        if (e == cudaSuccess) e = cudaMalloc((void**)&f.hop_buf, sizeof(uint32_t) * GRZ_HOP_VOTE);
+        if (e != cudaSuccess) {
+            cudaFree(f.hop_map);
+            f.hop_map = nullptr;
+            f.hop_buf = nullptr;
+            return e == cudaErrorMemoryAllocation ? (cudaGetLastError(), GRZ_OK) : grz_cuda_check(g, e, "hop scratch");
+        }
         GRZ_CK(g, cudaMemsetAsync(f.hop_map, 0, sizeof(unsigned long long) * W, g->stream));
-        GRZ_CK(g, cudaMalloc((void**)&f.hop_buf, sizeof(uint32_t) * GRZ_HOP_VOTE));
     }
     f.hop_list = f.hop_buf;
     return GRZ_OK;

@@ -397,6 +397,8 @@ struct grz_mlp;
 #define GRZ_TUNE_CC_SEGMENTS 16
 #define GRZ_TUNE_BFS_PULL_FIRST 17
 #define GRZ_TUNE_CC_PULL_FIRST 18
+#define GRZ_TUNE_WITHHOLD 19
+#define GRZ_WITHHOLD_CLUSTERS 1u
 #define GRZ_TUNE_HUBS_LOADED 100
 
 // kernel shapes chosen per graph (grz_tune_set; the autotuner searches them)
@@ -419,6 +421,7 @@ struct grz_tuning {
     uint32_t cc_segments; // CC full pull over the source segments: 0 when built, 1 never, 2 build them by size
     uint32_t bfs_pull_first;  // BFS pull: vectors a wanted destination reads in the early-exit pass (0: no such pass)
     uint32_t cc_pull_first;   // CC: each destination's first vector before the whole-list pass of a first pull (0: off)
+    uint32_t withhold;        // tests: GRZ_WITHHOLD_* that the graph finds missing
 };
 
 // Device control block of a CC/BFS run executed as one CUDA graph (grz_ccbfs.cu): the
@@ -655,6 +658,8 @@ void grz_prof_direct(grz_graph* g, int kind, float ms);
 int grz_set_error(grz_graph* g, int code, const char* fmt, ...);
 int grz_cuda_check(grz_graph* g, cudaError_t e, const char* what);
 int grz_scratch(grz_graph* g, size_t bytes, void** out);
+// whether clusters of `ctas` blocks of `kernel` can run on the current device (opts the kernel in)
+bool grz_clusters_fit(const void* kernel, int ctas, int threads, size_t smem);
 
 #define GRZ_TRY(expr) do { const int rc_try_ = (expr); if (rc_try_) return rc_try_; } while (0)
 #define GRZ_CK(g, call)                                         \

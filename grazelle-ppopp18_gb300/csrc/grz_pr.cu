@@ -1813,22 +1813,24 @@ int grz_pr_persistent_iterations(grz_graph* g, uint32_t iters)
     return GRZ_OK;
 }
 
+static bool pr_small_fits(const grz_graph* g)
+{
+    static int known[64] = {};  // per device: 1 fits, 2 does not
+    if (g->device < 0 || g->device >= 64 || (g->tune.withhold & GRZ_WITHHOLD_CLUSTERS)) return false;
+    if (!known[g->device]) known[g->device] = grz_clusters_fit((const void*)k_pr_small, PS_CTAS, PS_T, ps_smem(PS_MAX_V)) ? 1 : 2;
+    return known[g->device] == 1;
+}
+
 // Whether a graph's iterations run in one cluster (k_pr_small): packed props of a small graph, unless a
-// form or grid of the two kernels is asked for, or their times.
+// form or grid of the two kernels is asked for, or their times, or the device cannot hold the cluster.
 static bool pr_use_small(const grz_graph* g)
 {
     return g->pr_pkmode && !g->pr_segmode && !g->pull.nhub && !g->pr_nhot && g->tune.pr_persistent == 0 && g->tune.pr_grid == 0 &&
-           !(g->prof && g->prof->on) && g->V && g->V <= PS_MAX_V && g->pull.nvec <= PS_MAX_VEC;
+           !(g->prof && g->prof->on) && g->V && g->V <= PS_MAX_V && g->pull.nvec <= PS_MAX_VEC && pr_small_fits(g);
 }
 
 static int pr_small_iterations(grz_graph* g, uint32_t iters)
 {
-    static bool configured[64] = {};
-    if (g->device < 0 || g->device >= 64 || !configured[g->device]) {
-        GRZ_CK(g, cudaFuncSetAttribute(k_pr_small, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-        GRZ_CK(g, cudaFuncSetAttribute(k_pr_small, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ps_smem(PS_MAX_V)));
-        if (g->device >= 0 && g->device < 64) configured[g->device] = true;
-    }
     GRZ_TRY(pr_sync_pk(g));
     const uint32_t stride = blocks_for(g->V) + 1;
     const int k = g->pr_sum_cur, cur = g->pr_cur ^ (int)(iters & 1);
