@@ -136,8 +136,7 @@ static void free_graph_data(grz_graph* g, uint64_t next_V = ~0ull)
         g->pr_lists_changed = 1;
     } else {
         cudaFree(g->pr_fx[0]);  // and with it the arrays after it (grz_pr_prepare)
-        if (g->pr_pk_own)
-            for (void* p : { (void*)g->pr_pk[0], (void*)g->pr_pk[1] }) cudaFree(p);
+        if (g->pr_pk_own) cudaFree(g->pr_pk[0]);  // (both)
         g->pr_pk_own = 0;
         g->pr_pk[0] = g->pr_pk[1] = nullptr;
         g->pr_fx[0] = g->pr_fx[1] = nullptr; g->pr_sum = nullptr; g->pr_K = nullptr; g->pr_rowacc = nullptr;
@@ -973,7 +972,7 @@ extern "C" int grz_tune_set(grz_graph* g, int param, int64_t value)
         g->tune.pr_segment_bits = (uint32_t)value;  // from the next grz_pr_init
         return GRZ_OK;
     case GRZ_TUNE_WITHHOLD:
-        if (value > GRZ_WITHHOLD_CLUSTERS) return grz_set_error(g, GRZ_ERR_ARG, "unknown thing to withhold");
+        if (value > GRZ_WITHHOLD_ALL) return grz_set_error(g, GRZ_ERR_ARG, "unknown thing to withhold");
         g->tune.withhold = (uint32_t)value;
         return GRZ_OK;
     case GRZ_TUNE_RUN_LIMIT_US:

@@ -399,6 +399,10 @@ struct grz_mlp;
 #define GRZ_TUNE_CC_PULL_FIRST 18
 #define GRZ_TUNE_WITHHOLD 19
 #define GRZ_WITHHOLD_CLUSTERS 1u
+#define GRZ_WITHHOLD_HOT_LIST 2u
+#define GRZ_WITHHOLD_SEGMENTS 4u
+#define GRZ_WITHHOLD_PACKED 8u
+#define GRZ_WITHHOLD_ALL 15u
 #define GRZ_TUNE_HUBS_LOADED 100
 
 // kernel shapes chosen per graph (grz_tune_set; the autotuner searches them)

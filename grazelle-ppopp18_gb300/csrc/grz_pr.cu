@@ -1243,11 +1243,14 @@ static int pr_sync_fx(grz_graph* g)
     return GRZ_OK;
 }
 
+// whether the packed gather takes hot sources from the table: some were chosen, and the list it reads names them
+static bool pr_hot_on(const grz_graph* g) { return g->pr_nhot && (g->pr_segmode || g->pr_hot_nbr); }
+
 static int pr_sync_pk(grz_graph* g)
 {
     if (!g->pr_pk_stale) return GRZ_OK;
     k_pk_pack<<<blocks_for(g->V), PR_THREADS, 0, g->stream>>>(g->pr_fx[g->pr_cur], g->V, g->pr_pk[g->pr_cur],
-                                                             g->pr_nhot ? g->pr_hotmap : nullptr, g->pr_hot[g->pr_cur]); GRZ_COUNT_LAUNCH(g);
+                                                             pr_hot_on(g) ? g->pr_hotmap : nullptr, g->pr_hot[g->pr_cur]); GRZ_COUNT_LAUNCH(g);
     GRZ_CK(g, cudaGetLastError());
     g->pr_pk_stale = 0;
     return GRZ_OK;
@@ -1345,6 +1348,7 @@ static int pr_hot_choose(grz_graph* g)
 static int pr_hot_encode(grz_graph* g)
 {
     if (!g->pr_nhot || g->pr_hot_nbr) return GRZ_OK;
+    if (g->tune.withhold & GRZ_WITHHOLD_HOT_LIST) return GRZ_ERR_NOMEM;
     GRZ_TRY(grz_dev_alloc(g, (void**)&g->pr_hot_nbr, sizeof(uint4) * g->pull.nvec));
     k_hot_encode<<<blocks_for(g->pull.nvec), PR_THREADS, 0, g->stream>>>(g->pull.nbr, g->pull.nvec, g->pr_hotmap, g->pr_nhot, g->pr_hot_nbr);
     GRZ_COUNT_LAUNCH(g);
@@ -1392,29 +1396,55 @@ int grz_pr_ensure_segments(grz_graph* g, int force)
     return pr_build_segments(g, bits);
 }
 
+// The PageRank arrays of V vertices, with those of the packed props if `pk`, in one allocation.
+static int pr_arrays(grz_graph* g, bool pk)
+{
+    // (GB300, the first grz_pr_init of a graph of 300k vertices 338 us with eight allocations, 119 so; 16 iterations on
+    // R-MAT of 2^20 vertices with it 1380 and 1148 us)
+    const uint64_t V = g->V;
+    const size_t parts[] = { sizeof(u128) * (V + 1), sizeof(u128) * (V + 1), sizeof(u128) * (V + 1),
+                             pk ? sizeof(pk_t) * (V + 1) : 0, pk ? sizeof(pk_t) * (V + 1) : 0,
+                             sizeof(u128) * 2 * (blocks_for(V) + 1), sizeof(uint32_t) * ((V + 31) / 32 + 1), sizeof(double) * 2,
+                             sizeof(u128) * 2 * PS_CTAS };
+    void** const to[] = { (void**)&g->pr_fx[0], (void**)&g->pr_fx[1], (void**)&g->pr_rowacc, (void**)&g->pr_pk[0], (void**)&g->pr_pk[1],
+                          (void**)&g->pr_sum, (void**)&g->pr_cut, (void**)&g->pr_K, (void**)&g->pr_small_parts };
+    size_t total = 0;
+    for (size_t n : parts) total += (n + 255) & ~(size_t)255;
+    char* p = nullptr;
+    if (pk && (g->tune.withhold & GRZ_WITHHOLD_PACKED)) return GRZ_ERR_NOMEM;
+    GRZ_CK(g, cudaMalloc((void**)&p, total));
+    for (int i = 0; i < 9; ++i) {
+        *to[i] = parts[i] ? p : nullptr;
+        p += (parts[i] + 255) & ~(size_t)255;
+    }
+    g->pr_pk_own = 0;
+    g->pr_lists_changed = 1;
+    return GRZ_OK;
+}
+
+// the packed props by themselves, where the other arrays came without them
+static int pr_packed_arrays(grz_graph* g)
+{
+    if (g->tune.withhold & GRZ_WITHHOLD_PACKED) return GRZ_ERR_NOMEM;
+    const size_t half = (sizeof(pk_t) * (g->V + 1) + 255) & ~(size_t)255;
+    GRZ_CK(g, cudaMalloc((void**)&g->pr_pk[0], 2 * half));
+    g->pr_pk[1] = g->pr_pk[0] + half / sizeof(pk_t);
+    g->pr_pk_own = 1;
+    GRZ_CK(g, cudaMemsetAsync(g->pr_pk[0], 0, 2 * half, g->stream));
+    return GRZ_OK;
+}
+
+// Packed props, segments and the encoded list only make the iterations faster: where the memory for one of
+// them cannot be had, the graph runs without it.
+static int pr_or_without(int rc) { return rc == GRZ_ERR_NOMEM ? GRZ_OK : rc; }
+
 int grz_pr_prepare(grz_graph* g)
 {
     const uint64_t V = g->V;
     if (!g->pr_fx[0]) {
-        // one allocation and one clear (GB300, the first grz_pr_init of a graph of 300k vertices 338 us with eight
-        // allocations, 119 so; 16 iterations on R-MAT of 2^20 vertices with it 1380 and 1148 us)
-        const bool pk = g->tune.pr_props != 1;
-        const size_t parts[] = { sizeof(u128) * (V + 1), sizeof(u128) * (V + 1), sizeof(u128) * (V + 1),
-                                 pk ? sizeof(pk_t) * (V + 1) : 0, pk ? sizeof(pk_t) * (V + 1) : 0,
-                                 sizeof(u128) * 2 * (blocks_for(V) + 1), sizeof(uint32_t) * ((V + 31) / 32 + 1), sizeof(double) * 2,
-                                 sizeof(u128) * 2 * PS_CTAS };
-        void** const to[] = { (void**)&g->pr_fx[0], (void**)&g->pr_fx[1], (void**)&g->pr_rowacc, (void**)&g->pr_pk[0], (void**)&g->pr_pk[1],
-                              (void**)&g->pr_sum, (void**)&g->pr_cut, (void**)&g->pr_K, (void**)&g->pr_small_parts };
-        size_t total = 0;
-        for (size_t n : parts) total += (n + 255) & ~(size_t)255;
-        char* p = nullptr;
-        GRZ_CK(g, cudaMalloc((void**)&p, total));
-        for (int i = 0; i < 9; ++i) {
-            *to[i] = parts[i] ? p : nullptr;
-            p += (parts[i] + 255) & ~(size_t)255;
-        }
-        g->pr_pk_own = 0;
-        g->pr_lists_changed = 1;
+        int rc = pr_arrays(g, g->tune.pr_props != 1);
+        if (rc == GRZ_ERR_NOMEM && g->tune.pr_props != 1) rc = pr_arrays(g, false);
+        if (rc) return rc;
     }
     if (g->pr_lists_changed) {
         // (also after a reload with the same V, which kept the arrays)
@@ -1425,15 +1455,14 @@ int grz_pr_prepare(grz_graph* g)
         const bool pk = g->pr_pk[0] && !g->pr_pk_own;
         const char* const end = pk ? (const char*)(g->pr_pk[1] + V + 1) : (const char*)(g->pr_rowacc + V + 1);
         GRZ_CK(g, cudaMemsetAsync(g->pr_fx[0], 0, (size_t)(end - (const char*)g->pr_fx[0]), g->stream));
-        if (g->pr_pk_own)
-            for (pk_t* p : g->pr_pk) GRZ_CK(g, cudaMemsetAsync(p, 0, sizeof(pk_t) * (V + 1), g->stream));
+        if (g->pr_pk_own) GRZ_CK(g, cudaMemsetAsync(g->pr_pk[0], 0, (size_t)((char*)(g->pr_pk[1] + V + 1) - (char*)g->pr_pk[0]), g->stream));
         g->pr_lists_changed = 0;
     }
     // Packed props (8 bytes) unless 16-byte fixed point is asked for: half the gathered working set
     // for a few integer instructions per edge (GB300, a thread per vector, gather per iteration, 16 ->
     // 8 bytes: R-MAT 20 71 -> 63 us, R-MAT 24 1089 -> 938 us, uniform 3M vertices 153 -> 145 us).
     g->pr_pkmode = g->tune.pr_props != 1;
-    if (!g->pull.nhub && V) GRZ_TRY(pr_hot_choose(g));
+    if (!g->pull.nhub && V) GRZ_TRY(pr_or_without(pr_hot_choose(g)));
     // Source segments (pr_segment_bits): each segment's props mostly stay in L2 while its edges
     // stream, instead of one random DRAM sector per gathered prop.  They need sources in ascending
     // order along each destination's lanes: not a hub-encoded list, nor one that is only grouped.
@@ -1441,18 +1470,14 @@ int grz_pr_prepare(grz_graph* g)
     g->pr_segmode = 0;
     if (bits && g->pull.nhub == 0 && g->pull.nvec && g->pull.ascending) {
         const int rc = pr_build_segments(g, bits);
-        if (rc) return rc;
-        g->pr_segmode = 1;
-        g->pr_pkmode = 1;  // the segments gather the props packed
+        GRZ_TRY(pr_or_without(rc));
+        if (!rc) g->pr_segmode = g->pr_pkmode = 1;  // the segments gather the props packed
     }
     if (g->pr_pkmode && !g->pr_pk[0]) {
-        g->pr_pk_own = 1;  // not packed when the other arrays were allocated
-        GRZ_CK(g, cudaMalloc((void**)&g->pr_pk[0], sizeof(pk_t) * (V + 1)));
-        GRZ_CK(g, cudaMalloc((void**)&g->pr_pk[1], sizeof(pk_t) * (V + 1)));
-        GRZ_CK(g, cudaMemsetAsync(g->pr_pk[0], 0, sizeof(pk_t) * (V + 1), g->stream));
-        GRZ_CK(g, cudaMemsetAsync(g->pr_pk[1], 0, sizeof(pk_t) * (V + 1), g->stream));
+        GRZ_TRY(pr_or_without(pr_packed_arrays(g)));
+        if (!g->pr_pk[0]) g->pr_segmode = g->pr_pkmode = 0;
     }
-    if (g->pr_pkmode && !g->pr_segmode && !g->pull.nhub && V) GRZ_TRY(pr_hot_encode(g));
+    if (g->pr_pkmode && !g->pr_segmode && !g->pull.nhub && V) GRZ_TRY(pr_or_without(pr_hot_encode(g)));
     return GRZ_OK;
 }
 
@@ -1461,6 +1486,7 @@ int grz_pr_prepare(grz_graph* g)
 static int pr_build_segments(grz_graph* g, uint32_t bits)
 {
     if (g->seg_nbr && g->seg_bits == bits && g->seg_nhot == g->pr_nhot) return GRZ_OK;
+    if (g->tune.withhold & GRZ_WITHHOLD_SEGMENTS) return GRZ_ERR_NOMEM;
     grz_dev_free(g, g->seg_nbr);
     grz_dev_free(g, g->seg_dst);
     g->seg_nbr = nullptr;
@@ -1525,7 +1551,10 @@ static int pr_build_segments(grz_graph* g, uint32_t bits)
 int grz_pr_init_state(grz_graph* g, double damping)
 {
     int rc = grz_pr_prepare(g);
-    if (rc) return rc;
+    if (rc) {
+        g->pr_lists_changed = 1;  // no state to iterate
+        return rc;
+    }
     g->pr_damping = damping;
     g->pr_cur = 0;
     g->pr_fx_stale = g->pr_pkmode;
@@ -1535,7 +1564,7 @@ int grz_pr_init_state(grz_graph* g, double damping)
     if (g->V) {
         const unsigned grid = (unsigned)std::min<uint64_t>(blocks_for(g->V), (uint64_t)g->num_sms * 8);
         k_pr_init<<<grid, PR_THREADS, 0, g->stream>>>(g->inv_deg, g->degree, g->V, 1.0 / (double)g->V, g->accum, g->pr_fx[0],
-                                                      g->pr_pkmode ? g->pr_pk[0] : nullptr, g->pr_nhot ? g->pr_hotmap : nullptr,
+                                                      g->pr_pkmode ? g->pr_pk[0] : nullptr, pr_hot_on(g) ? g->pr_hotmap : nullptr,
                                                       g->pr_hot[0], g->pr_sum); GRZ_COUNT_LAUNCH(g);
         GRZ_CK(g, cudaGetLastError());
         g->pr_nparts[0] = grid;
@@ -1610,7 +1639,7 @@ static int pr_gather_pk(grz_graph* g, const uint4* nbr, const uint32_t* dstv, ui
     const uint32_t per = pr_gather_pk_range(span, grid);
     const pk_t* props = g->pr_pk[g->pr_cur];
     cudaError_t e;
-    if (g->pr_nhot) {
+    if (pr_hot_on(g)) {
         GRZ_TRY(pr_gather_pk_config(g));
         const size_t smem = sizeof(pk_t) * 2 * ((g->pr_nhot + 2) / 2);
         e = pdl_launch(k_pr_gather_pk<true, ADD>, grid, PK_THREADS, smem, g->stream, nbr, dstv, (uint32_t)first, (uint32_t)end, per, props,
@@ -1670,14 +1699,14 @@ int grz_pr_fused_iteration(grz_graph* g, int write_double_props)
         rc = pr_cut_for(g, pr_gather_pk_range(n, pr_gather_pk_grid(g, n)));
         if (rc) return rc;
         grz_prof_begin(g, GRZ_PROF_PR_GATHER);
-        rc = pr_gather_pk<false>(g, g->pr_nhot ? g->pr_hot_nbr : g->pull.nbr, g->pull.shared, 0, n, pc);
+        rc = pr_gather_pk<false>(g, pr_hot_on(g) ? g->pr_hot_nbr : g->pull.nbr, g->pull.shared, 0, n, pc);
         grz_prof_end(g);
     } else {
         rc = pr_cut_for(g, PR_THREADS);
         if (!rc) rc = g->pr_pkmode ? pr_gather(g, 0, n, pc, (const pk_t*)g->pr_pk[g->pr_cur]) : pr_gather(g, 0, n, pc, (const u128*)g->pr_fx[g->pr_cur]);
     }
     if (rc) return rc;
-    const bool hot = g->pr_pkmode && g->pr_nhot;
+    const bool hot = g->pr_pkmode && pr_hot_on(g);
     grz_prof_begin(g, GRZ_PROF_PR_APPLY);
     const uint64_t agrid = std::max<uint64_t>(1, std::min<uint64_t>((g->V + (uint64_t)PR_THREADS * PR_APPLY_U - 1) /
                                                                         ((uint64_t)PR_THREADS * PR_APPLY_U),
@@ -1803,7 +1832,7 @@ int grz_pr_persistent_iterations(grz_graph* g, uint32_t iters)
     }
     g->pr_nparts[g->pr_sum_cur] = grid;
     g->pr_fx_stale = g->pr_pkmode;
-    if (g->pr_nhot) {
+    if (pr_hot_on(g)) {
         // the persistent form does not keep the hot table: packed again before the next fused iteration
         GRZ_TRY(pr_sync_fx(g));
         g->pr_pk_stale = 1;

@@ -39,7 +39,7 @@ TUNE_CC_SEGMENTS = 16
 TUNE_BFS_PULL_FIRST = 17
 TUNE_CC_PULL_FIRST = 18
 TUNE_WITHHOLD = 19
-WITHHOLD_CLUSTERS = 1
+WITHHOLD_CLUSTERS, WITHHOLD_HOT_LIST, WITHHOLD_SEGMENTS, WITHHOLD_PACKED = 1, 2, 4, 8
 BATCH_TUNE_PPR_BLOCKS, BATCH_TUNE_BFS_BLOCKS, BATCH_TUNE_PPR_PROPS = 0, 1, 2
 FLAG_HOST_LOOP = 16  # grz_cc_run / grz_bfs_run: host round trip per iteration instead of one CUDA graph
 MLP_FEATURES, MLP_HIDDEN, MLP_PARAMS = 12, 32, 1505

@@ -169,7 +169,7 @@ int grz_read_levels(grz_graph* g, int64_t* host_levels, uint64_t capacity);
 #define GRZ_TUNE_PR_WITHHOLD 10  /* fault injection for tests: block + 1 of the persistent PageRank kernel that never arrives at its first barrier (0 = none) */
 #define GRZ_TUNE_RUN_MAX_ITERATIONS 11 /* CC/BFS iteration bound (0 = V + 2): a run that has not converged by then returns GRZ_ERR_TIMEOUT */
 #define GRZ_TUNE_RUN_LIMIT_US 12  /* CC/BFS time bound of a run in microseconds (0 = 300 s), checked after each iteration: GRZ_ERR_TIMEOUT */
-#define GRZ_TUNE_WITHHOLD 19  /* fault injection for tests, a mask of what the graph is to find missing: 1 = clusters of 16 blocks (small PageRank graphs and small CC/BFS iterations then run as larger ones do; results identical) */
+#define GRZ_TUNE_WITHHOLD 19  /* fault injection for tests, a mask of what the graph is to find missing: 1 = clusters of 16 blocks (small PageRank graphs and small CC/BFS iterations then run as larger ones do), and the memory for 2 = the PageRank list with hot sources, 4 = its source segments, 8 = its packed props (from the next grz_pr_init it gathers the plain list, unsegmented, or 16-byte props); results identical */
 #define GRZ_TUNE_HUBS_LOADED 100 /* read-only: hubs encoded in the loaded pull list */
 int grz_tune_set(grz_graph* g, int param, int64_t value);
 int grz_tune_get(const grz_graph* g, int param, int64_t* value);
