@@ -883,13 +883,11 @@ extern "C" int grz_read_levels(grz_graph* g, int64_t* host, uint64_t cap)
     GRZ_CK(g, cudaSetDevice(g->device));
     const size_t bytes = sizeof(int64_t) * g->V;
     int64_t* direct = (int64_t*)mapped_view(host, bytes);
-    void* buf = nullptr;
-    int rc = direct ? GRZ_OK : grz_dev_alloc(g, &buf, bytes);
-    if (!rc) rc = grz_frontier_levels(g, direct ? direct : (int64_t*)buf);
-    if (!rc && !direct) rc = grz_cuda_check(g, cudaMemcpyAsync(host, buf, bytes, cudaMemcpyDeviceToHost, g->stream), "read levels");
-    if (!rc) rc = grz_cuda_check(g, cudaStreamSynchronize(g->stream), "read levels");
-    grz_dev_free(g, buf);
-    return rc;
+    // (staged in g->prop, as large and only ever a staging area of CC and BFS results)
+    GRZ_TRY(grz_frontier_levels(g, direct ? direct : (int64_t*)g->prop));
+    if (!direct) GRZ_CK(g, cudaMemcpyAsync(host, g->prop, bytes, cudaMemcpyDeviceToHost, g->stream));
+    GRZ_CK(g, cudaStreamSynchronize(g->stream));
+    return GRZ_OK;
 }
 
 extern "C" int grz_result_digest(grz_graph* g, uint64_t* out3)

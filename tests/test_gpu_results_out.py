@@ -35,4 +35,7 @@ def test_results_at_any_address(offset, pinned):
         np.testing.assert_array_equal(at_offset(lambda p: G.lib.grz_read_props(G.h, p, V)).view(np.float64), G.props())
         G.bfs_run(0)
         np.testing.assert_array_equal(at_offset(lambda p: G.lib.grz_read_props(G.h, p, V)).view(np.float64), G.props())
+        parents, free = G.props(), torch.cuda.mem_get_info()[0]
         np.testing.assert_array_equal(at_offset(lambda p: G.lib.grz_read_levels(G.h, p, V)).view(np.int64), G.levels())
+        assert torch.cuda.mem_get_info()[0] == free  # levels need no memory of their own
+        np.testing.assert_array_equal(G.props(), parents)
