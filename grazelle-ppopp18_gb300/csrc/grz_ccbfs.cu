@@ -1816,6 +1816,19 @@ __global__ void k_levels_out(const uint32_t* __restrict__ level, uint64_t V, int
 static uint64_t words_of(uint64_t V) { return (V >> 6) + 2; }
 static int frontier_list_state(grz_graph* g);
 
+// tile_first with room for `tiles`
+static int tiles_alloc(grz_graph* g, uint64_t tiles)
+{
+    grz_frontier_state& f = g->fr;
+    if (tiles <= f.tile_cap) return GRZ_OK;
+    GRZ_CK(g, cudaFree(f.tile_first));
+    f.tile_first = nullptr;
+    f.tile_cap = 0;
+    GRZ_CK(g, cudaMalloc((void**)&f.tile_first, sizeof(uint32_t) * tiles));
+    f.tile_cap = tiles;
+    return GRZ_OK;
+}
+
 static int ensure_frontier_state(grz_graph* g)
 {
     grz_frontier_state& f = g->fr;
@@ -1825,17 +1838,11 @@ static int ensure_frontier_state(grz_graph* g)
     if (f.label) {
         // kept from the graph loaded before, which had the same V
         if (f.alloc_V != V) return grz_set_error(g, GRZ_ERR_STATE, "frontier buffers sized for another graph");
-        if (tiles > f.tile_cap) {
-            GRZ_CK(g, cudaFree(f.tile_first));
-            f.tile_first = nullptr;
-            GRZ_CK(g, cudaMalloc((void**)&f.tile_first, sizeof(uint32_t) * tiles));
-            f.tile_cap = tiles;
-        }
+        GRZ_TRY(tiles_alloc(g, tiles));
         f.lists_changed = 0;
         return frontier_list_state(g);
     }
     f.alloc_V = V;
-    f.tile_cap = tiles;
     // one allocation but for tile_first, which a reload may make larger: twenty took a part of a small graph's
     // first run (GB300, the first pass of CC of 4096 vertices 425 us with them, 373 so; of BFS of 100k 741 and 626)
     const size_t v4 = sizeof(uint32_t) * (V + 1), v8 = sizeof(unsigned long long) * (V + 1), w8 = sizeof(unsigned long long) * W;
@@ -1848,9 +1855,7 @@ static int ensure_frontier_state(grz_graph* g)
         { (void**)&f.dev_err, sizeof(unsigned) } };
     size_t total = 0;
     for (const auto& p : part) total += (p.bytes + 255) & ~(size_t)255;
-    cudaFree(f.tile_first);  // of a call that failed at the other arrays
-    f.tile_first = nullptr;
-    GRZ_CK(g, cudaMalloc((void**)&f.tile_first, sizeof(uint32_t) * tiles));
+    GRZ_TRY(tiles_alloc(g, tiles));
     char* at = nullptr;
     GRZ_CK(g, cudaMalloc((void**)&at, total));
     for (const auto& p : part) {
