@@ -72,6 +72,21 @@ void grz_dev_free(grz_graph* g, void* p)
     if (p) cudaFreeAsync(p, g->stream);
 }
 
+cudaError_t grz_alloc_arrays(const grz_part* part, int n, void** mem)
+{
+    auto size = [&](int i) { return (part[i].bytes + 255) & ~(size_t)255; };
+    size_t total = 0;
+    for (int i = 0; i < n; ++i) total += size(i);
+    *mem = nullptr;
+    const cudaError_t e = cudaMalloc(mem, total);
+    char* at = (char*)*mem;
+    for (int i = 0; i < n; ++i) {
+        *part[i].to = at && part[i].bytes ? at : nullptr;
+        at += size(i);
+    }
+    return e;
+}
+
 bool grz_clusters_fit(const void* kernel, int ctas, int threads, size_t smem)
 {
     cudaLaunchConfig_t cfg = {};
@@ -135,7 +150,8 @@ static void free_graph_data(grz_graph* g, uint64_t next_V = ~0ull)
         // the PageRank arrays are sized by V alone: kept, and refilled at the next grz_pr_init
         g->pr_lists_changed = 1;
     } else {
-        cudaFree(g->pr_fx[0]);  // and with it the arrays after it (grz_pr_prepare)
+        cudaFree(g->pr_mem);
+        g->pr_mem = nullptr;
         if (g->pr_pk_own) cudaFree(g->pr_pk[0]);  // (both)
         g->pr_pk_own = 0;
         g->pr_pk[0] = g->pr_pk[1] = nullptr;

@@ -1843,25 +1843,35 @@ static int ensure_frontier_state(grz_graph* g)
         return frontier_list_state(g);
     }
     f.alloc_V = V;
-    // one allocation but for tile_first, which a reload may make larger: twenty took a part of a small graph's
-    // first run (GB300, the first pass of CC of 4096 vertices 425 us with them, 373 so; of BFS of 100k 741 and 626)
+    // One allocation (and tile_first, which a reload may make larger): twenty were a part of a small graph's
+    // first run.  But above half a GB the driver can let it, and the small one after it, wait for what was freed
+    // before, 0.9 ms each; then there are three, the randomly read arrays still together (in allocations of their
+    // own they read slower: CC on a uniform graph of 16.8M vertices 3.62 and 3.86 ms).  GB300, what a first pass takes
+    // beyond the next, twenty / one / three: CC of 4096 vertices 310 / 260 / - us, 2^20 660 / 380 / -, 2^23 920 / 450 / -, 12M
+    // 950 / 510 / 570, R-MAT of 2^24 (590 MB) 1070 / 1430 / 790 (one, and the control block after it: 2290).
     const size_t v4 = sizeof(uint32_t) * (V + 1), v8 = sizeof(unsigned long long) * (V + 1), w8 = sizeof(unsigned long long) * W;
-    struct { void** to; size_t bytes; } const part[] = {
+    const grz_part part[] = {
         { (void**)&f.label, v4 }, { (void**)&f.level, v4 }, { (void**)&f.has, w8 }, { (void**)&f.has_next, w8 }, { (void**)&f.wants, w8 },
-        { (void**)&f.nonempty_push, w8 }, { (void**)&f.nonempty_pull, w8 }, { (void**)&f.unres, w8 }, { (void**)&f.frontier, v4 },
-        { (void**)&f.voff, v4 }, { (void**)&f.vdelta, v4 }, { (void**)&f.touched, v4 }, { (void**)&f.cand64, v8 }, { (void**)&f.cand32, v4 },
-        { (void**)&f.counters, sizeof(uint32_t) * 8 }, { (void**)&f.digest, sizeof(unsigned long long) * 4 },
-        { (void**)&f.vote, sizeof(unsigned long long) * GRZ_VOTE_SLOTS * GRZ_VOTE_STRIDE }, { (void**)&f.chg, sizeof(unsigned long long) * 2 },
-        { (void**)&f.dev_err, sizeof(unsigned) } };
+        { (void**)&f.nonempty_push, w8 }, { (void**)&f.nonempty_pull, w8 }, { (void**)&f.unres, w8 }, { (void**)&f.hop_map, w8 },
+        { (void**)&f.hop_buf, sizeof(uint32_t) * GRZ_HOP_VOTE }, { (void**)&f.counters, sizeof(uint32_t) * 8 },
+        { (void**)&f.digest, sizeof(unsigned long long) * 4 }, { (void**)&f.vote, sizeof(unsigned long long) * GRZ_VOTE_SLOTS * GRZ_VOTE_STRIDE },
+        { (void**)&f.chg, sizeof(unsigned long long) * 2 }, { (void**)&f.dev_err, sizeof(unsigned) }, { (void**)&f.ctl, sizeof(grz_runctl) },
+        { (void**)&f.frontier, v4 }, { (void**)&f.voff, v4 }, { (void**)&f.vdelta, v4 }, { (void**)&f.touched, v4 },
+        { (void**)&f.cand64, v8 }, { (void**)&f.cand32, v4 } };
+    constexpr int N = sizeof(part) / sizeof(part[0]), SECOND = N - 6, THIRD = N - 2;
     size_t total = 0;
-    for (const auto& p : part) total += (p.bytes + 255) & ~(size_t)255;
+    for (const grz_part& p : part) total += p.bytes;
     GRZ_TRY(tiles_alloc(g, tiles));
-    char* at = nullptr;
-    GRZ_CK(g, cudaMalloc((void**)&at, total));
-    for (const auto& p : part) {
-        *p.to = at;
-        at += (p.bytes + 255) & ~(size_t)255;
+    const bool one = total <= (512u << 20);
+    cudaError_t e = grz_alloc_arrays(part, one ? N : SECOND, &f.mem[0]);
+    if (!one && e == cudaSuccess) e = grz_alloc_arrays(part + SECOND, THIRD - SECOND, &f.mem[1]);
+    if (!one && e == cudaSuccess) e = grz_alloc_arrays(part + THIRD, N - THIRD, &f.mem[2]);
+    if (e != cudaSuccess) {
+        for (void*& m : f.mem) { cudaFree(m); m = nullptr; }
+        f.label = nullptr;  // no state
+        return grz_cuda_check(g, e, "frontier arrays");
     }
+    GRZ_CK(g, cudaMemsetAsync(f.hop_map, 0, w8, g->stream));
     GRZ_CK(g, cudaMemsetAsync(f.digest, 0, sizeof(unsigned long long) * 4, g->stream));
     return frontier_list_state(g);
 }
@@ -2463,12 +2473,10 @@ void grz_frontier_park(grz_graph* g)
 void grz_frontier_free(grz_graph* g)
 {
     grz_frontier_state& f = g->fr;
-    void* ptrs[] = { f.label /* and the arrays allocated with it */, f.tile_first, f.sw_out, f.snap, f.hop_buf, f.hop_map };
-    for (void* p : ptrs) cudaFree(p);
+    for (void* p : { f.mem[0], f.mem[1], f.mem[2], (void*)f.tile_first, f.sw_out, f.snap }) cudaFree(p);
     if (f.ev[0]) { cudaEventDestroy(f.ev[0]); cudaEventDestroy(f.ev[1]); }
     if (f.mail) cudaFreeHost(f.mail);
     if (f.run_exec) cudaGraphExecDestroy(f.run_exec);
-    cudaFree(f.ctl);
     grz_mlp* keep_mlp = f.mlp;
     const int keep_policy = f.policy;
     memset(&f, 0, sizeof(f));
@@ -2591,28 +2599,14 @@ static bool hop_fits(const grz_graph* g)
 
 // Whether a run's small iterations go through k_hop: its frontiers are bounded by the vote, so the
 // vote has to count vertices and out-edges (the default; forced engines included).  Where its cluster does
-// not fit (a cluster of 16 blocks needs the opt-in, and a GPC that can hold it) or its memory cannot be had,
-// the engines' kernels run every iteration.
-static int hop_prepare(grz_graph* g)
+// not fit (a cluster of 16 blocks needs the opt-in, and a GPC that can hold it), the engines' kernels run every
+// iteration.
+static void hop_prepare(grz_graph* g)
 {
     grz_frontier_state& f = g->fr;
     f.hop_list = nullptr;
-    if ((f.flags & (GRZ_FLAG_WITHOUT_COUNT | GRZ_FLAG_WITHOUT_OUTDEG)) || g->V >= 0x80000000ull) return GRZ_OK;  // (31-bit iteration numbers)
-    if (!hop_fits(g)) return GRZ_OK;
-    if (!f.hop_buf) {
-        const uint64_t W = words_of(g->V);
-        cudaError_t e = cudaMalloc((void**)&f.hop_map, sizeof(unsigned long long) * W);
-        if (e == cudaSuccess) e = cudaMalloc((void**)&f.hop_buf, sizeof(uint32_t) * GRZ_HOP_VOTE);
-        if (e != cudaSuccess) {
-            cudaFree(f.hop_map);
-            f.hop_map = nullptr;
-            f.hop_buf = nullptr;
-            return e == cudaErrorMemoryAllocation ? (cudaGetLastError(), GRZ_OK) : grz_cuda_check(g, e, "hop scratch");
-        }
-        GRZ_CK(g, cudaMemsetAsync(f.hop_map, 0, sizeof(unsigned long long) * W, g->stream));
-    }
-    f.hop_list = f.hop_buf;
-    return GRZ_OK;
+    if ((f.flags & (GRZ_FLAG_WITHOUT_COUNT | GRZ_FLAG_WITHOUT_OUTDEG)) || g->V >= 0x80000000ull) return;  // (31-bit iteration numbers)
+    if (hop_fits(g)) f.hop_list = f.hop_buf;
 }
 
 static int build_run_graph(grz_graph* g)
@@ -2706,9 +2700,6 @@ int grz_frontier_run_graph(grz_graph* g, cudaEvent_t started, uint64_t* launches
         return grz_set_error(g, GRZ_ERR_STATE, "the graph run needs both edge lists");
     int rc = grz_frontier_mail(g);
     if (rc) return rc;
-    if (!f.ctl) {
-        GRZ_CK(g, cudaMalloc((void**)&f.ctl, sizeof(grz_runctl)));
-    }
     rc = grz_switch_max_degree(g);
     if (rc) return rc;
     const bool same = f.run_exec && f.run_bm[0] == f.has && f.run_bm[1] == f.has_next && f.run_key[0] == f.app &&
@@ -2719,9 +2710,9 @@ int grz_frontier_run_graph(grz_graph* g, cudaEvent_t started, uint64_t* launches
         const size_t smem = sizeof(uint32_t) * std::min<uint32_t>(g->tune.cc_cache, g->pull.nhub);
         rc = g->tune.cc_threads == 256 ? cc_pull_config_any<256>(g, smem, &resident)
              : (g->tune.cc_threads == 1024 ? cc_pull_config_any<1024>(g, smem, &resident) : cc_pull_config_any<512>(g, smem, &resident));
-        if (!rc) rc = hop_prepare(g);
-        if (!rc) rc = build_run_graph(g);
         if (rc) return rc;
+        hop_prepare(g);
+        GRZ_TRY(build_run_graph(g));
     }
     grz_runctl c;
     memset(&c, 0, sizeof(c));

@@ -348,6 +348,12 @@ __device__ __forceinline__ uint32_t grz_hub_decode(uint32_t x, const uint32_t* _
     return sl < nhub ? __ldg(hub_vid + sl) : x;
 }
 
+// one of the arrays of an allocation (grz_alloc_arrays)
+struct grz_part {
+    void** to;
+    size_t bytes;  // 0: none, *to = null
+};
+
 struct grz_prof;
 
 // engine flags (the reference's EXPERIMENTS that change the CC/BFS driver, Makefile:59-176)
@@ -513,6 +519,7 @@ struct grz_frontier_state {
     void* snap;
     uint64_t snap_bytes;
     uint64_t snap_scalars[8];
+    void* mem[3];                    // the allocations that hold the arrays (but tile_first)
     // the buffers outlive a reload of a graph with the same V (cudaMalloc and cudaFree synchronise
     // the device); what depends on the lists is rebuilt at the next initialisation
     uint64_t alloc_V;                // V the per-vertex buffers are sized for
@@ -553,6 +560,7 @@ struct grz_graph {
     uint32_t seg_nhot;    // hot sources encoded
     uint32_t seg_gen;     // builds so far (a captured run names one of them)
     int pr_segmode;       // fused iterations gather segment by segment
+    void* pr_mem;         // the allocation that holds the PageRank arrays
     u128* pr_small_parts; // parts of S of the blocks that run a small graph's iterations
     void* pr_bar;         // grid barrier and phase timer of the persistent PageRank kernel (device)
     void* pr_bar_host;    // pinned read-back of its error word and phase times
@@ -662,6 +670,8 @@ void grz_prof_direct(grz_graph* g, int kind, float ms);
 int grz_set_error(grz_graph* g, int code, const char* fmt, ...);
 int grz_cuda_check(grz_graph* g, cudaError_t e, const char* what);
 int grz_scratch(grz_graph* g, size_t bytes, void** out);
+// one cudaMalloc for all parts, in their order, 256-byte aligned: *mem, null and all *to null on failure
+cudaError_t grz_alloc_arrays(const grz_part* part, int n, void** mem);
 // whether clusters of `ctas` blocks of `kernel` can run on the current device (opts the kernel in)
 bool grz_clusters_fit(const void* kernel, int ctas, int threads, size_t smem);
 

@@ -1396,27 +1396,19 @@ int grz_pr_ensure_segments(grz_graph* g, int force)
     return pr_build_segments(g, bits);
 }
 
-// The PageRank arrays of V vertices, with those of the packed props if `pk`, in one allocation.
+// The PageRank arrays of V vertices, with those of the packed props if `pk`.
 static int pr_arrays(grz_graph* g, bool pk)
 {
-    // (GB300, the first grz_pr_init of a graph of 300k vertices 338 us with eight allocations, 119 so; 16 iterations on
-    // R-MAT of 2^20 vertices with it 1380 and 1148 us)
+    // together (GB300, the first grz_pr_init of a graph of 300k vertices 338 us with eight allocations, 119 in one; 16
+    // iterations on R-MAT of 2^20 vertices with it 1380 and 1148 us)
     const uint64_t V = g->V;
-    const size_t parts[] = { sizeof(u128) * (V + 1), sizeof(u128) * (V + 1), sizeof(u128) * (V + 1),
-                             pk ? sizeof(pk_t) * (V + 1) : 0, pk ? sizeof(pk_t) * (V + 1) : 0,
-                             sizeof(u128) * 2 * (blocks_for(V) + 1), sizeof(uint32_t) * ((V + 31) / 32 + 1), sizeof(double) * 2,
-                             sizeof(u128) * 2 * PS_CTAS };
-    void** const to[] = { (void**)&g->pr_fx[0], (void**)&g->pr_fx[1], (void**)&g->pr_rowacc, (void**)&g->pr_pk[0], (void**)&g->pr_pk[1],
-                          (void**)&g->pr_sum, (void**)&g->pr_cut, (void**)&g->pr_K, (void**)&g->pr_small_parts };
-    size_t total = 0;
-    for (size_t n : parts) total += (n + 255) & ~(size_t)255;
-    char* p = nullptr;
+    const grz_part part[] = { { (void**)&g->pr_fx[0], sizeof(u128) * (V + 1) }, { (void**)&g->pr_fx[1], sizeof(u128) * (V + 1) },
+                              { (void**)&g->pr_rowacc, sizeof(u128) * (V + 1) }, { (void**)&g->pr_pk[0], pk ? sizeof(pk_t) * (V + 1) : 0 },
+                              { (void**)&g->pr_pk[1], pk ? sizeof(pk_t) * (V + 1) : 0 }, { (void**)&g->pr_sum, sizeof(u128) * 2 * (blocks_for(V) + 1) },
+                              { (void**)&g->pr_cut, sizeof(uint32_t) * ((V + 31) / 32 + 1) }, { (void**)&g->pr_K, sizeof(double) * 2 },
+                              { (void**)&g->pr_small_parts, sizeof(u128) * 2 * PS_CTAS } };
     if (pk && (g->tune.withhold & GRZ_WITHHOLD_PACKED)) return GRZ_ERR_NOMEM;
-    GRZ_CK(g, cudaMalloc((void**)&p, total));
-    for (int i = 0; i < 9; ++i) {
-        *to[i] = parts[i] ? p : nullptr;
-        p += (parts[i] + 255) & ~(size_t)255;
-    }
+    GRZ_CK(g, grz_alloc_arrays(part, sizeof(part) / sizeof(part[0]), &g->pr_mem));
     g->pr_pk_own = 0;
     g->pr_lists_changed = 1;
     return GRZ_OK;
