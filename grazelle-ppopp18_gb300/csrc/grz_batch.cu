@@ -483,6 +483,7 @@ struct grz_batch {
     u128* rowacc;                        // [V][instance]: sums of the cut destinations, zero between iterations
     uint32_t* ppr_bnd;                   // ranges of k_ppr_step (k_ppr_bounds) and the destinations they cut
     uint32_t* ppr_cut;
+    void *ppr_mem, *bfs_mem;             // the allocations that hold the PPR and the BFS arrays
     u128* S[3];                          // of the props gathered, written, and of the iteration after
     cudaGraphExec_t ppr_exec;
     uint32_t ppr_iters;
@@ -545,11 +546,11 @@ extern "C" int grz_batch_create(grz_batch** out, int device, void* stream)
 
 static void free_state(grz_batch* b)
 {
-    void* p[] = { b->d_voff, b->d_seeds, b->d_roots, b->stamps, b->prop[0], b->prop[1], b->rank, b->rowacc, b->ppr_bnd, b->ppr_cut, b->S[0], b->S[1], b->S[2],
-                  b->visited, b->frontier, b->next_words, b->level, b->ctl, b->iter };
+    void* p[] = { b->d_voff, b->d_seeds, b->d_roots, b->stamps, b->ppr_mem, b->bfs_mem };
     for (void* x : p) cudaFree(x);
     b->d_voff = b->d_seeds = b->d_roots = nullptr;
     b->stamps = nullptr;
+    b->ppr_mem = b->bfs_mem = nullptr;
     b->prop[0] = b->prop[1] = nullptr;
     b->rank = nullptr;
     b->rowacc = b->S[0] = b->S[1] = b->S[2] = nullptr;
@@ -723,22 +724,21 @@ static int build_ppr_graph(grz_batch* b, uint32_t iterations, double damping)
     return GRZ_OK;
 }
 
-// the PPR state (props, ranks, accumulators), allocated on first use
+// the PPR state (props, ranks, accumulators), allocated on first use, in one call (GB300, what a batch's first run takes
+// beyond the next, nine and one: three graphs of 1400 vertices in all 215 and 190 us, eight of 1.04M 770 and 610 us)
 static int ppr_alloc(grz_batch* b)
 {
     const uint64_t V = b->u->V;
     const uint32_t G = (uint32_t)b->Vg.size();
     if (b->prop[0]) return GRZ_OK;
-    for (pk_t*& p : b->prop) {
-        BCK(b, cudaMalloc((void**)&p, sizeof(pk_t) * (V + 1) * K));
-        BCK(b, cudaMemsetAsync(p + V * K, 0, sizeof(pk_t) * K, b->stream));
-    }
-    BCK(b, cudaMalloc((void**)&b->rank, sizeof(double) * V * K));
-    BCK(b, cudaMalloc((void**)&b->rowacc, sizeof(u128) * V * K));
     const uint64_t max_ranges = 4ull * (GT / 32) * b->u->num_sms * PPR_RESIDENT;
-    BCK(b, cudaMalloc((void**)&b->ppr_bnd, sizeof(uint32_t) * (max_ranges + 1)));
-    BCK(b, cudaMalloc((void**)&b->ppr_cut, sizeof(uint32_t) * max_ranges));
-    for (u128*& x : b->S) BCK(b, cudaMalloc((void**)&x, sizeof(u128) * G * K));
+    const size_t s = sizeof(u128) * G * K;
+    const grz_part part[] = { { (void**)&b->prop[0], sizeof(pk_t) * (V + 1) * K }, { (void**)&b->prop[1], sizeof(pk_t) * (V + 1) * K },
+                              { (void**)&b->S[0], s }, { (void**)&b->S[1], s }, { (void**)&b->S[2], s },
+                              { (void**)&b->ppr_bnd, sizeof(uint32_t) * (max_ranges + 1) }, { (void**)&b->ppr_cut, sizeof(uint32_t) * max_ranges },
+                              { (void**)&b->rank, sizeof(double) * V * K }, { (void**)&b->rowacc, sizeof(u128) * V * K } };
+    BCK(b, grz_alloc_arrays(part, sizeof(part) / sizeof(part[0]), &b->ppr_mem));
+    for (pk_t* p : b->prop) BCK(b, cudaMemsetAsync(p + V * K, 0, sizeof(pk_t) * K, b->stream));
     BCK(b, cudaMemsetAsync(b->rowacc, 0, sizeof(u128) * V * K, b->stream));
     return GRZ_OK;
 }
@@ -844,12 +844,10 @@ static int bfs_alloc(grz_batch* b)
     const uint64_t V = b->u->V;
     const uint64_t Vw = (V + 3) / 4 * 4;
     if (!b->visited) {
-        BCK(b, cudaMalloc((void**)&b->visited, Vw));
-        BCK(b, cudaMalloc((void**)&b->frontier, Vw));
-        BCK(b, cudaMalloc((void**)&b->next_words, Vw));
-        BCK(b, cudaMalloc((void**)&b->level, sizeof(int32_t) * V * K));
-        BCK(b, cudaMalloc((void**)&b->ctl, sizeof(unsigned long long) * 4));
-        BCK(b, cudaMalloc((void**)&b->iter, sizeof(uint32_t)));
+        const grz_part part[] = { { (void**)&b->visited, Vw }, { (void**)&b->frontier, Vw }, { (void**)&b->next_words, Vw },
+                                  { (void**)&b->level, sizeof(int32_t) * V * K }, { (void**)&b->ctl, sizeof(unsigned long long) * 4 },
+                                  { (void**)&b->iter, sizeof(uint32_t) } };
+        BCK(b, grz_alloc_arrays(part, sizeof(part) / sizeof(part[0]), &b->bfs_mem));
     }
     return GRZ_OK;
 }
