@@ -647,19 +647,19 @@ constexpr int FR_STEP = 4;  // words whose row pointers are loaded together
 // vertices' vectors, vdelta[i] = its first vector's index in the list minus voff[i] (mod 2^32);
 // tile_first[t] for the tiles that start in its range.  `skip` leaves out the first vectors of
 // every selected vertex (each selected one has more).  A zero gate selects nothing (the bitmaps
-// were not written in this phase).
+// were not written in this phase).  The words from `word0` on.
 template <int WORDS>
 __global__ void __launch_bounds__(T) k_fr_compact(const unsigned long long* __restrict__ bm1, const unsigned long long* __restrict__ bm2,
                                                   uint64_t V, const uint32_t* __restrict__ rowptr, uint32_t skip,
                                                   const uint32_t* __restrict__ gate, uint32_t* __restrict__ counters,
                                                   uint32_t* __restrict__ frontier, uint32_t* __restrict__ voff,
-                                                  uint32_t* __restrict__ vdelta, uint32_t* __restrict__ tile_first)
+                                                  uint32_t* __restrict__ vdelta, uint32_t* __restrict__ tile_first, uint64_t word0)
 {
     __shared__ uint32_t sn[T / 32], sv[T / 32];
     __shared__ unsigned long long s_base;
     if (gate && *gate == 0u) return;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const uint64_t first = ((uint64_t)blockIdx.x * (T / 32) + warp) * WORDS, word = first + lane;  // bits of vertices [32 word, 32 word + 32)
+    const uint64_t first = word0 + ((uint64_t)blockIdx.x * (T / 32) + warp) * WORDS, word = first + lane;  // bits of vertices [32 word, 32 word + 32)
     uint32_t bits = 0;
     if (lane < WORDS && 32 * word < V) bits = reinterpret_cast<const uint32_t*>(bm1)[word] & reinterpret_cast<const uint32_t*>(bm2)[word];
     if (32 * word + 32 > V && bits) bits &= (1u << (V - 32 * word)) - 1u;
@@ -2029,7 +2029,7 @@ static unsigned tile_grid(const grz_graph* g, const grz_list& l)
 
 // Compacts the vertices selected by bm1 & bm2 (defined below)
 static void compact(grz_graph* g, const unsigned long long* bm1, const unsigned long long* bm2, const uint32_t* rowptr,
-                    uint32_t skip = 0, const uint32_t* gate = nullptr);
+                    uint32_t skip = 0, const uint32_t* gate = nullptr, bool lowest_first = false);
 
 template <int BT, bool BULK>
 static int launch_cc_pull_bt(grz_graph* g, uint64_t first, uint64_t count, const VoteCfg& vc)
@@ -2147,15 +2147,29 @@ static int launch_cc_pull(grz_graph* g, uint64_t first, uint64_t count, const Vo
 
 // Compacts the vertices selected by bm1 & bm2, with their vector ranges in `rowptr`, into
 // fr.frontier / voff / vdelta / tile_first (counts on the device in counters[3], [2], which are zero).
+// lowest_first: in a large graph the first 1/256 of the vertices come before the others.  CC's push wants that:
+// labels are vertex IDs, so the lowest have the smallest labels, which spread in place while the rest of
+// the list is pushed and spare it its atomics.  GB300, R-MAT, forced pushes, a whole run with the list in vertex
+// order by three kernels / any order / this: 2^20 vertices 428 / 437 / 386 us, 2^21 709 / - / 671, 2^23 2408 / 2780 /
+// 2418, uniform 3M 1202 / - / 1014.
+constexpr uint64_t FR_LOWEST = 256;
+static bool compact_twice(const grz_graph* g, bool lowest_first) { return lowest_first && g->V >= FR_SMALL_V; }
 static void compact(grz_graph* g, const unsigned long long* bm1, const unsigned long long* bm2, const uint32_t* rowptr,
-                    uint32_t skip, const uint32_t* gate)
+                    uint32_t skip, const uint32_t* gate, bool lowest_first)
 {
     grz_frontier_state& f = g->fr;
-    const int words = g->V < FR_SMALL_V ? FR_WORDS_SMALL : FR_WORDS;
-    const unsigned nb = (unsigned)(g->V / ((uint64_t)T * words) + 1);
-    (words == FR_WORDS ? k_fr_compact<FR_WORDS> : k_fr_compact<FR_WORDS_SMALL>)<<<nb, T, 0, g->stream>>>(
-        bm1, bm2, g->V, rowptr, skip, gate, f.counters, f.frontier, f.voff, f.vdelta, f.tile_first);
-    GRZ_COUNT_LAUNCH(g);
+    auto launch = [&](auto kernel, unsigned nb, uint64_t word0) {
+        kernel<<<nb, T, 0, g->stream>>>(bm1, bm2, g->V, rowptr, skip, gate, f.counters, f.frontier, f.voff, f.vdelta, f.tile_first, word0);
+        GRZ_COUNT_LAUNCH(g);
+    };
+    if (g->V < FR_SMALL_V) {
+        launch(k_fr_compact<FR_WORDS_SMALL>, (unsigned)(g->V / (T * FR_WORDS_SMALL) + 1), 0);
+        return;
+    }
+    // blocks of FR_WORDS words per warp; the first part's words are spread over more blocks
+    const unsigned nb = (unsigned)(g->V / (T * FR_WORDS) + 1), lowest = compact_twice(g, lowest_first) ? (unsigned)((nb + FR_LOWEST - 1) / FR_LOWEST) : 0u;
+    if (lowest) launch(k_fr_compact<FR_WORDS_SMALL>, lowest * (FR_WORDS / FR_WORDS_SMALL), 0);
+    if (nb > lowest) launch(k_fr_compact<FR_WORDS>, nb - lowest, (uint64_t)lowest * (T / 32) * FR_WORDS);
 }
 
 // One edge phase on a vector range of the pull (pull=1) or push list.  Leaves the vote of the
@@ -2226,7 +2240,7 @@ static int edge_phase(grz_graph* g, int pull, uint64_t first, uint64_t count)
     } else {
         if (!g->push.nbr) return grz_set_error(g, GRZ_ERR_STATE, "push list not loaded");
         grz_prof_begin(g, GRZ_PROF_PUSH_COMPACT);
-        compact(g, f.has, f.nonempty_push, g->push.rowptr);
+        compact(g, f.has, f.nonempty_push, g->push.rowptr, 0, nullptr, !bfs);
         grz_prof_end(g);
         GRZ_TRY(grz_stats_count_selected(g, &g->push, f.frontier, f.counters));
         grz_prof_begin(g, bfs ? GRZ_PROF_BFS_PUSH : GRZ_PROF_CC_PUSH);
@@ -2763,7 +2777,7 @@ int grz_frontier_run_graph(grz_graph* g, cudaEvent_t started, uint64_t* launches
     // CC one pull launch, or one per source segment plus the whole-list one
     const uint64_t per_pull = bfs ? (g->tune.bfs_pull_scan ? 2 : (g->tune.bfs_pull_first ? 4 : 3))
                                   : (f.run_seg ? cc_segment_launches(g) + 1 : (g->tune.cc_pull_first == 2 ? 4 : (g->tune.cc_pull_first == 3 ? 5 : (g->tune.cc_pull_first == 4 ? 4 : (g->tune.cc_pull_first ? 2 : 1)))));
-    const uint64_t per_push = bfs ? 3 : 2;
+    const uint64_t per_push = bfs ? 3 : 2 + compact_twice(g, true);
     // decisions, iterations by an engine's kernels, and k_hop's launches
     const uint64_t k = 1 + c.bodies + (uint64_t)(c.npull - c.hop_levels[1]) * per_pull + (uint64_t)(c.npush - c.hop_levels[0]) * per_push +
                        (uint64_t)c.hop_runs * (2 + hop_pulls(g));

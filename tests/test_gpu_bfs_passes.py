@@ -137,3 +137,21 @@ def test_first_pass_over_sources_in_any_order(first_n, hubs):
             for par, lv in found:
                 np.testing.assert_array_equal(lv, levels)
                 np.testing.assert_array_equal(par, rule)
+
+
+@pytest.mark.parametrize("V", [(1 << 19) - 1, 1 << 19, (1 << 19) + 8191, 2200007])
+def test_cc_push_compaction_in_two_parts(V):
+    """From 2^19 vertices on a CC push lists the lowest 1/256 of them first: the labels under forced
+    pushes, as one graph and step by step, whichever part a vertex is in."""
+    from grazelle import graphgen as gg, native
+    from grazelle.engine import Graph
+    rng = np.random.RandomState(V & 0xffff)
+    a, b = rng.randint(0, V, size=2 * V), rng.randint(0, V, size=2 * V)
+    a[:4], b[:4] = [0, 8191, 8192, V - 1], [V - 1, 8192, 16384, V - 2]
+    g = gg.EdgeList(V, np.concatenate([a, b]).astype(np.uint64), np.concatenate([b, a]).astype(np.uint64))
+    pull = g.pull_order().pairs()
+    ref = O.cc_min_labels(pull, V).astype(np.float64)
+    with Graph(0) as G:
+        G.load_pairs(V, pull, g.push_order().pairs())
+        for flags in (native.FORCE_PUSH, native.FORCE_PUSH | native.FLAG_HOST_LOOP, 0):
+            np.testing.assert_array_equal(G.connected_components(flags), ref, err_msg="flags %d" % flags)
