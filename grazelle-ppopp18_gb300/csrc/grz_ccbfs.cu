@@ -1430,6 +1430,12 @@ __device__ __forceinline__ HopPart hop_exchange(cg::cluster_group& cl, HopPart x
 // Vectors of a vertex that its lane lists by itself; its warp lists more.  A hub's thousands of vectors listed
 // by one lane held up all 16 blocks: GB300, first small iterations of a BFS on 2^24 R-MAT vertices 58 -> 10 us.
 constexpr uint32_t HOP_NARROW = 4;
+// Vectors of a vertex of the starting frontier that its thread lists by itself; all blocks share the listing
+// of more.  A run of 32 takes about 1 us, and a root's 16000 vectors one after the other took longer than the
+// iteration they saved: GB300, BFS from a root of degree 64722 on 2^20 R-MAT
+// vertices 499 -> 208 us (285 without k_hop).
+constexpr uint32_t HOP_WIDE = 128;
+constexpr uint32_t HOP_MAX_WIDE = GRZ_HOP_VOTE / (4 * HOP_WIDE);  // more than 128 full vectors each, but for the last
 
 template <bool IsBfs>
 __global__ void __cluster_dims__(HOP_CTAS, 1, 1) __launch_bounds__(HOP_T, 1) k_hop(const HopIn in)
@@ -1437,6 +1443,7 @@ __global__ void __cluster_dims__(HOP_CTAS, 1, 1) __launch_bounds__(HOP_T, 1) k_h
     extern __shared__ uint32_t s_mem[];
     __shared__ uint32_t s_items[4];  // vectors listed for an iteration, by its number mod 4
     __shared__ HopPart s_block[2], s_part[2][HOP_CTAS];
+    __shared__ uint32_t s_nwide, s_wide[HOP_MAX_WIDE];  // (block 0's)
     __shared__ int s_pull;
     __shared__ float s_f[NF], s_par[MLP_WARP_FLOATS];
     cg::cluster_group cl = cg::this_cluster();
@@ -1445,6 +1452,7 @@ __global__ void __cluster_dims__(HOP_CTAS, 1, 1) __launch_bounds__(HOP_T, 1) k_h
     const uint32_t rank = cl.block_rank();
     const uint32_t n0 = ctl->hop_n;
     if (tid < 4) s_items[tid] = 0;
+    if (tid == 0) s_nwide = 0;
     if (tid < 2) s_block[tid] = hop_zero();
     const uint32_t level0 = ctl->level, max_level = ctl->max_level, mode0 = ctl->engine;
     const int force = ctl->force;
@@ -1456,23 +1464,38 @@ __global__ void __cluster_dims__(HOP_CTAS, 1, 1) __launch_bounds__(HOP_T, 1) k_h
     // The starting frontier's vectors, spread over the blocks in runs of at most 32, a full list's over
     // the next ones: they are fewer than the vote, which is half of what the lists hold.
     HopPart sum = hop_zero();
-    for (uint32_t i = rank + HOP_CTAS * tid; i < n0; i += HOP_CTAS * HOP_T) {
-        const uint32_t d = in.list[i], r0 = __ldg(in.rowptr + d), n = __ldg(in.rowptr + d + 1) - r0;
-        uint32_t to = (rank + tid) & (HOP_CTAS - 1);
-        for (uint32_t j = 0, tries = 0; j < n && tries < 64u; to = (to + 1) & (HOP_CTAS - 1)) {
-            const uint32_t k = min(32u, n - j);
+    auto place = [&](uint32_t d, uint32_t r, uint32_t k, uint32_t to) {
+        for (int tries = 0; tries < 64; ++tries, to = (to + 1) & (HOP_CTAS - 1)) {
             const uint32_t at = atomicAdd(cl.map_shared_rank(&s_items[0], to), k);
             uint32_t* vec = cl.map_shared_rank(s_mem, to);
-            if (at + k > HOP_CAP) {  // the places no one takes
-                for (uint32_t q = at; q < HOP_CAP; ++q) { vec[q] = HOP_NOVEC; vec[HOP_CAP + q] = 0; }
-                ++tries;
+            if (at + k <= HOP_CAP) {
+                for (uint32_t q = 0; q < k; ++q) { vec[at + q] = r + q; vec[HOP_CAP + at + q] = d; }
+                return;
+            }
+            for (uint32_t q = at; q < HOP_CAP; ++q) { vec[q] = HOP_NOVEC; vec[HOP_CAP + q] = 0; }  // the places no one takes
+        }
+    };
+    for (uint32_t i = rank + HOP_CTAS * tid; i < n0; i += HOP_CTAS * HOP_T) {
+        const uint32_t d = in.list[i], r0 = __ldg(in.rowptr + d), n = __ldg(in.rowptr + d + 1) - r0;
+        if (n > HOP_WIDE) {
+            const uint32_t w = atomicAdd(cl.map_shared_rank(&s_nwide, 0), 1u);
+            if (w < HOP_MAX_WIDE) {
+                *cl.map_shared_rank(s_wide + w, 0) = d;
                 continue;
             }
-            for (uint32_t q = 0; q < k; ++q) { vec[at + q] = r0 + j + q; vec[HOP_CAP + at + q] = d; }
-            j += k;
         }
+        for (uint32_t j = 0, to = rank + tid; j < n; j += 32, ++to) place(d, r0 + j, min(32u, n - j), to & (HOP_CTAS - 1));
     }
     cl.sync();  // other blocks have added to this one's list
+    const uint32_t nwide = min(*cl.map_shared_rank(&s_nwide, 0), HOP_MAX_WIDE);
+    if (nwide) {
+        for (uint32_t w = tid >> 5; w < nwide; w += HOP_T / 32) {  // a warp of every block, a lane per run
+            const uint32_t d = *cl.map_shared_rank(s_wide + w, 0), r0 = __ldg(in.rowptr + d), n = __ldg(in.rowptr + d + 1) - r0;
+            for (uint32_t j = 32 * (((rank - w) & (HOP_CTAS - 1)) + HOP_CTAS * lane); j < n; j += 32 * HOP_CTAS * 32)
+                place(d, r0 + j, min(32u, n - j), rank);
+        }
+        cl.sync();
+    }
     hop_exchange(cl, sum, &s_items[0], &s_block[1], s_part[1]);
     // lists the vectors [r0, r0 + n) of the lanes' vertices d that are `fresh` in this block's list q (by
     // whole warps, which share the writing of long ranges); false for those that it has no room for

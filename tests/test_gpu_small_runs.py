@@ -175,3 +175,28 @@ def test_parents_over_repeated_edges(V, hubs):
         for flags in (0, native.FORCE_PULL, native.FORCE_PUSH):
             np.testing.assert_array_equal(G.bfs(0, flags)[0], O.bfs(L, flags)[0], err_msg="flags %d" % flags)
         assert G.bfs(V - 2, native.FORCE_PULL)[0][V - 1] == 15  # of the first vector, 10 11 12 15
+
+
+@pytest.mark.parametrize("sizes", [[512], [513], [508, 509, 512, 516, 517], [520] * 50, [517] * 57, [20000], [8200, 8300, 513, 4, 600], [31000]])
+def test_hubs_in_the_starting_frontier(sizes):
+    """Vertices of 128 vectors and around it, of many times as many, and as many such as a starting frontier can
+    hold, listed by all blocks: CC, whose first frontier is every vertex, and BFS from each hub."""
+    from grazelle import native
+    from grazelle.engine import Graph
+    hubs = np.arange(len(sizes))
+    src = np.repeat(hubs, sizes)
+    V = len(sizes) + sum(sizes) + 1
+    dst = len(sizes) + np.arange(sum(sizes))
+    src, dst = np.concatenate([src, dst[::7]]), np.concatenate([dst, np.full(dst[::7].shape[0], V - 1)])
+    g = _edges(V, src, dst)
+    pull, push = g.pull_order().pairs(), g.push_order().pairs()
+    with Graph(0) as G:
+        G.load_pairs(V, pull, push)
+        for flags in (0, native.FORCE_PUSH):
+            np.testing.assert_array_equal(G.connected_components(flags), O.cc_min_labels(pull, V).astype(np.float64))
+            for r in sorted({0, len(sizes) // 2, len(sizes) - 1}):
+                par, lv = G.bfs(r, flags)
+                par2, lv2 = G.bfs(r, flags | native.FLAG_HOST_LOOP)
+                np.testing.assert_array_equal(lv, lv2)
+                np.testing.assert_array_equal(par, par2)
+                np.testing.assert_array_equal(lv, O.bfs_levels(push, V, r))
