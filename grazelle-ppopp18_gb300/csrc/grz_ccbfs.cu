@@ -865,7 +865,7 @@ __global__ void __launch_bounds__(T) k_push_expand(const uint32_t* __restrict__ 
 }
 
 // BFS pull over the compacted wanted destinations (WantsInfo and in-vectors): only their vectors
-// are read, in tiles of PUSH_TILE vectors.  The vectors of one destination are consecutive in the
+// are read, in tiles of pull_tile vectors.  The vectors of one destination are consecutive in the
 // concatenation, so the per-destination minimum candidate (the reference's parent rule, as in
 // k_bfs_pull) is reduced within the warp before one atomicMin.
 // Early exit: the candidate is (first vector with a frontier source, ~largest such source), so
@@ -878,6 +878,17 @@ __global__ void __launch_bounds__(T) k_push_expand(const uint32_t* __restrict__ 
 // destination next to a frontier hub stops after its first vectors.
 constexpr uint32_t LONG_RUN = 32;
 
+// Vectors of a tile of the pulls' expansions: one per thread, or four where that still gives every block several
+// tiles, for a tile costs a trip to the queue and three barriers whatever its size.  GB300, CC's first pull, tiles of
+// 256 / 512 / 1024 / 2048 vectors (of 1024 and two at a time before): uniform 1M vertices of degree 60 341 / 297 / 287 /
+// 473 us (305), 3.8M of 42 965 / 801 / 746 / 1252 (810), R-MAT of 2^24 316 / 324 / 317 / 440 (328).
+constexpr uint32_t PULL_TILE = 4 * PUSH_TILE;
+constexpr uint32_t PULL_MANY = 2;
+__device__ __forceinline__ uint32_t pull_tile(uint32_t total, uint32_t blocks)
+{
+    return total / (PULL_MANY * PULL_TILE) >= blocks ? PULL_TILE : PUSH_TILE;
+}
+
 __global__ void __launch_bounds__(T) k_bfs_pull_expand(const uint32_t* __restrict__ dests, const uint32_t* __restrict__ voff,
                                                        const uint32_t* __restrict__ vdelta, const uint32_t* __restrict__ tile_first,
                                                        const uint32_t* __restrict__ counters, const uint4* __restrict__ nbr,
@@ -887,21 +898,20 @@ __global__ void __launch_bounds__(T) k_bfs_pull_expand(const uint32_t* __restric
                                                        uint32_t nhub, unsigned long long* __restrict__ has_next,
                                                        uint32_t* __restrict__ queue)
 {
-    __shared__ uint32_t s_dst[PUSH_TILE];
-    __shared__ uint32_t s_off[PUSH_TILE];
-    __shared__ uint32_t s_delta[PUSH_TILE];
+    __shared__ uint32_t s_dst[PULL_TILE];
+    __shared__ uint32_t s_off[PULL_TILE];
+    __shared__ uint32_t s_delta[PULL_TILE];
     __shared__ uint32_t s_tile;
     __shared__ bool s_full;  // the touched list is long enough for the visit to sweep (read per tile)
-    const uint32_t nd = counters[3], total = counters[2];
-    const uint32_t ntiles = (total + PUSH_TILE - 1) / PUSH_TILE;
+    const uint32_t nd = counters[3], total = counters[2], span = pull_tile(total, gridDim.x);
+    const uint32_t ntiles = (total + span - 1) / span;
     const int lane = threadIdx.x & 31;
     for (uint32_t tile = blockIdx.x; tile < ntiles; tile = s_tile) {
         uint32_t next = 0;
         if (threadIdx.x == 0) next = atomicAdd(queue, 1u) + gridDim.x;
-        const uint32_t first = tile_first[tile];
-        const uint32_t t0 = tile * PUSH_TILE;
-        const uint32_t tend = min(total, t0 + PUSH_TILE);
-        const uint32_t nw = min(PUSH_TILE, nd - first);
+        const uint32_t t0 = tile * span, first = tile_first[t0 / PUSH_TILE];
+        const uint32_t tend = min(total, t0 + span);
+        const uint32_t nw = min(span, nd - first);
         for (uint32_t i = threadIdx.x; i < nw; i += T) {
             s_off[i] = voff[first + i];
             s_dst[i] = dests[first + i];
@@ -982,15 +992,15 @@ __global__ void __launch_bounds__(T) k_cc_pull_expand(const uint32_t* __restrict
                                                       uint32_t epoch, const uint32_t* __restrict__ epoch_dev,
                                                       uint32_t* __restrict__ queue, unsigned long long* __restrict__ work)
 {
-    __shared__ uint32_t s_dst[PUSH_TILE];
-    __shared__ uint32_t s_off[PUSH_TILE];
-    __shared__ uint32_t s_delta[PUSH_TILE];
+    __shared__ uint32_t s_dst[PULL_TILE];
+    __shared__ uint32_t s_off[PULL_TILE];
+    __shared__ uint32_t s_delta[PULL_TILE];
     __shared__ uint32_t s_tile;
     __shared__ unsigned long long red[T / 32];
     __shared__ uint32_t red32[T / 32];
     const uint32_t ep = epoch_dev ? *epoch_dev : epoch;
-    const uint32_t nd = counters[3], total = counters[2];
-    const uint32_t ntiles = (total + PUSH_TILE - 1) / PUSH_TILE;
+    const uint32_t nd = counters[3], total = counters[2], span = pull_tile(total, gridDim.x);
+    const uint32_t ntiles = (total + span - 1) / span;
     const int lane = threadIdx.x & 31;
     unsigned long long my_vote = 0, my_vecs = 0;
     uint32_t my_min = INF;
@@ -1002,10 +1012,9 @@ __global__ void __launch_bounds__(T) k_cc_pull_expand(const uint32_t* __restrict
     for (uint32_t tile = blockIdx.x; tile < ntiles; tile = s_tile) {
         uint32_t next = 0;
         if (threadIdx.x == 0) next = atomicAdd(queue, 1u) + gridDim.x;
-        const uint32_t first = tile_first[tile];
-        const uint32_t t0 = tile * PUSH_TILE;
-        const uint32_t tend = min(total, t0 + PUSH_TILE);
-        const uint32_t nw = min(PUSH_TILE, nd - first);
+        const uint32_t t0 = tile * span, first = tile_first[t0 / PUSH_TILE];
+        const uint32_t tend = min(total, t0 + span);
+        const uint32_t nw = min(span, nd - first);
         for (uint32_t i = threadIdx.x; i < nw; i += T) {
             s_off[i] = voff[first + i];
             s_dst[i] = dests[first + i];

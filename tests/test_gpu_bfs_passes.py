@@ -155,3 +155,33 @@ def test_cc_push_compaction_in_two_parts(V):
         G.load_pairs(V, pull, g.push_order().pairs())
         for flags in (native.FORCE_PUSH, native.FORCE_PUSH | native.FLAG_HOST_LOOP, 0):
             np.testing.assert_array_equal(G.connected_components(flags), ref, err_msg="flags %d" % flags)
+
+
+@pytest.mark.parametrize("V", [2470001, 2540003])
+def test_pulls_over_long_lists(V):
+    """From 2 tiles of 1024 vectors for each of 1216 blocks on, the pulls over compacted destinations take
+    such tiles instead of 256: a random tree, a vector per vertex, with a destination of 5000 vectors among
+    them, on either side of that length; vertex 0 reaches everything."""
+    from grazelle import graphgen as gg, native
+    from grazelle.engine import Graph
+    rng = np.random.RandomState(V & 0xffff)
+    dst = np.arange(1, V)
+    src = (rng.rand(V - 1) * dst).astype(np.int64)
+    hub = np.unique(rng.randint(0, V, size=20000))
+    hub = hub[hub != 1234567]
+    g = gg.EdgeList(V, np.concatenate([src, hub]).astype(np.uint64), np.concatenate([dst, np.full(hub.shape[0], 1234567)]).astype(np.uint64))
+    pull, push = g.pull_order().pairs(), g.push_order().pairs()
+    with Graph(0) as G:
+        G.load_pairs(V, pull, push)
+        labels = O.cc_min_labels(pull, V).astype(np.float64)
+        for flags in (native.FORCE_PULL, native.FORCE_PULL | native.FLAG_HOST_LOOP):
+            np.testing.assert_array_equal(G.connected_components(flags), labels)
+        G.tune(bfs_pull_scan=1)
+        par, lv = G.bfs(0, native.FORCE_PULL)
+        np.testing.assert_array_equal(lv, O.bfs_levels(push, V, 0))
+        for form in ({"bfs_pull_scan": 0, "bfs_pull_first": 0}, {"bfs_pull_first": 1}):
+            G.tune(**form)
+            for flags in (native.FORCE_PULL, native.FORCE_PULL | native.FLAG_HOST_LOOP):
+                par2, lv2 = G.bfs(0, flags)
+                np.testing.assert_array_equal(par2, par)
+                np.testing.assert_array_equal(lv2, lv)
