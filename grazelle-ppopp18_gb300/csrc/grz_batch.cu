@@ -678,8 +678,8 @@ static int enqueue_ppr(grz_batch* b, cudaStream_t cs, uint32_t iterations, doubl
 {
     grz_graph* u = b->u;
     const uint32_t V = (uint32_t)u->V, G = (uint32_t)b->Vg.size(), nvec = (uint32_t)u->pull.nvec;
-    for (pk_t* p : b->prop) BCK(b, cudaMemsetAsync(p, 0, sizeof(pk_t) * (uint64_t)V * K, cs));
-    BCK(b, cudaMemsetAsync(b->rank, 0, sizeof(double) * (uint64_t)V * K, cs));
+    // the props and the ranks, neighbours in memory (ppr_alloc)
+    BCK(b, cudaMemsetAsync(b->prop[0], 0, (size_t)((char*)(b->rank + (uint64_t)V * K) - (char*)b->prop[0]), cs));
     k_ppr_init<<<(G * K + 255) / 256, 256, 0, cs>>>(b->d_seeds, G, u->inv_deg, u->degree, b->prop[0], b->S[0], b->S[1]);
     const unsigned grid = ppr_grid(b);
     const uint32_t nranges = 4 * grid * (GT / 32);
@@ -734,9 +734,9 @@ static int ppr_alloc(grz_batch* b)
     const uint64_t max_ranges = 4ull * (GT / 32) * b->u->num_sms * PPR_RESIDENT;
     const size_t s = sizeof(u128) * G * K;
     const grz_part part[] = { { (void**)&b->prop[0], sizeof(pk_t) * (V + 1) * K }, { (void**)&b->prop[1], sizeof(pk_t) * (V + 1) * K },
+                              { (void**)&b->rank, sizeof(double) * V * K }, { (void**)&b->rowacc, sizeof(u128) * V * K },
                               { (void**)&b->S[0], s }, { (void**)&b->S[1], s }, { (void**)&b->S[2], s },
-                              { (void**)&b->ppr_bnd, sizeof(uint32_t) * (max_ranges + 1) }, { (void**)&b->ppr_cut, sizeof(uint32_t) * max_ranges },
-                              { (void**)&b->rank, sizeof(double) * V * K }, { (void**)&b->rowacc, sizeof(u128) * V * K } };
+                              { (void**)&b->ppr_bnd, sizeof(uint32_t) * (max_ranges + 1) }, { (void**)&b->ppr_cut, sizeof(uint32_t) * max_ranges } };
     BCK(b, grz_alloc_arrays(part, sizeof(part) / sizeof(part[0]), &b->ppr_mem));
     for (pk_t* p : b->prop) BCK(b, cudaMemsetAsync(p + V * K, 0, sizeof(pk_t) * K, b->stream));
     BCK(b, cudaMemsetAsync(b->rowacc, 0, sizeof(u128) * V * K, b->stream));
@@ -845,10 +845,18 @@ static int bfs_alloc(grz_batch* b)
     const uint64_t Vw = (V + 3) / 4 * 4;
     if (!b->visited) {
         const grz_part part[] = { { (void**)&b->visited, Vw }, { (void**)&b->frontier, Vw }, { (void**)&b->next_words, Vw },
-                                  { (void**)&b->level, sizeof(int32_t) * V * K }, { (void**)&b->ctl, sizeof(unsigned long long) * 4 },
-                                  { (void**)&b->iter, sizeof(uint32_t) } };
+                                  { (void**)&b->ctl, sizeof(unsigned long long) * 4 }, { (void**)&b->iter, sizeof(uint32_t) },
+                                  { (void**)&b->level, sizeof(int32_t) * V * K } };
         BCK(b, grz_alloc_arrays(part, sizeof(part) / sizeof(part[0]), &b->bfs_mem));
     }
+    return GRZ_OK;
+}
+
+// no vertex visited, no level: the bitmaps and the control words are neighbours in memory (bfs_alloc)
+static int bfs_clear(grz_batch* b, cudaStream_t st)
+{
+    BCK(b, cudaMemsetAsync(b->visited, 0, (size_t)((char*)(b->ctl + 4) - (char*)b->visited), st));
+    BCK(b, cudaMemsetAsync(b->level, 0xff, sizeof(int32_t) * b->u->V * K, st));
     return GRZ_OK;
 }
 
@@ -882,7 +890,6 @@ static int build_run_graph(grz_batch* b, uint32_t iterations, double damping)
     if (rr) return rr;
     grz_graph* u = b->u;
     const uint64_t V = u->V;
-    const uint64_t Vw = (V + 3) / 4 * 4;
     const uint32_t G = (uint32_t)b->Vg.size();
     cudaGraph_t top = nullptr;
     BCK(b, cudaGraphCreate(&top, 0));
@@ -902,13 +909,9 @@ static int build_run_graph(grz_batch* b, uint32_t iterations, double damping)
     if (!rc) rc = bck(b, cudaStreamBeginCaptureToGraph(cs, top, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal), "capture");
     if (!rc) {
         k_stamp<<<1, 1, 0, cs>>>(b->stamps + 2);
-        cudaMemsetAsync(b->visited, 0, Vw, cs);
-        cudaMemsetAsync(b->frontier, 0, Vw, cs);
-        cudaMemsetAsync(b->next_words, 0, Vw, cs);
-        cudaMemsetAsync(b->level, 0xff, sizeof(int32_t) * V * K, cs);
-        cudaMemsetAsync(b->ctl, 0, sizeof(unsigned long long) * 4, cs);
+        rc = bfs_clear(b, cs);
         k_msbfs_init<<<(G * K + 255) / 256, 256, 0, cs>>>(b->d_roots, G * K, b->visited, b->frontier, b->level, b->iter);
-        rc = bck(b, cudaGetLastError(), "bfs init");
+        if (!rc) rc = bck(b, cudaGetLastError(), "bfs init");
         const int rc2 = end_capture_sink(b, cs, &init);
         if (!rc) rc = rc2;
     }
@@ -939,7 +942,6 @@ extern "C" int grz_batch_msbfs(grz_batch* b, const uint32_t* roots, uint32_t k, 
     grz_graph* u = b->u;
     const uint64_t V = u->V;
     const uint32_t G = (uint32_t)b->Vg.size();
-    const uint64_t Vw = (V + 3) / 4 * 4;
     int rc = bfs_alloc(b);
     if (rc) return rc;
     rc = upload_seeds(b, roots, k);
@@ -954,11 +956,7 @@ extern "C" int grz_batch_msbfs(grz_batch* b, const uint32_t* roots, uint32_t k, 
     BCK(b, cudaEventCreate(&e1));
     const uint32_t one = 1;
     rc = bck(b, cudaEventRecord(e0, st), "event");
-    if (!rc) rc = bck(b, cudaMemsetAsync(b->visited, 0, Vw, st), "memset");
-    if (!rc) rc = bck(b, cudaMemsetAsync(b->frontier, 0, Vw, st), "memset");
-    if (!rc) rc = bck(b, cudaMemsetAsync(b->next_words, 0, Vw, st), "memset");
-    if (!rc) rc = bck(b, cudaMemsetAsync(b->level, 0xff, sizeof(int32_t) * V * K, st), "memset");
-    if (!rc) rc = bck(b, cudaMemsetAsync(b->ctl, 0, sizeof(unsigned long long) * 4, st), "memset");
+    if (!rc) rc = bfs_clear(b, st);
     if (!rc) {
         memcpy(b->mail, &one, sizeof(one));
         rc = bck(b, cudaMemcpyAsync(b->iter, b->mail, sizeof(uint32_t), cudaMemcpyHostToDevice, st), "H2D");
