@@ -655,10 +655,13 @@ static int upload_seeds(grz_batch* b, const uint32_t* local, uint32_t k, uint32_
     return GRZ_OK;
 }
 
-// blocks of k_ppr_step: a step of 16 vectors per warp at least
+// Blocks of k_ppr_step: a step of 16 vectors per warp at least, in lists that would fill the chip so, two: shorter
+// ranges cut more destinations, and the BFS beside it waits for the registers.  GB300, PPR alone / with BFS, one and
+// two steps at least: 3k vectors 136 / 171 and 157 / 193 us, 29k 89 / 158 and 93 / 158, 41k 95 / 162 and 97 / 155, 74k 356 / 402
+// and 339 / 388, 117k 125 / 278 and 128 / 260, 210k 261 / 346 and 261 / 349.
 static unsigned ppr_grid(const grz_batch* b)
 {
-    const uint64_t steps = (b->u->pull.nvec + 15) / 16;
+    const uint64_t nvec = b->u->pull.nvec, least = nvec < (1u << 15) ? 16 : 32, steps = (nvec + least - 1) / least;
     return persistent_grid(b, (steps + GT / 32 - 1) / (GT / 32), std::min(b->ppr_blocks, PPR_RESIDENT));
 }
 

@@ -101,3 +101,20 @@ def test_small_props():
     ref = P.ppr(g.num_vertices, g.pull_order().pairs(), 0, 9, 0.85)
     assert 0 < ref[ref > 0].min() < 2.0 ** -60
     np.testing.assert_allclose(ranks[0][:, 0], ref, rtol=1e-12, atol=9 * 2.0 ** -124)
+
+
+@pytest.mark.parametrize("n", [32767, 32768, 32769])
+def test_ranges_around_32768_vectors(n):
+    """From 2^15 vectors on a warp has at least 32: n vertices of one in-edge each, so n vectors."""
+    rng = np.random.RandomState(n)
+    g = edges(n, rng.randint(0, n, n), np.arange(n))
+    seeds, found = [[0, n - 1, 77]], []
+    with batch_of([g]) as B:
+        assert B.info()["vectors"] == n
+        for blocks in (8, 1):
+            B.tune(ppr_blocks=blocks)
+            found.append(B.ppr(seeds, 6, 0.85)[0][0])
+    np.testing.assert_array_equal(found[0], found[1])
+    for i, s in enumerate(seeds[0]):
+        ref = P.ppr(n, g.pull_order().pairs(), s, 6, 0.85)
+        assert np.abs(found[0][:, i] - ref).sum() < 1e-12 * np.abs(ref).sum()
