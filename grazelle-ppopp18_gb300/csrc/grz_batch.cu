@@ -124,7 +124,9 @@ constexpr int PPR_RESIDENT = 4;  // blocks per SM the launch bounds fit
 // = nvec.  The warps' ranges are equal in PPR_WV per vector + PPR_WD per vertex up to their destinations, about
 // the instructions k_ppr_step has for each; a warp's slots have the same number of vectors.  All ranges run at
 // once, so the longest sets the time: 8-graph batch of 1.04M vertices, 8 instances x 20 iterations, ranges of
-// equal vectors 4.46 ms, weights 4:5 3.49, 2:3 3.56, 4:7 3.65 ms.
+// equal vectors 4.46 ms.  Weights 1:1 / 4:5 / 2:3 / 4:7 / 1:2, PPR alone: that batch 3.42 / 3.47 / 3.55 / 3.64 / 3.75 ms, 6 graphs
+// of 2.2M vectors 2.86 / 2.87 / 2.91 / 2.94 / 2.97, one of 10^6 vertices and 1.2M vectors 1.96 / 2.06 / 1.99 / 2.06 / 2.15, three of
+// 5.3M 2.54 / 2.50 / 2.63 / 2.51 / 2.55.
 constexpr uint32_t PPR_WV = 4, PPR_WD = 5;
 
 __global__ void k_ppr_bounds(const uint32_t* __restrict__ dstv, uint32_t nvec, uint32_t V, uint32_t nwarps, uint32_t* __restrict__ bnd)

@@ -18,10 +18,10 @@
 //   * Pull: one thread per vector, a warp-segmented reduction per destination, one atomic per
 //     (warp, destination).  Labels are updated in place, as the reference's CAS loop does, so
 //     a later vector may already see a lowered label.
-//   * Push: HasInfo is compacted, in vertex order, into a list of active sources that have
-//     out-edges, with a scan of their vector counts.  The concatenation of their vector ranges
-//     is expanded in tiles of 1024 vectors over the whole grid, so neither threads nor blocks
-//     wait on high-degree sources.
+//   * Push: HasInfo is compacted, in vertex order block by block, into a list of active sources that have
+//     out-edges, with the offset of each one's vectors among all of theirs.  The concatenation of
+//     their vector ranges is expanded in tiles of one vector per thread over the whole grid, so
+//     neither threads nor blocks wait on high-degree sources.
 //   * Each changed vertex is counted once per iteration: the first setter of its HasInfo* bit
 //     adds 1 + outdeg to the vote.  The reference can count a destination that straddles two
 //     work units twice.  The vote only steers the engine choice.
@@ -643,7 +643,7 @@ constexpr uint32_t PUSH_TILE = T;
 // whole runs, three kernels -> one: 8 BFS at R-MAT 24 9.67 -> 9.15 ms, a BFS of 1400 levels on a mesh of
 // 250k vertices 33.4 -> 30.6 ms.
 // Words of a warp: its passes over them are a chain of loads, FR_STEP words at a time, so a graph that would
-// give few blocks takes fewer words per warp (GB300, 4096 vertices: 32 words 8 to 13 us, 4 words FRCUS); with
+// give few blocks takes fewer words per warp (GB300, 4096 vertices: 32 words 8 to 13 us, 4 words 2 us); with
 // more blocks the adds to the one counter cost more than the chain.
 constexpr int FR_WORDS = 32, FR_WORDS_SMALL = 4;
 constexpr uint64_t FR_SMALL_V = 1ull << 19;

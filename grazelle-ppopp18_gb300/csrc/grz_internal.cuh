@@ -368,8 +368,9 @@ struct grz_prof;
 #define GRZ_VOTE_STRIDE 16
 
 // Largest vote (frontier vertices and their out-edges) of an iteration that k_hop runs (grz_ccbfs.cu).
-// GB300, a BFS run with 2048 / 8192 / 32768 / 65536: R-MAT of 100k vertices 270 / 238 / 218 / 223 us, R-MAT
-// 24 940 / 939 / 939 / 901 us; 65536 is half of what its lists hold.
+// GB300, a BFS run with 4096 / 16384 / 32768 / 65536: R-MAT of 100k vertices 184 / 181 / 178 / 181 us, of 4.2M 423 /
+// 428 / 420 / 420, uniform 500k 237 / 218 / 221 / 221, 20k 168 / 168 / 158 / 154; CC on a mesh of 200k 18.9 / 17.9 / 16.9 /
+// 15.9 ms.  65536 is half of what its lists hold.
 #define GRZ_HOP_VOTE 65536u
 // what the run graph's SWITCH runs next
 #define GRZ_RUN_PULL 0

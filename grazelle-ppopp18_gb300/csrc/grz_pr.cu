@@ -13,8 +13,8 @@
 //     of its integer rate, so FP64 adds per edge would bound the kernel.
 //   * The gathers bound the iteration: about one line request per SM clock.  The iterations of
 //     grz_pr_iterate therefore gather 8-byte packed props (pk_to_fx), and take those of the sources
-//     with the highest out-degrees from shared memory (k_pr_gather_pk): in a power-law graph 12000
-//     sources are half of the edges at R-MAT 20.  Each thread sums four consecutive vectors, a
+//     with the highest out-degrees from shared memory (k_pr_gather_pk): in a power-law graph 20000
+//     sources are more than half of the edges at R-MAT 20.  Each thread sums four consecutive vectors, a
 //     warp-segmented scan joins the threads, and a warp walks a contiguous range of the list, so
 //     only the destinations cut by the ends of a range are combined with exact u128 atomics, in any
 //     order.  This replaces the reference's work-unit merge buffer (source/phases.c:41-70); no
@@ -1071,9 +1071,10 @@ __global__ void k_pr_vertex(const double* __restrict__ accum, const double* __re
 // execution_initialize_vertex_prop_pr (source/execution_pr.c:85-88): c / deg' with c = 1/V, in the
 // form the first gather reads (packed with the hot table, or fixed point).  The division is one
 // Newton step on the reciprocal 1/deg' (Markstein 1990): q0 = c * inv, r = c - q0 * deg' exactly by
-// one fma, q = q0 + r * inv.  It gives the division's result for every degree up to 4M at 40 vertex
-// counts and up to 100k at 360 others (checked against the division on the CPU), at 3 FP64
-// operations instead of a division's; the grid strides, with one partial of S_0 per block.  GB300, with
+// one fma, q = q0 + r * inv.  That is the division's result for every degree below 2^32: r is a multiple
+// of ulp(q0) below 2^34 of them, so it is exact; q0 + r * inv before its one rounding is within 2^-51 ulp of
+// the quotient; and the quotient of a 53-bit significand by a 32-bit integer is a number of 53 bits or at
+// least 2^-33 ulp from every rounding boundary.  3 FP64 operations instead of a division's; the grid strides, with one partial of S_0 per block.  GB300, with
 // the accumulators' clearing (a division per vertex, props also written as doubles and in fixed point
 // -> now): V = 2^24 512 -> 171 us, 2^20 52 -> 24 us.
 __global__ void __launch_bounds__(PR_THREADS, 8) k_pr_init(const double* __restrict__ inv_deg, const uint32_t* __restrict__ degree, uint64_t V,
@@ -1280,11 +1281,12 @@ static int pr_cut_for(grz_graph* g, uint32_t per)
 }
 
 // Chooses the hot sources of the loaded lists.  Once per loaded lists; one read-back.  Worth it
-// when the hot sources are at least a tenth of the edges: with 1% (a uniform graph) the gather is no
-// faster, with 20% (R-MAT 24) it is 13% faster, with 52% (R-MAT 20) 20-30%.  Lists below 2^21
-// vectors stay as they are: their props are mostly L1 hits and the table's copy is not for free (GB300,
-// R-MAT, us per iteration without / with the table: 0.5M vectors 13.6 / 15.3, 1.05M 18.7 / 20.0, 2.1M
-// 33.7 / 30.3; choosing and encoding take 120 us there).
+// when the hot sources are at least a tenth of the edges.  GB300, us per iteration without / with the table,
+// uniform graphs with that share of the edges moved to 20000 sources: 3M vertices, degree 12, 5% 167 / 166, 10%
+// 167 / 160, 30% 166 / 138; 2^20, degree 16, 5% 77.3 / 78.5, 10% 77.2 / 76.3; 2^22, degree 16, 2% 289 / 291, 10%
+// 289 / 274; R-MAT of 2^20 67.4 / 51.8.  (Only a thin rest of 8M to 12M vertices is better without: 10M, degree 8, 10%
+// 472 / 567.)  Lists below 2^21 vectors stay as they are: R-MAT of 0.5M vectors 13.7 / 14.8, 1.0M 19.2 / 18.8, 2.0M
+// 27.6 / 24.1, and choosing and encoding take 120 us there, the gain of 35 iterations.
 constexpr uint64_t PR_HOT_MIN_VECTORS = 1ull << 21;
 static int pr_hot_choose(grz_graph* g)
 {

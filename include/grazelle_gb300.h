@@ -159,7 +159,7 @@ int grz_read_levels(grz_graph* g, int64_t* host_levels, uint64_t capacity);
 #define GRZ_TUNE_BFS_PULL_SCAN 5 /* BFS pull over the whole list: 0 = only the wanted destinations' vectors (compacted), 1 = scan every vector */
 #define GRZ_TUNE_PR_PROPS 6     /* props the PageRank gather reads, from the next grz_pr_init: 0 or 2 = packed in 8 bytes, 1 = 16-byte fixed point; results identical */
 #define GRZ_TUNE_INGEST_CHUNKS 7 /* chunks of the pull-only ingest, from the next load (0 = one per 2^24 pairs, <= 64; the last is cut into up to four smaller pieces): each chunk is processed while the next crosses the host link */
-#define GRZ_TUNE_PR_PERSISTENT 8 /* form of grz_pr_iterate: 0 = default (two kernels), 1 = two kernels per iteration (gather, apply), 2 or 3 = every iteration in one cooperative launch (6 or 8 blocks per SM) whose phases are separated by a grid barrier with bounded waits (the call then waits for the iterations) */
+#define GRZ_TUNE_PR_PERSISTENT 8 /* form of grz_pr_iterate: 0 = default (graphs of up to 6144 vertices and 24576 vectors: all iterations of a call in one cluster of 16 blocks, where that fits and no hub encoding, grid, 16-byte props or profiling is asked for; others: two kernels per iteration), 1 = two kernels per iteration (gather, apply), 2 or 3 = every iteration in one cooperative launch (6 or 8 blocks per SM) whose phases are separated by a grid barrier with bounded waits (the call then waits for the iterations) */
 #define GRZ_TUNE_PULL_STAGING 13 /* CC pull's edge stream: 0 = streaming loads, 1 = bulk copies (cp.async.bulk) into shared memory, two tiles ahead; results identical */
 #define GRZ_TUNE_CC_SEGMENTS 16 /* CC's first (full) pull over the source-segmented lists of GRZ_TUNE_PR_SEGMENT_BITS: 0 = when they are built (by grz_pr_init), 1 = never, 2 = built at the CC initialisation (with the default segment size when the graph is below the size threshold); results identical */
 #define GRZ_TUNE_BFS_PULL_FIRST 17 /* BFS pull over the whole list: vectors each wanted destination reads, in order, in a first pass that stops at the first vector with a frontier source (1..64; 0 = no such pass, every vector of the wanted destinations is read); destinations left undecided are finished by the pass over their remaining vectors; results identical */

@@ -187,3 +187,21 @@ def test_segmented_after_unsegmented(V, degree, before):
             if seg == 1:
                 G.tune(**before)
             np.testing.assert_array_equal(G.pagerank(6, damping=0.85), ref, err_msg="segment bits %d" % seg)
+
+
+@pytest.mark.parametrize("V", [1501, 1777, 4099, 65537, 1000003])
+@pytest.mark.parametrize("props", [0, 1])
+def test_starting_props_are_the_quotients(V, props):
+    """The starting props, one Newton step on the reciprocal, equal the division's (1 / V) / degree bit for
+    bit: every degree up to 1500, and one of 300 thousand, on both sides of powers of two in V."""
+    from grazelle import graphgen as gg
+    from grazelle.engine import Graph
+    deg = np.concatenate([np.arange(1500), [300007 if V > 60000 else 1501]])
+    src = np.repeat(np.arange(deg.shape[0]), deg)
+    g = gg.EdgeList(V, src.astype(np.uint64), np.random.RandomState(V % 1000).randint(0, V, size=src.shape[0]).astype(np.uint64))
+    d = np.full(V, V, dtype=np.float64)
+    d[1:deg.shape[0]] = deg[1:]
+    with Graph(0) as G:
+        G.tune(pr_props=props)
+        G.load_pairs(V, g.pull_order().pairs())
+        np.testing.assert_array_equal(G.pr_init(0.85).props(), 1.0 / V / d)
